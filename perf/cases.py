@@ -217,3 +217,29 @@ def tolerance(case):
         exact_weights = case["M"] <= 16 and case["G"] == 128
         return {"rel": 1e-3 if exact_weights else 8e-3, "max": 3e-2}
     return {"rel": 1.5e-2, "max": 8e-2, "differ": 0.0}
+
+
+def _exact_linear(x, Wq, S, G):
+    """x . ((q - 8) * s)^T in 64 bits, a block of rows at a time."""
+    shifts = torch.arange(0, 32, 4, device="cuda", dtype=torch.int32)
+    x = x.double()
+    rows = []
+    for lo in range(0, Wq.shape[0], 4096):
+        q = ((Wq[lo:lo + 4096, :, None] >> shifts) & 15).flatten(1).double() - 8
+        rows.append(x @ (q * S[lo:lo + 4096].double().repeat_interleave(G, dim=1)).T)
+    return torch.cat(rows, dim=1)
+
+
+def exact(case, seed):
+    """What `run` returns, in 64 bits and without this package's code.  A quantized matrix is whole numbers; a model's
+    logits and cache depend on every intermediate's rounding to bf16, so no 64-bit value is theirs."""
+    kind, gen = case["kind"], _gen(seed)
+    if kind == "linear":
+        Wq, S = _weights(case["N"], case["K"], case["G"], gen)
+        return _exact_linear(_activations(case["M"], case["K"], gen), Wq, S, case["G"])
+    if kind == "layers":
+        shapes = _layer_linears(case)
+        xs = [_activations(case["M"], K, gen) for _, K in shapes]
+        return [[_exact_linear(x, *_weights(N, K, case["G"], gen), case["G"]) for x, (N, K) in zip(xs, shapes)]
+                for _ in range(case["n_layers"])]
+    return None
