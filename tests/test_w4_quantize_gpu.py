@@ -48,6 +48,40 @@ def test_ties_round_to_even(kernels):
     assert list(q) == [7, 0, 2, 2, 0, -2, -2, 4]
 
 
+@pytest.mark.parametrize("G", [32, 64, 128, 256])
+def test_every_significand_and_special_groups(kernels, G):
+    """The division-free rounding against the oracle's division: every pair of bf16 significands at the exponents where
+    w / s can be halfway between two integers, scales at both ends of the range, infinite and nan members, and a word
+    count that fills no block."""
+    rng = np.random.default_rng(G)
+    rows = []
+    for top in range(128, 256):  # a group's largest value sets s; the other members run through the significands
+        w = np.arange(128, 256, dtype=np.float64) * 2.0 ** rng.integers(-5, 1, 128) * rng.choice([-1, 1], 128)
+        w[np.abs(w) > 2 * top] /= 4
+        for part in w.reshape(-1, 32):
+            g = np.resize(part, G).copy()
+            g[rng.integers(0, G)] = top * 2.0
+            rows.append(g)
+    W = oracle.f32_to_bf16_bits(np.array(rows, dtype=np.float32))
+    halves = (np.array(rows) * 0 + rng.integers(-14, 15, (len(rows), G)) / 2)  # s = 1: every second one is a tie
+    halves[:, 0] = 7.0
+    special = oracle.f32_to_bf16_bits(rng.standard_normal((12, G), dtype=np.float32))
+    for r, (lo, hi) in enumerate([(0x0001, 0x0040), (0x0080, 0x0100), (0x0300, 0x0D80), (0x7000, 0x7F7F)]):
+        special[r] = rng.integers(lo, hi, G) | (rng.integers(0, 2, G) << 15)  # subnormal to largest magnitudes
+    W = np.concatenate([W, oracle.f32_to_bf16_bits(halves.astype(np.float32)), special])
+    Wq, S = quant(kernels, W, G)
+    Wq_o, S_o = oracle.w4_quantize(W, G)
+    assert np.array_equal(S, S_o) and np.array_equal(Wq, Wq_o)
+    # an infinite or nan member changes its own group only
+    bad = W.copy()
+    bad[1, 3], bad[5, 0], bad[9, G - 1] = 0x7F80, 0x7FC0, 0xFF80
+    Wq_b, S_b = quant(kernels, bad, G)
+    keep = np.setdiff1d(np.arange(len(W)), [1, 5, 9])
+    assert np.array_equal(Wq_b[keep], Wq_o[keep]) and np.array_equal(S_b[keep], S_o[keep])
+    assert oracle.bf16_bits_to_f32(S_b[1])[0] == np.inf and oracle.bf16_bits_to_f32(S_b[9])[0] == np.inf
+    assert (Wq_b[5, 0] & 15) == 8  # a nan is stored as the zero point, its group scaled by the other members
+
+
 def test_error_codes(kernels):
     W = torch.zeros(4, 96, dtype=torch.bfloat16, device="cuda")
     with pytest.raises(RuntimeError, match="ns_w4_quantize failed with code -1"):
