@@ -167,7 +167,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   volatile int* abort_flag = reinterpret_cast<volatile int*>(gen_base + geo::kBarOffset + 26 * 8);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gen_base + geo::kBarOffset + 27 * 8);
 
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   // CTA pair: this CTA loads and unpacks rows [wr0, wr0 + kWRows) of the weight tile; the peer the other half
   uint32_t crank = 0;
   if constexpr (PAIR) crank = cluster_ctarank_u32();
@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   __syncthreads();
   if constexpr (PAIR) cluster_sync_all();  // the peer's barriers are initialised before anybody arrives on them
   tc_fence_after_sync();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   const bool poisoned = *reinterpret_cast<volatile int*>(p.status) != 0;
 
   if (!poisoned) {
@@ -264,52 +264,61 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       __syncwarp();
     } else if (warp == 1) {
       // ------------------------------------------------------------ MMA issuer (pairs: the rank-0 CTA's, for both)
-      if (lane == 0 && (!PAIR || leader)) {
+      // The whole warp runs the loop and one elected lane issues: with everything the instructions take the same in all
+      // lanes the descriptors stay in uniform registers.  (Issuing under `if (lane == 0)` cost up to 176 cycles per
+      // instruction, more than the 128 the tensor core needs for it.)
+      if (!PAIR || leader) {
         constexpr uint32_t idesc = umma_idesc_bf16(PAIR ? 256 : 128, kBN);
+        const uint64_t desc_a0 = umma_desc_k128(base), desc_b0 = umma_desc_k128(base + geo::kBdOffset);
         int s = 0, b = 0;
         uint32_t ph = 0, bph = 0;
         for (int kb = 0; kb < nkb; ++kb) {
-          if constexpr (PAIR) {
-            // X tiles of both CTAs (counted here), dequantised halves of both CTAs (the peer's warps arrive here)
-            mbar_wait(bar_full + 8 * s, ph, abort_flag);
-            mbar_wait(bar_bd_full + 8 * b, bph, abort_flag);
-          } else {
-            mbar_wait(bar_full + 8 * s, ph, abort_flag);
-            mbar_wait(bar_bd_full + 8 * b, bph, abort_flag);
-          }
+          // X tiles (pairs: of both CTAs, counted here), dequantised tile (pairs: both halves; the peer's warps arrive
+          // here)
+          mbar_wait(bar_full + 8 * s, ph, abort_flag);
+          mbar_wait(bar_bd_full + 8 * b, bph, abort_flag);
+          __syncwarp();
           tc_fence_after_sync();
-          const uint32_t a_addr = base + s * geo::kStageBytes;
-          const uint32_t b_addr = base + geo::kBdOffset + b * geo::kBdBytes;
+          const uint64_t da0 = desc_a0 + s * (geo::kStageBytes >> 4), db0 = desc_b0 + b * (geo::kBdBytes >> 4);
+          if (elect_one()) {
 #pragma unroll
-          for (int kk = 0; kk < kBK / 16; ++kk) {
-            const uint64_t db = umma_desc_k128(b_addr + kk * 32);
+            for (int kk = 0; kk < kBK / 16; ++kk) {
 #pragma unroll
-            for (int mi = 0; mi < MI; ++mi) {
-              const uint64_t da = umma_desc_k128(a_addr + mi * kATileBytes + kk * 32);
-              if constexpr (PAIR)
-                umma_f16_ss_pair(tmem_base + mi * kBN, da, db, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
-              else
-                umma_f16_ss(tmem_base + mi * kBN, da, db, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
+              for (int mi = 0; mi < MI; ++mi) {
+                const uint64_t da = da0 + mi * (kATileBytes >> 4) + kk * 2, db = db0 + kk * 2;
+                if constexpr (PAIR)
+                  umma_f16_ss_pair(tmem_base + mi * kBN, da, db, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
+                else
+                  umma_f16_ss(tmem_base + mi * kBN, da, db, idesc, (kb > 0 || kk > 0) ? 1u : 0u);
+              }
+            }
+            if constexpr (PAIR) {
+              // the stage and the dequantised buffer are free in BOTH CTAs
+              umma_commit_pair(bar_empty + 8 * s);
+              umma_commit_pair(peer_base + (bar_empty - base) + 8 * s);
+              umma_commit_pair(bar_bd_empty + 8 * b);
+              umma_commit_pair(peer_base + (bar_bd_empty - base) + 8 * b);
+              if (kb + 1 == nkb) {
+                umma_commit_pair(bar_acc);
+                umma_commit_pair(peer_base + (bar_acc - base));
+              }
+            } else {
+              umma_commit(bar_empty + 8 * s);      // the X tile and the packed tile of this stage are consumed
+              umma_commit(bar_bd_empty + 8 * b);   // the dequantised tile may be overwritten
+              if (kb + 1 == nkb) umma_commit(bar_acc);
             }
           }
-          if constexpr (PAIR) {
-            // the stage and the dequantised buffer are free in BOTH CTAs
-            umma_commit_pair(bar_empty + 8 * s);
-            umma_commit_pair(peer_base + (bar_empty - base) + 8 * s);
-            umma_commit_pair(bar_bd_empty + 8 * b);
-            umma_commit_pair(peer_base + (bar_bd_empty - base) + 8 * b);
-          } else {
-            umma_commit(bar_empty + 8 * s);      // the X tile and the packed tile of this stage are consumed
-            umma_commit(bar_bd_empty + 8 * b);   // the dequantised tile may be overwritten
-          }
+          __syncwarp();
           if (++s == geo::kStages) { s = 0; ph ^= 1; }
           if (++b == geo::kBdCount) { b = 0; bph ^= 1; }
         }
-        if constexpr (PAIR) {
-          umma_commit_pair(bar_acc);
-          umma_commit_pair(peer_base + (bar_acc - base));
-        } else {
-          umma_commit(bar_acc);
+        if (nkb == 0 && elect_one()) {  // a split with no K blocks
+          if constexpr (PAIR) {
+            umma_commit_pair(bar_acc);
+            umma_commit_pair(peer_base + (bar_acc - base));
+          } else {
+            umma_commit(bar_acc);
+          }
         }
       }
       __syncwarp();
