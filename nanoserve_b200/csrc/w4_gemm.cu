@@ -571,19 +571,11 @@ int gemm_launch(const void* X, const void* Wq, const void* S, void* Y, int M, in
     return kErrBadPointer;
   if (!ws.status) return kErrWorkspace;
 
-  CUtensorMap tx, tw;
-  if (!make_tensor_map_2d(&tx, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, X, (uint64_t)M, (uint64_t)K, 128, kBK,
-                 CU_TENSOR_MAP_SWIZZLE_128B))
-    return kErrDevice;
   // CTA pairs (each unpacks half of the weight tile for both): where the token tiles pair up without much padding.
   // A lone token tile (M <= 256) would be paired with an empty one and do the whole unpack for half the product.
   const int mi_ = M <= 128 ? 1 : 2;
   const int tiles_m = (M + 128 * mi_ - 1) / (128 * mi_);
   const bool pair = !(flags & kFlagGemmNoPairs) && mi_ == 2 && (tiles_m % 2 == 0 || tiles_m >= 7);
-  if (!make_tensor_map_2d(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, Wq, (uint64_t)N, (uint64_t)K / 8, pair ? kBN / 2 : kBN,
-                 kBK / 8, CU_TENSOR_MAP_SWIZZLE_NONE))
-    return kErrDevice;
-
   GemmParams p{};
   p.S = static_cast<const __nv_bfloat16*>(S);
   p.Y = static_cast<__nv_bfloat16*>(Y);
@@ -624,7 +616,25 @@ int gemm_launch(const void* X, const void* Wq, const void* S, void* Y, int M, in
     p.tail_ks = best;
     p.partial = ws.partial;
     p.counters = ws.counters;
+    // The few-token kernel where it is estimated to be shorter.  This kernel: 0.93 us per K block of a 256 x 256 tile
+    // (0.6 of a 128-token one), 5 us to start and finish, 20 more where the last wave is split (its fp32 part-tiles), 35
+    // more per wave where N % 8 forces its epilogue to single values (1070 x 6051 x 1792: 108 us against 32).
+    // Measured at 512 tokens: 4608 x 3584 40 us against 17.8 us, 3584 x 18944 75 against 64, 37888 x 3584 110 against
+    // 121 (this one stays).
+    const double block = mi == 2 ? 0.93 : 0.6;
+    const long tail_waves = (n_tail * best + sms - 1) / sms;
+    const double waves = (double)((tiles - n_tail) / sms_even);
+    const double us = 5.0 + (best > 1 ? 20.0 : 0.0) + (N % 8 ? 35.0 * (waves + tail_waves) : 0.0) +
+                      block * (waves * p.nkb + (double)tail_waves * ((p.nkb + best - 1) / best));
+    if (gemm_narrow_applies(M, N, K, flags, us, sms))
+      return gemm_narrow_launch(X, Wq, S, Y, M, N, K, G, ws, flags, sms, stream);
   }
+  CUtensorMap tx, tw;
+  if (!make_tensor_map_2d(&tx, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, X, (uint64_t)M, (uint64_t)K, 128, kBK,
+                 CU_TENSOR_MAP_SWIZZLE_128B) ||
+      !make_tensor_map_2d(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, Wq, (uint64_t)N, (uint64_t)K / 8, pair ? kBN / 2 : kBN,
+                 kBK / 8, CU_TENSOR_MAP_SWIZZLE_NONE))
+    return kErrDevice;
   if (pair) return launch_gemm<2, true>(tx, tw, p, stream);
   return M <= 128 ? launch_gemm<1, false>(tx, tw, p, stream) : launch_gemm<2, false>(tx, tw, p, stream);
 }

@@ -1,0 +1,571 @@
+// W4A16 GEMM for sm_100a where the tokens are few:  Y[M,N] (bf16) = X[M,K] (bf16) . dequant(Wq, S)^T  for M > 16, the
+// token counts of batched decoding and short prompts.  Same operands and numerics as w4_gemm.cu: each weight is
+// RN_bf16((q - 8) * s), products accumulate in fp32, one rounding at the store.
+//
+// What bounds it: the packed weights' way from HBM (0.5 bytes per weight), and next to it the conversion of every
+// weight (17 instructions per eight).  w4_gemm.cu gives the tokens the 128-row side of the MMA and writes the converted
+// weights to shared memory: with 48 tokens it pads the MMA to 128, sends every weight through shared memory twice and
+// has one CTA per 256 weight rows with no way to fill the chip but fp32 part-tiles in global memory.  Here
+//   * the WEIGHTS are the M side of tcgen05.mma (128 rows per block) and the tokens its N side (16 to 128 columns, a
+//     multiple of 16): the MMA's work follows the token count;
+//   * converted weights go from registers to TENSOR MEMORY (tcgen05.st; a thread owns a weight row = a TMEM lane) and
+//     the MMA takes its A operand from there.  Shared memory carries the packed words once and the X tile;
+//   * K is cut over the CTAs of a CLUSTER (up to eight), which add their fp32 accumulators up through distributed shared
+//     memory in rank order: no scratch in global memory, no counters, the result does not depend on timing;
+//   * launched programmatically: packed weights and scales stream in while the previous kernel finishes; X and Y are
+//     touched only after it has.
+// Warps: 0 packed words (TMA), 1 MMA issue and TMEM, 2 X tiles (TMA), 3 idle, then DW conversion warps, which also do
+// the epilogue.  All rings run on mbarriers with bounded waits; a CTA that gives up records a status, still takes part in
+// the cluster barriers, frees its TMEM and returns.
+#include <cuda.h>
+
+#include <algorithm>
+#include <atomic>
+
+#include "ptx.cuh"
+#include "tensor_map.h"
+#include "w4_common.cuh"
+#include "w4_internal.h"
+
+namespace b2 {
+namespace {
+
+constexpr int kKB = 128;              // K per step and per X slot: two 128-byte rows of X per token
+constexpr int kMaxSlots = 10;
+constexpr int kHeaderBytes = 1024;    // barriers and flags
+constexpr int kSmemHalf = 115712;     // two CTAs per SM: (228 KB / 2) - 1 KB
+constexpr int kSmemFull = 232448;
+
+struct NarrowParams {
+  const __nv_bfloat16* S;
+  __nv_bfloat16* Y;
+  int* status;
+  int M, N, K, G, KG;
+  int nkb;        // K blocks of 128
+  int ks;         // CTAs of a cluster, each with its share of the K blocks
+  int nt;         // token columns of a tile (multiple of 16)
+  int t_tiles;    // token tiles (fastest in the tile order: neighbours read the same weights)
+  int sw, sx;     // ring slots of packed words, of X
+  int sv;         // scales per load: 4, 2 or 1, by the alignment of a row of S
+  int tmem_cols;  // power of two
+};
+
+__device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const uint32_t (&r)[32]) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%32], "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31};" ::"r"(r[0]),
+      "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]), "r"(r[10]),
+      "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]),
+      "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]),
+      "r"(r[29]), "r"(r[30]), "r"(r[31]), "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tmem_ld_32x16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+// D[tmem] (+)= A[tmem] * B[smem desc]: A is 128 lanes x 8 columns of bf16 pairs per K = 16.
+__device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc,
+                                            uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
+      "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr, uint32_t rank) {
+  float4 v;
+  asm volatile(
+      "{\n\t.reg .u32 a;\n\t"
+      "mapa.shared::cluster.u32 a, %4, %5;\n\t"
+      "ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [a];\n\t}"
+      : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+      : "r"(addr), "r"(rank)
+      : "memory");
+  return v;
+}
+
+// One packed word -> four bf16 pairs of (q - 8) * s in their natural order {w0,w1} {w2,w3} {w4,w5} {w6,w7}.  The byte
+// permutation puts nibble 2i into the low half (from w) and nibble 2i + 1 into the high half (from w >> 4): the unpack
+// order is the operand's order without a second permutation.
+__device__ __forceinline__ void dequant_word(uint32_t w, uint32_t s2, uint32_t mask, uint32_t magic, uint32_t* o) {
+  const uint32_t u = w >> 4;
+  o[0] = mul_bf16x2(sub136_bf16x2(lop3_and_or(__byte_perm(w, u, 0x4400), mask, magic)), s2);
+  o[1] = mul_bf16x2(sub136_bf16x2(lop3_and_or(__byte_perm(w, u, 0x5511), mask, magic)), s2);
+  o[2] = mul_bf16x2(sub136_bf16x2(lop3_and_or(__byte_perm(w, u, 0x6622), mask, magic)), s2);
+  o[3] = mul_bf16x2(sub136_bf16x2(lop3_and_or(__byte_perm(w, u, 0x7733), mask, magic)), s2);
+}
+
+// MB: blocks of 128 weight rows per tile (each X tile is then read by MB MMAs).  DW: conversion warps, in DW / (4 MB)
+// groups that take the K blocks in turn; the converted weights of two K blocks fit in TMEM.  MINB: CTAs per SM.
+// G128: groups of 128 (a scale per row and step), read four at a time.
+template <int MB, int DW, int MINB, bool G128>
+__global__ void __launch_bounds__(128 + DW * 32, MINB)
+    w4_gemm_narrow_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
+                          const NarrowParams p) {
+  constexpr int kRows = MB * 128, kGroups = DW / (4 * MB), kWSlot = kRows * 128;  // a slot of packed words: K = 256
+  static_assert(kGroups == 2, "a slot of packed words holds a step for either group");
+  extern __shared__ unsigned char smem_raw[];
+  const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;  // swizzled tiles
+  unsigned char* gen = smem_raw + (base - smem_u32(smem_raw));
+  const uint32_t bar_w_full = base, bar_w_empty = base + 8 * kMaxSlots;
+  const uint32_t bar_x_full = base + 16 * kMaxSlots, bar_x_empty = base + 24 * kMaxSlots;
+  const uint32_t bar_a_full = base + 32 * kMaxSlots, bar_a_empty = bar_a_full + 16;
+  const uint32_t bar_acc = bar_a_empty + 16;
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(gen + 512);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gen + 516);
+  const uint32_t ring_w = base + kHeaderBytes, ring_x = ring_w + p.sw * kWSlot;
+  const uint32_t x_slot = (uint32_t)p.nt * 256;
+
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+  const int crank = p.ks > 1 ? (int)cluster_rank() : 0;
+  const int tile = blockIdx.x / p.ks;
+  const int m0 = (tile % p.t_tiles) * p.nt, n0 = (tile / p.t_tiles) * kRows;
+  const int kb0 = (int)((long)crank * p.nkb / p.ks), nkb = (int)((long)(crank + 1) * p.nkb / p.ks) - kb0;
+
+  if (tid == 0) {
+    *abort_flag = 0;
+    for (int s = 0; s < kMaxSlots; ++s) {
+      mbar_init(bar_w_full + 8 * s, 1);
+      mbar_init(bar_w_empty + 8 * s, DW);
+      mbar_init(bar_x_full + 8 * s, 1);
+      mbar_init(bar_x_empty + 8 * s, 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(bar_a_full + 8 * b, 4 * MB);
+      mbar_init(bar_a_empty + 8 * b, 1);
+    }
+    mbar_init(bar_acc, 1);
+    fence_mbar_init();
+    tma_prefetch_desc(&tmap_w);
+    tma_prefetch_desc(&tmap_x);
+  }
+  if (warp == 1) {
+    tmem_alloc(smem_u32(tmem_slot), p.tmem_cols);
+    tmem_relinquish();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  pdl_launch_dependents();
+  const uint32_t tmem_d = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+  const uint32_t tmem_a = tmem_d + ((MB * p.nt + 31) & ~31);
+  const bool poisoned = *reinterpret_cast<volatile int*>(p.status) != 0;
+
+  if (!poisoned) {
+    if (warp == 0) {
+      if (lane == 0) {
+        int s = 0;
+        uint32_t ph = 1;
+        for (int i = 0; i < nkb; i += 2) {  // (128-byte rows: the copy engine's rate counts rows, not bytes)
+          mbar_wait(bar_w_empty + 8 * s, ph, abort_flag);
+          mbar_arrive_expect_tx(bar_w_full + 8 * s, kWSlot);
+          tma_load_2d(ring_w + s * kWSlot, &tmap_w, (kb0 + i) * (kKB / 8), n0, bar_w_full + 8 * s);
+          if (++s == p.sw) { s = 0; ph ^= 1; }
+        }
+      }
+      __syncwarp();
+    } else if (warp == 2) {
+      if (lane == 0) {
+        pdl_wait_prior_grid();
+        int s = 0;
+        uint32_t ph = 1;
+        for (int i = 0; i < nkb; ++i) {
+          mbar_wait(bar_x_empty + 8 * s, ph, abort_flag);
+          mbar_arrive_expect_tx(bar_x_full + 8 * s, x_slot);
+          const uint32_t dst = ring_x + s * x_slot;
+          tma_load_2d(dst, &tmap_x, (kb0 + i) * kKB, m0, bar_x_full + 8 * s);
+          tma_load_2d(dst + x_slot / 2, &tmap_x, (kb0 + i) * kKB + 64, m0, bar_x_full + 8 * s);
+          if (++s == p.sx) { s = 0; ph ^= 1; }
+        }
+      }
+      __syncwarp();
+    } else if (warp == 1) {
+      // The whole warp runs the loop and one elected lane issues: with everything the instructions take the same in all
+      // lanes the descriptors stay in uniform registers.  (Under `if (lane == 0)` an issue took 176 cycles, whatever the
+      // tile, and bounded the kernel.)
+      const uint32_t idesc = umma_idesc_bf16(128, p.nt);
+      const uint64_t desc0 = umma_desc_k128(ring_x);
+      int xs = 0;
+      uint32_t xph = 0;
+      for (int i = 0; i < nkb; ++i) {
+        const int buf = i & 1;
+        mbar_wait(bar_x_full + 8 * xs, xph, abort_flag);
+        mbar_wait(bar_a_full + 8 * buf, (i >> 1) & 1, abort_flag);
+        __syncwarp();
+        tc_fence_after_sync();
+        const uint64_t db = desc0 + ((xs * x_slot) >> 4);
+        const uint32_t a = tmem_a + buf * MB * 64;
+        if (elect_one()) {
+#pragma unroll
+          for (int kk = 0; kk < 8; ++kk) {
+            const uint64_t d = db + (kk & 3) * 2 + (kk >> 2) * (x_slot >> 5);
+#pragma unroll
+            for (int mb = 0; mb < MB; ++mb)
+              umma_f16_ts(tmem_d + mb * p.nt, a + mb * 64 + kk * 8, d, idesc, (i > 0 || kk > 0) ? 1u : 0u);
+          }
+          umma_commit(bar_a_empty + 8 * buf);
+          umma_commit(bar_x_empty + 8 * xs);
+          if (i + 1 == nkb) umma_commit(bar_acc);
+        }
+        __syncwarp();
+        if (++xs == p.sx) { xs = 0; xph ^= 1; }
+      }
+    }
+  }
+  if (warp >= 4) {
+    const int dw = warp - 4, quad = warp & 3;       // the quarter of the TMEM lanes this warp may touch
+    const int mb = (dw >> 2) % MB, grp = dw / (4 * MB);
+    const int row = mb * 128 + quad * 32 + lane;    // weight row of the tile
+    const uint32_t lane_off = (uint32_t)(quad * 32) << 16;
+    if (!poisoned) {
+      const int n = n0 + row;
+      const bool live = n < p.N;
+      uint32_t k_mask = kNibblePairMask, k_magic = kMagic128x2;
+      asm volatile("" : "+r"(k_mask), "+r"(k_magic));
+      const __nv_bfloat16* s_row = p.S + (size_t)(live ? n : 0) * p.KG;
+      // Scales, p.sv of them per load (a thread reads along its own row, so every load touches 32 lines), the next load
+      // in flight while one is used.  General groups: (g, kin) is the group of the current K position and the position
+      // inside it, vi the load that group is in.
+      const int sv = G128 ? 4 : p.sv;
+      auto load_sv = [&](int v) {
+        uint2 r = make_uint2(0u, 0u);
+        const int g = v * sv;
+        if (live && g < p.KG) {
+          if (sv == 4) r = __ldg(reinterpret_cast<const uint2*>(s_row + g));
+          else if (sv == 2) r.x = __ldg(reinterpret_cast<const uint32_t*>(s_row + g));
+          else r.x = __bfloat16_as_ushort(__ldg(s_row + g));
+        }
+        return r;
+      };
+      int k = (kb0 + grp) * kKB;
+      int g = G128 ? kb0 + grp : k / p.G, kin = G128 ? 0 : k - g * p.G, vi = g / sv;
+      uint2 cur = load_sv(vi), nxt = load_sv(vi + 1);
+      auto scale2 = [&]() {  // the pair (s, s) of the current position
+        const int e = g - vi * sv;
+        return __byte_perm(e & 2 ? cur.y : cur.x, 0, e & 1 ? 0x3232 : 0x1010);
+      };
+      auto advance = [&](int by) {
+        kin += by;
+        while (kin >= p.G) {
+          kin -= p.G;
+          ++g;
+        }
+        while (g >= (vi + 1) * sv) {
+          ++vi;
+          cur = nxt;
+          nxt = load_sv(vi + 1);
+        }
+      };
+      const uint32_t pick = (kb0 + grp) & 1 ? 0x3232 : 0x1010;
+      const uint32_t src_row = ring_w + row * 128, swz = (uint32_t)row & 7u;
+      uint32_t src_off[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) src_off[j] = src_row + (((uint32_t)(grp * 4 + j) ^ swz) << 4);
+      const uint32_t a_dst = tmem_a + lane_off + (grp * MB + mb) * 64;
+      int s = 0;
+      uint32_t ph = 0, aph = 1;
+      for (int i = grp; i < nkb; i += 2) {
+        uint32_t sc[4];
+        if constexpr (G128) {
+          sc[0] = sc[1] = sc[2] = sc[3] = __byte_perm(g & 2 ? cur.y : cur.x, 0, pick);
+          if (g & 2) {
+            cur = nxt;
+            nxt = load_sv((g >> 2) + 2);
+          }
+          g += 2;
+        } else {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            sc[j] = k + 32 * j < p.K ? scale2() : 0u;  // behind the end of K: zero weights
+            advance(j < 3 ? 32 : 32 + kKB);
+          }
+          k += 2 * kKB;
+        }
+        mbar_wait(bar_w_full + 8 * s, ph, abort_flag);
+        uint4 w[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) w[j] = lds128(src_off[j] + s * kWSlot);
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          uint32_t v[32];
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            const uint4 q = w[2 * half + j];
+            dequant_word(q.x, sc[2 * half + j], k_mask, k_magic, v + 16 * j);
+            dequant_word(q.y, sc[2 * half + j], k_mask, k_magic, v + 16 * j + 4);
+            dequant_word(q.z, sc[2 * half + j], k_mask, k_magic, v + 16 * j + 8);
+            dequant_word(q.w, sc[2 * half + j], k_mask, k_magic, v + 16 * j + 12);
+          }
+          if (half == 0) {
+            mbar_wait(bar_a_empty + 8 * grp, aph, abort_flag);
+            __syncwarp();
+            tc_fence_after_sync();
+          }
+          tmem_st_32x32(a_dst + half * 32, v);
+        }
+        tmem_st_wait();
+        tc_fence_before_sync();
+        __syncwarp();
+        if (lane == 0) {
+          mbar_arrive(bar_a_full + 8 * grp);
+          mbar_arrive(bar_w_empty + 8 * s);  // the slot's words went into the conversion above
+        }
+        aph ^= 1;
+        if (++s == p.sw) { s = 0; ph ^= 1; }
+      }
+      mbar_wait(bar_acc, 0, abort_flag);
+      __syncwarp();
+      tc_fence_after_sync();
+      pdl_wait_prior_grid();  // Y may still be read by the kernel in front
+
+      // ---- the accumulator columns (tokens) of the warp's 32 rows; two groups of warps take alternate 16 columns
+      const int rt = min(p.nt, p.M - m0);  // tokens of the tile
+      for (int c0 = 16 * grp; c0 < rt; c0 += 16 * kGroups) {
+        uint32_t v[16];
+        tmem_ld_32x16(tmem_d + lane_off + mb * p.nt + c0, v);
+        tmem_ld_wait();
+        if (p.ks == 1) {
+          __nv_bfloat16* y = p.Y + (size_t)(m0 + c0) * p.N + n;
+#pragma unroll
+          for (int e = 0; e < 16; ++e)
+            if (live && c0 + e < rt) y[(size_t)e * p.N] = __float2bfloat16(__uint_as_float(v[e]));
+        } else {  // [token][row], over the rings: every copy has landed and every MMA has read its operands
+#pragma unroll
+          for (int e = 0; e < 16; ++e)
+            asm volatile("st.shared.b32 [%0], %1;" ::"r"(ring_w + (uint32_t)((c0 + e) * kRows + row) * 4), "r"(v[e])
+                         : "memory");
+        }
+      }
+    }
+  }
+  tc_fence_before_sync();
+  if (p.ks > 1) {
+    cluster_barrier();
+    // every CTA adds up its share of the tile, four rows of a token per thread, in rank order
+    if (warp >= 4 && !poisoned) {
+      const int rt = min(p.nt, p.M - m0), units = rt * (kRows / 4);
+      const int u1 = (int)((long)(crank + 1) * units / p.ks);
+      for (int u = (int)((long)crank * units / p.ks) + tid - 128; u < u1; u += DW * 32) {
+        const int tok = u / (kRows / 4), r = (u % (kRows / 4)) * 4, n = n0 + r;
+        const uint32_t at = ring_w + (uint32_t)(tok * kRows + r) * 4;
+        float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int z = 0; z < 8; ++z)
+          if (z < p.ks) {
+            const float4 b = ld_cluster_f4(at, z);
+            a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
+          }
+        __nv_bfloat16* y = p.Y + (size_t)(m0 + tok) * p.N + n;
+        if (n + 4 <= p.N && (p.N & 3) == 0) {
+          const __nv_bfloat162 lo = __floats2bfloat162_rn(a.x, a.y), hi = __floats2bfloat162_rn(a.z, a.w);
+          *reinterpret_cast<uint2*>(y) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo),
+                                                    *reinterpret_cast<const uint32_t*>(&hi));
+        } else {
+          const float f[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            if (n + e < p.N) y[e] = __float2bfloat16(f[e]);
+        }
+      }
+    }
+    __syncwarp();
+    cluster_barrier();  // the peers have read this CTA's part
+  }
+  __syncthreads();
+  if (*abort_flag) {
+    if (tid == 0) atomicCAS(p.status, kStatusOk, kStatusGemmTimeout);
+    for (int i = 0; i < 64; ++i) __nanosleep(2000);  // copies in flight land before the shared memory is released
+    __syncthreads();
+  }
+  if (warp == 1) {
+    tc_fence_after_sync();
+    tmem_dealloc(tmem_d, p.tmem_cols);
+  }
+}
+
+using NarrowKernel = void (*)(const CUtensorMap, const CUtensorMap, const NarrowParams);
+struct NarrowForm {
+  NarrowKernel kernel;
+  int rows, warps, per_sm, smem;
+};
+// form 0: 128 weight rows, two CTAs per SM; form 1: 256 rows, one CTA.  All of an SM's (or half an SM's) shared memory
+// is asked for, needed or not: at most 512 columns' worth of CTAs then fit on an SM, whatever mix of these launches
+// overlaps, and no CTA of a cluster waits for tensor memory that a CTA at a cluster barrier holds.
+NarrowForm narrow_form(int form, bool g128) {
+  if (form == 0)
+    return {g128 ? w4_gemm_narrow_kernel<1, 8, 2, true> : w4_gemm_narrow_kernel<1, 8, 2, false>, 128, 8, 2, kSmemHalf};
+  return {g128 ? w4_gemm_narrow_kernel<2, 16, 1, true> : w4_gemm_narrow_kernel<2, 16, 1, false>, 256, 16, 1, kSmemFull};
+}
+
+int narrow_attributes(const NarrowForm& f, int form, bool g128, int dev) {
+  static std::atomic<bool> done[64][2][2];
+  if (dev >= 0 && dev < 64 && done[dev][form][g128].load(std::memory_order_acquire)) return 0;
+  const cudaError_t e = cudaFuncSetAttribute(f.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, f.smem);
+  if (e == cudaSuccess && dev >= 0 && dev < 64) done[dev][form][g128].store(true, std::memory_order_release);
+  return (int)e;
+}
+
+void narrow_config(const NarrowForm& f, int grid, int ks, bool pdl, cudaLaunchConfig_t* cfg, cudaLaunchAttribute (&attr)[2]) {
+  cfg->gridDim = dim3(grid);
+  cfg->blockDim = dim3(128 + f.warps * 32);
+  cfg->dynamicSmemBytes = f.smem;
+  int na = 0;
+  if (ks > 1) {
+    attr[na].id = cudaLaunchAttributeClusterDimension;
+    attr[na].val.clusterDim.x = ks;
+    attr[na].val.clusterDim.y = 1;
+    attr[na].val.clusterDim.z = 1;
+    ++na;
+  }
+  if (pdl) {
+    attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[na].val.programmaticStreamSerializationAllowed = 1;
+    ++na;
+  }
+  cfg->attrs = attr;
+  cfg->numAttrs = na;
+}
+
+// CTAs of a form the device runs at a time in clusters of ks (a cluster stays inside one GPC: eight to a cluster leave
+// some SMs of every GPC out), asked for once per device.
+int narrow_capacity(int form, int ks, int sm_count, int dev) {
+  const NarrowForm f = narrow_form(form, true);
+  const int all = sm_count * f.per_sm;
+  if (ks == 1) return all;
+  static std::atomic<int> known[64][2][9];
+  const bool cached = dev >= 0 && dev < 64;
+  if (cached)
+    if (const int v = known[dev][form][ks].load(std::memory_order_relaxed)) return v;
+  int clusters = 0;
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute attr[2];
+  narrow_config(f, ks, ks, false, &cfg, attr);
+  if (narrow_attributes(f, form, true, dev) != 0 ||
+      cudaOccupancyMaxActiveClusters(&clusters, f.kernel, &cfg) != cudaSuccess || clusters < 1) {
+    (void)cudaGetLastError();
+    clusters = std::max(1, all / ks * 3 / 4);
+  }
+  const int v = std::min(all, clusters * ks);
+  if (cached) known[dev][form][ks].store(v, std::memory_order_relaxed);
+  return v;
+}
+
+struct NarrowPlan {
+  int form = 0, ks = 1, nt = 16, t_tiles = 1;
+  long n_tiles = 0;
+  double us = 0;
+};
+
+// Estimated time of a form and a cluster size: waves of CTAs, each its K blocks at the rate measured with the chip full
+// (one 128-row CTA on an SM, two, one 256-row CTA; the rate falls with the token columns), plus start-up and, when K is
+// cut, the exchange through distributed shared memory.  Fitted to 512 to 8192 x 3584 to 28672 at 17 to 512 tokens; the
+// form it picks was within 6 % of the best form tried on each.
+void narrow_estimate(NarrowPlan* pl, int N, int K, int sm_count, int dev) {
+  const int nkb = (K + kKB - 1) / kKB;
+  pl->n_tiles = (long)pl->t_tiles * ((N + (pl->form ? 255 : 127)) / (pl->form ? 256 : 128));
+  const int cap = narrow_capacity(pl->form, pl->ks, sm_count, dev);
+  const long ctas = pl->n_tiles * pl->ks, waves = (ctas + cap - 1) / cap;
+  const int blocks = (nkb + pl->ks - 1) / pl->ks;
+  double block;
+  if (pl->form)
+    block = ctas > 100 ? 0.50 + 0.0040 * pl->nt : 0.40 + 0.0032 * pl->nt;
+  else
+    block = ctas > sm_count ? 0.55 + 0.0034 * pl->nt : 0.43 + 0.0022 * pl->nt;
+  pl->us = 3.0 + (pl->ks > 1 ? 1.0 + 0.025 * pl->nt : 0.0) + waves * blocks * block + (waves - 1) * 2.0;
+}
+
+NarrowPlan narrow_plan(int M, int N, int K, int flags, int sm_count, int dev) {
+  NarrowPlan best;
+  const bool forced = flags & kFlagGemmNarrow;
+  const int want_form = forced ? (flags >> 24) & 3 : 0, want_ks = forced ? (flags >> 20) & 15 : 0;
+  const int nkb = (K + kKB - 1) / kKB;
+  bool any = false;
+  for (int form = 0; form < 2; ++form) {
+    if (want_form && form != want_form - 1) continue;
+    for (int ks = 1; ks <= 8 && ks <= nkb; ++ks) {
+      if (want_ks && ks != std::min({want_ks, 8, nkb})) continue;
+      NarrowPlan pl;
+      pl.form = form;
+      pl.ks = ks;
+      pl.t_tiles = (M + 127) / 128;
+      pl.nt = ((M + pl.t_tiles - 1) / pl.t_tiles + 15) / 16 * 16;
+      narrow_estimate(&pl, N, K, sm_count, dev);
+      if (!any || pl.us < best.us) best = pl;
+      any = true;
+    }
+  }
+  return best;
+}
+
+int current_device() {
+  int dev = -1;
+  return cudaGetDevice(&dev) == cudaSuccess ? dev : -1;
+}
+
+}  // namespace
+
+// Whether this kernel takes a GEMM that the general kernel would run in about wide_us microseconds.
+bool gemm_narrow_applies(int M, int N, int K, int flags, double wide_us, int sm_count) {
+  if (flags & (kFlagGemmNoPairs | kFlagGemmWholeTiles | kFlagGemmWide)) return false;  // the other kernel's switches
+  if (flags & kFlagGemmNarrow) return true;
+  return narrow_plan(M, N, K, flags, sm_count, current_device()).us < wide_us;
+}
+
+// The arguments have been checked by gemm_launch.
+int gemm_narrow_launch(const void* X, const void* Wq, const void* S, void* Y, int M, int N, int K, int G,
+                       const Workspace& ws, int flags, int sm_count, cudaStream_t stream) {
+  const int dev = current_device();
+  const NarrowPlan pl = narrow_plan(M, N, K, flags, sm_count, dev);
+  if (pl.n_tiles * pl.ks > 0x3fffffff) return kErrBadShape;
+  NarrowParams p{};
+  p.S = static_cast<const __nv_bfloat16*>(S);
+  p.Y = static_cast<__nv_bfloat16*>(Y);
+  p.status = ws.status;
+  p.M = M; p.N = N; p.K = K; p.G = G;
+  p.KG = K / G;
+  p.nkb = (K + kKB - 1) / kKB;
+  p.t_tiles = pl.t_tiles;
+  p.nt = pl.nt;
+  p.ks = pl.ks;
+  const uintptr_t sa = reinterpret_cast<uintptr_t>(S);
+  p.sv = p.KG % 4 == 0 && sa % 8 == 0 ? 4 : p.KG % 2 == 0 && sa % 4 == 0 ? 2 : 1;
+  const bool g128 = G == 128 && p.sv == 4;
+  const NarrowForm f = narrow_form(pl.form, g128);
+  const int slot_w = f.rows * 128, slot_x = p.nt * 256, room = f.smem - kHeaderBytes - 1024;
+  const int x_bytes = pl.form ? 128 << 10 : p.nt > 64 ? 72 << 10 : 48 << 10;  // the rest holds packed words
+  p.sx = std::max(2, std::min(6, x_bytes / slot_x));
+  p.sw = std::min(kMaxSlots, (room - p.sx * slot_x) / slot_w);
+  p.tmem_cols = pl.form ? 512 : 256;
+  CUtensorMap tx, tw;
+  if (!make_tensor_map_2d(&tx, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, X, (uint64_t)M, (uint64_t)K, p.nt, 64,
+                          CU_TENSOR_MAP_SWIZZLE_128B) ||
+      !make_tensor_map_2d(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, Wq, (uint64_t)N, (uint64_t)K / 8, f.rows, 2 * kKB / 8,
+                          CU_TENSOR_MAP_SWIZZLE_128B))
+    return kErrDevice;
+  if (const int rc = narrow_attributes(f, pl.form, g128, dev)) return rc;
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute attr[2];
+  narrow_config(f, (int)(pl.n_tiles * pl.ks), pl.ks, (flags & kFlagNoPdl) == 0, &cfg, attr);
+  cfg.stream = stream;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, f.kernel, tx, tw, p);
+  return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
+}
+
+}  // namespace b2

@@ -62,6 +62,9 @@ enum : int {
   kFlagStreamKernel = 262144 * 2,  // GEMV: run the streaming kernel for every M <= 16 it can serve (by default M <= 2)
   kFlagGemmNoPairs = 1 << 29,     // GEMM: one CTA per tile unpacks the whole weight tile (no clusters of two)
   kFlagGemmWholeTiles = 1 << 30,  // GEMM: every CTA takes whole output tiles (no part-tiles, no scratch)
+  kFlagGemmNarrow = 1 << 28,      // GEMM: the few-token kernel (w4_gemm_narrow.cu) for every M > 16; bits 20-23: CTAs per
+                                  // cluster along K, bits 24-25: tile (1: 128 rows, 2: 256), 0 = the rule decides
+  kFlagGemmWide = 1 << 27,        // GEMM: never that kernel
   kFlagNoPdl = 8,          // GEMV: do NOT launch with programmatic stream serialization (by default the kernel may
                            // begin -- weight prefetch only -- while the previous kernel of the stream still runs)
 };
@@ -117,6 +120,9 @@ int gemv_launch(const void* X, const void* Wq, const void* S, void* Y, int M, in
                 const Workspace& ws, int flags, int sm_count, cudaStream_t stream);
 int gemm_launch(const void* X, const void* Wq, const void* S, void* Y, int M, int N, int K, int G,
                 const Workspace& ws, int flags, int sm_count, cudaStream_t stream);
+bool gemm_narrow_applies(int M, int N, int K, int flags, double wide_us, int sm_count);
+int gemm_narrow_launch(const void* X, const void* Wq, const void* S, void* Y, int M, int N, int K, int G,
+                       const Workspace& ws, int flags, int sm_count, cudaStream_t stream);
 int quantize_launch(const void* W, void* Wq, void* S, int N, int K, int G, cudaStream_t stream);
 
 int decode_attention_fused_launch(const void* qkv, const void* bias, const void* inv_freq, const void* pos,

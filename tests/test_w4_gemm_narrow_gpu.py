@@ -1,0 +1,48 @@
+"""GPU parity tests of the few-token GEMM (weights as the M side of the MMA, converted into tensor memory) against the
+CPU oracle: every tile form and cluster size, at the edges of the token, row and K tiles."""
+import numpy as np
+import pytest
+import torch
+
+import oracle
+from nanoserve_b200.ops import FLAG_GEMM_WIDE, narrow_flags
+from tests.test_w4_gemm_gpu import rounded_weight_reference
+from tests.util import bits_to_torch, check_bf16_output, torch_to_bits, u32_to_torch
+
+pytestmark = pytest.mark.gpu
+
+
+def run(k, X, Wq, S, G, flags):
+    y = k.w4_linear(bits_to_torch(X), u32_to_torch(Wq), bits_to_torch(S), G, flags=flags)
+    torch.cuda.synchronize()
+    assert k.device_status() == 0
+    return torch_to_bits(y)
+
+
+# token columns 32 to 128 and two token tiles; rows below, at and above a tile, N odd; K of a quarter block, of whole
+# blocks, with a tail of 32, 64 and 96, shorter than the cluster; scales that load by four, by two and one by one
+SHAPES = [(17, 300, 1024, 128), (33, 129, 384, 128), (48, 513, 1152, 128), (64, 256, 640, 64), (65, 131, 544, 32),
+          (96, 256, 96, 96), (113, 77, 1120, 32), (128, 512, 2048, 128), (129, 260, 1024, 128), (200, 1, 160, 32),
+          (31, 400, 32, 32), (40, 128, 4096, 256)]
+
+
+@pytest.mark.parametrize("tile", [1, 2])
+@pytest.mark.parametrize("split", [0, 1, 2, 5, 8])
+def test_tiles_and_splits(kernels, tile, split):
+    for M, N, K, G in SHAPES:
+        X, Wq, S = oracle.synth_inputs(M, N, K, G, seed=M + N)
+        y = run(kernels, X, Wq, S, G, narrow_flags(split, tile))
+        # weights rounded to bf16 once, fp32 sums: half a bf16 step plus the sums' error (K <= 4096 terms)
+        check_bf16_output(y, rounded_weight_reference(X, Wq, S, G), 3e-5)
+        assert np.array_equal(y, run(kernels, X, Wq, S, G, narrow_flags(split, tile))), "two identical launches differ"
+
+
+@pytest.mark.parametrize("M", [17, 48, 100, 128, 300, 512])
+def test_rule_agrees_with_the_wide_kernel(kernels, M):
+    """What the rule picks against the general kernel on layer shapes: the same products in another order of sums."""
+    for N, K, G in [(4608, 3584, 128), (3584, 18944, 128), (1000, 4096, 64)]:
+        X, Wq, S = oracle.synth_inputs(M, N, K, G, seed=3)
+        a = oracle.bf16_bits_to_f32(run(kernels, X, Wq, S, G, 0))
+        b = oracle.bf16_bits_to_f32(run(kernels, X, Wq, S, G, FLAG_GEMM_WIDE))
+        assert np.abs(a - b).max() <= 2.0**-7 * np.abs(b).max()
+        assert (a != b).mean() < 0.05  # sums that differ in the last fp32 bits round differently once in a while
