@@ -202,6 +202,17 @@ int b2_w4_gemv_noalloc(const void* X, const void* Wq, const void* S, void* Y, in
  *   b2_greedy_next: token = argmax(logits[0..V)) (lowest index on ties); out_tokens[*step] = token; *step += 1;
  *     *pos += 1; x_next[0..H) = embed[token].  pos, step: int32 on the device; out_tokens: int64 on the device.
  */
+/*
+ * The prompt's counterparts: between the q|k|v projection and attention, and between gate|up and down.
+ *   b2_qkv_prefill: qkv [T, (Hq+2Hk)*D] bf16, positions 0..T-1: += bias (may be NULL), rotate-half RoPE on q (in place)
+ *     and k, k and v written to cache_k / cache_v [Hk, max_len, D] (the row's own k and v are left as they were).
+ *     T <= max_len, D % 16 == 0.
+ *   b2_swiglu_blocks: out [T, I] = silu(gate) * up with gu [T, 2 I] = `block` gate columns, their `block` up columns,
+ *     the next `block` gate columns ... (block % 8 == 0, I % block == 0); ns_swiglu's arithmetic.
+ */
+int b2_qkv_prefill(void* qkv, const void* bias, const void* inv_freq, void* cache_k, void* cache_v, int T, int Hq,
+                   int Hk, int D, int max_len, void* stream);
+int b2_swiglu_blocks(const void* gu, void* out, int T, int I, int block, void* stream);
 int b2_rope_kv_store(void* qkv, const void* bias, const void* inv_freq, const void* pos, void* cache_k, void* cache_v,
                      int Hq, int Hk, int D, int max_len, void* stream);
 int b2_decode_attention(const void* q, const void* cache_k, const void* cache_v, const void* pos, void* out,

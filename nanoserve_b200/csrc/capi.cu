@@ -245,6 +245,16 @@ int ns_swiglu(const void* gate, const void* up, void* out, int T, int I, void* s
   return b2::swiglu_launch(gate, up, out, T, I, static_cast<cudaStream_t>(stream));
 }
 
+int b2_qkv_prefill(void* qkv, const void* bias, const void* inv_freq, void* cache_k, void* cache_v, int T, int Hq, int Hk,
+                   int D, int max_len, void* stream) {
+  return b2::qkv_prefill_launch(qkv, bias, inv_freq, cache_k, cache_v, T, Hq, Hk, D, max_len,
+                                static_cast<cudaStream_t>(stream));
+}
+
+int b2_swiglu_blocks(const void* gu, void* out, int T, int I, int block, void* stream) {
+  return b2::swiglu_blocks_launch(gu, out, T, I, block, static_cast<cudaStream_t>(stream));
+}
+
 int ns_flash_fwd(const void*, const void*, const void*, void*, int, int, int, int, long long, long long,
                  long long, int, int, void*) {
   return b2::kErrNotImplemented;

@@ -119,6 +119,74 @@ __global__ void __launch_bounds__(256) swiglu_kernel(const __nv_bfloat16* __rest
   }
 }
 
+// What stands between a prompt's q|k|v projection and its attention, in one pass over the row: bias (the projection is
+// stored in bf16, then the bias is added in bf16), rotation of q and k (rope_kernel's arithmetic, positions 0 .. T - 1),
+// k and v into the cache [Hk, max_len, D].  q is updated in place; the row's k and v are left as they were.  Bound by
+// memory; as a bias addition, rope_kernel and two strided copies it took 25 us a layer at T = 512 and 36 heads of 128,
+// four passes over the row instead of one.  One thread: eight (i, i + D/2) pairs of one head of one token.
+__global__ void __launch_bounds__(256) qkv_prefill_kernel(__nv_bfloat16* __restrict__ qkv,
+                                                          const __nv_bfloat16* __restrict__ bias,
+                                                          const float* __restrict__ inv_freq,
+                                                          __nv_bfloat16* __restrict__ cache_k,
+                                                          __nv_bfloat16* __restrict__ cache_v, int T, int Hq, int Hk,
+                                                          int D, int max_len) {
+  const int per_head = D / 16, heads = Hq + 2 * Hk;
+  const long long total = (long long)T * heads * per_head;
+  for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
+       idx += (long long)gridDim.x * blockDim.x) {
+    const int c = (int)(idx % per_head) * 8;
+    const long long ht = idx / per_head;
+    const int h = (int)(ht % heads), t = (int)(ht / heads);
+    __nv_bfloat16* src = qkv + ((long long)t * heads + h) * D;
+    float lo[8], hi[8], f[8];
+    load8(src + c, lo);
+    load8(src + D / 2 + c, hi);
+    if (bias != nullptr) {
+      load8(bias + (long long)h * D + c, f);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) lo[e] = __bfloat162float(__float2bfloat16(lo[e] + f[e]));
+      load8(bias + (long long)h * D + D / 2 + c, f);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) hi[e] = __bfloat162float(__float2bfloat16(hi[e] + f[e]));
+    }
+    if (h < Hq + Hk) {
+      const float pos = (float)t;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        float sn, cs;
+        sincosf(pos * inv_freq[c + e], &sn, &cs);
+        const float a = lo[e], b = hi[e];
+        lo[e] = a * cs - b * sn;
+        hi[e] = b * cs + a * sn;
+      }
+    }
+    __nv_bfloat16* dst = h < Hq        ? src
+                         : h < Hq + Hk ? cache_k + ((long long)(h - Hq) * max_len + t) * D
+                                       : cache_v + ((long long)(h - Hq - Hk) * max_len + t) * D;
+    store8(dst + c, lo);
+    store8(dst + D / 2 + c, hi);
+  }
+}
+
+// SwiGLU on the output of a row-interleaved gate|up matrix: `block` gate columns, their `block` up columns, the next
+// `block` gate columns ...  swiglu_kernel's arithmetic without the two strided copies that sort the columns first (61 us
+// a layer for all three at T = 512 and 18944 columns).
+__global__ void __launch_bounds__(256) swiglu_blocks_kernel(const __nv_bfloat16* __restrict__ gu,
+                                                            __nv_bfloat16* __restrict__ out, int I8, int block8,
+                                                            size_t n8) {
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n8; i += (size_t)gridDim.x * blockDim.x) {
+    const size_t t = i / I8;
+    const int c = (int)(i - t * I8), b = c / block8;
+    const __nv_bfloat16* src = gu + (t * 2 * I8 + (size_t)(b * 2 * block8 + (c - b * block8))) * 8;
+    float g[8], u[8];
+    load8(src, g);
+    load8(src + block8 * 8, u);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) g[e] = g[e] / (1.f + __expf(-g[e])) * u[e];
+    store8(out + i * 8, g);
+  }
+}
+
 // The kernels above load and store 16 bytes at a time: a pointer that is not 16-byte aligned (a view into the middle
 // of a row) would fault on the device, so it is refused on the host instead.
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
@@ -151,6 +219,30 @@ int rope_launch(void* q, void* k, const void* inv_freq, int T, int Hq, int Hk, i
                                                      static_cast<__nv_bfloat16*>(k),
                                                      static_cast<const float*>(inv_freq), T, Hq, Hk, D, pos0,
                                                      q_stride, k_stride);
+  return (int)cudaGetLastError();
+}
+
+int qkv_prefill_launch(void* qkv, const void* bias, const void* inv_freq, void* cache_k, void* cache_v, int T, int Hq,
+                       int Hk, int D, int max_len, cudaStream_t s) {
+  if (T < 1 || T > max_len || D < 16 || D % 16 || Hq < 0 || Hk < 1) return kErrBadShape;
+  if (!qkv || !inv_freq || !cache_k || !cache_v) return kErrBadPointer;
+  if (!aligned16(qkv) || !aligned16(bias) || !aligned16(cache_k) || !aligned16(cache_v) ||
+      (reinterpret_cast<uintptr_t>(inv_freq) & 3))
+    return kErrBadPointer;
+  const size_t total = (size_t)T * (Hq + 2 * Hk) * (D / 16);
+  qkv_prefill_kernel<<<blocks_for(total, 256), 256, 0, s>>>(
+      static_cast<__nv_bfloat16*>(qkv), static_cast<const __nv_bfloat16*>(bias), static_cast<const float*>(inv_freq),
+      static_cast<__nv_bfloat16*>(cache_k), static_cast<__nv_bfloat16*>(cache_v), T, Hq, Hk, D, max_len);
+  return (int)cudaGetLastError();
+}
+
+int swiglu_blocks_launch(const void* gu, void* out, int T, int I, int block, cudaStream_t s) {
+  if (T < 1 || I < 1 || block < 8 || block % 8 || I % block) return kErrBadShape;
+  if (!gu || !out) return kErrBadPointer;
+  if (!aligned16(gu) || !aligned16(out)) return kErrBadPointer;
+  const size_t n8 = (size_t)T * I / 8;
+  swiglu_blocks_kernel<<<blocks_for(n8, 256), 256, 0, s>>>(static_cast<const __nv_bfloat16*>(gu),
+                                                           static_cast<__nv_bfloat16*>(out), I / 8, block / 8, n8);
   return (int)cudaGetLastError();
 }
 

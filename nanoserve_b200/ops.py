@@ -65,6 +65,8 @@ SIGNATURES = {
     "b2_w4_gemv_scratch_bytes": ([_i32, _i32, _i32, _i32, _i32], ctypes.c_size_t),
     "b2_w4_gemv_noalloc": ([_vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _vp], _i32),
     "b2_rope_kv_store": ([_vp, _vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _vp], _i32),
+    "b2_qkv_prefill": ([_vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _vp], _i32),
+    "b2_swiglu_blocks": ([_vp, _vp, _i32, _i32, _i32, _vp], _i32),
     "b2_decode_attention": ([_vp, _vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _vp], _i32),
     "b2_greedy_next": ([_vp, _i32, _vp, _i32, _vp, _vp, _vp, _vp, _vp, _vp], _i32),
     "b2_decode_workspace_bytes": ([_i32, _i32], ctypes.c_size_t),
@@ -228,6 +230,27 @@ class Kernels:
         return y
 
     # ---- additions
+    def qkv_prefill(self, qkv, bias, inv_freq, cache_k, cache_v, n_heads, n_kv_heads, head_dim):
+        """qkv [T, (Hq + 2 Hk) D] of a prompt: bias, RoPE at positions 0 .. T - 1 (q in place), k and v into the cache
+        [Hk, max_len, D]."""
+        self._cuda(qkv, bias, inv_freq, cache_k, cache_v)
+        assert qkv.is_contiguous() and cache_k.is_contiguous() and cache_v.is_contiguous()
+        assert qkv.shape[1] == (n_heads + 2 * n_kv_heads) * head_dim and inv_freq.dtype == torch.float32
+        rc = self.lib.b2_qkv_prefill(qkv.data_ptr(), None if bias is None else bias.data_ptr(), inv_freq.data_ptr(),
+                                     cache_k.data_ptr(), cache_v.data_ptr(), qkv.shape[0], n_heads, n_kv_heads, head_dim,
+                                     cache_k.shape[1], self._stream())
+        self._check(rc, "b2_qkv_prefill")
+
+    def swiglu_blocks(self, gu, block):
+        """gu [T, 2 I], blocks of `block` gate columns and their `block` up columns -> silu(gate) * up, [T, I]."""
+        self._cuda(gu)
+        assert gu.is_contiguous() and gu.dtype == torch.bfloat16
+        T, I = gu.shape[0], gu.shape[1] // 2
+        out = torch.empty((T, I), dtype=gu.dtype, device=gu.device)
+        self._check(self.lib.b2_swiglu_blocks(gu.data_ptr(), out.data_ptr(), T, I, block, self._stream()),
+                    "b2_swiglu_blocks")
+        return out
+
     def w4_linear_fused(self, x, Wq, S, group=128, prologue=0, r=None, wn=None, eps=0.0, x_out=None, flags=0,
                         epilogue=0):
         """Decode GEMV with the neighbouring operators folded in: prologue 1 = add + RMSNorm (x + r normalised with

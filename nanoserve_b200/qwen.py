@@ -224,21 +224,14 @@ class Qwen2Runner:
         h = k.rmsnorm(x, None, self.layers[0]["ln_in"], cfg.rms_eps)
         for li, L in enumerate(self.layers):
             qkv = self._gather_parts(self.linear(h, L["qkv"]), [self.nq, self.nkv, self.nkv])
-            qkv = qkv + L["bias"]
-            q, kk, v = qkv[:, :self.nq], qkv[:, self.nq:self.nq + self.nkv], qkv[:, self.nq + self.nkv:]
-            k.rope(q, kk, self.inv_freq, cfg.n_heads, cfg.n_kv_heads, D, 0)
-            self.cache_k[li, :, :T] = kk.reshape(T, cfg.n_kv_heads, D).transpose(0, 1)
-            self.cache_v[li, :, :T] = v.reshape(T, cfg.n_kv_heads, D).transpose(0, 1)
-            qh = q.reshape(T, cfg.n_heads, D).transpose(0, 1)[None]
-            kh = kk.reshape(T, cfg.n_kv_heads, D).transpose(0, 1)[None]
-            vh = v.reshape(T, cfg.n_kv_heads, D).transpose(0, 1)[None]
+            k.qkv_prefill(qkv, L["bias"], self.inv_freq, self.cache_k[li], self.cache_v[li], cfg.n_heads, cfg.n_kv_heads, D)
+            qh = qkv[:, :self.nq].view(T, cfg.n_heads, D).transpose(0, 1)[None]
+            kh, vh = self.cache_k[li, :, :T][None], self.cache_v[li, :, :T][None]
             a = F.scaled_dot_product_attention(qh, kh, vh, is_causal=True, enable_gqa=True)
             a = a[0].transpose(0, 1).reshape(T, self.nq).contiguous()
             h = k.rmsnorm(x, self._gather(self.linear(a, L["o"])), L["ln_post"], cfg.rms_eps)
             gu = self.linear(h, L["gu"])
-            il = self.I // self.world
-            gu = gu.view(T, il // self.gu_block, 2, self.gu_block)  # gate and up row blocks alternate (see __init__)
-            act = self._gather(k.swiglu(gu[:, :, 0].reshape(T, il), gu[:, :, 1].reshape(T, il)))
+            act = self._gather(k.swiglu_blocks(gu, self.gu_block))  # gate and up row blocks alternate (see __init__)
             nxt = self.layers[li + 1]["ln_in"] if li + 1 < cfg.n_layers else self.final_norm
             h = k.rmsnorm(x, self._gather(self.linear(act, L["d"])), nxt, cfg.rms_eps)
         self.pos.fill_(T - 1)  # the pick advances it to T, the position of the first generated token

@@ -52,6 +52,39 @@ def test_rope_and_swiglu(kernels):
         kernels.swiglu(a[:1, :4].contiguous(), b[:1, :4].contiguous())  # T*I % 8 (csrc/nanoserve_ops.cu:39)
 
 
+@pytest.mark.parametrize("T,Hq,Hk,D,with_bias", [(1, 4, 1, 128, True), (7, 3, 2, 64, True), (33, 28, 4, 128, False),
+                                                 (5, 2, 1, 16, True)])
+def test_qkv_prefill_equals_its_parts(kernels, T, Hq, Hk, D, with_bias):
+    """Bias, rotation and cache stores in one kernel: bit for bit what the separate operators give; cache rows behind the
+    prompt stay."""
+    g = torch.Generator(device="cuda").manual_seed(T)
+    W = (Hq + 2 * Hk) * D
+    qkv = torch.randn(T, W, device="cuda", generator=g).to(torch.bfloat16)
+    bias = torch.randn(W, device="cuda", generator=g).to(torch.bfloat16) if with_bias else None
+    inv = 1.0 / (1e6 ** (torch.arange(0, D, 2, device="cuda").float() / D))
+    ck = torch.full((Hk, T + 3, D), 5.0, dtype=torch.bfloat16, device="cuda")
+    cv = ck.clone()
+    ref = qkv + bias if with_bias else qkv.clone()
+    q, k, v = ref[:, :Hq * D], ref[:, Hq * D:(Hq + Hk) * D], ref[:, (Hq + Hk) * D:]
+    kernels.rope(q, k, inv, Hq, Hk, D, 0)
+    kernels.qkv_prefill(qkv, bias, inv, ck, cv, Hq, Hk, D)
+    assert torch.equal(qkv[:, :Hq * D], q)
+    assert torch.equal(ck[:, :T], k.reshape(T, Hk, D).transpose(0, 1)) and bool((ck[:, T:] == 5).all())
+    assert torch.equal(cv[:, :T], v.reshape(T, Hk, D).transpose(0, 1)) and bool((cv[:, T:] == 5).all())
+    with pytest.raises(RuntimeError, match="b2_qkv_prefill failed with code -1"):
+        kernels.qkv_prefill(qkv, bias, inv, ck[:, :T - 1].contiguous(), cv, Hq, Hk, D)  # a cache shorter than the prompt
+
+
+@pytest.mark.parametrize("T,I,block", [(1, 16, 16), (3, 48, 8), (129, 1024, 16), (2, 8, 8)])
+def test_swiglu_blocks_equals_swiglu(kernels, T, I, block):
+    gu = torch.randn(T, 2 * I, device="cuda").to(torch.bfloat16) * 3
+    b = gu.view(T, I // block, 2, block)
+    want = kernels.swiglu(b[:, :, 0].reshape(T, I).contiguous(), b[:, :, 1].reshape(T, I).contiguous())
+    assert torch.equal(kernels.swiglu_blocks(gu, block), want)
+    with pytest.raises(RuntimeError, match="b2_swiglu_blocks failed with code -1"):
+        kernels.swiglu_blocks(gu, 12)
+
+
 def _reference_kernels():
     """The reference's own library (its C-ABI source built unchanged for sm_100a by oracle/Makefile) behind this
     repository's binding class: the live checker for the three element-wise operators."""
