@@ -1,6 +1,7 @@
-// W4A16 GEMM for sm_100a where the tokens are few:  Y[M,N] (bf16) = X[M,K] (bf16) . dequant(Wq, S)^T  for M > 16, the
-// token counts of batched decoding and short prompts.  Same operands and numerics as w4_gemm.cu: each weight is
-// RN_bf16((q - 8) * s), products accumulate in fp32, one rounding at the store.
+// W4A16 GEMM for sm_100a where the tokens are few:  Y[M,N] (bf16) = X[M,K] (bf16) . dequant(Wq, S)^T: the token counts of
+// batched decoding and short prompts (M > 16), and at most 16 tokens where the quantization group is finer than the
+// GEMVs' exact integer arithmetic serves.  Same operands and numerics as w4_gemm.cu: each weight is RN_bf16((q - 8) * s),
+// products accumulate in fp32, one rounding at the store.
 //
 // What bounds it: the packed weights' way from HBM (0.5 bytes per weight), and next to it the conversion of every
 // weight (17 instructions per eight).  w4_gemm.cu gives the tokens the 128-row side of the MMA and writes the converted
@@ -14,6 +15,9 @@
 //     memory in rank order: no scratch in global memory, no counters, the result does not depend on timing;
 //   * launched programmatically: packed weights and scales stream in while the previous kernel finishes; X and Y are
 //     touched only after it has.
+// Measured, weights from HBM, against w4_gemm.cu at 48 tokens: 4608 x 3584 7.9 us (25), 37888 x 3584 22.7 (46), 3584 x
+// 18944 17.8 (51), 8192 x 28672 39.5 (113).  Of the 22.7 us, 11 are the weights' way from HBM; with the conversion taken
+// out (a copy of the raw words) it takes 17.5: a step's chain of waits, then the conversion's issue slots (60 % taken).
 // Warps: 0 packed words (TMA), 1 MMA issue and TMEM, 2 X tiles (TMA), 3 idle, then DW conversion warps, which also do
 // the epilogue.  All rings run on mbarriers with bounded waits; a CTA that gives up records a status, still takes part in
 // the cluster barriers, frees its TMEM and returns.
@@ -114,13 +118,15 @@ __device__ __forceinline__ void dequant_word(uint32_t w, uint32_t s2, uint32_t m
 
 // MB: blocks of 128 weight rows per tile (each X tile is then read by MB MMAs).  DW: conversion warps, in DW / (4 MB)
 // groups that take the K blocks in turn; the converted weights of two K blocks fit in TMEM.  MINB: CTAs per SM.
-// G128: groups of 128 (a scale per row and step), read four at a time.
-template <int MB, int DW, int MINB, bool G128>
+// MODE: 4 or 2: groups of 128 (a scale per row and step), read that many at a time; 64, 32: groups of 64 or 32 and whole
+// steps, a step's two or four scales per read; 0: any group, any K.
+template <int MB, int DW, int MINB, int MODE>
 __global__ void __launch_bounds__(128 + DW * 32, MINB)
     w4_gemm_narrow_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
                           const NarrowParams p) {
   constexpr int kRows = MB * 128, kGroups = DW / (4 * MB), kWSlot = kRows * 128;  // a slot of packed words: K = 256
   static_assert(kGroups == 2, "a slot of packed words holds a step for either group");
+  constexpr bool G128 = MODE == 2 || MODE == 4;
   extern __shared__ unsigned char smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;  // swizzled tiles
   unsigned char* gen = smem_raw + (base - smem_u32(smem_raw));
@@ -243,20 +249,21 @@ __global__ void __launch_bounds__(128 + DW * 32, MINB)
       // Scales, p.sv of them per load (a thread reads along its own row, so every load touches 32 lines), the next load
       // in flight while one is used.  General groups: (g, kin) is the group of the current K position and the position
       // inside it, vi the load that group is in.
-      const int sv = G128 ? 4 : p.sv;
+      const int sv = G128 ? MODE : MODE == 64 ? 2 : MODE == 32 ? 4 : p.sv;
       auto load_sv = [&](int v) {
         uint2 r = make_uint2(0u, 0u);
         const int g = v * sv;
         if (live && g < p.KG) {
-          if (sv == 4) r = __ldg(reinterpret_cast<const uint2*>(s_row + g));
-          else if (sv == 2) r.x = __ldg(reinterpret_cast<const uint32_t*>(s_row + g));
-          else r.x = __bfloat16_as_ushort(__ldg(s_row + g));
+          if (sv == 4) r = __ldcg(reinterpret_cast<const uint2*>(s_row + g));
+          else if (sv == 2) r.x = __ldcg(reinterpret_cast<const uint32_t*>(s_row + g));
+          else r.x = __ldcg(reinterpret_cast<const unsigned short*>(s_row + g));
         }
         return r;
       };
       int k = (kb0 + grp) * kKB;
-      int g = G128 ? kb0 + grp : k / p.G, kin = G128 ? 0 : k - g * p.G, vi = g / sv;
-      uint2 cur = load_sv(vi), nxt = load_sv(vi + 1);
+      int g = MODE ? kb0 + grp : k / p.G, kin = MODE ? 0 : k - g * p.G;  // MODE: g counts steps
+      int vi = G128 || MODE == 0 ? g / sv : g;
+      uint2 cur = load_sv(vi), nxt = load_sv(MODE >= 32 ? vi + 2 : vi + 1);
       auto scale2 = [&]() {  // the pair (s, s) of the current position
         const int e = g - vi * sv;
         return __byte_perm(e & 2 ? cur.y : cur.x, 0, e & 1 ? 0x3232 : 0x1010);
@@ -273,7 +280,7 @@ __global__ void __launch_bounds__(128 + DW * 32, MINB)
           nxt = load_sv(vi + 1);
         }
       };
-      const uint32_t pick = (kb0 + grp) & 1 ? 0x3232 : 0x1010;
+      [[maybe_unused]] const uint32_t pick = (kb0 + grp) & 1 ? 0x3232 : 0x1010;
       const uint32_t src_row = ring_w + row * 128, swz = (uint32_t)row & 7u;
       uint32_t src_off[4];
 #pragma unroll
@@ -284,11 +291,19 @@ __global__ void __launch_bounds__(128 + DW * 32, MINB)
       for (int i = grp; i < nkb; i += 2) {
         uint32_t sc[4];
         if constexpr (G128) {
-          sc[0] = sc[1] = sc[2] = sc[3] = __byte_perm(g & 2 ? cur.y : cur.x, 0, pick);
-          if (g & 2) {
+          sc[0] = sc[1] = sc[2] = sc[3] = __byte_perm(MODE == 4 && (g & 2) ? cur.y : cur.x, 0, pick);
+          if (MODE == 2 || (g & 2)) {
             cur = nxt;
-            nxt = load_sv((g >> 2) + 2);
+            nxt = load_sv(g / MODE + 2);
           }
+          g += 2;
+        } else if constexpr (MODE == 64 || MODE == 32) {
+          sc[0] = __byte_perm(cur.x, 0, 0x1010);
+          sc[1] = MODE == 64 ? sc[0] : __byte_perm(cur.x, 0, 0x3232);
+          sc[2] = __byte_perm(MODE == 64 ? cur.x : cur.y, 0, MODE == 64 ? 0x3232 : 0x1010);
+          sc[3] = MODE == 64 ? sc[2] : __byte_perm(cur.y, 0, 0x3232);
+          cur = nxt;
+          nxt = load_sv(g + 4);
           g += 2;
         } else {
 #pragma unroll
@@ -403,22 +418,37 @@ __global__ void __launch_bounds__(128 + DW * 32, MINB)
 using NarrowKernel = void (*)(const CUtensorMap, const CUtensorMap, const NarrowParams);
 struct NarrowForm {
   NarrowKernel kernel;
-  int rows, warps, per_sm, smem;
+  int variant, rows, warps, per_sm, smem;
 };
 // form 0: 128 weight rows, two CTAs per SM; form 1: 256 rows, one CTA.  All of an SM's (or half an SM's) shared memory
 // is asked for, needed or not: at most 512 columns' worth of CTAs then fit on an SM, whatever mix of these launches
 // overlaps, and no CTA of a cluster waits for tensor memory that a CTA at a cluster barrier holds.
-NarrowForm narrow_form(int form, bool g128) {
-  if (form == 0)
-    return {g128 ? w4_gemm_narrow_kernel<1, 8, 2, true> : w4_gemm_narrow_kernel<1, 8, 2, false>, 128, 8, 2, kSmemHalf};
-  return {g128 ? w4_gemm_narrow_kernel<2, 16, 1, true> : w4_gemm_narrow_kernel<2, 16, 1, false>, 256, 16, 1, kSmemFull};
+// variant: 0 any group, 1 and 2 groups of 128 by two and by four scales, 3 groups of 64, 4 groups of 32
+NarrowForm narrow_form(int form, int variant) {
+  static constexpr NarrowKernel kHalf[5] = {w4_gemm_narrow_kernel<1, 8, 2, 0>, w4_gemm_narrow_kernel<1, 8, 2, 2>,
+                                            w4_gemm_narrow_kernel<1, 8, 2, 4>, w4_gemm_narrow_kernel<1, 8, 2, 64>,
+                                            w4_gemm_narrow_kernel<1, 8, 2, 32>};
+  static constexpr NarrowKernel kFull[5] = {w4_gemm_narrow_kernel<2, 16, 1, 0>, w4_gemm_narrow_kernel<2, 16, 1, 2>,
+                                            w4_gemm_narrow_kernel<2, 16, 1, 4>, w4_gemm_narrow_kernel<2, 16, 1, 64>,
+                                            w4_gemm_narrow_kernel<2, 16, 1, 32>};
+  if (form == 0) return {kHalf[variant], variant, 128, 8, 2, kSmemHalf};
+  return {kFull[variant], variant, 256, 16, 1, kSmemFull};
+}
+int narrow_variant(const void* S, int K, int G) {
+  const uintptr_t sa = reinterpret_cast<uintptr_t>(S);
+  const int kg = K / G;
+  const int sv = kg % 4 == 0 && sa % 8 == 0 ? 4 : kg % 2 == 0 && sa % 4 == 0 ? 2 : 1;
+  if (G == 128 && sv > 1) return sv / 2;
+  if (G == 64 && K % kKB == 0 && sv > 1) return 3;
+  if (G == 32 && K % kKB == 0 && sv == 4) return 4;
+  return 0;
 }
 
-int narrow_attributes(const NarrowForm& f, int form, bool g128, int dev) {
-  static std::atomic<bool> done[64][2][2];
-  if (dev >= 0 && dev < 64 && done[dev][form][g128].load(std::memory_order_acquire)) return 0;
+int narrow_attributes(const NarrowForm& f, int form, int dev) {
+  static std::atomic<bool> done[64][2][5];
+  if (dev >= 0 && dev < 64 && done[dev][form][f.variant].load(std::memory_order_acquire)) return 0;
   const cudaError_t e = cudaFuncSetAttribute(f.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, f.smem);
-  if (e == cudaSuccess && dev >= 0 && dev < 64) done[dev][form][g128].store(true, std::memory_order_release);
+  if (e == cudaSuccess && dev >= 0 && dev < 64) done[dev][form][f.variant].store(true, std::memory_order_release);
   return (int)e;
 }
 
@@ -443,28 +473,31 @@ void narrow_config(const NarrowForm& f, int grid, int ks, bool pdl, cudaLaunchCo
   cfg->numAttrs = na;
 }
 
-// CTAs of a form the device runs at a time in clusters of ks (a cluster stays inside one GPC: eight to a cluster leave
-// some SMs of every GPC out), asked for once per device.
-int narrow_capacity(int form, int ks, int sm_count, int dev) {
-  const NarrowForm f = narrow_form(form, true);
-  const int all = sm_count * f.per_sm;
-  if (ks == 1) return all;
-  static std::atomic<int> known[64][2][9];
+// Clusters of ks one-per-SM CTAs the device runs at a time (a cluster stays inside one GPC, so some SMs of a GPC are left
+// out), asked for once per device.
+int narrow_clusters(int ks, int sm_count, int dev) {
+  if (ks == 1) return sm_count;
+  static std::atomic<int> known[64][9];
   const bool cached = dev >= 0 && dev < 64;
   if (cached)
-    if (const int v = known[dev][form][ks].load(std::memory_order_relaxed)) return v;
+    if (const int v = known[dev][ks].load(std::memory_order_relaxed)) return v;
+  const NarrowForm f = narrow_form(1, 2);
   int clusters = 0;
   cudaLaunchConfig_t cfg{};
   cudaLaunchAttribute attr[2];
   narrow_config(f, ks, ks, false, &cfg, attr);
-  if (narrow_attributes(f, form, true, dev) != 0 ||
-      cudaOccupancyMaxActiveClusters(&clusters, f.kernel, &cfg) != cudaSuccess || clusters < 1) {
+  if (narrow_attributes(f, 1, dev) != 0 || cudaOccupancyMaxActiveClusters(&clusters, f.kernel, &cfg) != cudaSuccess ||
+      clusters < 1) {
     (void)cudaGetLastError();
-    clusters = std::max(1, all / ks * 3 / 4);
+    clusters = std::max(1, sm_count / ks * 7 / 8);
   }
-  const int v = std::min(all, clusters * ks);
-  if (cached) known[dev][form][ks].store(v, std::memory_order_relaxed);
-  return v;
+  if (cached) known[dev][ks].store(clusters, std::memory_order_relaxed);
+  return clusters;
+}
+// CTAs of a form the device runs at a time.  (Half-SM CTAs: twice the full ones; 288 CTAs in clusters of four were
+// measured to take two waves, so the clusters of one do not fill what those of the other leave.)
+int narrow_capacity(int form, int ks, int sm_count, int dev) {
+  return std::min(sm_count, narrow_clusters(ks, sm_count, dev) * ks) * (form == 0 ? 2 : 1);
 }
 
 struct NarrowPlan {
@@ -473,27 +506,30 @@ struct NarrowPlan {
   double us = 0;
 };
 
-// Estimated time of a form and a cluster size: waves of CTAs, each its K blocks at the rate measured with the chip full
-// (one 128-row CTA on an SM, two, one 256-row CTA; the rate falls with the token columns), plus start-up and, when K is
-// cut, the exchange through distributed shared memory.  Fitted to 512 to 8192 x 3584 to 28672 at 17 to 512 tokens; the
-// form it picks was within 6 % of the best form tried on each.
+// Estimated time of a form and a cluster size: start-up, the exchange through distributed shared memory when K is cut,
+// and waves of CTAs that take their K blocks at a rate that falls with the token columns and with the share of the chip
+// at work.  The constants (us) are a least-squares fit to 900 measured launches, 256 to 57344 x 512 to 28672 at 17 to 2300
+// tokens, weights from HBM (residual 13 to 15 %); over those shapes the form it picks takes 1.03 times the best one's
+// time in the geometric mean.
 void narrow_estimate(NarrowPlan* pl, int N, int K, int sm_count, int dev) {
   const int nkb = (K + kKB - 1) / kKB;
   pl->n_tiles = (long)pl->t_tiles * ((N + (pl->form ? 255 : 127)) / (pl->form ? 256 : 128));
   const int cap = narrow_capacity(pl->form, pl->ks, sm_count, dev);
   const long ctas = pl->n_tiles * pl->ks, waves = (ctas + cap - 1) / cap;
   const int blocks = (nkb + pl->ks - 1) / pl->ks;
-  double block;
+  const double nt = pl->nt, busy = std::min(1.0, (double)ctas / waves / (sm_count * (pl->form ? 1 : 2)));
+  const double cut = pl->ks - 1;
   if (pl->form)
-    block = ctas > 100 ? 0.50 + 0.0040 * pl->nt : 0.40 + 0.0032 * pl->nt;
+    pl->us = 1.27 + 0.0303 * nt + (cut > 0 ? 0.07 + 0.0071 * nt : 0.0) + cut * (0.130 + 0.0011 * nt) +
+             (waves - 1) * (4.42 + 0.0127 * nt) + waves * blocks * (0.449 + 0.0022 * nt + busy * (0.312 - 0.0008 * nt));
   else
-    block = ctas > sm_count ? 0.55 + 0.0034 * pl->nt : 0.43 + 0.0022 * pl->nt;
-  pl->us = 3.0 + (pl->ks > 1 ? 1.0 + 0.025 * pl->nt : 0.0) + waves * blocks * block + (waves - 1) * 2.0;
+    pl->us = 1.24 + 0.0291 * nt + (cut > 0 ? 0.41 + 0.0022 * nt : 0.0) + cut * (0.101 + 0.0010 * nt) +
+             (waves - 1) * (1.03 + 0.0163 * nt) + waves * blocks * (0.301 + 0.0017 * nt + busy * (0.509 - 0.0004 * nt));
 }
 
 NarrowPlan narrow_plan(int M, int N, int K, int flags, int sm_count, int dev) {
   NarrowPlan best;
-  const bool forced = flags & kFlagGemmNarrow;
+  const bool forced = flags & (kFlagGemmNarrow | kFlagDecodeNarrow);
   const int want_form = forced ? (flags >> 24) & 3 : 0, want_ks = forced ? (flags >> 20) & 15 : 0;
   const int nkb = (K + kKB - 1) / kKB;
   bool any = false;
@@ -521,8 +557,26 @@ int current_device() {
 
 }  // namespace
 
+// Up to 16 tokens.  Groups that are no multiple of 128 have their weights rounded to bf16 in the GEMV as here, and it
+// takes about 4 + 0.195 w + M K / 1e4 us (w = millions of weights, from HBM; 0.1 w more above eight tokens): G = 64,
+// 37888 x 3584 M = 4 35.0 against 22.7 here, 3584 x 18944 M = 16 64.4 against 18.4, 3584 x 3584 M = 1 7.3 against 6.9;
+// 57344 x 8192 M = 1 stays, 97.6 against 85 and estimated at 100.  Multiples of 128 keep exact weights: the GEMVs' alone.
+bool gemm_narrow_takes_decode(const void* X, const void* Wq, const void* S, const void* Y, int M, int N, int K, int G,
+                              int flags, int sm_count) {
+  if (flags < 0) return true;
+  if (flags != 0 || M < 1 || N < 1 || K < 32 || G < 32 || K % 32 || G % 32 || K % G || G % 128 == 0) return false;
+  if (!X || !Wq || !S || !Y ||
+      ((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(Wq) | reinterpret_cast<uintptr_t>(Y)) & 15) ||
+      (reinterpret_cast<uintptr_t>(S) & 1))
+    return false;
+  const double w = (double)N * K * 1e-6, gemv = 4.0 + 0.195 * w + 1e-4 * M * K + (M > 8 ? 0.1 * w : 0.0);
+  const double slower = narrow_variant(S, K, G) == 0 ? 1.5 : 1.05;  // than the form the estimate was fitted to
+  return slower * narrow_plan(M, N, K, 0, sm_count, current_device()).us < gemv;
+}
+
 // Whether this kernel takes a GEMM that the general kernel would run in about wide_us microseconds.
 bool gemm_narrow_applies(int M, int N, int K, int flags, double wide_us, int sm_count) {
+  if (M <= 16) return true;  // (decided by gemm_narrow_takes_decode)
   if (flags & (kFlagGemmNoPairs | kFlagGemmWholeTiles | kFlagGemmWide)) return false;  // the other kernel's switches
   if (flags & kFlagGemmNarrow) return true;
   return narrow_plan(M, N, K, flags, sm_count, current_device()).us < wide_us;
@@ -546,8 +600,7 @@ int gemm_narrow_launch(const void* X, const void* Wq, const void* S, void* Y, in
   p.ks = pl.ks;
   const uintptr_t sa = reinterpret_cast<uintptr_t>(S);
   p.sv = p.KG % 4 == 0 && sa % 8 == 0 ? 4 : p.KG % 2 == 0 && sa % 4 == 0 ? 2 : 1;
-  const bool g128 = G == 128 && p.sv == 4;
-  const NarrowForm f = narrow_form(pl.form, g128);
+  const NarrowForm f = narrow_form(pl.form, narrow_variant(S, K, G));
   const int slot_w = f.rows * 128, slot_x = p.nt * 256, room = f.smem - kHeaderBytes - 1024;
   const int x_bytes = pl.form ? 128 << 10 : p.nt > 64 ? 72 << 10 : 48 << 10;  // the rest holds packed words
   p.sx = std::max(2, std::min(6, x_bytes / slot_x));
@@ -559,7 +612,7 @@ int gemm_narrow_launch(const void* X, const void* Wq, const void* S, void* Y, in
       !make_tensor_map_2d(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, Wq, (uint64_t)N, (uint64_t)K / 8, f.rows, 2 * kKB / 8,
                           CU_TENSOR_MAP_SWIZZLE_128B))
     return kErrDevice;
-  if (const int rc = narrow_attributes(f, pl.form, g128, dev)) return rc;
+  if (const int rc = narrow_attributes(f, pl.form, dev)) return rc;
   cudaLaunchConfig_t cfg{};
   cudaLaunchAttribute attr[2];
   narrow_config(f, (int)(pl.n_tiles * pl.ks), pl.ks, (flags & kFlagNoPdl) == 0, &cfg, attr);

@@ -36,6 +36,7 @@ FLAG_GEMM_NO_PAIRS = 1 << 29  # prefill GEMM: one CTA per tile unpacks the whole
 FLAG_GEMM_WHOLE_TILES = 1 << 30  # prefill GEMM: every CTA takes whole output tiles (no fp32 part-tiles)
 FLAG_GEMM_NARROW = 1 << 28  # prefill GEMM: the few-token kernel for every M > 16 (narrow_flags picks its split and tile)
 FLAG_GEMM_WIDE = 1 << 27  # prefill GEMM: never the few-token kernel
+FLAG_DECODE_NARROW = -(1 << 31)  # M <= 16: the few-token GEMM instead of a GEMV (with narrow_flags)
 FLAG_NO_MID_KERNEL = 262144  # decode GEMV: never the many-token kernel (2 <= M <= 16 on plain launches)
 FLAG_MID_KERNEL = 131072 | 524288  # decode GEMV (both kernel flags): the many-token kernel for every shape it can serve
 FLAG_STREAM_KERNEL = 524288  # decode GEMV: the streaming kernel for every M <= 16 it can serve (default: M <= 2)

@@ -5,7 +5,7 @@ import pytest
 import torch
 
 import oracle
-from nanoserve_b200.ops import FLAG_GEMM_WIDE, narrow_flags
+from nanoserve_b200.ops import FLAG_DECODE_NARROW, FLAG_GEMM_WIDE, narrow_flags
 from tests.test_w4_gemm_gpu import rounded_weight_reference
 from tests.util import bits_to_torch, check_bf16_output, torch_to_bits, u32_to_torch
 
@@ -46,3 +46,31 @@ def test_rule_agrees_with_the_wide_kernel(kernels, M):
         b = oracle.bf16_bits_to_f32(run(kernels, X, Wq, S, G, FLAG_GEMM_WIDE))
         assert np.abs(a - b).max() <= 2.0**-7 * np.abs(b).max()
         assert (a != b).mean() < 0.05  # sums that differ in the last fp32 bits round differently once in a while
+
+
+@pytest.mark.parametrize("tile", [1, 2])
+@pytest.mark.parametrize("split", [0, 1, 3, 8])
+def test_decode_tokens(kernels, tile, split):
+    """At most 16 tokens: row tiles cut off, one K block, odd and even numbers of blocks, every way to read scales."""
+    for M, N, K, G in [(1, 300, 1024, 64), (2, 129, 256, 32), (16, 512, 3584, 64), (13, 260, 2304, 32), (7, 77, 768, 128),
+                       (5, 256, 1088, 64), (16, 130, 640, 32), (9, 131, 352, 32), (3, 64, 192, 96)]:
+        X, Wq, S = oracle.synth_inputs(M, N, K, G, seed=M + K)
+        y = run(kernels, X, Wq, S, G, FLAG_DECODE_NARROW | narrow_flags(split, tile))
+        check_bf16_output(y, rounded_weight_reference(X, Wq, S, G), 3e-5)
+
+
+def test_decode_of_fine_groups_takes_any_alignment(kernels):
+    """Fine groups at decode token counts run the few-token GEMM where pointers are 16-byte aligned, and the GEMV where they
+    are not: the results agree to a rounding of the output and of the sums."""
+    M, N, K, G = 4, 1000, 2048, 64
+    X, Wq, S = oracle.synth_inputs(M, N, K, G, seed=8)
+    x, wq, s = bits_to_torch(X), u32_to_torch(Wq), bits_to_torch(S)
+    want = oracle.bf16_bits_to_f32(torch_to_bits(kernels.w4_linear(x, wq, s, G)))
+    room = torch.empty(M * N + 8, dtype=torch.bfloat16, device="cuda")
+    out = room[1:1 + M * N].view(M, N)
+    s_off = torch.empty(S.size + 1, dtype=torch.bfloat16, device="cuda")[1:].view(*S.shape).copy_(s)
+    kernels.w4_linear(x, wq, s_off, G, out=out)
+    torch.cuda.synchronize()
+    assert kernels.device_status() == 0
+    got = oracle.bf16_bits_to_f32(torch_to_bits(out))
+    assert np.abs(got - want).max() <= 2.0**-7 * np.abs(want).max()
