@@ -83,6 +83,8 @@ int linear_dispatch(const void* X, const void* Wq, const void* S, void* Y, int M
   DeviceState* st = device_state(&rc);
   if (!st) return rc;
   const auto s = static_cast<cudaStream_t>(stream);
+  if (M <= 16 && b2::gemv_tc_applies(X, Wq, S, Y, M, N, K, G, flags, st->sm_count))
+    return b2::gemv_tc_launch(X, Wq, S, Y, M, N, K, st->ws, flags, st->sm_count, s);
   if (M <= 16 && !b2::gemm_narrow_takes_decode(X, Wq, S, Y, M, N, K, G, flags, st->sm_count))
     return b2::gemv_launch(X, Wq, S, Y, M, N, K, G, st->ws, flags, st->sm_count, s);
   return b2::gemm_launch(X, Wq, S, Y, M, N, K, G, st->ws, flags, st->sm_count, s);

@@ -65,7 +65,8 @@ enum : int {
   kFlagGemmNarrow = 1 << 28,      // GEMM: the few-token kernel (w4_gemm_narrow.cu) for every M > 16; bits 20-23: CTAs per
                                   // cluster along K, bits 24-25: tile (1: 128 rows, 2: 256), 0 = the rule decides
   kFlagGemmWide = 1 << 27,        // GEMM: never that kernel
-  kFlagDecodeNarrow = (int)0x80000000u,  // M <= 16: that kernel instead of a GEMV (bits 20-25 as for kFlagGemmNarrow)
+  kFlagDecodeNarrow = (int)0x80000000u,  // M <= 16: the tcgen05 GEMV (w4_gemv_tc.cu) where its shapes allow, else that
+                                         // kernel, instead of another GEMV (bits 20-25 as for kFlagGemmNarrow)
   kFlagNoPdl = 8,          // GEMV: do NOT launch with programmatic stream serialization (by default the kernel may
                            // begin -- weight prefetch only -- while the previous kernel of the stream still runs)
 };
@@ -127,6 +128,10 @@ bool gemm_narrow_takes_decode(const void* X, const void* Wq, const void* S, cons
 bool gemm_narrow_applies(int M, int N, int K, int flags, double wide_us, int sm_count);
 int gemm_narrow_launch(const void* X, const void* Wq, const void* S, void* Y, int M, int N, int K, int G,
                        const Workspace& ws, int flags, int sm_count, cudaStream_t stream);
+bool gemv_tc_applies(const void* X, const void* Wq, const void* S, const void* Y, int M, int N, int K, int G, int flags,
+                     int sm_count);
+int gemv_tc_launch(const void* X, const void* Wq, const void* S, void* Y, int M, int N, int K, const Workspace& ws,
+                   int flags, int sm_count, cudaStream_t stream);
 int quantize_launch(const void* W, void* Wq, void* S, int N, int K, int G, cudaStream_t stream);
 
 int decode_attention_fused_launch(const void* qkv, const void* bias, const void* inv_freq, const void* pos,
