@@ -76,7 +76,7 @@ __device__ __forceinline__ uint32_t abs_max_bits(const uint4& v) {
 //
 // 18944 x 3584 at G = 128: 34.8 us (4.9 TB/s of bf16 in, words and scales out), where a division per weight with half
 // of the lanes idle took 162 us (1.05 TB/s).
-constexpr int kUnroll = 4;
+constexpr int kUnroll = 4;  // 1, 2, 4, 8 loads in flight per lane: 45.1, 36.4, 35.0, 37.2 us
 template <int LPG>
 __global__ void __launch_bounds__(256) w4_quantize_fast_kernel(const uint4* __restrict__ W, uint32_t* __restrict__ Wq,
                                                                __nv_bfloat16* __restrict__ S, size_t words) {
