@@ -103,10 +103,12 @@ int ns_flash_fwd(const void* q, const void* k, const void* v, void* o, int N, in
 #define B2_FLAG_GEMM_WHOLE_TILES 1073741824 /* prefill GEMM (M > 16): every CTA takes whole output tiles; by default the CTAs
                                            take equal shares of the (tile, K block) pairs and tiles that several CTAs cover
                                            are finished from fp32 part-tiles in the scratch */
-#define B2_FLAG_NO_PDL 8          /* GEMV: plain launch.  By default the GEMV is launched with programmatic stream
-                                     serialization: it may begin (weight prefetch only) while the previous kernel of
-                                     the stream is still running, and touches X, Y and scratch only after that kernel
-                                     has completed */
+#define B2_FLAG_NO_PDL 8          /* plain launch.  By default every kernel but the prefill GEMM is launched with programmatic
+                                     stream serialization: it may begin while the previous kernel of the stream is still
+                                     running, and touches X, Y and scratch only after that kernel has completed.  At up to
+                                     16 tokens Wq and S may be read earlier (the streaming and the ring kernel do), so
+                                     they must not be written by a kernel that lets its dependents start before it is
+                                     done; above 16 tokens Wq and S are read after it has completed too */
 
 /*
  * Sets up the calling thread's current device: queries the SM count and allocates the per-device scratch

@@ -116,6 +116,12 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst_smem, const void* tmap,
       "l"(tmap), "r"(bar), "r"(x), "r"(y)
       : "memory");
 }
+// Brings a tile (or the 128-byte line of an address) into L2 only.  Nothing is read as far as the program can tell, so a
+// kernel that still runs may be writing it: what is loaded later is what L2 then holds.
+__device__ __forceinline__ void tma_prefetch_2d(const void* tmap, int x, int y) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global [%0, {%1, %2}];" ::"l"(tmap), "r"(x), "r"(y) : "memory");
+}
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p) : "memory"); }
 // Asynchronous BYTES-byte copy (4, 8 or 16) global -> shared by the calling thread (src_bytes < BYTES: the rest is
 // zero-filled; 0 reads nothing).  Both addresses BYTES-aligned.
 template <int BYTES>

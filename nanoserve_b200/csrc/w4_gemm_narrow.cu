@@ -13,8 +13,10 @@
 //     the MMA takes its A operand from there.  Shared memory carries the packed words once and the X tile;
 //   * K is cut over the CTAs of a CLUSTER (up to eight), which add their fp32 accumulators up through distributed shared
 //     memory in rank order: no scratch in global memory, no counters, the result does not depend on timing;
-//   * launched programmatically: packed weights and scales stream in while the previous kernel finishes; X and Y are
-//     touched only after it has.
+//   * launched programmatically: while the previous kernel finishes, the first packed words and scales are brought into
+//     L2.  All reads and writes come after it has, so it may be the kernel that writes the weights.  (Sixteen launches of
+//     a decoder stack at 48 tokens, us: ring filled before the wait 233, nothing 248, the whole ring into L2 251, its first
+//     slot 243.)
 // Measured, weights from HBM, against w4_gemm.cu at 48 tokens: 4608 x 3584 7.9 us (25), 37888 x 3584 22.7 (46), 3584 x
 // 18944 17.8 (51), 8192 x 28672 39.5 (113).  Of the 22.7 us, 11 are the weights' way from HBM; with the conversion taken
 // out (a copy of the raw words) it takes 17.5: a step's chain of waits, then the conversion's issue slots (60 % taken).
@@ -136,6 +138,8 @@ __global__ void __launch_bounds__(128 + DW * 32, MINB)
   if (!poisoned) {
     if (warp == 0) {
       if (lane == 0) {
+        tma_prefetch_2d(&tmap_w, kb0 * (kKB / 8), n0);
+        pdl_wait_prior_grid();  // it may be the kernel that writes the weights
         int s = 0;
         uint32_t ph = 1;
         for (int i = 0; i < nkb; i += 2) {  // (128-byte rows: the copy engine's rate counts rows, not bytes)
@@ -222,6 +226,8 @@ __global__ void __launch_bounds__(128 + DW * 32, MINB)
       int k = (kb0 + grp) * kKB;
       int g = MODE ? kb0 + grp : k / p.G, kin = MODE ? 0 : k - g * p.G;  // MODE: g counts steps
       int vi = G128 || MODE == 0 ? g / sv : g;
+      if (const int first = MODE >= 32 ? g * sv : g; live && first < p.KG) prefetch_l2(s_row + first);
+      pdl_wait_prior_grid();
       uint2 cur = load_sv(vi), nxt = load_sv(MODE >= 32 ? vi + 2 : vi + 1);
       auto scale2 = [&]() {  // the pair (s, s) of the current position
         const int e = g - vi * sv;
@@ -307,7 +313,6 @@ __global__ void __launch_bounds__(128 + DW * 32, MINB)
       mbar_wait(bar_acc, 0, abort_flag);
       __syncwarp();
       tc_fence_after_sync();
-      pdl_wait_prior_grid();  // Y may still be read by the kernel in front
 
       // ---- the accumulator columns (tokens) of the warp's 32 rows; two groups of warps take alternate 16 columns
       const int rt = min(p.nt, p.M - m0);  // tokens of the tile

@@ -120,6 +120,11 @@ __global__ void __launch_bounds__(128 + DW * 32, MINB)
   if (!poisoned) {
     if (warp == 0) {
       if (lane == 0) {
+        // The kernel in front may be the one that writes the weights: until it has finished they are only brought into
+        // L2 (two slots; sixteen launches of a decoder stack at 13 tokens, us: 226, one slot 227, the whole ring 229,
+        // nothing 231, the ring filled before the wait 224).
+        for (int i = 0; i < nkb && i < 4; i += 2) tma_prefetch_2d(&tmap_w, (kb0 + i) * (kStepK / 8), n0);
+        pdl_wait_prior_grid();
         int s = 0;
         uint32_t ph = 1;
         for (int i = 0; i < nkb; i += 2) {
@@ -172,13 +177,14 @@ __global__ void __launch_bounds__(128 + DW * 32, MINB)
         return r;
       };
       int g = kb0 + grp;
+      if (live && g < p.KG) prefetch_l2(s_row + g);
+      pdl_wait_prior_grid();
       uint2 cur = load_sv(g / SV), nxt = load_sv(g / SV + 1);
       const uint32_t pick = g & 1 ? 0x7632 : 0x5410;  // the odd or the even scale of a pair, as the high half of a float
 
       // ---- X: 16 consecutive k of a token per item, the eight items of a chunk in eight consecutive lanes; the largest
       // magnitude of a (token, chunk) is scaled to below 2^15, its values are rounded to 16-bit integers (the low mantissa
       // bits of x * 2^.. + 1.5 * 2^23) and split into bytes, in the order the nibble masks produce.
-      pdl_wait_prior_grid();
       {
         constexpr int UN = 4;
         const int per_tok = nkb * 8, items = kTokens * per_tok;

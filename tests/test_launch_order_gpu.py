@@ -1,0 +1,69 @@
+"""GPU tests of the order of launches on one stream: kernels of this library that are launched programmatically (they may
+start while the kernel in front still runs) behind kernels whose outputs they read."""
+import pytest
+import torch
+
+from nanoserve_b200.ops import FLAG_DECODE_NARROW, FLAG_GEMM_NARROW, narrow_flags
+
+pytestmark = pytest.mark.gpu
+
+
+def rand_w4(N, K, G, gen):
+    Wq = torch.randint(-2**31, 2**31 - 1, (N, K // 8), dtype=torch.int32, device="cuda", generator=gen)
+    S = (0.005 + (torch.randn(N, K // G, device="cuda", generator=gen) * 0.01).abs()).to(torch.bfloat16)
+    return Wq, S
+
+
+def rand_x(M, K, gen):
+    return torch.randn(M, K, device="cuda", generator=gen).to(torch.bfloat16)
+
+
+@pytest.mark.parametrize("M,G,flags", [(13, 128, FLAG_DECODE_NARROW), (4, 64, FLAG_DECODE_NARROW), (48, 128, FLAG_GEMM_NARROW),
+                                       (48, 32, FLAG_GEMM_NARROW), (300, 128, 0)])
+def test_weights_written_by_the_kernel_in_front(kernels, M, G, flags):
+    """The kernel in front lets its dependents start at once and stores at its end: a linear whose output is the next one's
+    scales, or its packed words.  The result is that of the same launches with a synchronisation in between."""
+    gen = torch.Generator(device="cuda").manual_seed(M)
+    N, K = 1024, 1024
+    x, (Wq, S) = rand_x(M, K, gen), rand_w4(N, K, G, gen)
+    front_x, (front_q, front_s) = rand_x(64, 18944, gen), rand_w4(N * (K // G) // 64, 18944, 128, gen)
+    words_x, (words_q, words_s) = rand_x(64, 8192, gen), rand_w4(N * K // 4 // 64, 8192, 128, gen)
+    scales, words = torch.empty_like(S), torch.empty_like(Wq)
+
+    def chain(sync):
+        sync()
+        kernels.w4_linear(front_x, front_q, front_s, 128, flags=narrow_flags(split=1), out=scales.view(64, -1))
+        sync()
+        a = kernels.w4_linear(x, Wq, scales, G, flags=flags)
+        sync()
+        kernels.w4_linear(words_x, words_q, words_s, 128, flags=narrow_flags(split=1),
+                          out=words.view(torch.bfloat16).view(64, -1))
+        sync()
+        b = kernels.w4_linear(x, words, S, G, flags=flags)
+        sync()
+        return a, b
+
+    want = chain(torch.cuda.synchronize)
+    assert all(bool(w.isfinite().all()) and float(w.float().abs().max()) > 0 for w in want)
+    for _ in range(20):
+        scales.zero_()
+        words.zero_()
+        got = chain(lambda: None)
+        assert all(torch.equal(g, w) for g, w in zip(got, want))
+    assert kernels.device_status() == 0
+
+
+@pytest.mark.parametrize("M", [13, 48])
+def test_linear_behind_its_quantizer(kernels, M):
+    gen = torch.Generator(device="cuda").manual_seed(M)
+    W, x = rand_x(5000, 3584, gen), rand_x(M, 3584, gen)
+    Wq, S = kernels.w4_quantize(W)
+    torch.cuda.synchronize()
+    want = kernels.w4_linear(x, Wq, S)
+    for _ in range(10):
+        Wq.zero_()
+        S.zero_()
+        torch.cuda.synchronize()
+        rc = kernels.lib.ns_w4_quantize(W.data_ptr(), Wq.data_ptr(), S.data_ptr(), 5000, 3584, 128, kernels._stream())
+        assert rc == 0 and torch.equal(kernels.w4_linear(x, Wq, S), want)
+    assert kernels.device_status() == 0
