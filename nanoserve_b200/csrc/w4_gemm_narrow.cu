@@ -173,6 +173,7 @@ __global__ void __launch_bounds__(128 + DW * 32, MINB)
       const uint64_t desc0 = umma_desc_k128(ring_x);
       int xs = 0;
       uint32_t xph = 0;
+      pdl_wait_prior_grid();  // the kernel in front may run longer than a bounded wait for X
       for (int i = 0; i < nkb; ++i) {
         const int buf = i & 1;
         mbar_wait(bar_x_full + 8 * xs, xph, abort_flag);

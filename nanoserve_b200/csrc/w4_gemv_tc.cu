@@ -138,6 +138,7 @@ __global__ void __launch_bounds__(128 + DW * 32, MINB)
     } else if (warp == 1) {
       constexpr uint32_t id_lo = umma_idesc_s8(0, 128, kTokens), id_hi = umma_idesc_s8(1, 128, kTokens);
       const uint64_t desc0 = umma_desc_k128(xs);
+      pdl_wait_prior_grid();  // the kernel in front may run longer than a bounded wait for X
       mbar_wait(bar_x, 0, abort_flag);
       for (int i = 0; i < nkb; ++i) {
         const int buf = i % kBufs;

@@ -67,3 +67,33 @@ def test_linear_behind_its_quantizer(kernels, M):
         rc = kernels.lib.ns_w4_quantize(W.data_ptr(), Wq.data_ptr(), S.data_ptr(), 5000, 3584, 128, kernels._stream())
         assert rc == 0 and torch.equal(kernels.w4_linear(x, Wq, S), want)
     assert kernels.device_status() == 0
+
+
+@pytest.fixture(scope="module")
+def long_launch(kernels):
+    """A launch that lets its dependents start at once and then runs longer than any bounded wait of the library (10^9
+    cycles, 0.51 s at 1.965 GHz): one CTA walks a K of 2^28."""
+    K, G = 2**28, 64
+    x = torch.zeros(1, K, dtype=torch.bfloat16, device="cuda")
+    Wq = torch.zeros(1, K // 8, dtype=torch.int32, device="cuda")
+    S = torch.ones(1, K // G, dtype=torch.bfloat16, device="cuda")
+    go = lambda: kernels.w4_linear(x, Wq, S, G, flags=FLAG_DECODE_NARROW | narrow_flags(split=1, tile=1))
+    go()
+    start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    start.record()
+    y = go()
+    end.record()
+    end.synchronize()
+    assert kernels.device_status() == 0 and float(y) == 0 and start.elapsed_time(end) > 600
+    return go
+
+
+@pytest.mark.parametrize("M,G,flags", [(13, 128, FLAG_DECODE_NARROW), (4, 64, FLAG_DECODE_NARROW), (48, 128, FLAG_GEMM_NARROW)])
+def test_wait_for_a_long_launch_is_no_time_out(kernels, long_launch, M, G, flags):
+    gen = torch.Generator(device="cuda").manual_seed(M)
+    x, (Wq, S) = rand_x(M, 1024, gen), rand_w4(1024, 1024, G, gen)
+    want = kernels.w4_linear(x, Wq, S, G, flags=flags)
+    torch.cuda.synchronize()
+    long_launch()
+    got = kernels.w4_linear(x, Wq, S, G, flags=flags)
+    assert kernels.device_status() == 0 and torch.equal(got, want)
