@@ -237,17 +237,24 @@ class Kernels:
         """qkv [T, (Hq + 2 Hk) D] of a prompt: bias, RoPE at positions 0 .. T - 1 (q in place), k and v into the cache
         [Hk, max_len, D]."""
         self._cuda(qkv, bias, inv_freq, cache_k, cache_v)
-        assert qkv.is_contiguous() and cache_k.is_contiguous() and cache_v.is_contiguous()
-        assert qkv.shape[1] == (n_heads + 2 * n_kv_heads) * head_dim and inv_freq.dtype == torch.float32
+        width = (n_heads + 2 * n_kv_heads) * head_dim
+        for t in (qkv, bias, inv_freq, cache_k, cache_v):
+            assert t is None or t.is_contiguous() and t.dtype == (torch.float32 if t is inv_freq else torch.bfloat16)
+        assert qkv.dim() == 2 and qkv.shape[1] == width and (bias is None or bias.numel() == width)
+        assert inv_freq.numel() == head_dim // 2
+        # the kernel writes both caches by one layout (a cache shorter than the prompt is refused by the library, with -1)
+        assert cache_k.dim() == cache_v.dim() == 3 and cache_k.shape[::2] == cache_v.shape[::2] == (n_kv_heads, head_dim)
+        max_len = min(cache_k.shape[1], cache_v.shape[1])
+        assert cache_k.shape == cache_v.shape or max_len < qkv.shape[0]
         rc = self.lib.b2_qkv_prefill(qkv.data_ptr(), None if bias is None else bias.data_ptr(), inv_freq.data_ptr(),
                                      cache_k.data_ptr(), cache_v.data_ptr(), qkv.shape[0], n_heads, n_kv_heads, head_dim,
-                                     cache_k.shape[1], self._stream())
+                                     max_len, self._stream())
         self._check(rc, "b2_qkv_prefill")
 
     def swiglu_blocks(self, gu, block):
         """gu [T, 2 I], blocks of `block` gate columns and their `block` up columns -> silu(gate) * up, [T, I]."""
         self._cuda(gu)
-        assert gu.is_contiguous() and gu.dtype == torch.bfloat16
+        assert gu.is_contiguous() and gu.dtype == torch.bfloat16 and gu.dim() == 2 and gu.shape[1] % 2 == 0
         T, I = gu.shape[0], gu.shape[1] // 2
         out = torch.empty((T, I), dtype=gu.dtype, device=gu.device)
         self._check(self.lib.b2_swiglu_blocks(gu.data_ptr(), out.data_ptr(), T, I, block, self._stream()),

@@ -75,6 +75,26 @@ def test_qkv_prefill_equals_its_parts(kernels, T, Hq, Hk, D, with_bias):
         kernels.qkv_prefill(qkv, bias, inv, ck[:, :T - 1].contiguous(), cv, Hq, Hk, D)  # a cache shorter than the prompt
 
 
+def test_qkv_prefill_refuses_what_it_would_misread(kernels):
+    """Everything the kernel takes on trust is checked on the host: it writes the caches by the layout of one of them."""
+    T, Hq, Hk, D, L = 8, 4, 2, 64, 16
+    W = (Hq + 2 * Hk) * D
+    z = lambda *shape, dtype=torch.bfloat16: torch.zeros(*shape, dtype=dtype, device="cuda")
+    good = dict(qkv=z(T, W), bias=z(W), inv_freq=z(D // 2, dtype=torch.float32), cache_k=z(Hk, L, D), cache_v=z(Hk, L, D))
+    kernels.qkv_prefill(**good, n_heads=Hq, n_kv_heads=Hk, head_dim=D)
+    bad = [dict(cache_v=z(Hk, L - 4, D)), dict(cache_v=z(Hk - 1, L, D)), dict(cache_k=z(Hk - 1, L, D), cache_v=z(Hk - 1, L, D)),
+           dict(cache_k=z(Hk, L, D // 2), cache_v=z(Hk, L, D // 2)), dict(cache_k=z(Hk, L, D, dtype=torch.float32)),
+           dict(cache_v=z(Hk, L, D, dtype=torch.float16)), dict(qkv=z(T, W, dtype=torch.float32)),
+           dict(qkv=z(T, W, dtype=torch.float16)), dict(bias=z(W - D)), dict(bias=z(W, dtype=torch.float32)),
+           dict(bias=z(2 * W)[::2]), dict(inv_freq=z(D // 4, dtype=torch.float32)), dict(inv_freq=z(D // 2)),
+           dict(inv_freq=z(D, dtype=torch.float32)[::2]), dict(cache_v=z(Hk, D, L).transpose(1, 2)), dict(qkv=z(T * W))]
+    for change in bad:
+        with pytest.raises(AssertionError):
+            kernels.qkv_prefill(**{**good, **change}, n_heads=Hq, n_kv_heads=Hk, head_dim=D)
+    with pytest.raises(AssertionError):
+        kernels.swiglu_blocks(z(2, 33), 8)
+
+
 @pytest.mark.parametrize("T,I,block", [(1, 16, 16), (3, 48, 8), (129, 1024, 16), (2, 8, 8)])
 def test_swiglu_blocks_equals_swiglu(kernels, T, I, block):
     gu = torch.randn(T, 2 * I, device="cuda").to(torch.bfloat16) * 3
