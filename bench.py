@@ -807,7 +807,9 @@ def main():
         # which kernel and launch shape the library picks for each launch of the pass (this rank's shard)
         from nanoserve_b200.tp import ShardedLayer as _SL
         groups = [(n, (n,)) for n in ORDER] if seven else list(_SL.FUSED)
-        plans = {f: k.gemv_describe(M, sum(shapes[n][0] for n in names) // world, shapes[names[0]][1], G, args.flags)
+        from nanoserve_b200.ops import FLAG_NO_MID_KERNEL as _tp_only  # launches that store to peers: two kernels serve them
+        plans = {f: k.gemv_describe(M, sum(shapes[n][0] for n in names) // world, shapes[names[0]][1], G,
+                                    args.flags | (_tp_only if fused_gather else 0))
                  for f, names in groups}
         line = {
             "metric": metric if M == 1 else metric.replace("M=1", f"M={M}"), "value": nbytes * args.steps / t_dev / 1e9,

@@ -162,7 +162,7 @@ int b2_w4_linear_fused(const void* X, const void* Wq, const void* S, void* Y, in
 int b2_device_status(void);
 int b2_clear_status(void);
 
-/* Scratch bytes the GEMV would use for this shape on the current device (0 = no split-K). */
+/* Scratch bytes b2_w4_linear would use for up to 16 tokens of this shape on the current device (0 = none). */
 size_t b2_w4_gemv_scratch_bytes(int M, int N, int K, int G, int flags);
 
 /*
@@ -291,10 +291,11 @@ int b2_w4_linear_tp(const void* X, const void* Wq, const void* S, int M, int N, 
 /* The consumer side of a descriptor as a small kernel of its own (announce, wait, and with advance_epoch != 0 add one
  * to *epoch afterwards): behind the last producer of a step, or in front of a consumer that is not a GEMV. */
 int b2_tp_wait_desc(const b2_tp_desc* tp, int advance_epoch, void* stream);
-/* CTAs the decode GEMV launches for this shape on the current device (0: not served by the GEMV). */
+/* CTAs the decode GEMV launches for this shape as a fused or tensor-parallel call on the current device (0: not served). */
 size_t b2_w4_gemv_grid(int M, int N, int K, int G, int flags);
-/* One line of text into buf: which kernel and launch shape a decode GEMV of this shape gets (benchmark records).  Plain
- * calls that ns_w4_linear hands to the tcgen05 kernels instead (9 to 16 tokens, groups finer than 128) are not described. */
+/* One line of text into buf: which kernel and launch shape b2_w4_linear runs for this shape, any M, with 16-byte aligned
+ * operands (benchmark records).  Fused and tensor-parallel calls run the streaming or the ring kernel only: ask with
+ * B2_FLAG_NO_MID_KERNEL. */
 int b2_w4_gemv_describe(int M, int N, int K, int G, int flags, char* buf, int buflen);
 int b2_rope_kv_store_tp(void* qkv, const void* bias, const void* inv_freq, const void* pos, void* cache_k,
                         void* cache_v, int Hq, int Hk, int D, int max_len, const void* wait_sig, const void* epoch,

@@ -76,6 +76,15 @@ int* device_status_word(int* rc) {
 
 namespace {
 
+// Which launcher takes a plain call.  (Pointers: null = "assume aligned", for the queries that have no operands.)
+enum Route { kRouteGemv, kRouteGemvTc, kRouteGemm };
+Route plain_route(const DeviceState& st, const void* X, const void* Wq, const void* S, const void* Y, int M, int N, int K,
+                  int G, int flags) {
+  if (M > 16) return kRouteGemm;
+  if (b2::gemv_tc_applies(X, Wq, S, Y, M, N, K, G, flags, st.sm_count)) return kRouteGemvTc;
+  return b2::gemm_narrow_takes_decode(X, Wq, S, Y, M, N, K, G, flags, st.sm_count) ? kRouteGemm : kRouteGemv;
+}
+
 int linear_dispatch(const void* X, const void* Wq, const void* S, void* Y, int M, int N, int K, int G,
                     int flags, void* stream) {
   if (M < 1) return b2::kErrUnsupportedM;
@@ -83,10 +92,11 @@ int linear_dispatch(const void* X, const void* Wq, const void* S, void* Y, int M
   DeviceState* st = device_state(&rc);
   if (!st) return rc;
   const auto s = static_cast<cudaStream_t>(stream);
-  if (M <= 16 && b2::gemv_tc_applies(X, Wq, S, Y, M, N, K, G, flags, st->sm_count))
-    return b2::gemv_tc_launch(X, Wq, S, Y, M, N, K, st->ws, flags, st->sm_count, s);
-  if (M <= 16 && !b2::gemm_narrow_takes_decode(X, Wq, S, Y, M, N, K, G, flags, st->sm_count))
-    return b2::gemv_launch(X, Wq, S, Y, M, N, K, G, st->ws, flags, st->sm_count, s);
+  // (a null operand is answered by the checks of the GEMV and the GEMM)
+  const bool operands = X && Wq && S && Y;
+  const Route route = operands || M > 16 ? plain_route(*st, X, Wq, S, Y, M, N, K, G, flags) : kRouteGemv;
+  if (route == kRouteGemvTc) return b2::gemv_tc_launch(X, Wq, S, Y, M, N, K, st->ws, flags, st->sm_count, s);
+  if (route == kRouteGemv) return b2::gemv_launch(X, Wq, S, Y, M, N, K, G, st->ws, flags, st->sm_count, s);
   return b2::gemm_launch(X, Wq, S, Y, M, N, K, G, st->ws, flags, st->sm_count, s);
 }
 
@@ -182,6 +192,11 @@ int b2_w4_gemv_describe(int M, int N, int K, int G, int flags, char* buf, int bu
   int rc = 0;
   DeviceState* st = device_state(&rc);
   if (!st) return rc;
+  if (!buf || buflen < 1) return b2::kErrBadPointer;
+  const Route route =
+      M < 1 ? kRouteGemv : plain_route(*st, nullptr, nullptr, nullptr, nullptr, M, N, K, G, flags);
+  if (route == kRouteGemvTc && b2::gemv_tc_describe(N, K, flags, st->sm_count, buf, buflen) > 0) return 0;
+  if (route == kRouteGemm && b2::gemm_describe(M, N, K, G, st->ws, flags, st->sm_count, buf, buflen) > 0) return 0;
   return b2::gemv_describe(M, N, K, G, flags, st->sm_count, st->ws.partial_bytes, st->ws.n_counters - 1, buf, buflen);
 }
 
@@ -299,6 +314,7 @@ size_t b2_w4_gemv_scratch_bytes(int M, int N, int K, int G, int flags) {
   int rc = 0;
   DeviceState* st = device_state(&rc);
   if (!st) return 0;
+  if (M > 0 && plain_route(*st, nullptr, nullptr, nullptr, nullptr, M, N, K, G, flags) != kRouteGemv) return 0;
   return b2::gemv_scratch_bytes(M, N, K, G, flags, st->sm_count, st->ws.partial_bytes);
 }
 

@@ -556,6 +556,64 @@ int launch_gemm(const CUtensorMap& tx, const CUtensorMap& tw, const GemmParams& 
   return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }
 
+// How a GEMM of this shape is cut up, and about how long it takes.
+struct GemmPlan {
+  int mi = 1, tiles_x = 0, n_whole = 0, n_tail = 0, tail_ks = 1, nkb = 0;
+  bool pair = false;
+  double us = 0;
+};
+
+int gemm_plan(int M, int N, int K, const Workspace& ws, int flags, int sm_count, GemmPlan* out) {
+  GemmPlan pl;
+  // CTA pairs (each unpacks half of the weight tile for both): where the token tiles pair up without much padding.
+  // A lone token tile (M <= 256) would be paired with an empty one and do the whole unpack for half the product.
+  pl.mi = M <= 128 ? 1 : 2;
+  const int tiles_m = (M + 128 * pl.mi - 1) / (128 * pl.mi);
+  pl.pair = !(flags & kFlagGemmNoPairs) && pl.mi == 2 && (tiles_m % 2 == 0 || tiles_m >= 7);
+  pl.nkb = (K + kBK - 1) / kBK;
+  // Whole waves of tiles run one tile per CTA.  The tiles of the last, partial wave are split along K when that
+  // shortens it: pick the split whose makespan in K blocks is smallest, charging a split its fp32 round trip
+  // (e.g. the 3584 x 18944 projection: 28 tiles at M = 512 run as 5 splits each; at M = 8192 the 4 tiles that
+  // 3 waves of 148 leave over run as 8 splits each instead of a fourth wave).
+  pl.tiles_x = pl.pair ? (tiles_m + 1) / 2 * 2 : tiles_m;  // pairs never straddle a row of tiles
+  const long tiles = (long)pl.tiles_x * ((N + kBN - 1) / kBN);
+  if (tiles > 0x3fffffff) return kErrBadShape;
+  const int sms = std::max(1, sm_count);
+  const int sms_even = pl.pair ? sms / 2 * 2 : sms;  // whole waves of pairs
+  const long n_tail = tiles % sms_even ? tiles % sms_even : std::min<long>(tiles, sms_even);
+  long best_cost = -1;
+  int best = 1;
+  for (int ks = 1; ks <= 8; ++ks) {
+    if (ks > 1 && ((flags & kFlagGemmWholeTiles) || !ws.partial || !ws.counters ||
+                   (size_t)ks * n_tail * (size_t)(pl.mi * 128 * kBN) * sizeof(float) > ws.partial_bytes ||
+                   n_tail > ws.n_counters || pl.nkb / ks < 8))
+      break;
+    const long waves = (n_tail * ks + sms - 1) / sms;
+    const long cost = waves * ((pl.nkb + ks - 1) / ks + (ks > 1 ? 6 + 2 * ks : 4));
+    // a split must win by a margin: its fp32 partials cost memory traffic the model only roughly accounts for
+    // (measured: 3584 x 18944 at M = 512 goes from 267 to 747 TFLOP/s with 5 splits)
+    if (best_cost < 0 || cost * 100 < best_cost * (best == 1 ? 95 : 100)) {
+      best_cost = cost;
+      best = ks;
+    }
+  }
+  pl.n_tail = (int)n_tail;
+  pl.n_whole = (int)(tiles - n_tail);
+  pl.tail_ks = best;
+  // For the choice between this kernel and the few-token one: 0.93 us per K block of a 256 x 256 tile
+  // (0.6 of a 128-token one), 5 us to start and finish, 20 more where the last wave is split (its fp32 part-tiles), 35
+  // more per wave where N % 8 forces its epilogue to single values (1070 x 6051 x 1792: 108 us against 32).
+  // Measured at 512 tokens: 4608 x 3584 40 us against 17.8 us, 3584 x 18944 75 against 64, 37888 x 3584 110 against
+  // 121 (this one stays).
+  const double block = pl.mi == 2 ? 0.93 : 0.6;
+  const long tail_waves = (n_tail * best + sms - 1) / sms;
+  const double waves = (double)((tiles - n_tail) / sms_even);
+  pl.us = 5.0 + (best > 1 ? 20.0 : 0.0) + (N % 8 ? 35.0 * (waves + tail_waves) : 0.0) +
+          block * (waves * pl.nkb + (double)tail_waves * ((pl.nkb + best - 1) / best));
+  *out = pl;
+  return 0;
+}
+
 }  // namespace
 
 int gemm_launch(const void* X, const void* Wq, const void* S, void* Y, int M, int N, int K, int G,
@@ -571,72 +629,43 @@ int gemm_launch(const void* X, const void* Wq, const void* S, void* Y, int M, in
     return kErrBadPointer;
   if (!ws.status) return kErrWorkspace;
 
-  // CTA pairs (each unpacks half of the weight tile for both): where the token tiles pair up without much padding.
-  // A lone token tile (M <= 256) would be paired with an empty one and do the whole unpack for half the product.
-  const int mi_ = M <= 128 ? 1 : 2;
-  const int tiles_m = (M + 128 * mi_ - 1) / (128 * mi_);
-  const bool pair = !(flags & kFlagGemmNoPairs) && mi_ == 2 && (tiles_m % 2 == 0 || tiles_m >= 7);
+  GemmPlan pl;
+  if (const int rc = gemm_plan(M, N, K, ws, flags, sm_count, &pl)) return rc;
+  if (gemm_narrow_applies(M, N, K, flags, pl.us, std::max(1, sm_count)))
+    return gemm_narrow_launch(X, Wq, S, Y, M, N, K, G, ws, flags, std::max(1, sm_count), stream);
   GemmParams p{};
   p.S = static_cast<const __nv_bfloat16*>(S);
   p.Y = static_cast<__nv_bfloat16*>(Y);
   p.M = M; p.N = N; p.K = K; p.G = G;
   p.KG = K / G;
-  p.nkb = (K + kBK - 1) / kBK;
-  p.status = ws.status;
-  // Whole waves of tiles run one tile per CTA.  The tiles of the last, partial wave are split along K when that
-  // shortens it: pick the split whose makespan in K blocks is smallest, charging a split its fp32 round trip
-  // (e.g. the 3584 x 18944 projection: 28 tiles at M = 512 run as 5 splits each; at M = 8192 the 4 tiles that
-  // 3 waves of 148 leave over run as 8 splits each instead of a fourth wave).
-  {
-    const int mi = mi_;
-    p.tiles_x = pair ? (tiles_m + 1) / 2 * 2 : tiles_m;  // pairs never straddle a row of tiles
-    const long tiles = (long)p.tiles_x * ((N + kBN - 1) / kBN);
-    if (tiles > 0x3fffffff) return kErrBadShape;
-    const int sms = std::max(1, sm_count);
-    const int sms_even = pair ? sms / 2 * 2 : sms;  // whole waves of pairs
-    const long n_tail = tiles % sms_even ? tiles % sms_even : std::min<long>(tiles, sms_even);
-    long best_cost = -1;
-    int best = 1;
-    for (int ks = 1; ks <= 8; ++ks) {
-      if (ks > 1 && ((flags & kFlagGemmWholeTiles) || !ws.partial || !ws.counters ||
-                     (size_t)ks * n_tail * (size_t)(mi * 128 * kBN) * sizeof(float) > ws.partial_bytes ||
-                     n_tail > ws.n_counters || p.nkb / ks < 8))
-        break;
-      const long waves = (n_tail * ks + sms - 1) / sms;
-      const long cost = waves * ((p.nkb + ks - 1) / ks + (ks > 1 ? 6 + 2 * ks : 4));
-      // a split must win by a margin: its fp32 partials cost memory traffic the model only roughly accounts for
-      // (measured: 3584 x 18944 at M = 512 goes from 267 to 747 TFLOP/s with 5 splits)
-      if (best_cost < 0 || cost * 100 < best_cost * (best == 1 ? 95 : 100)) {
-        best_cost = cost;
-        best = ks;
-      }
-    }
-    p.n_tail = (int)n_tail;
-    p.n_whole = (int)(tiles - n_tail);
-    p.tail_ks = best;
+  p.nkb = pl.nkb;
+  p.tiles_x = pl.tiles_x;
+  p.n_whole = pl.n_whole;
+  p.n_tail = pl.n_tail;
+  p.tail_ks = pl.tail_ks;
+  if (pl.tail_ks > 1) {
     p.partial = ws.partial;
     p.counters = ws.counters;
-    // The few-token kernel where it is estimated to be shorter.  This kernel: 0.93 us per K block of a 256 x 256 tile
-    // (0.6 of a 128-token one), 5 us to start and finish, 20 more where the last wave is split (its fp32 part-tiles), 35
-    // more per wave where N % 8 forces its epilogue to single values (1070 x 6051 x 1792: 108 us against 32).
-    // Measured at 512 tokens: 4608 x 3584 40 us against 17.8 us, 3584 x 18944 75 against 64, 37888 x 3584 110 against
-    // 121 (this one stays).
-    const double block = mi == 2 ? 0.93 : 0.6;
-    const long tail_waves = (n_tail * best + sms - 1) / sms;
-    const double waves = (double)((tiles - n_tail) / sms_even);
-    const double us = 5.0 + (best > 1 ? 20.0 : 0.0) + (N % 8 ? 35.0 * (waves + tail_waves) : 0.0) +
-                      block * (waves * p.nkb + (double)tail_waves * ((p.nkb + best - 1) / best));
-    if (gemm_narrow_applies(M, N, K, flags, us, sms))
-      return gemm_narrow_launch(X, Wq, S, Y, M, N, K, G, ws, flags, sms, stream);
   }
+  p.status = ws.status;
   CUtensorMap tx, tw;
   if (!make_tensor_map_2d(&tx, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, X, (uint64_t)M, (uint64_t)K, 128, kBK,
                  CU_TENSOR_MAP_SWIZZLE_128B) ||
-      !make_tensor_map_2d(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, Wq, (uint64_t)N, (uint64_t)K / 8, pair ? kBN / 2 : kBN,
+      !make_tensor_map_2d(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, Wq, (uint64_t)N, (uint64_t)K / 8, pl.pair ? kBN / 2 : kBN,
                  kBK / 8, CU_TENSOR_MAP_SWIZZLE_NONE))
     return kErrDevice;
-  if (pair) return launch_gemm<2, true>(tx, tw, p, stream);
-  return M <= 128 ? launch_gemm<1, false>(tx, tw, p, stream) : launch_gemm<2, false>(tx, tw, p, stream);
+  if (pl.pair) return launch_gemm<2, true>(tx, tw, p, stream);
+  return pl.mi == 1 ? launch_gemm<1, false>(tx, tw, p, stream) : launch_gemm<2, false>(tx, tw, p, stream);
+}
+
+int gemm_describe(int M, int N, int K, int G, const Workspace& ws, int flags, int sm_count, char* buf, int buflen) {
+  GemmPlan pl;
+  if (M < 1 || N < 1 || K < 32 || G < 32 || K % 32 || G % 32 || K % G || gemm_plan(M, N, K, ws, flags, sm_count, &pl) != 0)
+    return snprintf(buf, buflen, "not served");
+  if (gemm_narrow_applies(M, N, K, flags, pl.us, std::max(1, sm_count)))
+    return gemm_narrow_describe(M, N, K, G, flags, std::max(1, sm_count), buf, buflen);
+  return snprintf(buf, buflen, "prefill GEMM: %d tiles of 256 rows x %d tokens%s, the last %d in %d K part(s)",
+                  pl.n_whole + pl.n_tail, 128 * pl.mi, pl.pair ? " in CTA pairs" : "", pl.n_tail, pl.tail_ks);
 }
 
 }  // namespace b2

@@ -27,6 +27,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <cstdio>
 
 #include "ptx.cuh"
 #include "tensor_map.h"
@@ -526,12 +527,12 @@ int current_device() {
 // takes about 4 + 0.195 w + M K / 1e4 us (w = millions of weights, from HBM; 0.1 w more above eight tokens): G = 64,
 // 37888 x 3584 M = 4 35.0 against 22.7 here, 3584 x 18944 M = 16 64.4 against 18.4, 3584 x 3584 M = 1 7.3 against 6.9;
 // 57344 x 8192 M = 1 stays, 97.6 against 85 and estimated at 100.  Multiples of 128 keep exact weights: the GEMVs' alone.
+// (Pointers: null = "assume aligned", for the queries that have no operands.)
 bool gemm_narrow_takes_decode(const void* X, const void* Wq, const void* S, const void* Y, int M, int N, int K, int G,
                               int flags, int sm_count) {
   if (flags < 0) return true;
   if (flags != 0 || M < 1 || N < 1 || K < 32 || G < 32 || K % 32 || G % 32 || K % G || G % 128 == 0) return false;
-  if (!X || !Wq || !S || !Y ||
-      ((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(Wq) | reinterpret_cast<uintptr_t>(Y)) & 15) ||
+  if (((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(Wq) | reinterpret_cast<uintptr_t>(Y)) & 15) ||
       (reinterpret_cast<uintptr_t>(S) & 1))
     return false;
   const double w = (double)N * K * 1e-6, gemv = 4.0 + 0.195 * w + 1e-4 * M * K + (M > 8 ? 0.1 * w : 0.0);
@@ -545,6 +546,15 @@ bool gemm_narrow_applies(int M, int N, int K, int flags, double wide_us, int sm_
   if (flags & (kFlagGemmNoPairs | kFlagGemmWholeTiles | kFlagGemmWide)) return false;  // the other kernel's switches
   if (flags & kFlagGemmNarrow) return true;
   return narrow_plan(M, N, K, flags, sm_count, current_device()).us < wide_us;
+}
+
+int gemm_narrow_describe(int M, int N, int K, int G, int flags, int sm_count, char* buf, int buflen) {
+  const NarrowPlan pl = narrow_plan(M, N, K, flags, sm_count, current_device());
+  static const char* const kScales[5] = {"one by one", "by two", "by four", "by step", "by step"};
+  return snprintf(buf, buflen,
+                  "few-token GEMM: %ld CTAs (%d per SM), tiles of %d rows x %d tokens, clusters of %d along K, scales %s",
+                  pl.n_tiles * pl.ks, pl.form ? 1 : 2, pl.form ? 256 : 128, pl.nt, pl.ks,
+                  kScales[narrow_variant(nullptr, K, G)]);
 }
 
 // The arguments have been checked by gemm_launch.

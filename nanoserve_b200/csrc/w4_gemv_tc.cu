@@ -22,6 +22,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <cstdio>
 
 #include "ptx.cuh"
 #include "tensor_map.h"
@@ -419,16 +420,28 @@ bool tc_plan(int N, int K, int sm_count, int wanted_form, int wanted_ks, TcPlan*
 // Nine to sixteen tokens and groups of 128, where the estimate is below what the mma.sync kernel takes: 6 + 0.145 w + 3 K /
 // 1e4 us (w = millions of weights; 57344 x 8192 stays, 88 us against 96, and 8192 x 28672, 50 against 57).  Fewer tokens: the
 // mma.sync kernel pads to eight and is as fast or faster (37888 x 3584 at eight 20.0 against 21.0).
+// (Pointers: null = "assume aligned", for the queries that have no operands.)
 bool gemv_tc_applies(const void* X, const void* Wq, const void* S, const void* Y, int M, int N, int K, int G, int flags,
                      int sm_count) {
   if (G != kStepK || K < 2 * kStepK || K % (2 * kStepK) || N < 1 || M < 1 || M > kTokens) return false;
-  if (!X || !Wq || !S || !Y || ((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(Wq)) & 15) ||
-      (reinterpret_cast<uintptr_t>(Y) & 7) || (reinterpret_cast<uintptr_t>(S) & 3))
+  if (((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(Wq)) & 15) || (reinterpret_cast<uintptr_t>(Y) & 7) ||
+      (reinterpret_cast<uintptr_t>(S) & 3))
     return false;
   TcPlan pl;
   if (flags < 0) return tc_plan(N, K, sm_count, (flags >> 24) & 3, (flags >> 20) & 15, &pl);
   return flags == 0 && M > 8 && tc_plan(N, K, sm_count, 0, 0, &pl) &&
          pl.us < 6.0 + 0.145e-6 * ((double)N * K) + 3e-4 * K;
+}
+
+int gemv_tc_describe(int N, int K, int flags, int sm_count, char* buf, int buflen) {
+  const bool forced = flags < 0;
+  TcPlan pl;
+  if (!tc_plan(N, K, sm_count, forced ? (flags >> 24) & 3 : 0, forced ? (flags >> 20) & 15 : 0, &pl)) return 0;
+  const int rows = pl.form ? 256 : 128;
+  return snprintf(buf, buflen,
+                  "tcgen05 GEMV: %d CTAs (%d per SM), tiles of %d rows x %d tokens, clusters of %d along K, 2 planes (16-bit X), "
+                  "%d ring slots",
+                  (N + rows - 1) / rows * pl.ks, pl.form ? 1 : 2, rows, kTokens, pl.ks, pl.sw);
 }
 
 // flags: bits 20-23 CTAs per cluster, bits 24-25 tile (1: 128 rows, two CTAs per SM; 2: 256 rows, one), 0 = the rule.

@@ -128,6 +128,9 @@ bool gemm_narrow_takes_decode(const void* X, const void* Wq, const void* S, cons
 bool gemm_narrow_applies(int M, int N, int K, int flags, double wide_us, int sm_count);
 int gemm_narrow_launch(const void* X, const void* Wq, const void* S, void* Y, int M, int N, int K, int G,
                        const Workspace& ws, int flags, int sm_count, cudaStream_t stream);
+int gemm_describe(int M, int N, int K, int G, const Workspace& ws, int flags, int sm_count, char* buf, int buflen);
+int gemm_narrow_describe(int M, int N, int K, int G, int flags, int sm_count, char* buf, int buflen);
+int gemv_tc_describe(int N, int K, int flags, int sm_count, char* buf, int buflen);
 bool gemv_tc_applies(const void* X, const void* Wq, const void* S, const void* Y, int M, int N, int K, int G, int flags,
                      int sm_count);
 int gemv_tc_launch(const void* X, const void* Wq, const void* S, void* Y, int M, int N, int K, const Workspace& ws,

@@ -325,7 +325,8 @@ class Kernels:
                     "b2_tp_wait_desc")
 
     def gemv_describe(self, M, N, K, group=128, flags=0) -> str:
-        """Which kernel and launch shape a decode GEMV of this shape gets on the current device."""
+        """Which kernel and launch shape w4_linear runs for this shape on the current device (fused and tensor-parallel
+        calls: ask with FLAG_NO_MID_KERNEL)."""
         buf = ctypes.create_string_buffer(512)
         self._check(self.lib.b2_w4_gemv_describe(M, N, K, group, flags, buf, 512), "b2_w4_gemv_describe")
         return buf.value.decode()

@@ -63,6 +63,7 @@ def test_decode_of_fine_groups_takes_any_alignment(kernels):
     """Fine groups at decode token counts run the few-token GEMM where pointers are 16-byte aligned, and the GEMV where they
     are not: the results agree to a rounding of the output and of the sums."""
     M, N, K, G = 4, 1000, 2048, 64
+    assert kernels.gemv_describe(M, N, K, G, 0).startswith("few-token GEMM")
     X, Wq, S = oracle.synth_inputs(M, N, K, G, seed=8)
     x, wq, s = bits_to_torch(X), u32_to_torch(Wq), bits_to_torch(S)
     want = oracle.bf16_bits_to_f32(torch_to_bits(kernels.w4_linear(x, wq, s, G)))

@@ -36,6 +36,7 @@ def test_rule_on_layer_shapes(kernels, M):
     """What the rule picks, against the oracle on sampled rows and against the mma.sync kernel: the same integers in
     another order of fp32 sums."""
     for N, K in [(3584, 3584), (512, 3584), (3584, 18944)]:
+        assert kernels.gemv_describe(M, N, K, 128, 0).startswith("tcgen05 GEMV")
         X, Wq, S = oracle.synth_inputs(M, N, K, 128, seed=4)
         y = run(kernels, X, Wq, S, 0)
         rows = np.unique(np.concatenate([[0, N - 1], np.random.default_rng(0).integers(0, N, 40)]))
