@@ -531,7 +531,7 @@ int current_device() {
 bool gemm_narrow_takes_decode(const void* X, const void* Wq, const void* S, const void* Y, int M, int N, int K, int G,
                               int flags, int sm_count) {
   if (flags < 0) return true;
-  if (flags != 0 || M < 1 || N < 1 || K < 32 || G < 32 || K % 32 || G % 32 || K % G || G % 128 == 0) return false;
+  if ((flags & ~kFlagNoPdl) != 0 || M < 1 || N < 1 || K < 32 || G < 32 || K % 32 || G % 32 || K % G || G % 128 == 0) return false;
   if (((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(Wq) | reinterpret_cast<uintptr_t>(Y)) & 15) ||
       (reinterpret_cast<uintptr_t>(S) & 1))
     return false;

@@ -429,7 +429,7 @@ bool gemv_tc_applies(const void* X, const void* Wq, const void* S, const void* Y
     return false;
   TcPlan pl;
   if (flags < 0) return tc_plan(N, K, sm_count, (flags >> 24) & 3, (flags >> 20) & 15, &pl);
-  return flags == 0 && M > 8 && tc_plan(N, K, sm_count, 0, 0, &pl) &&
+  return (flags & ~kFlagNoPdl) == 0 && M > 8 && tc_plan(N, K, sm_count, 0, 0, &pl) &&
          pl.us < 6.0 + 0.145e-6 * ((double)N * K) + 3e-4 * K;
 }
 
@@ -495,9 +495,11 @@ int gemv_tc_launch(const void* X, const void* Wq, const void* S, void* Y, int M,
     attr[na].val.clusterDim.z = 1;
     ++na;
   }
-  attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[na].val.programmaticStreamSerializationAllowed = 1;
-  ++na;
+  if ((flags & kFlagNoPdl) == 0) {
+    attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[na].val.programmaticStreamSerializationAllowed = 1;
+    ++na;
+  }
   cfg.attrs = attr;
   cfg.numAttrs = na;
   e = cudaLaunchKernelEx(&cfg, kernel, tw, p);

@@ -67,8 +67,8 @@ enum : int {
   kFlagGemmWide = 1 << 27,        // GEMM: never that kernel
   kFlagDecodeNarrow = (int)0x80000000u,  // M <= 16: the tcgen05 GEMV (w4_gemv_tc.cu) where its shapes allow, else that
                                          // kernel, instead of another GEMV (bits 20-25 as for kFlagGemmNarrow)
-  kFlagNoPdl = 8,          // GEMV: do NOT launch with programmatic stream serialization (by default the kernel may
-                           // begin -- weight prefetch only -- while the previous kernel of the stream still runs)
+  kFlagNoPdl = 8,          // do NOT launch with programmatic stream serialization (by default every kernel but the prefill
+                           // GEMM may begin while the previous kernel of the stream still runs); same kernel and plan
 };
 
 // Optional prologue of the GEMV (G % 128 == 0 only): the operator that precedes the linear, folded into the

@@ -3,7 +3,7 @@ start while the kernel in front still runs) behind kernels whose outputs they re
 import pytest
 import torch
 
-from nanoserve_b200.ops import FLAG_DECODE_NARROW, FLAG_GEMM_NARROW, narrow_flags
+from nanoserve_b200.ops import FLAG_DECODE_NARROW, FLAG_GEMM_NARROW, FLAG_NO_PDL, narrow_flags
 
 pytestmark = pytest.mark.gpu
 
@@ -97,3 +97,13 @@ def test_wait_for_a_long_launch_is_no_time_out(kernels, long_launch, M, G, flags
     long_launch()
     got = kernels.w4_linear(x, Wq, S, G, flags=flags)
     assert kernels.device_status() == 0 and torch.equal(got, want)
+
+
+@pytest.mark.parametrize("M,N,K,G", [(1, 3584, 3584, 128), (4, 1000, 2048, 64), (8, 3584, 18944, 128), (13, 3584, 3584, 128),
+                                     (16, 3584, 18944, 32), (48, 4608, 3584, 128), (2, 1000, 2048, 32)])
+def test_a_plain_launch_runs_the_same_kernel(kernels, M, N, K, G):
+    assert kernels.gemv_describe(M, N, K, G, FLAG_NO_PDL) == kernels.gemv_describe(M, N, K, G)
+    gen = torch.Generator(device="cuda").manual_seed(N)
+    x, (Wq, S) = rand_x(M, K, gen), rand_w4(N, K, G, gen)
+    assert torch.equal(kernels.w4_linear(x, Wq, S, G, flags=FLAG_NO_PDL), kernels.w4_linear(x, Wq, S, G))
+    assert kernels.device_status() == 0
