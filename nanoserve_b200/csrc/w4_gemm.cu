@@ -600,16 +600,25 @@ int gemm_plan(int M, int N, int K, const Workspace& ws, int flags, int sm_count,
   pl.n_tail = (int)n_tail;
   pl.n_whole = (int)(tiles - n_tail);
   pl.tail_ks = best;
-  // For the choice between this kernel and the few-token one: 0.93 us per K block of a 256 x 256 tile
-  // (0.6 of a 128-token one), 5 us to start and finish, 20 more where the last wave is split (its fp32 part-tiles), 35
-  // more per wave where N % 8 forces its epilogue to single values (1070 x 6051 x 1792: 108 us against 32).
-  // Measured at 512 tokens: 4608 x 3584 40 us against 17.8 us, 3584 x 18944 75 against 64, 37888 x 3584 110 against
-  // 121 (this one stays).
-  const double block = pl.mi == 2 ? 0.93 : 0.6;
-  const long tail_waves = (n_tail * best + sms - 1) / sms;
-  const double waves = (double)((tiles - n_tail) / sms_even);
-  pl.us = 5.0 + (best > 1 ? 20.0 : 0.0) + (N % 8 ? 35.0 * (waves + tail_waves) : 0.0) +
-          block * (waves * pl.nkb + (double)tail_waves * ((pl.nkb + best - 1) / best));
+  // About how long that takes, for the choice between this kernel and the few-token one: a start, then per wave a fixed
+  // part and its K blocks, which take longer the more SMs are at work (a pair shares its operands through the same
+  // memory), a split's exchange of part-tiles, and the single-value epilogue where N % 8.  Least-squares fit, us, to 486
+  // launches of this kernel from 17 to 8192 tokens, 256 to 57344 x 256 to 28672, weights from HBM, weighted towards
+  // shapes where the two kernels are close; 6 to 8 % off there.  (One rate of 0.93 us per block for every shape, as it
+  // takes at K = 3584, sent 3584 x 18944 at 2048 tokens to the few-token kernel: 255 us against 221.)
+  struct Cost {
+    double start, wave, block, block_busy, split, split_part, odd_wave, odd_split;
+  };
+  static constexpr Cost kCost[3] = {{5.8, 0.0, 0.794, 0.0, 8.7, 1.3, 8.4, 10.9},       // 128 tokens
+                                    {2.1, 8.7, 0.880, 0.037, 3.6, 3.7, 53.9, 44.1},    // 256 tokens
+                                    {1.3, 11.1, 0.430, 0.357, 3.7, 3.0, 64.4, 57.1}};  // CTA pairs
+  const Cost& c = kCost[pl.mi == 1 ? 0 : pl.pair ? 2 : 1];
+  const long tail_waves = (n_tail * best + sms - 1) / sms, whole_waves = (tiles - n_tail) / sms_even;
+  const double busy = std::min(1.0, (double)(n_tail * best) / (double)(tail_waves * sms));
+  pl.us = c.start + whole_waves * (c.wave + (c.block + c.block_busy) * pl.nkb) +
+          tail_waves * (c.wave + (c.block + c.block_busy * busy) * ((pl.nkb + best - 1) / best)) +
+          (best > 1 ? c.split + c.split_part * best : 0.0);
+  if (N % 8) pl.us += c.odd_wave * (whole_waves + (best > 1 ? 0 : tail_waves)) + (best > 1 ? c.odd_split : 0.0);
   *out = pl;
   return 0;
 }
@@ -631,7 +640,7 @@ int gemm_launch(const void* X, const void* Wq, const void* S, void* Y, int M, in
 
   GemmPlan pl;
   if (const int rc = gemm_plan(M, N, K, ws, flags, sm_count, &pl)) return rc;
-  if (gemm_narrow_applies(M, N, K, flags, pl.us, std::max(1, sm_count)))
+  if (gemm_narrow_applies(S, M, N, K, G, flags, pl.us, std::max(1, sm_count)))
     return gemm_narrow_launch(X, Wq, S, Y, M, N, K, G, ws, flags, std::max(1, sm_count), stream);
   GemmParams p{};
   p.S = static_cast<const __nv_bfloat16*>(S);
@@ -662,7 +671,7 @@ int gemm_describe(int M, int N, int K, int G, const Workspace& ws, int flags, in
   GemmPlan pl;
   if (M < 1 || N < 1 || K < 32 || G < 32 || K % 32 || G % 32 || K % G || gemm_plan(M, N, K, ws, flags, sm_count, &pl) != 0)
     return snprintf(buf, buflen, "not served");
-  if (gemm_narrow_applies(M, N, K, flags, pl.us, std::max(1, sm_count)))
+  if (gemm_narrow_applies(nullptr, M, N, K, G, flags, pl.us, std::max(1, sm_count)))
     return gemm_narrow_describe(M, N, K, G, flags, std::max(1, sm_count), buf, buflen);
   return snprintf(buf, buflen, "prefill GEMM: %d tiles of 256 rows x %d tokens%s, the last %d in %d K part(s)",
                   pl.n_whole + pl.n_tail, 128 * pl.mi, pl.pair ? " in CTA pairs" : "", pl.n_tail, pl.tail_ks);

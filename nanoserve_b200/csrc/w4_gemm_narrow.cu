@@ -400,10 +400,13 @@ NarrowForm narrow_form(int form, int variant) {
   if (form == 0) return {kHalf[variant], variant, 128, 8, 2, kSmemHalf};
   return {kFull[variant], variant, 256, 16, 1, kSmemFull};
 }
-int narrow_variant(const void* S, int K, int G) {
+int narrow_scales_per_load(const void* S, int K, int G) {
   const uintptr_t sa = reinterpret_cast<uintptr_t>(S);
   const int kg = K / G;
-  const int sv = kg % 4 == 0 && sa % 8 == 0 ? 4 : kg % 2 == 0 && sa % 4 == 0 ? 2 : 1;
+  return kg % 4 == 0 && sa % 8 == 0 ? 4 : kg % 2 == 0 && sa % 4 == 0 ? 2 : 1;
+}
+int narrow_variant(const void* S, int K, int G) {
+  const int sv = narrow_scales_per_load(S, K, G);
   if (G == 128 && sv > 1) return sv / 2;
   if (G == 64 && K % kKB == 0 && sv > 1) return 3;
   if (G == 32 && K % kKB == 0 && sv == 4) return 4;
@@ -540,12 +543,17 @@ bool gemm_narrow_takes_decode(const void* X, const void* Wq, const void* S, cons
   return slower * narrow_plan(M, N, K, 0, sm_count, current_device()).us < gemv;
 }
 
-// Whether this kernel takes a GEMM that the general kernel would run in about wide_us microseconds.
-bool gemm_narrow_applies(int M, int N, int K, int flags, double wide_us, int sm_count) {
+// Whether this kernel takes a GEMM that the general kernel would run in about wide_us microseconds.  The estimate of its
+// plan is brought to what it takes where the two are close; the form for any group takes longer by its loads of scales per
+// step (groups of 128 one by one, as K = 13696 has them, 1.31; of 64 1.6; of 32 2.4; of 256 by two 1.12).  Over 1900 shapes,
+// 17 to 8192 tokens, both kernels timed in turn, the one this picks takes 1.003 times the shorter one's time in the
+// geometric mean and is more than 10 % behind in 1 % (before the two fits: 1.51 at 4096 tokens on 4096 x 13696).
+bool gemm_narrow_applies(const void* S, int M, int N, int K, int G, int flags, double wide_us, int sm_count) {
   if (M <= 16) return true;  // (decided by gemm_narrow_takes_decode)
   if (flags & (kFlagGemmNoPairs | kFlagGemmWholeTiles | kFlagGemmWide)) return false;  // the other kernel's switches
   if (flags & kFlagGemmNarrow) return true;
-  return narrow_plan(M, N, K, flags, sm_count, current_device()).us < wide_us;
+  const double slower = narrow_variant(S, K, G) != 0 ? 1.0 : 1.05 + 0.31 * 128.0 / G / narrow_scales_per_load(S, K, G);
+  return 1.4 + 0.957 * slower * narrow_plan(M, N, K, flags, sm_count, current_device()).us < wide_us;
 }
 
 int gemm_narrow_describe(int M, int N, int K, int G, int flags, int sm_count, char* buf, int buflen) {
@@ -573,8 +581,7 @@ int gemm_narrow_launch(const void* X, const void* Wq, const void* S, void* Y, in
   p.t_tiles = pl.t_tiles;
   p.nt = pl.nt;
   p.ks = pl.ks;
-  const uintptr_t sa = reinterpret_cast<uintptr_t>(S);
-  p.sv = p.KG % 4 == 0 && sa % 8 == 0 ? 4 : p.KG % 2 == 0 && sa % 4 == 0 ? 2 : 1;
+  p.sv = narrow_scales_per_load(S, K, G);
   const NarrowForm f = narrow_form(pl.form, narrow_variant(S, K, G));
   const int slot_w = f.rows * 128, slot_x = p.nt * 256, room = f.smem - kHeaderBytes - 1024;
   const int x_bytes = pl.form ? 128 << 10 : p.nt > 64 ? 72 << 10 : 48 << 10;  // the rest holds packed words

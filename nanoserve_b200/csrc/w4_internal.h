@@ -125,7 +125,7 @@ int gemm_launch(const void* X, const void* Wq, const void* S, void* Y, int M, in
 // Whether the few-token GEMM takes a call of at most 16 tokens from the GEMVs (gemm_launch then runs it).
 bool gemm_narrow_takes_decode(const void* X, const void* Wq, const void* S, const void* Y, int M, int N, int K, int G,
                               int flags, int sm_count);
-bool gemm_narrow_applies(int M, int N, int K, int flags, double wide_us, int sm_count);
+bool gemm_narrow_applies(const void* S, int M, int N, int K, int G, int flags, double wide_us, int sm_count);
 int gemm_narrow_launch(const void* X, const void* Wq, const void* S, void* Y, int M, int N, int K, int G,
                        const Workspace& ws, int flags, int sm_count, cudaStream_t stream);
 int gemm_describe(int M, int N, int K, int G, const Workspace& ws, int flags, int sm_count, char* buf, int buflen);

@@ -75,3 +75,28 @@ def test_decode_of_fine_groups_takes_any_alignment(kernels):
     assert kernels.device_status() == 0
     got = oracle.bf16_bits_to_f32(torch_to_bits(out))
     assert np.abs(got - want).max() <= 2.0**-7 * np.abs(want).max()
+
+
+# tokens, rows, K, group, the kernel that was the shorter one, us of the general and of this kernel timed in turn
+@pytest.mark.parametrize("M,N,K,G,kernel", [
+    (2048, 3584, 18944, 128, "prefill GEMM"),  # 221, 255
+    (1536, 3584, 18944, 128, "prefill GEMM"),  # 178, 191
+    (512, 3584, 18944, 128, "few-token GEMM"),  # 77, 64
+    (2048, 4096, 13696, 128, "prefill GEMM"),  # 167, 235 (scales one by one)
+    (768, 4096, 13696, 128, "prefill GEMM"),  # 87, 102
+    (256, 4096, 13696, 128, "few-token GEMM"),  # 63, 36
+    (2048, 8192, 28672, 128, "prefill GEMM"),  # 774, 843
+    (256, 8192, 28672, 128, "few-token GEMM"),  # 135, 99
+    (2048, 4096, 14336, 128, "prefill GEMM"),  # 184, 196
+    (4096, 4096, 14336, 128, "prefill GEMM"),  # 363, 420
+    (512, 4096, 14336, 128, "few-token GEMM"),  # 68, 52
+    (1536, 5120, 13824, 128, "prefill GEMM"),  # 164, 178
+    (2048, 8192, 8192, 128, "prefill GEMM"),  # 201, 234
+    (768, 28672, 8192, 128, "few-token GEMM"),  # 344, 288
+    (512, 37888, 3584, 128, "prefill GEMM"),  # 108, 118
+    (512, 4608, 3584, 128, "few-token GEMM"),  # 41, 19
+    (8192, 18944, 3584, 128, "prefill GEMM"),
+    (1070, 6051, 1792, 128, "few-token GEMM"),  # 108, 32 (an odd number of rows: the general kernel stores value by value)
+])
+def test_rule_takes_the_shorter_kernel(kernels, M, N, K, G, kernel):
+    assert kernels.gemv_describe(M, N, K, G).startswith(kernel)
