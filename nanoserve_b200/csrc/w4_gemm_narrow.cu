@@ -530,6 +530,9 @@ int current_device() {
 // takes about 4 + 0.195 w + M K / 1e4 us (w = millions of weights, from HBM; 0.1 w more above eight tokens): G = 64,
 // 37888 x 3584 M = 4 35.0 against 22.7 here, 3584 x 18944 M = 16 64.4 against 18.4, 3584 x 3584 M = 1 7.3 against 6.9;
 // 57344 x 8192 M = 1 stays, 97.6 against 85 and estimated at 100.  Multiples of 128 keep exact weights: the GEMVs' alone.
+// Groups whose scales this kernel would read one by one or by two (K / 64 odd, K / 32 not a multiple of four) stay with the
+// GEMV: 313 x 28224 in groups of 64, M = 14, 13.7 us against 31.2 here, 8436 x 8032 in groups of 32, M = 6, 24.4 against 39.9;
+// over 140 such shapes 1.1 times the GEMV's time, over 100 of the others 0.66 times.
 // (Pointers: null = "assume aligned", for the queries that have no operands.)
 bool gemm_narrow_takes_decode(const void* X, const void* Wq, const void* S, const void* Y, int M, int N, int K, int G,
                               int flags, int sm_count) {
@@ -538,9 +541,9 @@ bool gemm_narrow_takes_decode(const void* X, const void* Wq, const void* S, cons
   if (((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(Wq) | reinterpret_cast<uintptr_t>(Y)) & 15) ||
       (reinterpret_cast<uintptr_t>(S) & 1))
     return false;
+  if (narrow_variant(S, K, G) == 0) return false;
   const double w = (double)N * K * 1e-6, gemv = 4.0 + 0.195 * w + 1e-4 * M * K + (M > 8 ? 0.1 * w : 0.0);
-  const double slower = narrow_variant(S, K, G) == 0 ? 1.5 : 1.05;  // than the form the estimate was fitted to
-  return slower * narrow_plan(M, N, K, 0, sm_count, current_device()).us < gemv;
+  return 1.05 * narrow_plan(M, N, K, 0, sm_count, current_device()).us < gemv;
 }
 
 // Whether this kernel takes a GEMM that the general kernel would run in about wide_us microseconds.  The estimate of its

@@ -100,3 +100,16 @@ def test_decode_of_fine_groups_takes_any_alignment(kernels):
 ])
 def test_rule_takes_the_shorter_kernel(kernels, M, N, K, G, kernel):
     assert kernels.gemv_describe(M, N, K, G).startswith(kernel)
+
+
+# tokens, rows, K, group, the kernel that was the shorter one, us of the ring GEMV and of this kernel
+@pytest.mark.parametrize("M,N,K,G,kernel", [
+    (14, 313, 28224, 64, "ring kernel"),  # 13.7, 31.2 (441 groups a row: scales one by one)
+    (6, 8436, 8032, 32, "ring kernel"),  # 24.4, 39.9
+    (16, 449, 13920, 32, "ring kernel"),  # 14.4, 24.1
+    (4, 18944, 3584, 64, "few-token GEMM"),
+    (16, 3584, 18944, 64, "few-token GEMM"),  # 64.4, 18.4
+    (16, 3584, 18944, 32, "few-token GEMM"),
+])
+def test_rule_at_decode_tokens(kernels, M, N, K, G, kernel):
+    assert kernels.gemv_describe(M, N, K, G).startswith(kernel)
