@@ -381,13 +381,14 @@ __global__ void __launch_bounds__(128 + DW * 32, MINB)
 using TcKernel = void (*)(const CUtensorMap, const TcParams);
 
 struct TcPlan {
-  int form = 0, ks = 1, sw = 0;  // form 0: 128 rows, two CTAs per SM; 1: 256 rows, one
+  int form = 0, ks = 1, sw = 0, steps = 0;  // form 0: 128 rows, two CTAs per SM; 1: 256 rows, one
   double us = 0;
 };
 
 // Estimated time (us, fitted to 512 to 57344 x 2048 to 28672): waves of CTAs, 4.6 each for start, X and the exchange, 0.62
-// per step of a 256-row CTA; a 128-row one takes 0.5 alone on its SM and twice that with a neighbour.  A CTA's steps are
-// limited by the planes of X beside two ring slots.  wanted_*: 0 = any.
+// per step of a 256-row CTA; a 128-row one takes 0.5 alone on its SM and twice that with a neighbour, and up to 2 more to
+// start and sum up where K is cut into single steps and the chip is full (5097 x 768 in clusters of six: 6.3).  A CTA's steps
+// are limited by the planes of X beside two ring slots.  wanted_*: 0 = any.
 bool tc_plan(int N, int K, int sm_count, int wanted_form, int wanted_ks, TcPlan* out) {
   const int nkb = K / kStepK;
   bool any = false;
@@ -401,13 +402,14 @@ bool tc_plan(int N, int K, int sm_count, int wanted_form, int wanted_ks, TcPlan*
       TcPlan pl;
       pl.form = form;
       pl.ks = ks;
+      pl.steps = steps;
       pl.sw = std::min(kMaxSlots, (room - steps * (kXStep + kInfoStep)) / (rows * 128));
       if (pl.sw < 2) continue;
       // clusters leave some SMs of a GPC out
       const long cap = (form ? 1 : 2) * (ks == 1 ? sm_count : ks == 7 ? sm_count * 0.7 : ks == 8 ? sm_count * 0.8 : sm_count * 0.87);
       const long ctas = tiles * ks, waves = (ctas + cap - 1) / cap;
       const double busy = std::min(1.0, (double)ctas / waves / (2.0 * sm_count));
-      pl.us = waves * (form ? 4.6 + 0.62 * steps : 3.8 + (0.5 + 0.5 * busy) * steps);
+      pl.us = waves * (form ? 4.6 + 0.62 * steps : 3.8 + (0.5 + 0.5 * busy) * steps + (steps == 1 ? 2.0 * busy : 0.0));
       if (!any || pl.us < out->us) *out = pl;
       any = true;
     }
@@ -419,7 +421,10 @@ bool tc_plan(int N, int K, int sm_count, int wanted_form, int wanted_ks, TcPlan*
 
 // Nine to sixteen tokens and groups of 128, where the estimate is below what the mma.sync kernel takes: 6 + 0.145 w + 3 K /
 // 1e4 us (w = millions of weights; 57344 x 8192 stays, 88 us against 96, and 8192 x 28672, 50 against 57).  Fewer tokens: the
-// mma.sync kernel pads to eight and is as fast or faster (37888 x 3584 at eight 20.0 against 21.0).
+// mma.sync kernel pads to eight and is as fast or faster (37888 x 3584 at eight 20.0 against 21.0).  The estimate is 4 %
+// short over 200 shapes, 10 % where a 128-row CTA has nine steps and more (1500 x 11008: 13.9 us against 11.0, estimated at
+// 11.1 and 11.7).  Two chunks of K on few rows are all start-up, of which this kernel has more (700 x 256: 3.9 to 4.1 us against
+// 3.3; 6000 x 256 level).  Over 110 shapes the pick takes 1.006 times the shorter one's time in the geometric mean.
 // (Pointers: null = "assume aligned", for the queries that have no operands.)
 bool gemv_tc_applies(const void* X, const void* Wq, const void* S, const void* Y, int M, int N, int K, int G, int flags,
                      int sm_count) {
@@ -429,8 +434,9 @@ bool gemv_tc_applies(const void* X, const void* Wq, const void* S, const void* Y
     return false;
   TcPlan pl;
   if (flags < 0) return tc_plan(N, K, sm_count, (flags >> 24) & 3, (flags >> 20) & 15, &pl);
-  return (flags & ~kFlagNoPdl) == 0 && M > 8 && tc_plan(N, K, sm_count, 0, 0, &pl) &&
-         pl.us < 6.0 + 0.145e-6 * ((double)N * K) + 3e-4 * K;
+  if ((flags & ~kFlagNoPdl) != 0 || M <= 8 || (K <= 256 && N < 5000) || !tc_plan(N, K, sm_count, 0, 0, &pl)) return false;
+  const double longer = pl.form == 0 && pl.steps >= 9 ? 1.1 : 1.04;
+  return longer * pl.us < 6.0 + 0.145e-6 * ((double)N * K) + 3e-4 * K;
 }
 
 int gemv_tc_describe(int N, int K, int flags, int sm_count, char* buf, int buflen) {

@@ -61,3 +61,21 @@ def test_extreme_inputs(kernels):
     assert np.isnan(oracle.bf16_bits_to_f32(y[[0, 2, 5]])).all()
     for m in (1, 3, 4, 6, 7, 15):
         check_bf16_output(y[m:m + 1], ref[m:m + 1], SLACK)
+
+
+# tokens, rows, columns, the kernel that was the shorter one, us of the many-token and of this kernel
+@pytest.mark.parametrize("M,N,K,kernel", [
+    (10, 1500, 11008, "many-token kernel"),  # 11.0, 13.9
+    (11, 1444, 9472, "many-token kernel"),  # 10.6, 12.8
+    (16, 57344, 8192, "many-token kernel"),  # 88, 96
+    (16, 700, 256, "many-token kernel"),  # 3.3, 4.1
+    (13, 512, 3584, "tcgen05 GEMV"),
+    (9, 545, 768, "tcgen05 GEMV"),  # 5.7, 4.2
+    (13, 3584, 3584, "tcgen05 GEMV"),  # 9.4, 7.8
+    (13, 10240, 8192, "tcgen05 GEMV"),  # 24.6, 19.2
+    (13, 14336, 4096, "tcgen05 GEMV"),  # 17.6, 14.6
+    (13, 37888, 3584, "tcgen05 GEMV"),  # 25.9, 21.7
+    (16, 3584, 18944, "tcgen05 GEMV"),  # 20.8, 18.1
+])
+def test_rule_takes_the_shorter_kernel(kernels, M, N, K, kernel):
+    assert kernels.gemv_describe(M, N, K, 128).startswith(kernel)
