@@ -193,10 +193,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   const int ksplit = split ? p.tail_ks : 1;
   const int m0 = (tile % p.tiles_x) * (128 * MI);
   const int n0 = (tile / p.tiles_x) * kBN;
-  // this CTA's share of the K blocks
+  // this CTA's share of the K blocks, never empty: at most eight splits of at least eight blocks each
   const int kb_per = (p.nkb + ksplit - 1) / ksplit;
   const int kb0 = tail_z * kb_per;
-  const int nkb = max(0, min(p.nkb, kb0 + kb_per) - kb0);
+  const int nkb = min(p.nkb, kb0 + kb_per) - kb0;
 
   if (tid == 0) {
     *abort_flag = 0;
@@ -312,14 +312,6 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
           if (++s == geo::kStages) { s = 0; ph ^= 1; }
           if (++b == geo::kBdCount) { b = 0; bph ^= 1; }
         }
-        if (nkb == 0 && elect_one()) {  // a split with no K blocks
-          if constexpr (PAIR) {
-            umma_commit_pair(bar_acc);
-            umma_commit_pair(peer_base + (bar_acc - base));
-          } else {
-            umma_commit(bar_acc);
-          }
-        }
       }
       __syncwarp();
     } else {
@@ -424,13 +416,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       const int ntiles = p.n_tail, tile_id = tail_t;
       for (int c0 = col_begin; c0 < col_end; c0 += 32) {
         uint32_t v[32];
-        if (nkb > 0) {
-          tmem_ld_32x32(tmem_base + (uint32_t(quad * 32) << 16) + uint32_t(mi * kBN + c0), v);
-          tmem_ld_wait();
-        } else {
-#pragma unroll
-          for (int e = 0; e < 32; ++e) v[e] = 0u;  // a split with no K blocks contributes zeros
-        }
+        tmem_ld_32x32(tmem_base + (uint32_t(quad * 32) << 16) + uint32_t(mi * kBN + c0), v);
+        tmem_ld_wait();
         if (parts) {
           // fp32 partial of this (split, tile), stored column-major inside the tile (row fastest): for a given
           // column the 32 lanes of a warp write 32 consecutive floats
