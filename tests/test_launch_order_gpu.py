@@ -107,3 +107,41 @@ def test_a_plain_launch_runs_the_same_kernel(kernels, M, N, K, G):
     x, (Wq, S) = rand_x(M, K, gen), rand_w4(N, K, G, gen)
     assert torch.equal(kernels.w4_linear(x, Wq, S, G, flags=FLAG_NO_PDL), kernels.w4_linear(x, Wq, S, G))
     assert kernels.device_status() == 0
+
+
+@pytest.mark.parametrize("M,G", [(1, 128), (4, 128), (13, 128), (16, 128), (4, 64), (16, 32), (48, 128), (300, 64)])
+def test_chain_of_dependent_launches(kernels, M, G):
+    """Linears that read one another's outputs and write into buffers that are still being read, eager and captured: bit for
+    bit the chain with a synchronisation after each launch."""
+    gen = torch.Generator(device="cuda").manual_seed(M)
+    dims = [1024, 2304, 512, 1024, 1024, 3584, 1024]
+    weights = [rand_w4(n, k, G, gen) for k, n in zip(dims, dims[1:])]
+    x = rand_x(M, dims[0], gen)
+    buffers = [torch.zeros(M * max(dims), dtype=torch.bfloat16, device="cuda") for _ in range(2)]
+    kernels.w4_linear(x, *weights[0], G)  # kernels loaded before the capture
+
+    def chain(sync):
+        h = x
+        for i, w in enumerate(weights):
+            y = buffers[i % 2][:M * dims[i + 1]].view(M, dims[i + 1])
+            h = kernels.w4_linear(h, *w, G, out=y)
+            sync()
+        return h
+
+    want = chain(torch.cuda.synchronize).clone()
+    assert bool(want.isfinite().all()) and float(want.float().abs().max()) > 0
+    for _ in range(20):
+        buffers[0].zero_()
+        buffers[1].zero_()
+        assert torch.equal(chain(lambda: None), want)
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        got = chain(lambda: None)
+    for _ in range(20):
+        buffers[0].zero_()
+        buffers[1].zero_()
+        graph.replay()
+        assert torch.equal(got, want)
+    assert kernels.device_status() == 0

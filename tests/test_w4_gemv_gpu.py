@@ -1,9 +1,10 @@
 """GPU parity tests of the decode GEMV (M <= 16) through the C ABI, against the CPU oracle.
 
-Three kernels serve the GEMV.  The streaming kernel (default for one token, and up to four on tall matrices, when
+Four kernels serve the GEMV.  The streaming kernel (default for one token, and up to four on tall matrices, when
 G % 128 == 0 and K % 256 == 0; every M <= 16 with FLAG_STREAM_KERNEL) carries X as block fixed point per (token,
 128-chunk): 32 bits for one and two tokens, 15 bits plus sign above.  The many-token kernel (five to sixteen tokens, two
-to four on a long K; its own tests are in test_w4_gemv_mid_gpu.py) and the ring kernel (everything else, or
+to four on a long K; its own tests are in test_w4_gemv_mid_gpu.py), the tcgen05 kernel (nine to sixteen tokens where it is
+estimated shorter; test_w4_gemv_tc_gpu.py) and the ring kernel (everything else, or
 FLAG_RING_KERNEL) carry it as 16-bit block fixed point (ring kernel: 24 bits with FLAG_WIDE_X, or, with FLAG_FLOAT_X,
 in fp16 on the floating-point mma).
 

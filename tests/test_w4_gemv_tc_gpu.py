@@ -63,6 +63,24 @@ def test_extreme_inputs(kernels):
         check_bf16_output(y[m:m + 1], ref[m:m + 1], SLACK)
 
 
+@pytest.mark.parametrize("y_off,s_off", [(4, 0), (2, 0), (0, 2), (0, 1), (1, 1)])
+def test_alignments(kernels, y_off, s_off):
+    """Y from 8 bytes and S from 4 run this kernel, anything less the kernel that serves it: within the same bounds."""
+    M, N, K = 13, 1000, 1536
+    X, Wq, S = oracle.synth_inputs(M, N, K, 128, seed=6)
+    out = torch.zeros(M * N + 8, dtype=torch.bfloat16, device="cuda")
+    y = out[y_off:y_off + M * N].view(M, N)
+    s = torch.empty(S.size + 8, dtype=torch.bfloat16, device="cuda")[s_off:s_off + S.size].view(*S.shape)
+    s.copy_(bits_to_torch(S))
+    kernels.w4_linear(bits_to_torch(X), u32_to_torch(Wq), s, 128, out=y)
+    torch.cuda.synchronize()
+    assert kernels.device_status() == 0
+    check_bf16_output(torch_to_bits(y), oracle.w4_linear_f32(X, Wq, S, 128), SLACK)
+    assert not out[:y_off].any() and not out[y_off + M * N:].any()
+    if y_off % 4 == 0 and s_off % 2 == 0:
+        assert np.array_equal(torch_to_bits(y), run(kernels, X, Wq, S, FLAG_DECODE_NARROW))
+
+
 # tokens, rows, columns, the kernel that was the shorter one, us of the many-token and of this kernel
 @pytest.mark.parametrize("M,N,K,kernel", [
     (10, 1500, 11008, "many-token kernel"),  # 11.0, 13.9

@@ -50,18 +50,19 @@ def test_ties_round_to_even(kernels):
 
 @pytest.mark.parametrize("G", [32, 64, 128, 256])
 def test_every_significand_and_special_groups(kernels, G):
-    """The division-free rounding against the oracle's division: every pair of bf16 significands at the exponents where
-    w / s can be halfway between two integers, scales at both ends of the range, infinite and nan members, and a word
-    count that fills no block."""
+    """The division-free rounding against the oracle's division: every significand of a group's largest value, which sets s,
+    with every significand of another member at every exponent where w / s can be halfway between two integers (|w| from
+    1/32 of the largest value up), scales at both ends of the range, infinite and nan members, and a word count that fills
+    no block."""
     rng = np.random.default_rng(G)
     rows = []
-    for top in range(128, 256):  # a group's largest value sets s; the other members run through the significands
-        w = np.arange(128, 256, dtype=np.float64) * 2.0 ** rng.integers(-5, 1, 128) * rng.choice([-1, 1], 128)
-        w[np.abs(w) > 2 * top] /= 4
-        for part in w.reshape(-1, 32):
-            g = np.resize(part, G).copy()
-            g[rng.integers(0, G)] = top * 2.0
-            rows.append(g)
+    for top in range(128, 256):
+        w = (np.arange(128, 256, dtype=np.float64)[:, None] * 2.0 ** np.arange(-5, 1)).reshape(-1)
+        w = w[w <= top] * rng.choice([-1, 1], (w <= top).sum())
+        for i in range(0, len(w), G - 1):
+            g = np.resize(w[i:i + G - 1], G)
+            g[G - 1] = top  # (np.resize wraps round: the last member of a full part is a repeat of its first)
+            rows.append(rng.permutation(g))
     W = oracle.f32_to_bf16_bits(np.array(rows, dtype=np.float32))
     halves = (np.array(rows) * 0 + rng.integers(-14, 15, (len(rows), G)) / 2)  # s = 1: every second one is a tie
     halves[:, 0] = 7.0
