@@ -36,7 +36,8 @@ extern "C" {
  * Y[M,N] (bf16) = X[M,K] (bf16) . dequant(Wq, S)^T, fp32 accumulation, one rounding to bf16 at the store.
  * Replaces ns_w4_linear, csrc/nanoserve_ops.cu:75-90.  The reference serves M in {1,2,4,8} (GEMV) and
  * M % 128 == 0 with N % 128 == 0 (GEMM) and returns -2 otherwise; this library serves every M >= 1 and
- * every N >= 1: M <= 16 runs the decode GEMV, larger M the tensor-core GEMM.  Needs K % 32 == 0,
+ * every N >= 1: M <= 16 runs a decode GEMV (groups finer than 128 also the few-token GEMM), larger M one of two
+ * tensor-core GEMMs.  Needs K % 32 == 0,
  * G % 32 == 0, K % G == 0 (the reference calls exit() on these inside w4a16.cuh:100-103; this library
  * returns -1 instead).
  */
@@ -66,14 +67,17 @@ int ns_flash_fwd(const void* q, const void* k, const void* v, void* o, int N, in
 /* ---- additions (no counterpart in the reference library) --------------------------------------- */
 
 /*
- * Flags for b2_w4_linear.  Three kernels serve the decode GEMV (M <= 16).  The streaming kernel (G % 128 == 0,
+ * Flags for b2_w4_linear.  Four kernels serve the decode GEMV (M <= 16).  The streaming kernel (G % 128 == 0,
  * K % 256 == 0, Wq 16-byte aligned) runs one token always and two to four tokens on tall matrices with K < 8192; it
  * carries X as block fixed point per (token, 128-wide chunk of K) -- 32 bits for M <= 2 (exact to fp32 summation
  * order), 15 bits + sign above -- on an 8-bit integer mma.  The many-token kernel (G == 128, K % 256 == 0, plain
  * launches) runs five to sixteen tokens, and two to four where K >= 8192, with X as 16-bit block
- * fixed point.  The ring kernel runs everything else, with X as 16-bit block fixed point (every element off by at most
+ * fixed point.  The tcgen05 kernel takes nine to sixteen tokens from it where that is estimated shorter (Y 8-byte aligned;
+ * the same arithmetic).  The ring kernel runs everything else, with X as 16-bit block fixed point (every element off by at most
  * 2^-16 of its chunk's largest magnitude) or as the flags below say.  No kernel measures anything or synchronises:
- * every call is asynchronous.  A K that is cut into slices across CTAs (long K, few rows) is followed by a small
+ * every call is asynchronous.  Groups finer than 128, whose weights the ring kernel rounds to bf16, run the few-token GEMM
+ * instead where that is estimated shorter (X, Wq, Y 16-byte aligned).  More than 16 tokens run the few-token GEMM or the
+ * prefill GEMM, whichever is estimated shorter.  A K that is cut into slices across CTAs (long K, few rows) is followed by a small
  * kernel that adds the slices' fp32 partial sums in fixed order; B2_FLAG_NO_SPLIT_K forbids that.
  */
 #define B2_FLAG_FOLD_ZERO_POINT 1 /* ring kernel with B2_FLAG_FLOAT_X: apply the -8 as one fp32 correction per 128-wide chunk */
@@ -98,6 +102,11 @@ int ns_flash_fwd(const void* q, const void* k, const void* v, void* o, int N, in
 #define B2_FLAG_NO_MID_KERNEL 262144 /* GEMV: never the many-token kernel (2 <= M <= 16, G == 128, K % 256 == 0, plain launches) */
 #define B2_FLAG_MID_KERNEL (131072 | 524288) /* GEMV (both kernel flags): the many-token kernel for every shape it can serve */
 #define B2_FLAG_STREAM_KERNEL 524288 /* GEMV: the streaming kernel for every M <= 16 it can serve */
+#define B2_FLAG_DECODE_NARROW (-2147483647 - 1) /* bit 31, M <= 16: the tcgen05 GEMV where its shapes allow, else the few-token
+                                           GEMM; bits 20-25 as for B2_FLAG_GEMM_NARROW */
+#define B2_FLAG_GEMM_NARROW 268435456 /* M > 16: the few-token GEMM; bits 20-23: CTAs per cluster along K (1-8), bits 24-25: tile
+                                           (1: 128 rows, 2: 256), 0 = the rule decides */
+#define B2_FLAG_GEMM_WIDE 134217728 /* M > 16: never the few-token GEMM */
 #define B2_FLAG_GEMM_NO_PAIRS 536870912 /* prefill GEMM: no clusters of two CTAs (by default two CTAs on neighbouring token
                                            tiles unpack half of the weight tile each, for both) */
 #define B2_FLAG_GEMM_WHOLE_TILES 1073741824 /* prefill GEMM (M > 16): every CTA takes whole output tiles; by default the CTAs
@@ -204,17 +213,6 @@ int b2_w4_gemv_noalloc(const void* X, const void* Wq, const void* S, void* Y, in
  *   b2_greedy_next: token = argmax(logits[0..V)) (lowest index on ties); out_tokens[*step] = token; *step += 1;
  *     *pos += 1; x_next[0..H) = embed[token].  pos, step: int32 on the device; out_tokens: int64 on the device.
  */
-/*
- * The prompt's counterparts: between the q|k|v projection and attention, and between gate|up and down.
- *   b2_qkv_prefill: qkv [T, (Hq+2Hk)*D] bf16, positions 0..T-1: += bias (may be NULL), rotate-half RoPE on q (in place)
- *     and k, k and v written to cache_k / cache_v [Hk, max_len, D] (the row's own k and v are left as they were).
- *     T <= max_len, D % 16 == 0.
- *   b2_swiglu_blocks: out [T, I] = silu(gate) * up with gu [T, 2 I] = `block` gate columns, their `block` up columns,
- *     the next `block` gate columns ... (block % 8 == 0, I % block == 0); ns_swiglu's arithmetic.
- */
-int b2_qkv_prefill(void* qkv, const void* bias, const void* inv_freq, void* cache_k, void* cache_v, int T, int Hq,
-                   int Hk, int D, int max_len, void* stream);
-int b2_swiglu_blocks(const void* gu, void* out, int T, int I, int block, void* stream);
 int b2_rope_kv_store(void* qkv, const void* bias, const void* inv_freq, const void* pos, void* cache_k, void* cache_v,
                      int Hq, int Hk, int D, int max_len, void* stream);
 int b2_decode_attention(const void* q, const void* cache_k, const void* cache_v, const void* pos, void* out,
@@ -226,6 +224,20 @@ int b2_decode_attention_fused(const void* qkv, const void* bias, const void* inv
                               const b2_tp_desc* tp, int flags, void* stream);
 int b2_greedy_next(const void* logits, int V, const void* embed, int H, void* pos, void* out_tokens, void* step,
                    void* x_next, void* workspace, void* stream);
+
+/*
+ * The same for a prompt (no counterpart in the reference library): between the q|k|v projection and attention, and between
+ * gate|up and down.
+ *   b2_qkv_prefill: qkv [T, (Hq+2Hk)*D] bf16, positions 0..T-1: += bias (may be NULL), rotate-half RoPE on q (in place)
+ *     and k, k and v written to cache_k / cache_v [Hk, max_len, D] (the row's own k and v are left as they were).
+ *     T <= max_len, D % 16 == 0.
+ *   b2_swiglu_blocks: out [T, I] = silu(gate) * up with gu [T, 2 I] = `block` gate columns, their `block` up columns,
+ *     the next `block` gate columns ... (block % 8 == 0, I % block == 0); ns_swiglu's arithmetic.
+ */
+int b2_qkv_prefill(void* qkv, const void* bias, const void* inv_freq, void* cache_k, void* cache_v, int T, int Hq,
+                   int Hk, int D, int max_len, void* stream);
+int b2_swiglu_blocks(const void* gu, void* out, int T, int I, int block, void* stream);
+
 /*
  * The bf16 vocabulary projection of a decode step with the greedy argmax in its epilogue.  No counterpart in the
  * reference library: the reference runs F.linear on the bf16 lm_head and argmax over the logits on the host side of
