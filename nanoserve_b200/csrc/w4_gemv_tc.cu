@@ -1,27 +1,32 @@
-// W4A16 decode GEMV on the fifth-generation tensor cores, nine to sixteen tokens, groups of 128:
+// W4A16 decode GEMV on the fifth-generation tensor cores, two to sixteen tokens, groups of 128:
 // Y[M,N] (bf16) = X[M,K] (bf16) . dequant(Wq, S)^T with exact weights.
 //
-// The arithmetic is that of w4_gemv_mid.cu: nibbles as signed bytes 16 (q - 8), X as block fixed point per (token,
-// 128-chunk) in an unsigned low and a signed high byte plane, integer products, one conversion to float and one fused
-// multiply-add per (row, token, chunk).  There the products run on mma.sync and the loop is bound by shared-memory reads of
-// X's fragments and by issue slots.  Here they run on tcgen05.mma (kind::i8) in the frame of w4_gemm_narrow.cu:
-//   * 128 weight rows are the M side; the bytes go from registers to tensor memory (three instructions per eight
-//     weights; a thread owns a row) and the MMA reads them there.  The byte order the nibble masks give is the order X is
-//     stored in: the contraction index is a dummy;
-//   * the planes of the CTA's K range stay in shared memory as the N side, 16 token columns each, read by the tensor core
-//     only;
-//   * a step is one chunk.  Its integer sums start at zero and a group of warps converts and scales them while the next
-//     step's products run: the wait for its buffer of bytes is also the wait for the sums of that buffer's last use;
-//   * K is cut over a cluster and summed through distributed shared memory in rank order (no second launch).
-// Measured at 13 tokens against the mma.sync kernel, weights from HBM, us: 37888 x 3584 21.7 (25.9), 3584 x 18944 18.1
-// (20.8), 3584 x 3584 7.8 (9.4), 10240 x 8192 19.2 (24.6), 14336 x 4096 14.6 (17.6).  What bounds it: about 0.6 us per step
-// of 256 rows, the chain of a group's waits, TMEM stores and loads and 16 int-to-float conversions per row.  One product
-// instruction for both planes (the high one offset to unsigned, corrected by the rows' weight sums) was 5 % slower.
+// The arithmetic is that of the mma.sync kernels: nibbles as signed bytes 16 (q - 8), X as block fixed point per (token,
+// 128-chunk) in byte planes -- 16 bits above four tokens, 32 up to four --, integer products, one conversion to float per joined
+// pair of planes and one fused multiply-add per (row, token, chunk).  Here the products run on tcgen05.mma (kind::i8):
+//   * 128 weight rows are the M side; the bytes go from registers to tensor memory (three instructions per eight weights; a
+//     thread owns a row) and the MMA reads them there.  The byte order the nibble masks give is the order X is stored in: the
+//     contraction index is a dummy.  The planes' sixteen rows of bytes (signed, unsigned) are the N side;
+//   * X is converted chunk by chunk by warps of its own, ahead of the products, into a ring in shared memory.  (Converted whole
+//     before the first product it took 1 to 2 us that did not overlap, and its size forced K into clusters.);
+//   * a hand-over is a pair of chunks, K = 256.  Two groups of warps take the pairs in turn: while one group's products run the
+//     other converts words, and each reads and scales its sums when it comes back for its buffer;
+//   * K is cut over a cluster.  A CTA sends its sums into the shared memory of the CTA that adds them, in the order of ranks and
+//     groups (no second launch, one cluster barrier behind the sums).
+// What bounds it: from the wait for the kernel in front to the last pair it runs at HBM's rate (37888 x 3584 at four tokens: 10.4
+// of 15.9 us for 70 MB); the rest is the boundary between launches (1.7 us), barriers and tensor memory before it (0.7), the
+// last sums and stores (1.3).  What the pairs are for: asking a barrier takes a warp some 130 cycles even where the answer is
+// yes, an arrival with its fence 100, and a chunk at a time with one group (0.55 us per chunk of 256 rows, HBM 0.37) these were
+// most of a step.  Measured, weights from HBM, us at 4 / 8 / 13 tokens, in brackets the shortest of the mma.sync kernels and, at
+// 13, this kernel before (a chunk per step, X converted first): 37888 x 3584 15.9 / 16.5 / 18.1 (15.8 / 19.3 / 21.5), 3584 x
+// 18944 12.9 / 13.4 / 14.7 (15.0 / 16.2 / 18.2), 3584 x 3584 5.6 / 5.8 / 6.5 (7.5 / 6.8 / 8.2), 8192 x 28672 28 / 30 / 34 (41 / 42
+// / 50), 57344 x 8192 56 / 59 / 68 (59 / 60 / 89).
 // Every wait is bounded; a CTA that gives up records a status, still takes part in the cluster barriers and frees its TMEM.
 #include <cuda.h>
 
 #include <algorithm>
 #include <atomic>
+#include <cmath>
 #include <cstdio>
 
 #include "ptx.cuh"
@@ -32,14 +37,14 @@
 namespace b2 {
 namespace {
 
-constexpr int kStepK = 128;
-constexpr int kMaxSlots = 8;
-constexpr int kTokens = 16;
-constexpr int kHeaderBytes = 1024;
-constexpr int kXStep = 2 * kTokens * 128;   // bytes of a step's two planes
-constexpr int kInfoStep = kTokens * 4;      // and of its factors
-constexpr int kSmemHalf = 115712, kSmemFull = 232448;
-constexpr int kBufs = 2;      // bytes and sums of two steps in TMEM, one per group of warps (two each were no faster)
+constexpr int kStepK = 128, kTokens = 16;
+constexpr int kWSlot = 128 * 128;          // packed words: 128 rows, K = 256
+constexpr int kXStep = 2 * 16 * 128;       // operand of a step: sixteen rows of unsigned bytes, sixteen of signed ones
+constexpr int kXAhead = 2;                 // items of X a warp has in flight
+constexpr int kBarOffset = 64;             // barriers of the rings; one per slot of X at kSlotBars
+constexpr int kSlotBars = 512;
+constexpr int kMaxPairs = 256;             // slots (pairs of steps) of a CTA
+constexpr int kSmemHalf = 115712, kSmemFull = 232448;  // (228 KB / 2) - 1 KB, 227 KB
 
 struct TcParams {
   const __nv_bfloat16* S;
@@ -47,11 +52,11 @@ struct TcParams {
   __nv_bfloat16* Y;
   int* status;
   int M, N, K, KG;
-  int nkb;      // steps of 128
-  int ks;       // CTAs of a cluster, each with its share of the steps
-  int sw;       // ring slots of packed words (K = 256 each)
-  int off_x;    // planes, then factors, behind the ring
-  int off_info;
+  int pairs;    // of steps of 128
+  int ks;       // CTAs of a cluster, each with its share of the pairs
+  int sw, sx;   // ring slots of a pair: packed words (per block of 128 rows), X
+  int ahead;    // slots of packed words that are brought into L2 ahead of the ring
+  int off_w, off_x, off_info, off_red;
 };
 
 __device__ __forceinline__ void umma_i8_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc,
@@ -68,45 +73,89 @@ __host__ __device__ constexpr uint32_t umma_idesc_s8(int b_signed, int M, int N)
   return (2u << 4) | (1u << 7) | (static_cast<uint32_t>(b_signed) << 10) | (static_cast<uint32_t>(N >> 3) << 17) |
          (static_cast<uint32_t>(M >> 4) << 24);
 }
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+__device__ __forceinline__ void st_cluster_f32(uint32_t addr, uint32_t rank, float v) {
+  asm volatile(
+      "{\n\t.reg .u32 a;\n\t"
+      "mapa.shared::cluster.u32 a, %0, %1;\n\t"
+      "st.shared::cluster.f32 [a], %2;\n\t}" ::"r"(addr), "r"(rank), "f"(v)
+      : "memory");
+}
+template <int N>
+__device__ __forceinline__ void regs_up() {
+  asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N));
+}
+template <int N>
+__device__ __forceinline__ void regs_down() {
+  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
+}
+// The sums of a step: unsigned planes' columns from column 0, the signed plane's from column 16.
+template <int LO>
+__device__ __forceinline__ void tmem_ld_sums(uint32_t taddr, uint32_t (&d)[32]) {
+  tmem_ld_32x32(taddr, d);
+}
+template <int LO>
+__device__ __forceinline__ void tmem_ld_sums(uint32_t taddr, uint32_t (&d)[16]) {
+  tmem_ld_32x8(taddr, d);
+  if constexpr (LO == 8) {
+    tmem_ld_32x8(taddr + 16, d + 8);
+  } else {
+    tmem_ld_32x4(taddr + 8, d + 8);
+    tmem_ld_32x4(taddr + 16, d + 12);
+  }
+}
 
-// MB: blocks of 128 weight rows per tile.  DW: conversion warps, two groups of 4 MB that take the steps in turn.
-// SV: scales per load.
-template <int MB, int DW, int MINB, int SV>
-__global__ void __launch_bounds__(128 + DW * 32, MINB)
+// All questions of a pair of steps in one go: asking a barrier takes some 100 cycles, complete or not, and one after the
+// other they add up.
+__device__ __forceinline__ bool mbar_try_wait2(uint32_t bar0, uint32_t parity0, uint32_t bar1, uint32_t parity1) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 q, [%3], %4;\n\t"
+      "and.pred p, p, q;\n\t"
+      "selp.b32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(bar0), "r"(parity0), "r"(bar1), "r"(parity1)
+      : "memory");
+  return ok != 0;
+}
+
+// MT: token columns (4, 8 or 16).  Four and fewer tokens keep X in 32 bits (three unsigned planes and a signed one), more
+// in 16 (one and one).  MB: blocks of 128 weight rows.  SV: scales per load.
+template <int MB, int MT, int SV>
+__global__ void __launch_bounds__(MB == 2 ? 896 : 512, MB == 2 ? 1 : 2)
     w4_gemv_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const TcParams p) {
-  constexpr int kRows = MB * 128, kWSlot = kRows * 128, kThreads = DW * 32;
-  constexpr int kTmemCols = 256;  // 128 or 256 used; see the launch
-  static_assert(DW == 8 * MB, "two groups of warps");
+  constexpr int P = MT == 4 ? 4 : 2;
+  constexpr int kLo = MT * (P - 1), kCols = MT * P;  // columns of a row's sums: unsigned planes, then the signed one
+  constexpr int kRows = MB * 128, kMain = 8 * MB, kBlocks = kRows / 32, kTmemCols = 256 * MB;
+  constexpr int kWarps = MB == 2 ? 28 : 16, kXWarps = 4 * MB;
+  constexpr int kWarpW = kMain + kXWarps, kWarpMma = kWarpW + 1;
   extern __shared__ unsigned char smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   unsigned char* gen = smem_raw + (base - smem_u32(smem_raw));
-  const uint32_t bar_w_full = base, bar_w_empty = base + 8 * kMaxSlots, bar_a_full = base + 16 * kMaxSlots;
-  const uint32_t bar_a_empty = bar_a_full + 8 * kBufs, bar_acc = bar_a_empty + 8 * kBufs, bar_x = bar_acc + 8;
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(gen + 512);
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gen + 516);
-  const uint32_t ring_w = base + kHeaderBytes, xs = base + p.off_x, info = base + p.off_info;
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(gen);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gen + 4);
+  const uint32_t bar_w_full = base + kBarOffset, bar_w_empty = bar_w_full + 8 * 8;  // [block][slot], at most 4 slots
+  const uint32_t bar_a_full = bar_w_empty + 8 * 8, bar_a_empty = bar_a_full + 8 * 4;  // [block][group]
+  const uint32_t bar_x_empty = bar_a_empty + 8 * 4;                                   // [slot], at most 16
+  const uint32_t bar_x_full = base + kSlotBars;                                       // [pair]
+  const uint32_t ring_w = base + p.off_w, ring_x = base + p.off_x, info = base + p.off_info, red = base + p.off_red;
 
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const int crank = p.ks > 1 ? (int)cluster_rank() : 0;
   const int n0 = (blockIdx.x / p.ks) * kRows;
-  const int kb0 = (int)((long)crank * p.nkb / p.ks), nkb = (int)((long)(crank + 1) * p.nkb / p.ks) - kb0;
+  const int pr0 = (int)((long)crank * p.pairs / p.ks), np = (int)((long)(crank + 1) * p.pairs / p.ks) - pr0;
+  const int groups = (p.M + 3) >> 2;  // of four tokens: one warp's piece of a step's X
 
-  if (tid == 0) {
-    *abort_flag = 0;
-    for (int s = 0; s < kMaxSlots; ++s) {
-      mbar_init(bar_w_full + 8 * s, 1);
-      mbar_init(bar_w_empty + 8 * s, DW);
-    }
-    for (int b = 0; b < kBufs; ++b) {
-      mbar_init(bar_a_full + 8 * b, 4 * MB);
-      mbar_init(bar_a_empty + 8 * b, 1);
-    }
-    mbar_init(bar_acc, 1);
-    mbar_init(bar_x, 1);
-    fence_mbar_init();
-    tma_prefetch_desc(&tmap_w);
-  }
-  if (warp == 1) {
+  for (int i = tid; i < np; i += kWarps * 32) mbar_init(bar_x_full + 8 * i, 2 * groups);
+  // (the barriers of the rings lie one behind the other: 8 + 8 + 4 + 4 + 16)
+  if (tid < 40) mbar_init(base + kBarOffset + 8 * tid, tid < 8 ? 1 : tid < 20 ? 4 : tid < 24 ? 1 : MB);
+  if (tid == 0) *abort_flag = 0;
+  fence_mbar_init();
+  if (warp == kWarpW && lane == 0) tma_prefetch_desc(&tmap_w);
+  if (warp == kWarpMma) {
     tmem_alloc(smem_u32(tmem_slot), kTmemCols);
     tmem_relinquish();
   }
@@ -114,61 +163,21 @@ __global__ void __launch_bounds__(128 + DW * 32, MINB)
   __syncthreads();
   tc_fence_after_sync();
   pdl_launch_dependents();
-  const uint32_t tmem_d = __shfl_sync(0xffffffffu, *tmem_slot, 0);  // [buffer][block][low 16 | high 16] columns
-  const uint32_t tmem_a = tmem_d + kBufs * MB * 32;                   // [buffer][block][32] columns
+  if (p.ks > 1) cluster_arrive();  // (waited for before the first store into a peer: it runs by then)
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);  // [block][group]: 64 columns of sums, 64 of bytes
   const bool poisoned = *reinterpret_cast<volatile int*>(p.status) != 0;
 
+  // The rows' warps need more registers than an even share.  256 rows, 896 threads of 72: 4 x 88 + 2 x 48 + 56 = 7 x 72 by
+  // warpgroup; 128 rows, 512 of 64: 2 x 80 + 2 x 48 = 4 x 64.
+  if (warp < kMain) regs_up<MB == 2 ? 88 : 80>();
+  else if (warp < kWarpW) regs_down<48>();
+  else regs_down<MB == 2 ? 56 : 48>();
   if (!poisoned) {
-    if (warp == 0) {
-      if (lane == 0) {
-        // The kernel in front may be the one that writes the weights: until it has finished they are only brought into
-        // L2 (two slots; sixteen launches of a decoder stack at 13 tokens, us: 226, one slot 227, the whole ring 229,
-        // nothing 231, the ring filled before the wait 224).
-        for (int i = 0; i < nkb && i < 4; i += 2) tma_prefetch_2d(&tmap_w, (kb0 + i) * (kStepK / 8), n0);
-        pdl_wait_prior_grid();
-        int s = 0;
-        uint32_t ph = 1;
-        for (int i = 0; i < nkb; i += 2) {
-          mbar_wait(bar_w_empty + 8 * s, ph, abort_flag);
-          mbar_arrive_expect_tx(bar_w_full + 8 * s, kWSlot);
-          tma_load_2d(ring_w + s * kWSlot, &tmap_w, (kb0 + i) * (kStepK / 8), n0, bar_w_full + 8 * s);
-          if (++s == p.sw) { s = 0; ph ^= 1; }
-        }
-      }
-      __syncwarp();
-    } else if (warp == 1) {
-      constexpr uint32_t id_lo = umma_idesc_s8(0, 128, kTokens), id_hi = umma_idesc_s8(1, 128, kTokens);
-      const uint64_t desc0 = umma_desc_k128(xs);
-      pdl_wait_prior_grid();  // the kernel in front may run longer than a bounded wait for X
-      mbar_wait(bar_x, 0, abort_flag);
-      for (int i = 0; i < nkb; ++i) {
-        const int buf = i % kBufs;
-        mbar_wait(bar_a_full + 8 * buf, (i / kBufs) & 1, abort_flag);
-        __syncwarp();
-        tc_fence_after_sync();
-        const uint64_t db = desc0 + i * (kXStep >> 4);
-        const uint32_t a = tmem_a + buf * MB * 32, d = tmem_d + buf * MB * 32;
-        if (elect_one()) {
-#pragma unroll
-          for (int kk = 0; kk < 4; ++kk) {
-#pragma unroll
-            for (int mb = 0; mb < MB; ++mb) {
-              umma_i8_ts(d + mb * 32, a + mb * 32 + kk * 8, db + kk * 2, id_lo, kk > 0 ? 1u : 0u);
-              umma_i8_ts(d + mb * 32 + 16, a + mb * 32 + kk * 8, db + (kTokens * 128 >> 4) + kk * 2, id_hi,
-                         kk > 0 ? 1u : 0u);
-            }
-          }
-          umma_commit(bar_a_empty + 8 * buf);
-          if (i + 1 == nkb) umma_commit(bar_acc);
-        }
-        __syncwarp();
-      }
-    } else if (warp >= 4) {
-      const int dw = warp - 4, quad = warp & 3;  // the quarter of the TMEM lanes this warp may touch
-      const int mb = (dw >> 2) % MB, grp = dw / (4 * MB);
-      const int row = mb * 128 + quad * 32 + lane, n = n0 + row, ct = tid - 128;
+    if (warp < kMain) {
+      // ---- the rows: words -> bytes in TMEM; sums of a step -> registers.  Two groups of warps take the pairs in turn.
+      const int quad = warp & 3, mb = (warp >> 2) % MB, grp = warp / (4 * MB);
+      const int row = mb * 128 + quad * 32 + lane, n = n0 + row;  // (a warp may touch a quarter of the TMEM lanes)
       const bool live = n < p.N;
-      const uint32_t lane_off = (uint32_t)(quad * 32) << 16;
       const __nv_bfloat16* s_row = p.S + (size_t)(live ? n : 0) * p.KG;
       auto load_sv = [&](int v) {
         uint2 r = make_uint2(0u, 0u);
@@ -178,238 +187,428 @@ __global__ void __launch_bounds__(128 + DW * 32, MINB)
         }
         return r;
       };
-      int g = kb0 + grp;
-      if (live && g < p.KG) prefetch_l2(s_row + g);
+      int g = 2 * (pr0 + grp);  // the pair's first step: even
+      if (live) prefetch_l2(s_row + g);
       pdl_wait_prior_grid();
-      uint2 cur = load_sv(g / SV), nxt = load_sv(g / SV + 1);
-      const uint32_t pick = g & 1 ? 0x7632 : 0x5410;  // the odd or the even scale of a pair, as the high half of a float
-
-      // ---- X: 16 consecutive k of a token per item, the eight items of a chunk in eight consecutive lanes; the largest
-      // magnitude of a (token, chunk) is scaled to below 2^15, its values are rounded to 16-bit integers (the low mantissa
-      // bits of x * 2^.. + 1.5 * 2^23) and split into bytes, in the order the nibble masks produce.
-      {
-        constexpr int UN = 4;
-        const int per_tok = nkb * 8, items = kTokens * per_tok;
-        for (int it0 = ct; it0 < items; it0 += kThreads * UN) {  // (items and threads: multiples of 32)
-          uint4 va[UN], vb[UN];
+      // SV == 4: two pairs, this group's one of them; SV == 2: one
+      auto pair_scales = [&](int step) {
+        const uint2 v = load_sv(step / SV);
+        return SV == 4 && (step & 2) ? v.y : v.x;
+      };
+      uint32_t cur = pair_scales(g), nxt = pair_scales(g + 4);
+      const uint32_t slot0 = ring_w + mb * p.sw * kWSlot + (quad * 32 + lane) * 128, swz = (uint32_t)lane & 7u;
+      const uint32_t d_src = tmem + ((uint32_t)(quad * 32) << 16) + (mb * 2 + grp) * 128, a_dst = d_src + 64;
+      const uint32_t b_wf = bar_w_full + 32 * mb, b_we = bar_w_empty + 32 * mb;
+      const uint32_t b_af = bar_a_full + 8 * (mb * 2 + grp), b_ae = bar_a_empty + 8 * (mb * 2 + grp);
+      float acc[MT];
 #pragma unroll
-          for (int u = 0; u < UN; ++u) {
-            const int it = it0 + u * kThreads, m = it / per_tok, r = it - m * per_tok;
-            va[u] = vb[u] = make_uint4(0u, 0u, 0u, 0u);
-            if (it < items && m < p.M) {
-              const uint4* src = reinterpret_cast<const uint4*>(p.X + (size_t)m * p.K + (size_t)kb0 * kStepK + r * 16);
-              va[u] = __ldcg(src);
-              vb[u] = __ldcg(src + 1);
+      for (int e = 0; e < MT; ++e) acc[e] = 0.f;
+      // the sums of a step: planes joined as integers, one conversion per pair, then scale times the token's factor
+      auto add_step = [&](int step, float scale) {
+        uint32_t d[kCols];
+        tmem_ld_sums<kLo>(d_src + (step & 1) * 32, d);
+        tmem_ld_wait();
+        const float2 scale2 = make_float2(scale, scale);
+#pragma unroll
+        for (int q = 0; q < MT / 4; ++q) {
+          const uint4 f = lds128(info + (step * MT + q * 4) * 4);
+          const float2 ff[2] = {make_float2(__uint_as_float(f.x), __uint_as_float(f.y)),
+                                make_float2(__uint_as_float(f.z), __uint_as_float(f.w))};
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            float v[2];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              const int t = q * 4 + h * 2 + e;
+              v[e] = (float)((int)d[t] + ((int)d[MT + t] << 8));
+              if constexpr (P == 4)
+                v[e] = fmaf((float)((int)d[2 * MT + t] + ((int)d[3 * MT + t] << 8)), 65536.f, v[e]);
             }
+            float2 a = make_float2(acc[q * 4 + h * 2], acc[q * 4 + h * 2 + 1]);
+            a = fma_f32x2(mul_f32x2(scale2, ff[h]), make_float2(v[0], v[1]), a);
+            acc[q * 4 + h * 2] = a.x;
+            acc[q * 4 + h * 2 + 1] = a.y;
           }
-#pragma unroll
-          for (int u = 0; u < UN; ++u) {
-            const int it = it0 + u * kThreads, m = it / per_tok, r = it - m * per_tok;
-            if (it < items) {  // (warp-uniform)
-              const uint32_t w[8] = {va[u].x, va[u].y, va[u].z, va[u].w, vb[u].x, vb[u].y, vb[u].z, vb[u].w};
-              uint32_t mx2 = 0;
-#pragma unroll
-              for (int i = 0; i < 8; ++i) mx2 = __vmaxu2(mx2, w[i] & 0x7FFF7FFFu);
-              uint32_t mx = max(mx2 & 0xFFFFu, mx2 >> 16);
-              mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
-              mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
-              mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
-              uint32_t eb = mx >> 7;
-              const bool bad = eb == 255u;
-              eb = min(254u, max(40u, eb));
-              const float down = __uint_as_float((uint32_t)(16 + 252 - (int)eb) << 23);
-              uint32_t v[16];
-#pragma unroll
-              for (int i = 0; i < 8; ++i) {
-                v[2 * i] = __float_as_uint(fmaf(__uint_as_float(w[i] << 16), down, 12582912.f));
-                v[2 * i + 1] = __float_as_uint(fmaf(__uint_as_float(w[i] & 0xFFFF0000u), down, 12582912.f));
-              }
-              const uint32_t at = xs + (r >> 3) * kXStep + m * 128 + (((uint32_t)r ^ (uint32_t)m) & 7u) * 16;
-#pragma unroll
-              for (int pl = 0; pl < 2; ++pl) {
-                uint32_t o[4];
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                  const int b = (j & 1) * 8 + (j >> 1);  // first k of the word: 0, 8, 1, 9; then every second one
-                  const uint32_t t0 = __byte_perm(v[b], v[b + 2], 0x5140), t1 = __byte_perm(v[b + 4], v[b + 6], 0x5140);
-                  o[j] = __byte_perm(t0, t1, pl ? 0x7632 : 0x5410);
-                }
-                sts128(at + pl * kTokens * 128, make_uint4(o[0], o[1], o[2], o[3]));
-              }
-              if ((r & 7) == 0)
-                asm volatile("st.shared.b32 [%0], %1;" ::"r"(info + (r >> 3) * kInfoStep + m * 4),
-                             "r"(bad ? 0x7FC00000u : (uint32_t)((int)eb - 18) << 23)
-                             : "memory");
-            }
-          }
-        }
-      }
-      fence_proxy_async_smem();
-      asm volatile("bar.sync 1, %0;" ::"r"(kThreads) : "memory");
-      if (ct == 0) mbar_arrive(bar_x);
-
-      // ---- steps
-      const uint32_t src_row = ring_w + row * 128, swz = (uint32_t)row & 7u;
-      uint32_t src_off[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) src_off[j] = src_row + (((uint32_t)(grp * 4 + j) ^ swz) << 4);
-      const uint32_t a_dst = tmem_a + lane_off + mb * 32, d_src = tmem_d + lane_off + mb * 32;
-      float acc[kTokens];
-#pragma unroll
-      for (int e = 0; e < kTokens; ++e) acc[e] = 0.f;
-      // the sums of step i: lo + 256 hi exactly, then scale times the token's factor
-      uint32_t d[32];
-      auto add_step = [&](int i, float scale) {
-#pragma unroll
-        for (int q = 0; q < kTokens / 4; ++q) {
-          const uint4 f = lds128(info + i * kInfoStep + q * 16);
-          const float ff[4] = {__uint_as_float(f.x), __uint_as_float(f.y), __uint_as_float(f.z), __uint_as_float(f.w)};
-#pragma unroll
-          for (int e = 0; e < 4; ++e)
-            acc[4 * q + e] = fmaf(scale * ff[e], (float)((int)d[4 * q + e] + ((int)d[16 + 4 * q + e] << 8)), acc[4 * q + e]);
         }
       };
-      float s_prev = 0.f;
-      int s = 0;
-      uint32_t ph = 0;
-      for (int i = grp; i < nkb; i += 2) {
-        const float scale = __uint_as_float(__byte_perm(0, SV == 4 && (g & 2) ? cur.y : cur.x, pick) & 0xFFFF0000u);
-        if (SV == 2 || (g & 2)) {
-          cur = nxt;
-          nxt = load_sv(g / SV + 2);
-        }
-        g += 2;
-        mbar_wait(bar_w_full + 8 * s, ph, abort_flag);
+      auto add_pair = [&](int i) {
+        add_step(2 * i, __uint_as_float(cur << 16));
+        add_step(2 * i + 1, __uint_as_float(cur & 0xFFFF0000u));
+        cur = nxt;
+        g += 4;
+        nxt = pair_scales(g + 4);
+      };
+      uint4 w[4];  // the packed words of a step
+      auto load_words = [&](uint32_t slot, int half) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) w[j] = lds128(slot + (((uint32_t)(half * 4 + j) ^ swz) << 4));
+      };
+      auto put_words = [&](int half) {
         uint32_t v[32];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          const uint4 w4 = lds128(src_off[j] + s * kWSlot);
-          const uint32_t w[4] = {w4.x, w4.y, w4.z, w4.w};
+          const uint32_t ww[4] = {w[j].x, w[j].y, w[j].z, w[j].w};
 #pragma unroll
           for (int h = 0; h < 2; ++h) {  // two words: their even nibbles, their odd nibbles
-            v[8 * j + 4 * h] = ((w[2 * h] << 4) & 0xF0F0F0F0u) ^ 0x80808080u;
-            v[8 * j + 4 * h + 1] = ((w[2 * h + 1] << 4) & 0xF0F0F0F0u) ^ 0x80808080u;
-            v[8 * j + 4 * h + 2] = (w[2 * h] & 0xF0F0F0F0u) ^ 0x80808080u;
-            v[8 * j + 4 * h + 3] = (w[2 * h + 1] & 0xF0F0F0F0u) ^ 0x80808080u;
+            v[8 * j + 4 * h] = ((ww[2 * h] << 4) & 0xF0F0F0F0u) ^ 0x80808080u;
+            v[8 * j + 4 * h + 1] = ((ww[2 * h + 1] << 4) & 0xF0F0F0F0u) ^ 0x80808080u;
+            v[8 * j + 4 * h + 2] = (ww[2 * h] & 0xF0F0F0F0u) ^ 0x80808080u;
+            v[8 * j + 4 * h + 3] = (ww[2 * h + 1] & 0xF0F0F0F0u) ^ 0x80808080u;
           }
         }
-        const int buf = i % kBufs;
-        mbar_wait(bar_a_empty + 8 * buf, ((i / kBufs) & 1) ^ 1, abort_flag);
-        __syncwarp();
-        tc_fence_after_sync();
-        tmem_st_32x32(a_dst + buf * (MB * 32), v);
-        tmem_st_wait();
-        if (i >= kBufs) {
-          tmem_ld_32x32(d_src + buf * (MB * 32), d);
-          tmem_ld_wait();
+        tmem_st_32x32(a_dst + half * 32, v);
+      };
+      int s = grp;  // (the ring has an even number of slots: a group's slots are its own)
+      uint32_t wph = 0, aph = 1;
+      for (int i = grp; i < np; i += 2) {
+        const uint32_t slot = slot0 + s * kWSlot;
+        // the bytes of the group's last pair have been read and its sums are complete; this pair's words are there
+        const bool ready = mbar_try_wait2(b_ae, aph, b_wf + 8 * s, wph);
+        if (!__all_sync(0xffffffffu, ready)) {
+          mbar_wait(b_ae, aph, abort_flag);
+          mbar_wait(b_wf + 8 * s, wph, abort_flag);
+          __syncwarp();
         }
+        tc_fence_after_sync();
+        load_words(slot, 0);
+        if (i >= 2) {
+          mbar_wait(bar_x_full + 8 * (i - 2), 0, abort_flag);  // (complete: its factors were written before it)
+          __syncwarp();
+          add_pair(i - 2);
+        }
+        put_words(0);
+        load_words(slot, 1);
+        put_words(1);
+        tmem_st_wait();
         tc_fence_before_sync();
         __syncwarp();
-        if (lane == 0) {
-          mbar_arrive(bar_a_full + 8 * buf);
-          mbar_arrive(bar_w_empty + 8 * s);
+        mbar_arrive_if(b_af, lane == 0);
+        mbar_arrive_if(b_we + 8 * s, lane == 0);
+        aph ^= 1;
+        s += 2;
+        if (s >= p.sw) {
+          s -= p.sw;
+          wph ^= 1;
         }
-        if (i >= kBufs) add_step(i - kBufs, s_prev);
-        s_prev = scale;
-        if (++s == p.sw) { s = 0; ph ^= 1; }
       }
-      mbar_wait(bar_acc, 0, abort_flag);
+      if (const int last = np - 1 - ((np - 1 - grp) & 1); last >= 0) {  // the group's last pair
+        mbar_wait(b_ae, aph, abort_flag);
+        mbar_wait(bar_x_full + 8 * last, 0, abort_flag);
+        __syncwarp();
+        tc_fence_after_sync();
+        add_pair(last);
+      }
+      tc_fence_before_sync();
       __syncwarp();
-      tc_fence_after_sync();
-      const int last = nkb - 1 - ((nkb - 1 - grp) & 1);  // the group's last step (below zero: none)
-      if (last >= 0) {
-        tmem_ld_32x32(d_src + (last % kBufs) * (MB * 32), d);
-        tmem_ld_wait();
-        add_step(last, s_prev);
+      if (p.ks == 1) {  // the second group's sums through shared memory
+        float* part = reinterpret_cast<float*>(gen + p.off_red) + (row >> 5) * (MT * 32) + lane;
+        if (grp == 1) {
+#pragma unroll
+          for (int e = 0; e < MT; ++e)
+            if (e < p.M) part[e * 32] = acc[e];
+        }
+        asm volatile("bar.sync %0, 256;" ::"r"(1 + mb) : "memory");
+        if (grp == 0) {
+          __nv_bfloat16* y = p.Y + n;
+#pragma unroll
+          for (int e = 0; e < MT; ++e)
+            if (live && e < p.M) y[(size_t)e * p.N] = __float2bfloat16(acc[e] + part[e * 32]);
+        }
+      } else {
+        // Every part goes to the CTA that sums its block of 32 rows, block * ks / kBlocks of the cluster, which adds the parts
+        // in the order of ranks and groups: [block][rank][group][token][32 rows]
+        const int blk = row >> 5, owner = blk * p.ks / kBlocks, first = (owner * kBlocks + p.ks - 1) / p.ks;
+        const uint32_t at = red + (uint32_t)((((blk - first) * p.ks + crank) * 2 + grp) * MT * 32 + lane) * 4;
+        cluster_wait();
+#pragma unroll
+        for (int e = 0; e < MT; ++e)
+          if (e < p.M) st_cluster_f32(at + e * 128, owner, acc[e]);
       }
-      // [group][token][row], over the ring: every copy has landed
+    } else if (warp < kWarpW) {
+      // ---- X: a warp takes four tokens of a step, a lane 16 consecutive k of a token, the eight lanes of a token side by
+      // side.  The largest magnitude of a (token, step) is scaled to below 2^15 (2^31), its values are rounded to integers
+      // and split into bytes, in the order the nibble masks produce.
+      pdl_wait_prior_grid();
+      constexpr int kGroups = MT / 4, kStride = kXWarps / kGroups;  // steps between a warp's items
+      const int r = lane & 7, m = ((warp - kMain) % kGroups) * 4 + (lane >> 3), steps = 2 * np;
+      const bool mine = ((warp - kMain) % kGroups) < groups, valid = m < p.M;
+      const uint4* src = reinterpret_cast<const uint4*>(p.X + (size_t)(valid ? m : 0) * p.K + (size_t)(2 * pr0) * kStepK + r * 16);
+      uint4 va[kXAhead], vb[kXAhead];  // items in flight
+      auto load = [&](int step, uint4& a, uint4& b) {
+        a = b = make_uint4(0u, 0u, 0u, 0u);
+        if (step < steps && valid) {
+          a = __ldcg(src + step * (kStepK / 8));
+          b = __ldcg(src + step * (kStepK / 8) + 1);
+        }
+      };
+      const int step0 = mine ? (warp - kMain) / kGroups : steps;
 #pragma unroll
-      for (int e = 0; e < kTokens; ++e)
-        asm volatile("st.shared.f32 [%0], %1;" ::"r"(ring_w + (uint32_t)((grp * kTokens + e) * kRows + row) * 4), "f"(acc[e])
-                     : "memory");
-    }
-  }
-  tc_fence_before_sync();
-  __syncwarp();
-  if (p.ks > 1)
-    cluster_barrier();
-  else
-    __syncthreads();
-  // every CTA adds up its share of the tile, four rows of a token per thread, in rank and group order
-  if (warp >= 4 && !poisoned) {
-    const int units = p.M * (kRows / 4), u1 = (int)((long)(crank + 1) * units / p.ks);
-    for (int u = (int)((long)crank * units / p.ks) + tid - 128; u < u1; u += kThreads) {
-      const int tok = u / (kRows / 4), r = (u % (kRows / 4)) * 4, n = n0 + r;
-      const uint32_t at = ring_w + (uint32_t)(tok * kRows + r) * 4;
-      float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int u = 0; u < kXAhead; ++u) load(step0 + u * kStride, va[u], vb[u]);
+      int sl = step0 >> 1;
+      uint32_t xph = 1;
+      for (int step = step0; step < steps; step += kStride) {
+        while (sl >= p.sx) {
+          sl -= p.sx;
+          xph ^= 1;
+        }
+        const uint32_t w[8] = {va[0].x, va[0].y, va[0].z, va[0].w, vb[0].x, vb[0].y, vb[0].z, vb[0].w};
 #pragma unroll
-      for (int z = 0; z < 8; ++z)
-        if (z < p.ks) {
+        for (int u = 0; u + 1 < kXAhead; ++u) {
+          va[u] = va[u + 1];
+          vb[u] = vb[u + 1];
+        }
+        load(step + kXAhead * kStride, va[kXAhead - 1], vb[kXAhead - 1]);
+        const bool room = mbar_try_wait(bar_x_empty + 8 * sl, xph);
+        uint32_t mx2 = 0;
 #pragma unroll
-          for (int h = 0; h < 2; ++h) {
-            const float4 b = ld_cluster_f4(at + h * kTokens * kRows * 4, z);
-            a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
+        for (int i = 0; i < 8; ++i) mx2 = __vmaxu2(mx2, w[i] & 0x7FFF7FFFu);
+        uint32_t mx = max(mx2 & 0xFFFFu, mx2 >> 16);
+        mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 4));
+        mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+        mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+        uint32_t eb = mx >> 7;
+        const bool bad = eb == 255u;
+        eb = min(254u, max(40u, eb));
+        const float down = __uint_as_float((uint32_t)((P == 4 ? 284 : 268) - (int)eb) << 23);
+        uint32_t v[16];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const float lo = __uint_as_float(w[i] << 16), hi = __uint_as_float(w[i] & 0xFFFF0000u);
+          if constexpr (P == 2) {  // the low mantissa bits of x * 2^.. + 1.5 * 2^23
+            v[2 * i] = __float_as_uint(fmaf(lo, down, 12582912.f));
+            v[2 * i + 1] = __float_as_uint(fmaf(hi, down, 12582912.f));
+          } else {
+            v[2 * i] = (uint32_t)__float2int_rn(lo * down);
+            v[2 * i + 1] = (uint32_t)__float2int_rn(hi * down);
           }
         }
-      __nv_bfloat16* y = p.Y + (size_t)tok * p.N + n;
-      if (n + 4 <= p.N && (p.N & 3) == 0) {
-        const __nv_bfloat162 lo = __floats2bfloat162_rn(a.x, a.y), hi = __floats2bfloat162_rn(a.z, a.w);
-        *reinterpret_cast<uint2*>(y) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo),
-                                                  *reinterpret_cast<const uint32_t*>(&hi));
-      } else {
-        const float f[4] = {a.x, a.y, a.z, a.w};
+        if (!room) mbar_wait(bar_x_empty + 8 * sl, xph, abort_flag);
+        if (valid) {
+          const uint32_t at = ring_x + (2 * sl + (step & 1)) * kXStep;
 #pragma unroll
-        for (int e = 0; e < 4; ++e)
-          if (n + e < p.N) y[e] = __float2bfloat16(f[e]);
+          for (int pl = 0; pl < P; ++pl) {
+            // plane pl of token m: row pl MT + m of the unsigned operand, row m of the signed one behind its 16 rows
+            const int row = pl + 1 < P ? pl * MT + m : 16 + m;
+            uint32_t o[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const int b = (j & 1) * 8 + (j >> 1);  // first k of the word: 0, 8, 1, 9; then every second one
+              const uint32_t sel = pl < 2 ? 0x5140 : 0x7362;
+              const uint32_t t0 = __byte_perm(v[b], v[b + 2], sel), t1 = __byte_perm(v[b + 4], v[b + 6], sel);
+              o[j] = __byte_perm(t0, t1, pl & 1 ? 0x7632 : 0x5410);
+            }
+            sts128(at + row * 128 + (((uint32_t)r ^ (uint32_t)row) & 7u) * 16, make_uint4(o[0], o[1], o[2], o[3]));
+          }
+          if (r == 0)
+            asm volatile("st.shared.b32 [%0], %1;" ::"r"(info + (step * MT + m) * 4),
+                         "r"(bad ? 0x7FC00000u : (uint32_t)((int)eb - (P == 4 ? 34 : 18)) << 23)
+                         : "memory");
+        }
+        fence_proxy_async_smem();
+        __syncwarp();
+        mbar_arrive_if(bar_x_full + 8 * (step >> 1), lane == 0);
+        sl += ((step + kStride) >> 1) - (step >> 1);
+      }
+    } else if (warp == kWarpW) {
+      // ---- packed words.  The kernel in front may be the one that writes them: until it has finished they are only
+      // brought into L2, p.ahead slots of them.
+      if (lane == 0) {
+        for (int i = 0; i < np && i < p.ahead; ++i) {
+#pragma unroll
+          for (int mb = 0; mb < MB; ++mb) tma_prefetch_2d(&tmap_w, (pr0 + i) * 32, n0 + mb * 128);
+        }
+        pdl_wait_prior_grid();
+        int s = 0;
+        uint32_t ph = 1;
+        for (int i = 0; i < np; ++i) {
+#pragma unroll
+          for (int mb = 0; mb < MB; ++mb) {
+            mbar_wait(bar_w_empty + 32 * mb + 8 * s, ph, abort_flag);
+            mbar_arrive_expect_tx(bar_w_full + 32 * mb + 8 * s, kWSlot);
+            tma_load_2d(ring_w + (mb * p.sw + s) * kWSlot, &tmap_w, (pr0 + i) * 32, n0 + mb * 128,
+                        bar_w_full + 32 * mb + 8 * s);
+          }
+          if (++s == p.sw) { s = 0; ph ^= 1; }
+        }
+      }
+      __syncwarp();
+    } else if (warp < kWarpMma + MB) {
+      // ---- products, one warp per block of rows: the whole warp runs the loop and one elected lane issues (the
+      // descriptors then stay in uniform registers)
+      const int mb = warp - kWarpMma;
+      constexpr uint32_t id_lo = umma_idesc_s8(0, 128, 16), id_hi = umma_idesc_s8(1, 128, 16);
+      const uint64_t desc0 = umma_desc_k128(ring_x);
+      pdl_wait_prior_grid();  // the kernel in front may run longer than a bounded wait for X
+      int xs = 0;
+      for (int i = 0; i < np; ++i) {
+        const uint32_t b_af = bar_a_full + 8 * (mb * 2 + (i & 1)), aph = (i >> 1) & 1;
+        if (!__all_sync(0xffffffffu, mbar_try_wait2(bar_x_full + 8 * i, 0, b_af, aph))) {
+          mbar_wait(bar_x_full + 8 * i, 0, abort_flag);
+          mbar_wait(b_af, aph, abort_flag);
+          __syncwarp();
+        }
+        tc_fence_after_sync();
+        const uint64_t db = desc0 + xs * (2 * kXStep >> 4);
+        const uint32_t d = tmem + (mb * 2 + (i & 1)) * 128, a = d + 64;
+        if (elect_one()) {
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk)
+              umma_i8_ts(d + h * 32, a + h * 32 + kk * 8, db + h * (kXStep >> 4) + kk * 2, id_lo, kk > 0 ? 1u : 0u);
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk)
+              umma_i8_ts(d + h * 32 + 16, a + h * 32 + kk * 8, db + h * (kXStep >> 4) + (16 * 128 >> 4) + kk * 2, id_hi,
+                         kk > 0 ? 1u : 0u);
+          }
+          umma_commit(bar_a_empty + 8 * (mb * 2 + (i & 1)));
+          umma_commit(bar_x_empty + 8 * xs);
+        }
+        __syncwarp();
+        if (++xs == p.sx) xs = 0;
       }
     }
   }
   __syncwarp();
-  if (p.ks > 1) cluster_barrier();  // the peers have read this CTA's part
+  if (p.ks > 1) {
+    if (warp >= kMain || poisoned) cluster_wait();
+    __syncwarp();
+    cluster_arrive();
+    cluster_wait();
+    const int first = (crank * kBlocks + p.ks - 1) / p.ks, count = ((crank + 1) * kBlocks + p.ks - 1) / p.ks - first;
+    for (int blk = 0; blk < count && !poisoned; ++blk)
+      for (int tok = warp; tok < p.M; tok += kWarps) {
+        const float* part = reinterpret_cast<const float*>(gen + p.off_red) + (blk * p.ks * 2 * MT + tok) * 32 + lane;
+        const int n = n0 + (first + blk) * 32 + lane;
+        float sum = 0.f;
+#pragma unroll 4
+        for (int z = 0; z < 2 * p.ks; ++z) sum += part[z * MT * 32];
+        if (n < p.N) p.Y[(size_t)tok * p.N + n] = __float2bfloat16(sum);
+      }
+  }
   __syncthreads();
   if (*abort_flag) {
     if (tid == 0) atomicCAS(p.status, kStatusOk, kStatusGemvTimeout);
-    for (int i = 0; i < 64; ++i) __nanosleep(2000);
+    for (int i = 0; i < 64; ++i) __nanosleep(2000);  // copies in flight land before the shared memory is released
     __syncthreads();
   }
-  if (warp == 1) {
+  if (warp == kWarpMma) {
     tc_fence_after_sync();
-    tmem_dealloc(tmem_d, kTmemCols);
+    tmem_dealloc(tmem, kTmemCols);
   }
 }
 
 using TcKernel = void (*)(const CUtensorMap, const TcParams);
 
 struct TcPlan {
-  int form = 0, ks = 1, sw = 0, steps = 0;  // form 0: 128 rows, two CTAs per SM; 1: 256 rows, one
+  int form = 0, ks = 1, pairs = 0;  // form 0: 128 rows, two CTAs per SM; 1: 256 rows, one
   double us = 0;
 };
 
-// Estimated time (us, fitted to 512 to 57344 x 2048 to 28672): waves of CTAs, 4.6 each for start, X and the exchange, 0.62
-// per step of a 256-row CTA; a 128-row one takes 0.5 alone on its SM and twice that with a neighbour, and up to 2 more to
-// start and sum up where K is cut into single steps and the chip is full (5097 x 768 in clusters of six: 6.3).  A CTA's steps
-// are limited by the planes of X beside two ring slots.  wanted_*: 0 = any.
-bool tc_plan(int N, int K, int sm_count, int wanted_form, int wanted_ks, TcPlan* out) {
-  const int nkb = K / kStepK;
+int tc_tokens(int M) { return M <= 4 ? 4 : M <= 8 ? 8 : 16; }
+
+// Shared memory of a plan: offsets from the 1024-aligned base.
+void tc_layout(const TcPlan& pl, int M, TcParams* p) {
+  const int mt = tc_tokens(M), mb = pl.form + 1, blocks = 4 * mb, room = (mb == 2 ? kSmemFull : kSmemHalf) - 1024;
+  const int info = 2 * pl.pairs * mt * 4, red = (blocks + pl.ks - 1) / pl.ks * pl.ks * 2 * mt * 128;
+  p->off_w = (kSlotBars + 8 * pl.pairs + 1023) / 1024 * 1024;
+  for (p->sw = 4;; p->sw = 2) {  // even: a slot belongs to one group
+    p->off_x = p->off_w + mb * p->sw * kWSlot;
+    p->sx = std::min(8, (room - 16 - p->off_x - info - red) / (2 * kXStep));
+    if (p->sx >= 2 || p->sw == 2) break;
+  }
+  p->off_info = p->off_x + p->sx * 2 * kXStep;
+  p->off_red = (p->off_info + info + 15) / 16 * 16;
+}
+
+template <int MB, int SV>
+TcKernel tc_kernel_mt(int mt) {
+  return mt == 4 ? w4_gemv_tc_kernel<MB, 4, SV> : mt == 8 ? w4_gemv_tc_kernel<MB, 8, SV> : w4_gemv_tc_kernel<MB, 16, SV>;
+}
+TcKernel tc_kernel(int form, int mt, bool sv4) {
+  return form ? (sv4 ? tc_kernel_mt<2, 4>(mt) : tc_kernel_mt<2, 2>(mt)) : (sv4 ? tc_kernel_mt<1, 4>(mt) : tc_kernel_mt<1, 2>(mt));
+}
+int tc_attributes(TcKernel kernel, int form, int mt, bool sv4, int dev) {
+  static std::atomic<bool> done[64][2][2][3];
+  const bool cached = dev >= 0 && dev < 64;
+  if (cached && done[dev][form][sv4][mt / 8].load(std::memory_order_acquire)) return 0;
+  const cudaError_t e =
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, form ? kSmemFull : kSmemHalf);
+  if (e == cudaSuccess && cached) done[dev][form][sv4][mt / 8].store(true, std::memory_order_release);
+  return (int)e;
+}
+void tc_config(int form, int grid, int ks, bool pdl, cudaLaunchConfig_t* cfg, cudaLaunchAttribute (&attr)[2]) {
+  cfg->gridDim = dim3(grid);
+  cfg->blockDim = dim3(form ? 896 : 512);
+  cfg->dynamicSmemBytes = form ? kSmemFull : kSmemHalf;  // all of it: at most 512 TMEM columns' worth of CTAs fit on an SM
+  int na = 0;
+  if (ks > 1) {
+    attr[na].id = cudaLaunchAttributeClusterDimension;
+    attr[na].val.clusterDim.x = ks;
+    attr[na].val.clusterDim.y = 1;
+    attr[na].val.clusterDim.z = 1;
+    ++na;
+  }
+  if (pdl) {
+    attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[na].val.programmaticStreamSerializationAllowed = 1;
+    ++na;
+  }
+  cfg->attrs = attr;
+  cfg->numAttrs = na;
+}
+
+// CTAs of a form that the device runs at a time in clusters of ks: a cluster stays inside one GPC, so some SMs are left out (256
+// rows: 148 of 148 in twos, 135, 132, 130, 132, 105, 120 in threes to eights).  Asked for once per device.
+int tc_capacity(int form, int ks, int sm_count, int dev) {
+  if (ks == 1) return sm_count * (form ? 1 : 2);
+  static std::atomic<int> known[64][2][9];
+  const bool cached = dev >= 0 && dev < 64;
+  if (cached)
+    if (const int v = known[dev][form][ks].load(std::memory_order_relaxed)) return v;
+  const TcKernel kernel = tc_kernel(form, 8, true);
+  int clusters = 0;
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute attr[2];
+  tc_config(form, ks, ks, false, &cfg, attr);
+  if (tc_attributes(kernel, form, 8, true, dev) != 0 ||
+      cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) != cudaSuccess || clusters < 1) {
+    (void)cudaGetLastError();
+    clusters = std::max(1, sm_count * (form ? 1 : 2) / ks * 7 / 8);
+  }
+  if (cached) known[dev][form][ks].store(clusters * ks, std::memory_order_relaxed);
+  return clusters * ks;
+}
+
+// Estimated time (us), a fit to 466 shapes in every form and cluster size (256 to 60000 x 256 to 28672, weights from HBM): start,
+// exchange through the cluster, waves of CTAs that take their pairs of steps at the rate of a warp group's chain or of HBM.  The
+// 128-row form shares an SM with a second CTA where K is cut or there are more CTAs than SMs.  What it picks takes 1.016 times
+// the best plan's time in the geometric mean; its own time is 2 % short there.
+bool tc_plan(int M, int N, int K, int sm_count, int wanted_form, int wanted_ks, TcPlan* out) {
+  static constexpr double kChain[2][3] = {{0.541, 0.582, 0.879}, {0.734, 0.775, 0.913}}, kShared[3] = {1.042, 1.121, 1.593};
+  static constexpr double kToken[3] = {0.0, 0.141, 0.359};
+  int dev = -1;
+  if (cudaGetDevice(&dev) != cudaSuccess) dev = -1;
+  const int total = K / (2 * kStepK), mc = M <= 4 ? 0 : M <= 8 ? 1 : 2;
   bool any = false;
   for (int form = 0; form < 2; ++form) {
     if (wanted_form && form != wanted_form - 1) continue;
-    const int rows = form ? 256 : 128, room = (form ? kSmemFull : kSmemHalf) - 1024 - kHeaderBytes;
+    const int rows = form ? 256 : 128;
     const long tiles = (N + rows - 1) / rows;
-    for (int ks = 1; ks <= 8 && ks <= nkb; ++ks) {
-      if (wanted_ks && ks != std::min({wanted_ks, 8, nkb})) continue;
-      const int steps = (nkb + ks - 1) / ks;
+    for (int ks = 1; ks <= 8 && ks <= total; ++ks) {
+      if (wanted_ks && ks != std::min({wanted_ks, 8, total})) continue;
       TcPlan pl;
       pl.form = form;
       pl.ks = ks;
-      pl.steps = steps;
-      pl.sw = std::min(kMaxSlots, (room - steps * (kXStep + kInfoStep)) / (rows * 128));
-      if (pl.sw < 2) continue;
-      // clusters leave some SMs of a GPC out
-      const long cap = (form ? 1 : 2) * (ks == 1 ? sm_count : ks == 7 ? sm_count * 0.7 : ks == 8 ? sm_count * 0.8 : sm_count * 0.87);
-      const long ctas = tiles * ks, waves = (ctas + cap - 1) / cap;
-      const double busy = std::min(1.0, (double)ctas / waves / (2.0 * sm_count));
-      pl.us = waves * (form ? 4.6 + 0.62 * steps : 3.8 + (0.5 + 0.5 * busy) * steps + (steps == 1 ? 2.0 * busy : 0.0));
+      pl.pairs = (total + ks - 1) / ks;
+      if (pl.pairs > kMaxPairs || tiles * ks > 0x3fffffff) continue;
+      const long cap = tc_capacity(form, ks, sm_count, dev), ctas = tiles * ks, waves = (ctas + cap - 1) / cap;
+      const double act = (double)std::min(ctas, cap), mix = form ? 0.053 : 0.736;
+      const double eff = waves == 1 ? 1.0 : (1.0 - mix) * waves + mix * ctas / cap;
+      double chain = kChain[form][mc];
+      if (form == 0 && (ks > 1 || ctas > sm_count)) chain = kShared[mc] * std::min(1.0, 0.385 + 0.615 * act / (2.0 * sm_count));
+      const double pair = std::max(chain, act * rows * 128 * 1.03 / 7.705e6);
+      pl.us = (form ? 2.0 : 1.76) + (ks > 1 ? 0.85 + 0.043 * ks : 0.0) + kToken[mc] + (eff - 1.0) * 4.23 + eff * pl.pairs * pair;
       if (!any || pl.us < out->us) *out = pl;
       any = true;
     }
@@ -417,40 +616,93 @@ bool tc_plan(int N, int K, int sm_count, int wanted_form, int wanted_ks, TcPlan*
   return any;
 }
 
+bool tc_operands(const void* X, const void* Wq, const void* S, const void* Y, int M, int N, int K, int G) {
+  if (G != kStepK || K < 2 * kStepK || K % (2 * kStepK) || N < 1 || M < 1 || M > kTokens) return false;
+  return !(((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(Wq)) & 15) || (reinterpret_cast<uintptr_t>(Y) & 7) ||
+           (reinterpret_cast<uintptr_t>(S) & 3));
+}
+
 }  // namespace
 
-// Nine to sixteen tokens and groups of 128, where the estimate is below what the mma.sync kernel takes: 6 + 0.145 w + 3 K /
-// 1e4 us (w = millions of weights; 57344 x 8192 stays, 88 us against 96, and 8192 x 28672, 50 against 57).  Fewer tokens: the
-// mma.sync kernel pads to eight and is as fast or faster (37888 x 3584 at eight 20.0 against 21.0).  The estimate is 4 %
-// short over 200 shapes, 10 % where a 128-row CTA has nine steps and more (1500 x 11008: 13.9 us against 11.0, estimated at
-// 11.1 and 11.7).  Two chunks of K on few rows are all start-up, of which this kernel has more (700 x 256: 3.9 to 4.1 us against
-// 3.3; 6000 x 256 level).  Over 110 shapes the pick takes 1.006 times the shorter one's time in the geometric mean.
+// The calls that come here by name: flags that ask for this kernel, and nine to sixteen tokens on the shapes below (a line
+// through steps of 256 rows and of 128, drawn when a step took 0.62 and 0.5 to 1.0 us, against 6 + 0.145 w + 3 K / 1e4 us of the
+// mma.sync kernel, w = millions of weights).  What the line leaves to the other kernels comes here from there where it is the
+// shorter way (gemv_tc_shorter).
 // (Pointers: null = "assume aligned", for the queries that have no operands.)
 bool gemv_tc_applies(const void* X, const void* Wq, const void* S, const void* Y, int M, int N, int K, int G, int flags,
                      int sm_count) {
-  if (G != kStepK || K < 2 * kStepK || K % (2 * kStepK) || N < 1 || M < 1 || M > kTokens) return false;
-  if (((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(Wq)) & 15) || (reinterpret_cast<uintptr_t>(Y) & 7) ||
-      (reinterpret_cast<uintptr_t>(S) & 3))
-    return false;
-  TcPlan pl;
-  if (flags < 0) return tc_plan(N, K, sm_count, (flags >> 24) & 3, (flags >> 20) & 15, &pl);
-  if ((flags & ~kFlagNoPdl) != 0 || M <= 8 || (K <= 256 && N < 5000) || !tc_plan(N, K, sm_count, 0, 0, &pl)) return false;
-  const double longer = pl.form == 0 && pl.steps >= 9 ? 1.1 : 1.04;
-  return longer * pl.us < 6.0 + 0.145e-6 * ((double)N * K) + 3e-4 * K;
+  if (!tc_operands(X, Wq, S, Y, M, N, K, G)) return false;
+  if (flags < 0) {
+    TcPlan pl;
+    return tc_plan(M, N, K, sm_count, (flags >> 24) & 3, (flags >> 20) & 15, &pl);
+  }
+  if ((flags & ~kFlagNoPdl) != 0 || M <= 8 || (K <= 256 && N < 5000)) return false;
+  const int nkb = K / kStepK;
+  double best = 1e30;
+  for (int ks = 1; ks <= 8 && ks <= nkb; ++ks) {
+    const int steps = (nkb + ks - 1) / ks;
+    for (int form = 0; form < 2; ++form) {
+      if (steps > (form ? 39 : 19)) continue;  // (the converted X of a CTA's steps was held in shared memory)
+      const double cap = (form ? 1 : 2) * sm_count * (ks == 1 ? 1.0 : ks == 7 ? 0.7 : ks == 8 ? 0.8 : 0.87);
+      const long ctas = (long)((N + (form ? 255 : 127)) / (form ? 256 : 128)) * ks, waves = (long)std::ceil(ctas / (double)(long)cap);
+      const double busy = std::min(1.0, (double)ctas / waves / (2.0 * sm_count));
+      const double us =
+          waves * (form ? 4.6 + 0.62 * steps : 3.8 + (0.5 + 0.5 * busy) * steps + (steps == 1 ? 2.0 * busy : 0.0));
+      best = std::min(best, us * (form == 0 && steps >= 9 ? 1.1 : 1.04));
+    }
+  }
+  return best < 6.0 + 0.145e-6 * ((double)N * K) + 3e-4 * K;
 }
 
-int gemv_tc_describe(int N, int K, int flags, int sm_count, char* buf, int buflen) {
+// Whether this kernel is shorter than the GEMV that would take a plain call of 2 to 16 tokens, `other` one of kTcOther*.  Their
+// times (us) are fits to the same shapes as tc_plan's (w = millions of weights): many-token kernel at nine and more tokens 4.7 +
+// 0.176 w + 0.195 K / 1e3 + 0.09 M K / 1e4, at five to eight 4.2 + 0.11 w + 0.41 M K / 1e4, at two to four 6.65 + 0.11 w + 0.027 K
+// / 1e3 + 0.074 M K / 1e4; ring kernel 4.2 + 0.11 w + 0.164 K / 1e3 + 1.39 M K / 1e4.  Taken that way the calls run 1.40, 1.33,
+// 1.25 and 1.62 times as fast in the geometric mean (151, 114, 51 and 111 shapes); 7 of 427 lose more than 5 %, at most 16 %.
+// The streaming kernel (two to four tokens on tall matrices of short K) is level or shorter up to eighty million weights
+// (18944 x 3584 at two tokens 8.9 us against 10.0, 22705 x 1024 at four 4.8 against 5.4; between launches of this kernel
+// 22016 x 4096 at four is 1.4 us longer there).
+// Two tokens on up to two million weights stay with the ring kernel: the tensor-parallel form of such a call gives its bits.
+// Up to 512 rows at five to eight tokens stay with the many-token kernel's slices of K, 6.6 us against 3.9 at 512 x 3584: callers
+// rely on the plan that gemv_describe names there.
+bool gemv_tc_shorter(const void* X, const void* Wq, const void* S, const void* Y, int M, int N, int K, int G, int flags,
+                     int sm_count, TcOther other) {
+  if (M < 2 || (flags & ~kFlagNoPdl) != 0 || !tc_operands(X, Wq, S, Y, M, N, K, G)) return false;
+  const double w = 1e-6 * N * K, k3 = 1e-3 * K, mk = 1e-4 * M * K;
+  double us;
+  if (other == kTcOtherStream) {
+    if (w < 80.0) return false;
+    us = 2.6 + 0.094 * w + 0.011 * k3 + 1.75 * mk;
+  } else if (other == kTcOtherRing) {
+    if (M == 2 && w <= 2.0) return false;
+    us = 4.2 + 0.11 * w + 0.164 * k3 + 1.39 * mk;
+  } else if (M >= 9) {
+    us = 4.7 + 0.176 * w + 0.195 * k3 + 0.09 * mk;
+  } else if (M >= 5) {
+    if (N <= 512) return false;
+    us = 4.2 + 0.11 * w + 0.41 * mk;
+  } else {
+    us = 6.65 + 0.11 * w + 0.027 * k3 + 0.074 * mk;
+  }
+  TcPlan pl;
+  return tc_plan(M, N, K, sm_count, 0, 0, &pl) && 1.02 * pl.us < us;
+}
+
+int gemv_tc_describe(int M, int N, int K, int flags, int sm_count, bool many, char* buf, int buflen) {
   const bool forced = flags < 0;
   TcPlan pl;
-  if (!tc_plan(N, K, sm_count, forced ? (flags >> 24) & 3 : 0, forced ? (flags >> 20) & 15 : 0, &pl)) return 0;
+  if (!tc_plan(M, N, K, sm_count, forced ? (flags >> 24) & 3 : 0, forced ? (flags >> 20) & 15 : 0, &pl)) return 0;
   const int rows = pl.form ? 256 : 128;
+  TcParams p{};
+  tc_layout(pl, M, &p);
   return snprintf(buf, buflen,
-                  "tcgen05 GEMV: %d CTAs (%d per SM), tiles of %d rows x %d tokens, clusters of %d along K, 2 planes (16-bit X), "
+                  "%s: %d CTAs (%d per SM), tiles of %d rows x %d tokens, clusters of %d along K, %d planes (%d-bit X), "
                   "%d ring slots",
-                  (N + rows - 1) / rows * pl.ks, pl.form ? 1 : 2, rows, kTokens, pl.ks, pl.sw);
+                  many ? "many-token kernel on tcgen05" : "tcgen05 GEMV", (N + rows - 1) / rows * pl.ks, pl.form ? 1 : 2, rows,
+                  tc_tokens(M), pl.ks, M <= 4 ? 4 : 2, M <= 4 ? 32 : 16, p.sw);
 }
 
-// flags: bits 20-23 CTAs per cluster, bits 24-25 tile (1: 128 rows, two CTAs per SM; 2: 256 rows, one), 0 = the rule.
+// flags: bits 20-23 CTAs per cluster, bits 24-25 tile (1: 128 rows; 2: 256), 0 = the rule.
 int gemv_tc_launch(const void* X, const void* Wq, const void* S, void* Y, int M, int N, int K, const Workspace& ws,
                    int flags, int sm_count, cudaStream_t stream) {
   TcParams p{};
@@ -460,54 +712,28 @@ int gemv_tc_launch(const void* X, const void* Wq, const void* S, void* Y, int M,
   p.status = ws.status;
   p.M = M; p.N = N; p.K = K;
   p.KG = K / kStepK;
-  p.nkb = K / kStepK;
+  p.pairs = K / (2 * kStepK);
   const bool forced = flags < 0;
   TcPlan pl;
-  if (!tc_plan(N, K, sm_count, forced ? (flags >> 24) & 3 : 0, forced ? (flags >> 20) & 15 : 0, &pl)) return kErrTooLarge;
-  const int form = pl.form, rows = form ? 256 : 128, slot = rows * 128, steps = (p.nkb + pl.ks - 1) / pl.ks;
+  if (!tc_plan(M, N, K, sm_count, forced ? (flags >> 24) & 3 : 0, forced ? (flags >> 20) & 15 : 0, &pl)) return kErrTooLarge;
+  const int form = pl.form, rows = form ? 256 : 128, mt = tc_tokens(M);
   p.ks = pl.ks;
-  p.sw = pl.sw;
-  p.off_x = kHeaderBytes + p.sw * slot;
-  p.off_info = p.off_x + steps * kXStep;
+  tc_layout(pl, M, &p);
+  p.ahead = 3;
   CUtensorMap tw;
-  if (!make_tensor_map_2d(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, Wq, (uint64_t)N, (uint64_t)K / 8, rows, 32,
+  if (!make_tensor_map_2d(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, Wq, (uint64_t)N, (uint64_t)K / 8, 128, 32,
                           CU_TENSOR_MAP_SWIZZLE_128B))
     return kErrDevice;
-  static constexpr TcKernel kKernels[2][2] = {{w4_gemv_tc_kernel<1, 8, 2, 2>, w4_gemv_tc_kernel<1, 8, 2, 4>},
-                                              {w4_gemv_tc_kernel<2, 16, 1, 2>, w4_gemv_tc_kernel<2, 16, 1, 4>}};
-  const int sv4 = p.KG % 4 == 0 && reinterpret_cast<uintptr_t>(S) % 8 == 0;
-  const TcKernel kernel = kKernels[form][sv4];
-  const int smem = form ? kSmemFull : kSmemHalf;  // all of it: at most 512 columns' worth of CTAs fit on an SM
-  static std::atomic<bool> done[64][2][2];
+  const bool sv4 = p.KG % 4 == 0 && reinterpret_cast<uintptr_t>(S) % 8 == 0;
+  const TcKernel kernel = tc_kernel(form, mt, sv4);
   int dev = -1;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return (int)e;
-  if (dev >= 64 || !done[dev][form][sv4].load(std::memory_order_acquire)) {
-    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return (int)e;
-    if (dev < 64) done[dev][form][sv4].store(true, std::memory_order_release);
-  }
+  if (const int rc = tc_attributes(kernel, form, mt, sv4, dev)) return rc;
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((N + rows - 1) / rows * p.ks);
-  cfg.blockDim = dim3(form ? 640 : 384);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
   cudaLaunchAttribute attr[2];
-  int na = 0;
-  if (p.ks > 1) {
-    attr[na].id = cudaLaunchAttributeClusterDimension;
-    attr[na].val.clusterDim.x = p.ks;
-    attr[na].val.clusterDim.y = 1;
-    attr[na].val.clusterDim.z = 1;
-    ++na;
-  }
-  if ((flags & kFlagNoPdl) == 0) {
-    attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[na].val.programmaticStreamSerializationAllowed = 1;
-    ++na;
-  }
-  cfg.attrs = attr;
-  cfg.numAttrs = na;
+  tc_config(form, (N + rows - 1) / rows * p.ks, p.ks, (flags & kFlagNoPdl) == 0, &cfg, attr);
+  cfg.stream = stream;
   e = cudaLaunchKernelEx(&cfg, kernel, tw, p);
   return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
 }

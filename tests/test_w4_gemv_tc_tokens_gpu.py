@@ -1,0 +1,87 @@
+"""GPU parity tests of the tcgen05 GEMV at one to eight tokens (up to four with X in 32 bits, above in 16) against the CPU
+oracle, and of the rule that brings plain calls of two to sixteen tokens there."""
+import numpy as np
+import pytest
+import torch
+
+import oracle
+from nanoserve_b200.ops import FLAG_DECODE_NARROW, FLAG_NO_PDL, narrow_flags
+from tests.util import bits_to_torch, check_bf16_output, torch_to_bits, u32_to_torch
+
+pytestmark = pytest.mark.gpu
+
+
+def slack(M):
+    # relative to the largest output: fp32 summation order for X in 32 bits; half a unit of 2^-15 per activation in 16
+    return 3e-6 if M <= 4 else 2e-5
+
+
+def run(k, X, Wq, S, flags):
+    y = k.w4_linear(bits_to_torch(X), u32_to_torch(Wq), bits_to_torch(S), 128, flags=flags)
+    torch.cuda.synchronize()
+    assert k.device_status() == 0
+    return torch_to_bits(y)
+
+
+@pytest.mark.parametrize("tile", [1, 2])
+@pytest.mark.parametrize("split", [1, 2, 3, 5, 8])
+def test_tiles_and_splits(kernels, tile, split):
+    # one row; a row tile less one, plus one; one pair of steps (a group of warps without work), odd numbers of them, rings
+    # that wrap; scales by two (K / 128 = 2, 6) and by four
+    for M, N, K in [(1, 1, 256), (2, 127, 512), (4, 129, 768), (3, 257, 2304), (5, 255, 1280), (8, 257, 4096), (7, 40, 9216)]:
+        X, Wq, S = oracle.synth_inputs(M, N, K, 128, seed=M + N)
+        flags = FLAG_DECODE_NARROW | narrow_flags(split, tile)
+        y = run(kernels, X, Wq, S, flags)
+        check_bf16_output(y, oracle.w4_linear_f32(X, Wq, S, 128), slack(M))
+        assert np.array_equal(y, run(kernels, X, Wq, S, flags))
+        assert np.array_equal(y, run(kernels, X, Wq, S, flags | FLAG_NO_PDL))
+
+
+@pytest.mark.parametrize("M", [4, 8, 16])
+def test_longest_k_of_a_cta(kernels, M):
+    N, K = 130, 28672  # 112 pairs in one CTA
+    X, Wq, S = oracle.synth_inputs(M, N, K, 128, seed=9)
+    ref = oracle.w4_linear_f32(X, Wq, S, 128, threads=oracle.max_threads())
+    for tile in (1, 2):
+        check_bf16_output(run(kernels, X, Wq, S, FLAG_DECODE_NARROW | narrow_flags(1, tile)), ref, slack(M))
+
+
+@pytest.mark.parametrize("M", [3, 4, 8])
+def test_extreme_inputs(kernels, M):
+    N, K = 200, 1024
+    X, Wq, S = oracle.synth_inputs(M, N, K, 128, seed=5)
+    f = oracle.bf16_bits_to_f32(X).copy()
+    f[0] *= np.float32(2.0**110)
+    f[1] *= np.float32(2.0**-60)
+    f[1, 128:256] = 0
+    X = oracle.f32_to_bf16_bits(f)
+    ref = oracle.w4_linear_f32(X, Wq, S, 128)
+    X[2, 300] = 0x7FC0 if M == 4 else 0xFF80
+    y = run(kernels, X, Wq, S, FLAG_DECODE_NARROW | narrow_flags())
+    assert np.isnan(oracle.bf16_bits_to_f32(y[2])).all()
+    for m in (0, 1):
+        check_bf16_output(y[m:m + 1], ref[m:m + 1], slack(M))
+
+
+@pytest.mark.parametrize("M,N,K", [(2, 3584, 18944), (4, 37888, 3584), (6, 4608, 3584), (8, 10240, 8192), (16, 18944, 3584)])
+def test_rule_on_layer_shapes(kernels, M, N, K):
+    assert "tcgen05" in kernels.gemv_describe(M, N, K, 128) and kernels.gemv_scratch_bytes(M, N, K) == 0
+    X, Wq, S = oracle.synth_inputs(M, N, K, 128, seed=4)
+    y = run(kernels, X, Wq, S, 0)
+    rows = np.unique(np.concatenate([[0, N - 1], np.random.default_rng(0).integers(0, N, 40)]))
+    check_bf16_output(y[:, rows], oracle.w4_linear_f32(X, Wq[rows], S[rows], 128, threads=oracle.max_threads()), slack(M))
+
+
+# the shorter kernel, us of the other and of this one
+@pytest.mark.parametrize("M,N,K,here", [
+    (2, 18944, 3584, False),  # 8.9 and 10.0
+    (4, 22705, 1024, False),  # 4.8, 5.4
+    (8, 512, 3584, False),    # (6.6, 3.9: stays, see the rule)
+    (1, 37888, 3584, False),  # 13.7, 15.7
+    (4, 3584, 3584, True),    # 7.5, 5.6
+    (8, 700, 256, True),      # 3.1, 2.5
+    (4, 8192, 28672, True),   # 40.7, 28
+    (16, 57344, 8192, True),  # 91, 68
+])
+def test_rule_takes_the_shorter_kernel(kernels, M, N, K, here):
+    assert ("tcgen05" in kernels.gemv_describe(M, N, K, 128)) == here
