@@ -50,6 +50,17 @@ __device__ __forceinline__ uint32_t bf16_dup(__nv_bfloat16 s) {
   return b | (b << 16);
 }
 
+// One packed word -> four bf16 pairs of (q - 8) * s in their natural order {w0,w1} {w2,w3} {w4,w5} {w6,w7}.  The byte
+// permutation puts nibble 2i into the low half (from w) and nibble 2i + 1 into the high half (from w >> 4): the unpack
+// order is the operand's order without a second permutation.
+__device__ __forceinline__ void dequant_word(uint32_t w, uint32_t s2, uint32_t mask, uint32_t magic, uint32_t* o) {
+  const uint32_t u = w >> 4;
+  o[0] = mul_bf16x2(sub136_bf16x2(lop3_and_or(__byte_perm(w, u, 0x4400), mask, magic)), s2);
+  o[1] = mul_bf16x2(sub136_bf16x2(lop3_and_or(__byte_perm(w, u, 0x5511), mask, magic)), s2);
+  o[2] = mul_bf16x2(sub136_bf16x2(lop3_and_or(__byte_perm(w, u, 0x6622), mask, magic)), s2);
+  o[3] = mul_bf16x2(sub136_bf16x2(lop3_and_or(__byte_perm(w, u, 0x7733), mask, magic)), s2);
+}
+
 // 16-byte shared-memory accesses by 32-bit shared address.
 __device__ __forceinline__ uint2 lds64(uint32_t addr) {
   uint2 v;

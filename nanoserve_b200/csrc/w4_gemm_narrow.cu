@@ -67,17 +67,6 @@ __device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, ui
       "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// One packed word -> four bf16 pairs of (q - 8) * s in their natural order {w0,w1} {w2,w3} {w4,w5} {w6,w7}.  The byte
-// permutation puts nibble 2i into the low half (from w) and nibble 2i + 1 into the high half (from w >> 4): the unpack
-// order is the operand's order without a second permutation.
-__device__ __forceinline__ void dequant_word(uint32_t w, uint32_t s2, uint32_t mask, uint32_t magic, uint32_t* o) {
-  const uint32_t u = w >> 4;
-  o[0] = mul_bf16x2(sub136_bf16x2(lop3_and_or(__byte_perm(w, u, 0x4400), mask, magic)), s2);
-  o[1] = mul_bf16x2(sub136_bf16x2(lop3_and_or(__byte_perm(w, u, 0x5511), mask, magic)), s2);
-  o[2] = mul_bf16x2(sub136_bf16x2(lop3_and_or(__byte_perm(w, u, 0x6622), mask, magic)), s2);
-  o[3] = mul_bf16x2(sub136_bf16x2(lop3_and_or(__byte_perm(w, u, 0x7733), mask, magic)), s2);
-}
-
 // MB: blocks of 128 weight rows per tile (each X tile is then read by MB MMAs).  DW: conversion warps, in DW / (4 MB)
 // groups that take the K blocks in turn; the converted weights of two K blocks fit in TMEM.  MINB: CTAs per SM.
 // MODE: 4 or 2: groups of 128 (a scale per row and step), read that many at a time; 64, 32: groups of 64 or 32 and whole
