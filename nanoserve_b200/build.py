@@ -13,6 +13,8 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 CSRC = os.path.join(ROOT, "nanoserve_b200", "csrc")
 LIB_DIR = os.path.join(ROOT, "build")
 LIB_PATH = os.path.join(LIB_DIR, "libnanoserve.so")
+CALL_SRC = os.path.join(CSRC, "binding.cpp")
+CALL_PATH = os.path.join(LIB_DIR, "nanoserve_call.so")  # Python extension: the host side of an eager call
 
 NVCC_FLAGS = [
     "-O3", "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo",
@@ -33,8 +35,31 @@ def _stale():
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def build_call(force: bool = False) -> str:
+    """Compile the Python extension (host code on torch's C++ objects; no CUDA sources) if its source is newer."""
+    if not force and os.path.exists(CALL_PATH) and os.path.getmtime(CALL_PATH) >= os.path.getmtime(CALL_SRC):
+        return CALL_PATH
+    import sysconfig
+    import torch
+    os.makedirs(LIB_DIR, exist_ok=True)
+    t = os.path.dirname(torch.__file__)
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    include = [os.path.join(t, "include"), os.path.join(t, "include", "torch", "csrc", "api", "include"),
+               sysconfig.get_paths()["include"], os.path.join(cuda, "include")]
+    lib = os.path.join(t, "lib")
+    cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+           *[f"-I{i}" for i in include], CALL_SRC, "-o", CALL_PATH, f"-L{lib}", f"-Wl,-rpath,{lib}",
+           "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
+    res = subprocess.run(cmd, cwd=ROOT, capture_output=True, text=True)
+    if res.returncode != 0:
+        sys.stderr.write(res.stdout + res.stderr)
+        raise RuntimeError("g++ failed building nanoserve_call.so")
+    return CALL_PATH
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
-    """Compile the library if any source is newer than it. Returns the library path."""
+    """Compile the library and the Python extension if any source is newer. Returns the library path."""
+    build_call(force)
     if not force and not _stale():
         return LIB_PATH
     os.makedirs(LIB_DIR, exist_ok=True)

@@ -144,9 +144,29 @@ def load_library(path: str = _LIB_DEFAULT) -> ctypes.CDLL:
     return lib
 
 
+def _load_call():
+    """The native host side of w4_linear and w4_quantize (csrc/binding.cpp), built beside the default library; None where it was
+    not built: calls then go through ctypes, to the same kernels."""
+    path = os.path.join(os.path.dirname(os.path.abspath(_LIB_DEFAULT)), "nanoserve_call.so")
+    if not os.path.exists(path):
+        return None, None
+    import importlib.util
+    spec = importlib.util.spec_from_file_location("nanoserve_call", path)
+    module = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(module)
+    return module.w4_linear, module.w4_quantize
+
+
+_call_linear, _call_quantize = _load_call()
+
+
 class Kernels:
     def __init__(self, path: str = _LIB_DEFAULT):
         self.lib = load_library(path)
+        # the addresses the native calls take (a library that has only the reference's symbols: ctypes for the linear)
+        address = lambda name: (ctypes.cast(getattr(self.lib, name), ctypes.c_void_p).value
+                                if _call_linear is not None and hasattr(self.lib, name) else None)
+        self._linear, self._quantize = address("b2_w4_linear"), address("ns_w4_quantize")
         for name in ("ns_rmsnorm", "ns_rope", "ns_swiglu", "ns_flash_fwd", "ns_w4_quantize", "ns_w4_linear"):
             getattr(self.lib, name)  # AttributeError if the library is not a drop-in
 
@@ -204,6 +224,10 @@ class Kernels:
         return o
 
     def w4_quantize(self, W, group=128):
+        if self._quantize is not None:
+            both = _call_quantize(self._quantize, W, group)
+            if both is not NotImplemented:
+                return both
         self._cuda(W)
         N, K = W.shape
         Wq = torch.empty((N, K // 8), dtype=torch.int32, device=W.device)
@@ -217,6 +241,10 @@ class Kernels:
     def w4_linear(self, x, Wq, S, group=128, flags=0, out=None):
         """`out` may also be a pinned host tensor: the kernel then stores its outputs straight into host memory
         (unified addressing), which saves a copy node when the outputs are wanted on the host anyway."""
+        if self._linear is not None:
+            y = _call_linear(self._linear, x, Wq, S, group, flags, out)
+            if y is not NotImplemented:
+                return y
         if not (x.is_cuda and Wq.is_cuda and S.is_cuda and (out is None or out.is_cuda or out.is_pinned())):
             self._cuda(x, Wq, S, out)  # raises
         M, K = x.shape

@@ -1,0 +1,76 @@
+"""The native host side of w4_linear and w4_quantize hands everything that is not a plain call on CUDA tensors back to the
+ctypes path, which answers as ever; on CUDA tensors both give the same bits, for outputs given or not, strided inputs and flags."""
+import pytest
+import torch
+
+from nanoserve_b200 import ops
+
+needs_call = pytest.mark.skipif(ops._call_linear is None, reason="the extension was not built here")
+
+
+@needs_call
+def test_hands_back_what_it_does_not_take():
+    x = torch.zeros(2, 256, dtype=torch.bfloat16)
+    for args in [(), (1,), (1, x, x, x, 128, 0, None), (1, None, x, x, 128, 0, None), (1, x, x, x, 128.0, 0, None),
+                 (1, x, x, x, 1 << 40, 0, None), (1, x, x, x, 128, 0, 3)]:
+        assert ops._call_linear(*args) is NotImplemented
+    for args in [(), (1, x, 128), (1, x, 0), (1, None, 128), (1, x, 128.0)]:
+        assert ops._call_quantize(*args) is NotImplemented
+
+
+@pytest.mark.gpu
+@needs_call
+def test_same_answers_as_through_ctypes(kernels):
+    g = torch.Generator(device="cuda").manual_seed(1)
+    N, K = 300, 1024
+    wq = torch.randint(-2**31, 2**31 - 1, (N, K // 8), dtype=torch.int32, device="cuda", generator=g)
+    s = torch.rand(N, K // 128, device="cuda", generator=g).to(torch.bfloat16)
+    slow = ops.Kernels()
+    slow._linear = slow._quantize = None
+    assert kernels._linear is not None and kernels._quantize is not None
+    wide = torch.randn(5, 2 * K, device="cuda", generator=g).to(torch.bfloat16)
+    for group in (128, 64):
+        for W in (wide[:, :K], wide.contiguous()):
+            for a, b in zip(kernels.w4_quantize(W, group), slow.w4_quantize(W, group)):
+                assert torch.equal(a, b) and a.dtype == b.dtype and a.shape == b.shape
+    for x in (wide[:, :K], wide[:1, :K].contiguous(), wide[:4, K:], torch.nn.Parameter(wide[:2, :K].clone())):
+        for flags in (0, ops.FLAG_RING_KERNEL, ops.FLAG_DECODE_NARROW):
+            want = slow.w4_linear(x, wq, s, 128, flags=flags)
+            got = kernels.w4_linear(x, wq, s, 128, flags=flags)
+            assert torch.equal(got, want) and got.dtype == torch.bfloat16 and not got.requires_grad
+        out = torch.empty(x.shape[0], N, dtype=torch.bfloat16, device="cuda")
+        assert kernels.w4_linear(x, wq, s, out=out) is out and torch.equal(out, slow.w4_linear(x, wq, s))
+    pinned = torch.empty(1, N, dtype=torch.bfloat16, pin_memory=True)
+    assert kernels.w4_linear(wide[:1, :K], wq, s, out=pinned) is pinned
+    torch.cuda.synchronize()
+    assert torch.equal(pinned.cuda(), slow.w4_linear(wide[:1, :K], wq, s))
+
+
+@pytest.mark.gpu
+@needs_call
+def test_errors_and_streams(kernels):
+    wq = torch.zeros(64, 32, dtype=torch.int32, device="cuda")
+    s = torch.ones(64, 2, dtype=torch.bfloat16, device="cuda")
+    x = torch.ones(1, 256, dtype=torch.bfloat16, device="cuda")
+    with pytest.raises(RuntimeError, match="ns_w4_linear failed with code -1"):
+        kernels.w4_linear(x, wq, s, group=96)
+    with pytest.raises(RuntimeError, match="ns_w4_quantize failed with code -1"):
+        kernels.w4_quantize(x, 96)
+    with pytest.raises(RuntimeError, match="CUDA tensors only"):
+        kernels.w4_quantize(x.cpu())
+    with pytest.raises(RuntimeError, match="CUDA tensors only"):
+        kernels.w4_linear(x.cpu(), wq, s)
+    with pytest.raises(ValueError):
+        kernels.w4_linear(x[0], wq, s)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):  # captured on the stream that is current
+        kernels.w4_linear(x, wq, s)
+        side.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=side):
+            y = kernels.w4_linear(x, wq, s)
+    x.fill_(2.0)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, kernels.w4_linear(x, wq, s))
