@@ -582,11 +582,13 @@ int tc_capacity(int form, int ks, int sm_count, int dev) {
 
 // Estimated time (us), a fit to 466 shapes in every form and cluster size (256 to 60000 x 256 to 28672, weights from HBM): start,
 // exchange through the cluster, waves of CTAs that take their pairs of steps at the rate of a warp group's chain or of HBM.  The
-// 128-row form shares an SM with a second CTA where K is cut or there are more CTAs than SMs.  What it picks takes 1.016 times
+// 128-row form shares an SM with a second CTA where K is cut or there are more CTAs than SMs.  Several waves with K whole have
+// a line of their own (26 shapes of 38000 to 60000 rows): the 256-row form takes whole waves, the 128-row one lets a CTA start
+// wherever one ends (53886 x 5632 at three tokens 35 us against 41; 57344 x 8192 60 against 58).  What it picks takes 1.016 times
 // the best plan's time in the geometric mean; its own time is 2 % short there.
 bool tc_plan(int M, int N, int K, int sm_count, int wanted_form, int wanted_ks, TcPlan* out) {
   static constexpr double kChain[2][3] = {{0.541, 0.582, 0.879}, {0.734, 0.775, 0.913}}, kShared[3] = {1.042, 1.121, 1.593};
-  static constexpr double kToken[3] = {0.0, 0.141, 0.359};
+  static constexpr double kToken[3] = {0.0, 0.141, 0.359}, kWave[3] = {0.84, 0.84, 1.04}, kFluid[3] = {0.87, 0.93, 1.35};
   int dev = -1;
   if (cudaGetDevice(&dev) != cudaSuccess) dev = -1;
   const int total = K / (2 * kStepK), mc = M <= 4 ? 0 : M <= 8 ? 1 : 2;
@@ -604,11 +606,15 @@ bool tc_plan(int M, int N, int K, int sm_count, int wanted_form, int wanted_ks, 
       if (pl.pairs > kMaxPairs || tiles * ks > 0x3fffffff) continue;
       const long cap = tc_capacity(form, ks, sm_count, dev), ctas = tiles * ks, waves = (ctas + cap - 1) / cap;
       const double act = (double)std::min(ctas, cap), mix = form ? 0.053 : 0.736;
-      const double eff = waves == 1 ? 1.0 : (1.0 - mix) * waves + mix * ctas / cap;
+      const double eff = waves == 1 ? 1.0 : (1.0 - mix) * waves + mix * ctas / cap, in_caps = (double)ctas / cap;
       double chain = kChain[form][mc];
       if (form == 0 && (ks > 1 || ctas > sm_count)) chain = kShared[mc] * std::min(1.0, 0.385 + 0.615 * act / (2.0 * sm_count));
       const double pair = std::max(chain, act * rows * 128 * 1.03 / 7.705e6);
-      pl.us = (form ? 2.0 : 1.76) + (ks > 1 ? 0.85 + 0.043 * ks : 0.0) + kToken[mc] + (eff - 1.0) * 4.23 + eff * pl.pairs * pair;
+      if (waves > 1 && ks == 1)
+        pl.us = 3.0 + kToken[mc] + pl.pairs * (form ? kWave[mc] * waves : kFluid[mc] * (in_caps + 0.45));
+      else
+        pl.us = (waves > 1 ? 1.15 : 1.0) * ((form ? 2.0 : 1.76) + (ks > 1 ? 0.85 + 0.043 * ks : 0.0) + kToken[mc] + (eff - 1.0) * 4.23 +
+                                            eff * pl.pairs * pair);
       if (!any || pl.us < out->us) *out = pl;
       any = true;
     }
@@ -658,7 +664,8 @@ bool gemv_tc_applies(const void* X, const void* Wq, const void* S, const void* Y
 // times (us) are fits to the same shapes as tc_plan's (w = millions of weights): many-token kernel at nine and more tokens 4.7 +
 // 0.176 w + 0.195 K / 1e3 + 0.09 M K / 1e4, at five to eight 4.2 + 0.11 w + 0.41 M K / 1e4, at two to four 6.65 + 0.11 w + 0.027 K
 // / 1e3 + 0.074 M K / 1e4; ring kernel 4.2 + 0.11 w + 0.164 K / 1e3 + 1.39 M K / 1e4.  Taken that way the calls run 1.40, 1.33,
-// 1.25 and 1.62 times as fast in the geometric mean (151, 114, 51 and 111 shapes); 7 of 427 lose more than 5 %, at most 16 %.
+// 1.25 and 1.62 times as fast in the geometric mean (151, 114, 51 and 111 shapes); 7 of 427 lost more than 5 %, at most 16 %.
+// (Since the line for several waves: 57989 x 4608 at eight tokens 37.5 us against 34.4, 290 x 22784 at sixteen 12.3 against 10.5.)
 // The streaming kernel (two to four tokens on tall matrices of short K) is level or shorter up to eighty million weights
 // (18944 x 3584 at two tokens 8.9 us against 10.0, 22705 x 1024 at four 4.8 against 5.4; between launches of this kernel
 // 22016 x 4096 at four is 1.4 us longer there).
