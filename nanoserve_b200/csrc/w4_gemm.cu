@@ -167,6 +167,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   const uint32_t bar_full_w = bar_base + 32 * 8;             // [kStages], pairs only: this CTA's packed half
   volatile int* abort_flag = reinterpret_cast<volatile int*>(gen_base + geo::kBarOffset + 26 * 8);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gen_base + geo::kBarOffset + 27 * 8);
+  volatile int* status_seen = reinterpret_cast<volatile int*>(gen_base + geo::kBarOffset + 29 * 8);
 
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   // CTA pair: this CTA loads and unpacks rows [wr0, wr0 + kWRows) of the weight tile; the peer the other half
@@ -216,6 +217,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     tma_prefetch_desc(&tmap_x);
     tma_prefetch_desc(&tmap_w);
   }
+  // One thread reads the status for the CTA: another CTA may set it at any time, and warps that saw different values would
+  // wait for one another at the epilogue's named barrier, which has no limit.
+  if (tid == 64) *status_seen = *reinterpret_cast<volatile int*>(p.status);
   if (warp == 1) {
     if constexpr (PAIR) {
       tmem_alloc_pair(smem_u32(tmem_slot), geo::kTmemCols);
@@ -230,7 +234,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
   if constexpr (PAIR) cluster_sync_all();  // the peer's barriers are initialised before anybody arrives on them
   tc_fence_after_sync();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
-  const bool poisoned = *reinterpret_cast<volatile int*>(p.status) != 0;
+  const bool poisoned = *status_seen != 0;
 
   if (!poisoned) {
     if (warp == 0) {

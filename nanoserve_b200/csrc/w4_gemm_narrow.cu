@@ -87,6 +87,7 @@ __global__ void __launch_bounds__(128 + DW * 32, MINB)
   const uint32_t bar_acc = bar_a_empty + 16;
   volatile int* abort_flag = reinterpret_cast<volatile int*>(gen + 512);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gen + 516);
+  volatile int* status_seen = reinterpret_cast<volatile int*>(gen + 520);
   const uint32_t ring_w = base + kHeaderBytes, ring_x = ring_w + p.sw * kWSlot;
   const uint32_t x_slot = (uint32_t)p.nt * 256;
 
@@ -113,6 +114,7 @@ __global__ void __launch_bounds__(128 + DW * 32, MINB)
     tma_prefetch_desc(&tmap_w);
     tma_prefetch_desc(&tmap_x);
   }
+  if (tid == 64) *status_seen = *reinterpret_cast<volatile int*>(p.status);  // (one answer for all warps of the CTA)
   if (warp == 1) {
     tmem_alloc(smem_u32(tmem_slot), p.tmem_cols);
     tmem_relinquish();
@@ -123,7 +125,7 @@ __global__ void __launch_bounds__(128 + DW * 32, MINB)
   pdl_launch_dependents();
   const uint32_t tmem_d = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   const uint32_t tmem_a = tmem_d + ((MB * p.nt + 31) & ~31);
-  const bool poisoned = *reinterpret_cast<volatile int*>(p.status) != 0;
+  const bool poisoned = *status_seen != 0;
 
   if (!poisoned) {
     if (warp == 0) {

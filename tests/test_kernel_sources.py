@@ -1,0 +1,30 @@
+"""What no run may show, since a violation could hang or fault the GPU, read from the kernels' sources."""
+import glob
+import os
+import re
+
+import pytest
+
+from nanoserve_b200 import build
+
+SOURCES = {os.path.basename(f): open(f).read() for f in sorted(glob.glob(os.path.join(build.CSRC, "*.cu")))}
+
+
+@pytest.mark.parametrize("name", [n for n, s in SOURCES.items() if "poisoned" in s])
+def test_named_barriers_and_the_status_word(name):
+    """Another CTA may set the status word at any time and a named barrier is unbounded.  Either one thread reads the word ahead
+    of a __syncthreads and the whole CTA decides by that value, or every warp reads it for itself and meets each named barrier
+    of the skipped work all the same."""
+    body = SOURCES[name]
+    read = re.search(r"\*reinterpret_cast<volatile int\*>\(p\.status\)", body)
+    decision = body.index("const bool poisoned = ")
+    assert len(re.findall(r"\*\>\(p\.status\)", body)) == 1
+    if read.start() < decision:
+        assert re.search(r"if \(tid == \d+\) \*status_seen = $", body[:read.start()])
+        assert "__syncthreads();" in body[read.start():decision]
+        assert body.startswith("const bool poisoned = *status_seen != 0;", decision)
+    else:
+        assert body.startswith("const bool poisoned = __any_sync(", decision)
+        barriers = re.findall(r'(if \([^;{}]*\)[^;{}]*)?asm volatile\("(bar\.sync[^"]*)"', body[decision:])
+        met = sorted(b for skipped, b in barriers if skipped.startswith("if (poisoned && "))
+        assert met and met == sorted(b for skipped, b in barriers if not skipped.startswith("if (poisoned && "))
