@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(MB == 2 ? 896 : 512, MB == 2 ? 1 : 2)
         return r;
       };
       int g = 2 * (pr0 + grp);  // the pair's first step: even
-      if (live) prefetch_l2(s_row + g);
+      if (live && g < p.KG) prefetch_l2(s_row + g);  // (the second group has none where the CTA's share is one pair)
       pdl_wait_prior_grid();
       // SV == 4: two pairs, this group's one of them; SV == 2: one
       auto pair_scales = [&](int step) {

@@ -28,3 +28,15 @@ def test_named_barriers_and_the_status_word(name):
         barriers = re.findall(r'(if \([^;{}]*\)[^;{}]*)?asm volatile\("(bar\.sync[^"]*)"', body[decision:])
         met = sorted(b for skipped, b in barriers if skipped.startswith("if (poisoned && "))
         assert met and met == sorted(b for skipped, b in barriers if not skipped.startswith("if (poisoned && "))
+
+
+def test_scale_prefetches_are_bounded():
+    """A step index taken from the CTA's share of K may lie one pair of steps behind a weight row's scales (a share of one pair
+    has nothing for the second group of warps): behind the last row that is past the end of S."""
+    K = 256  # one pair of steps; the second group's first step
+    assert 2 * (0 + 1) >= K // 128
+    guards = [re.findall(r"if \(([^{}]*?)\) prefetch_l2\(s_row \+ (\w+)\)", s) for s in SOURCES.values()]
+    found = [(cond, at) for g in guards for cond, at in g]
+    assert len(found) == sum(s.count("prefetch_l2(s_row") for s in SOURCES.values()) >= 2
+    for cond, at in found:
+        assert re.search(r"\b%s < p\.KG" % at, cond), (cond, at)
