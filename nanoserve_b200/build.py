@@ -58,10 +58,21 @@ def build_call(force: bool = False) -> str:
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
-    """Compile the library and the Python extension if any source is newer. Returns the library path."""
-    build_call(force)
+    """Compile the library and the Python extension if any source is newer. Returns the library path.
+
+    The library needs nvcc alone.  Where the extension cannot be built as well (no g++, no headers of Python or torch) eager
+    calls go through ctypes."""
+    _build_library(force, verbose)
+    try:
+        build_call(force)
+    except Exception as e:  # whatever is missing: the library is complete without it
+        sys.stderr.write(f"nanoserve_call.so was not built, eager calls go through ctypes: {e!r}\n")
+    return LIB_PATH
+
+
+def _build_library(force, verbose):
     if not force and not _stale():
-        return LIB_PATH
+        return
     os.makedirs(LIB_DIR, exist_ok=True)
     nvcc = os.environ.get("NVCC", "nvcc")
     cmd = [nvcc] + NVCC_FLAGS + (["-Xptxas", "-v"] if verbose else []) + ["-o", LIB_PATH] + sources()
@@ -73,7 +84,6 @@ def build(force: bool = False, verbose: bool = False) -> str:
         raise RuntimeError("nvcc failed building libnanoserve.so")
     if verbose:
         sys.stderr.write(res.stderr)
-    return LIB_PATH
 
 
 if __name__ == "__main__":

@@ -1,0 +1,37 @@
+"""The two build products: the C library, which needs nvcc alone, and the Python extension of eager calls, which is optional."""
+import subprocess
+
+import pytest
+
+from nanoserve_b200 import build
+
+
+def compilers(monkeypatch, tmp_path, gxx):
+    """Builds go to tmp_path; the compilers are replaced: nvcc succeeds, g++ does what `gxx` does.  Returns their command lines."""
+    monkeypatch.setattr(build, "LIB_DIR", str(tmp_path))
+    monkeypatch.setattr(build, "LIB_PATH", str(tmp_path / "libnanoserve.so"))
+    monkeypatch.setattr(build, "CALL_PATH", str(tmp_path / "nanoserve_call.so"))
+    ran = []
+
+    def run(cmd, **kw):
+        ran.append(cmd)
+        return gxx(cmd) if cmd[0] == "g++" else subprocess.CompletedProcess(cmd, 0, "", "")
+
+    monkeypatch.setattr(build.subprocess, "run", run)
+    return ran
+
+
+def no_compiler(cmd):
+    raise FileNotFoundError(2, "No such file or directory", cmd[0])
+
+
+def no_header(cmd):
+    return subprocess.CompletedProcess(cmd, 1, "", "fatal error: Python.h: No such file or directory")
+
+
+@pytest.mark.parametrize("gxx", [no_compiler, no_header])
+def test_the_library_is_built_without_the_extension(monkeypatch, tmp_path, capsys, gxx):
+    ran = compilers(monkeypatch, tmp_path, gxx)
+    assert build.build() == build.LIB_PATH
+    assert [c[0] for c in ran] == [build.os.environ.get("NVCC", "nvcc"), "g++"]
+    assert "nanoserve_call.so was not built" in capsys.readouterr().err
