@@ -11,6 +11,7 @@ raises.
 """
 import ctypes
 import os
+import warnings
 
 import torch
 
@@ -146,15 +147,20 @@ def load_library(path: str = _LIB_DEFAULT) -> ctypes.CDLL:
 
 def _load_call():
     """The native host side of w4_linear and w4_quantize (csrc/binding.cpp), built beside the default library; None where it was
-    not built: calls then go through ctypes, to the same kernels."""
+    not built or does not load: calls then go through ctypes, to the same kernels."""
     path = os.path.join(os.path.dirname(os.path.abspath(_LIB_DEFAULT)), "nanoserve_call.so")
     if not os.path.exists(path):
         return None, None
     import importlib.util
     spec = importlib.util.spec_from_file_location("nanoserve_call", path)
-    module = importlib.util.module_from_spec(spec)
-    spec.loader.exec_module(module)
-    return module.w4_linear, module.w4_quantize
+    try:
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        return module.w4_linear, module.w4_quantize
+    except (ImportError, OSError, AttributeError) as e:
+        warnings.warn(f"{path} does not load, eager calls go through ctypes (python -m nanoserve_b200.build --force "
+                      f"rebuilds it): {e}", RuntimeWarning, stacklevel=2)
+        return None, None
 
 
 _call_linear, _call_quantize = _load_call()

@@ -3,7 +3,7 @@ import subprocess
 
 import pytest
 
-from nanoserve_b200 import build
+from nanoserve_b200 import build, ops
 
 
 def compilers(monkeypatch, tmp_path, gxx):
@@ -35,3 +35,11 @@ def test_the_library_is_built_without_the_extension(monkeypatch, tmp_path, capsy
     assert build.build() == build.LIB_PATH
     assert [c[0] for c in ran] == [build.os.environ.get("NVCC", "nvcc"), "g++"]
     assert "nanoserve_call.so was not built" in capsys.readouterr().err
+
+
+def test_an_extension_that_does_not_load_is_left_out(monkeypatch, tmp_path):
+    monkeypatch.setattr(ops, "_LIB_DEFAULT", str(tmp_path / "libnanoserve.so"))
+    assert ops._load_call() == (None, None)  # not built
+    (tmp_path / "nanoserve_call.so").write_bytes(b"\x7fELF, cut off")
+    with pytest.warns(RuntimeWarning, match="does not load"):
+        assert ops._load_call() == (None, None)
