@@ -35,9 +35,26 @@ def _stale():
     return any(os.path.getmtime(d) > t for d in deps)
 
 
+def built_for() -> str:
+    """What the Python extension is bound to: torch's C++ classes and the interpreter."""
+    import torch
+    return f"torch {torch.__version__} {sys.implementation.cache_tag}"
+
+
+def call_matches(path: str) -> bool:
+    """Whether the extension at `path` was built for this torch and this interpreter (a note beside it says for which)."""
+    try:
+        with open(path + ".built_for") as f:
+            return f.read() == built_for()
+    except OSError:
+        return False
+
+
 def build_call(force: bool = False) -> str:
-    """Compile the Python extension (host code on torch's C++ objects; no CUDA sources) if its source is newer."""
-    if not force and os.path.exists(CALL_PATH) and os.path.getmtime(CALL_PATH) >= os.path.getmtime(CALL_SRC):
+    """Compile the Python extension (host code on torch's C++ objects; no CUDA sources) if its source is newer or it was built
+    for another torch or Python."""
+    if not force and os.path.exists(CALL_PATH) and call_matches(CALL_PATH) and \
+            os.path.getmtime(CALL_PATH) >= os.path.getmtime(CALL_SRC):
         return CALL_PATH
     import sysconfig
     import torch
@@ -47,13 +64,20 @@ def build_call(force: bool = False) -> str:
     include = [os.path.join(t, "include"), os.path.join(t, "include", "torch", "csrc", "api", "include"),
                sysconfig.get_paths()["include"], os.path.join(cuda, "include")]
     lib = os.path.join(t, "lib")
+    part = f"{CALL_PATH}.{os.getpid()}"  # whole before it has its name: another process may be loading it
     cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
-           *[f"-I{i}" for i in include], CALL_SRC, "-o", CALL_PATH, f"-L{lib}", f"-Wl,-rpath,{lib}",
+           *[f"-I{i}" for i in include], CALL_SRC, "-o", part, f"-L{lib}", f"-Wl,-rpath,{lib}",
            "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda"]
     res = subprocess.run(cmd, cwd=ROOT, capture_output=True, text=True)
     if res.returncode != 0:
         sys.stderr.write(res.stdout + res.stderr)
         raise RuntimeError("g++ failed building nanoserve_call.so")
+    if os.path.exists(CALL_PATH + ".built_for"):
+        os.remove(CALL_PATH + ".built_for")  # never a note beside an extension that it is not about
+    os.replace(part, CALL_PATH)
+    with open(part, "w") as f:
+        f.write(built_for())
+    os.replace(part, CALL_PATH + ".built_for")
     return CALL_PATH
 
 

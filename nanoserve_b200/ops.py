@@ -15,6 +15,8 @@ import warnings
 
 import torch
 
+from . import build
+
 _LIB_DEFAULT = os.path.join(os.path.dirname(os.path.abspath(__file__)), "..", "build", "libnanoserve.so")
 
 FLAG_FOLD_ZERO_POINT = 1
@@ -147,13 +149,15 @@ def load_library(path: str = _LIB_DEFAULT) -> ctypes.CDLL:
 
 def _load_call():
     """The native host side of w4_linear and w4_quantize (csrc/binding.cpp), built beside the default library; None where it was
-    not built or does not load: calls then go through ctypes, to the same kernels."""
+    not built, was built for another torch or Python, or does not load: calls then go through ctypes, to the same kernels."""
     path = os.path.join(os.path.dirname(os.path.abspath(_LIB_DEFAULT)), "nanoserve_call.so")
     if not os.path.exists(path):
         return None, None
     import importlib.util
     spec = importlib.util.spec_from_file_location("nanoserve_call", path)
     try:
+        if not build.call_matches(path):
+            raise ImportError("built for another torch or Python")
         module = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(module)
         return module.w4_linear, module.w4_quantize

@@ -41,5 +41,30 @@ def test_an_extension_that_does_not_load_is_left_out(monkeypatch, tmp_path):
     monkeypatch.setattr(ops, "_LIB_DEFAULT", str(tmp_path / "libnanoserve.so"))
     assert ops._load_call() == (None, None)  # not built
     (tmp_path / "nanoserve_call.so").write_bytes(b"\x7fELF, cut off")
+    (tmp_path / "nanoserve_call.so.built_for").write_text(build.built_for())
     with pytest.warns(RuntimeWarning, match="does not load"):
         assert ops._load_call() == (None, None)
+
+
+def test_the_extension_follows_torch_and_python(monkeypatch, tmp_path):
+    """Built again where its note names another torch or Python, never loaded there, and never there in part."""
+    written = []
+
+    def gxx(cmd):
+        out = cmd[cmd.index("-o") + 1]
+        written.append(out)
+        open(out, "wb").close()
+        return subprocess.CompletedProcess(cmd, 0, "", "")
+
+    ran = compilers(monkeypatch, tmp_path, gxx)
+    build.build_call()
+    build.build_call()
+    assert len(ran) == 1 and build.call_matches(build.CALL_PATH)
+    monkeypatch.setattr(build, "built_for", lambda: "torch 0.0 cpython-00")
+    monkeypatch.setattr(ops, "_LIB_DEFAULT", build.LIB_PATH)
+    with pytest.warns(RuntimeWarning, match="another torch or Python"):
+        assert ops._load_call() == (None, None)
+    build.build_call()
+    assert len(ran) == 2 and build.call_matches(build.CALL_PATH)
+    assert build.CALL_PATH not in written
+    assert sorted(p.name for p in tmp_path.iterdir()) == ["nanoserve_call.so", "nanoserve_call.so.built_for"]
