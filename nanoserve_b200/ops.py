@@ -170,12 +170,21 @@ def _load_call():
 _call_linear, _call_quantize = _load_call()
 
 
+def _find_call():
+    """The native calls, also where they were built after this module was imported."""
+    global _call_linear, _call_quantize
+    if _call_linear is None:
+        _call_linear, _call_quantize = _load_call()
+    return _call_linear is not None
+
+
 class Kernels:
     def __init__(self, path: str = _LIB_DEFAULT):
         self.lib = load_library(path)
         # the addresses the native calls take (a library that has only the reference's symbols: ctypes for the linear)
+        native = _find_call()
         address = lambda name: (ctypes.cast(getattr(self.lib, name), ctypes.c_void_p).value
-                                if _call_linear is not None and hasattr(self.lib, name) else None)
+                                if native and hasattr(self.lib, name) else None)
         self._linear, self._quantize = address("b2_w4_linear"), address("ns_w4_quantize")
         for name in ("ns_rmsnorm", "ns_rope", "ns_swiglu", "ns_flash_fwd", "ns_w4_quantize", "ns_w4_linear"):
             getattr(self.lib, name)  # AttributeError if the library is not a drop-in

@@ -68,3 +68,14 @@ def test_the_extension_follows_torch_and_python(monkeypatch, tmp_path):
     assert len(ran) == 2 and build.call_matches(build.CALL_PATH)
     assert build.CALL_PATH not in written
     assert sorted(p.name for p in tmp_path.iterdir()) == ["nanoserve_call.so", "nanoserve_call.so.built_for"]
+
+
+def test_an_extension_built_after_the_import_is_used(monkeypatch, lib_path):
+    """A clean checkout: the tests' modules import ops before the fixture builds anything."""
+    if not build.os.path.exists(build.CALL_PATH):
+        pytest.skip("the extension cannot be built here")
+    monkeypatch.setattr(ops, "_call_linear", None)
+    monkeypatch.setattr(ops, "_call_quantize", None)
+    k = ops.Kernels(lib_path)
+    assert k._linear is not None and k._quantize is not None
+    assert ops._call_linear is not None and ops._call_quantize is not None

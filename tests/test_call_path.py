@@ -1,15 +1,23 @@
 """The native host side of w4_linear and w4_quantize hands everything that is not a plain call on CUDA tensors back to the
 ctypes path, which answers as ever; on CUDA tensors both give the same bits, for outputs given or not, strided inputs and flags."""
+import shutil
+
 import pytest
 import torch
 
 from nanoserve_b200 import ops
 
-needs_call = pytest.mark.skipif(ops._call_linear is None, reason="the extension was not built here")
+
+@pytest.fixture
+def call(lib_path):
+    """The extension, built with the library on demand; missing only where there is no g++ to build it."""
+    if not ops._find_call():
+        if shutil.which("g++"):
+            pytest.fail("nanoserve_call.so was not built or does not load")
+        pytest.skip("no g++ to build the extension")
 
 
-@needs_call
-def test_hands_back_what_it_does_not_take():
+def test_hands_back_what_it_does_not_take(call):
     x = torch.zeros(2, 256, dtype=torch.bfloat16)
     for args in [(), (1,), (1, x, x, x, 128, 0, None), (1, None, x, x, 128, 0, None), (1, x, x, x, 128.0, 0, None),
                  (1, x, x, x, 1 << 40, 0, None), (1, x, x, x, 128, 0, 3)]:
@@ -19,8 +27,7 @@ def test_hands_back_what_it_does_not_take():
 
 
 @pytest.mark.gpu
-@needs_call
-def test_same_answers_as_through_ctypes(kernels):
+def test_same_answers_as_through_ctypes(kernels, call):
     g = torch.Generator(device="cuda").manual_seed(1)
     N, K = 300, 1024
     wq = torch.randint(-2**31, 2**31 - 1, (N, K // 8), dtype=torch.int32, device="cuda", generator=g)
@@ -47,8 +54,7 @@ def test_same_answers_as_through_ctypes(kernels):
 
 
 @pytest.mark.gpu
-@needs_call
-def test_errors_and_streams(kernels):
+def test_errors_and_streams(kernels, call):
     wq = torch.zeros(64, 32, dtype=torch.int32, device="cuda")
     s = torch.ones(64, 2, dtype=torch.bfloat16, device="cuda")
     x = torch.ones(1, 256, dtype=torch.bfloat16, device="cuda")
