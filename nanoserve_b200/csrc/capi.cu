@@ -88,7 +88,8 @@ Route plain_route(const DeviceState& st, const void* X, const void* Wq, const vo
     const b2::TcOther other = many                                             ? b2::kTcOtherMany
                               : b2::gemv_stream_applies(Wq, M, N, K, G, flags) ? b2::kTcOtherStream
                                                                                : b2::kTcOtherRing;
-    if (b2::gemv_tc_shorter(X, Wq, S, Y, M, N, K, G, flags, st.sm_count, other)) return many ? kRouteManyTc : kRouteGemvTc;
+    if (b2::gemv_tc_shorter(X, Wq, S, Y, M, N, K, G, flags, st.sm_count, st.ws.partial_bytes, other))
+      return many ? kRouteManyTc : kRouteGemvTc;
   }
   return b2::gemm_narrow_takes_decode(X, Wq, S, Y, M, N, K, G, flags, st.sm_count) ? kRouteGemm : kRouteGemv;
 }

@@ -506,7 +506,9 @@ using TcKernel = void (*)(const CUtensorMap, const TcParams);
 
 struct TcPlan {
   int form = 0, ks = 1, pairs = 0;  // form 0: 128 rows, two CTAs per SM; 1: 256 rows, one
-  double us = 0;
+  double us = 0;                    // (what plans are compared by)
+  double busy = 0;                  // the share of the places for CTAs that are taken
+  bool several = false;             // waves, with K whole: the line of its own
 };
 
 int tc_tokens(int M) { return M <= 4 ? 4 : M <= 8 ? 8 : 16; }
@@ -609,12 +611,15 @@ bool tc_plan(int M, int N, int K, int sm_count, int wanted_form, int wanted_ks, 
       pl.pairs = (total + ks - 1) / ks;
       if (pl.pairs > kMaxPairs || tiles * ks > 0x3fffffff) continue;
       const long cap = tc_capacity(form, ks, sm_count, dev), ctas = tiles * ks, waves = (ctas + cap - 1) / cap;
-      const double act = (double)std::min(ctas, cap), mix = form ? 0.053 : 0.736;
+      const double act = (double)std::min(ctas, cap);
+      pl.busy = act / cap;
+      pl.several = waves > 1 && ks == 1;
+      const double mix = form ? 0.053 : 0.736;
       const double eff = waves == 1 ? 1.0 : (1.0 - mix) * waves + mix * ctas / cap, in_caps = (double)ctas / cap;
       double chain = kChain[form][mc];
       if (form == 0 && (ks > 1 || ctas > sm_count)) chain = kShared[mc] * std::min(1.0, 0.385 + 0.615 * act / (2.0 * sm_count));
       const double pair = std::max(chain, act * rows * 128 * 1.03 / 7.705e6);
-      if (waves > 1 && ks == 1)
+      if (pl.several)
         pl.us = 3.0 + kToken[mc] + pl.pairs * (form ? kWave[mc] * waves : kFluid[mc] * (in_caps + 0.45));
       else
         pl.us = (waves > 1 ? 1.15 : 1.0) * ((form ? 2.0 : 1.76) + (ks > 1 ? 0.85 + 0.043 * ks : 0.0) + kToken[mc] + (eff - 1.0) * 4.23 +
@@ -664,39 +669,39 @@ bool gemv_tc_applies(const void* X, const void* Wq, const void* S, const void* Y
   return best < 6.0 + 0.145e-6 * ((double)N * K) + 3e-4 * K;
 }
 
-// Whether this kernel is shorter than the GEMV that would take a plain call of 2 to 16 tokens, `other` one of kTcOther*.  Their
-// times (us) are fits to the same shapes as tc_plan's (w = millions of weights): many-token kernel at nine and more tokens 4.7 +
-// 0.176 w + 0.195 K / 1e3 + 0.09 M K / 1e4, at five to eight 4.2 + 0.11 w + 0.41 M K / 1e4, at two to four 6.65 + 0.11 w + 0.027 K
-// / 1e3 + 0.074 M K / 1e4; ring kernel 4.2 + 0.11 w + 0.164 K / 1e3 + 1.39 M K / 1e4.  Taken that way the calls run 1.40, 1.33,
-// 1.25 and 1.62 times as fast in the geometric mean (151, 114, 51 and 111 shapes); 7 of 427 lost more than 5 %, at most 16 %.
-// (Since the line for several waves: 57989 x 4608 at eight tokens 37.5 us against 34.4, 290 x 22784 at sixteen 12.3 against 10.5.)
-// The streaming kernel (two to four tokens on tall matrices of short K) is level or shorter up to eighty million weights
-// (18944 x 3584 at two tokens 8.9 us against 10.0, 22705 x 1024 at four 4.8 against 5.4; between launches of this kernel
-// 22016 x 4096 at four is 1.4 us longer there).
+// Whether this kernel is shorter than the GEMV that would take a plain call of 2 to 16 tokens, `other` one of kTcOther*.  Lines drawn
+// through 6472 calls on 1627 random shapes (48 to 60000 rows, K 256 to 28672, weights from HBM), every kernel and every plan of this
+// one timed, and 4308 more of the many-token kernel's; "lost" is a call that takes 5 % more time than with the other kernel.
+//   * Many-token kernel, five and more tokens: by the estimates of both, this one's with what plans have in common (they come out
+//     short where the chip is full).  Of 4127 calls at five to eight tokens 44 are lost (at most 20 %), of 3439 above 34 (19 %); the
+//     time is 1.003 and 1.002 times the shorter kernel's in the geometric mean.  (With a line in M, N and K alone 134 and 498 were
+//     lost, up to 55 %, small matrices of long K most: 10 x 178 x 26112 14.5 us against 9.4, 16 x 290 x 22784 12.0 against 10.7.)
+//   * Many-token kernel, two to four tokens (K >= 8192): X has 32 bits here and 16 there, so what a line in w (millions of weights),
+//     M and K brought here stays.  1.19 times as fast in the geometric mean, 18 of 801 calls lost (15 %).
+//   * Streaming kernel at two tokens: shorter (18944 x 3584 9.2 us against 11.4, 37888 x 3584 14.6 against 15.5) except where one
+//     CTA to an SM is all it has and K is longer than its ring and X leave room for (17570 x 4096 13.4 against 11.3, 14739 x 6912
+//     20.0 against 14.6): 32 of 303 calls run here, none lost.  At three and four tokens X has 32 bits here and 16 there: level
+//     above eighty million weights (2 of 11 lost, 6 %), shorter there below.
+//   * Ring kernel: never shorter (1840 calls, 1.65 times as fast here, one lost).
 // Two tokens on up to two million weights stay with the ring kernel: the tensor-parallel form of such a call gives its bits.
 // Up to 512 rows at five to eight tokens stay with the many-token kernel's slices of K, 6.6 us against 3.9 at 512 x 3584: callers
 // rely on the plan that gemv_describe names there.
 bool gemv_tc_shorter(const void* X, const void* Wq, const void* S, const void* Y, int M, int N, int K, int G, int flags,
-                     int sm_count, TcOther other) {
+                     int sm_count, size_t partial_cap, TcOther other) {
   if (M < 2 || (flags & ~kFlagNoPdl) != 0 || !tc_operands(X, Wq, S, Y, M, N, K, G)) return false;
   const double w = 1e-6 * N * K, k3 = 1e-3 * K, mk = 1e-4 * M * K;
-  double us;
-  if (other == kTcOtherStream) {
-    if (w < 80.0) return false;
-    us = 2.6 + 0.094 * w + 0.011 * k3 + 1.75 * mk;
-  } else if (other == kTcOtherRing) {
-    if (M == 2 && w <= 2.0) return false;
-    us = 4.2 + 0.11 * w + 0.164 * k3 + 1.39 * mk;
-  } else if (M >= 9) {
-    us = 4.7 + 0.176 * w + 0.195 * k3 + 0.09 * mk;
-  } else if (M >= 5) {
-    if (N <= 512) return false;
-    us = 4.2 + 0.11 * w + 0.41 * mk;
-  } else {
-    us = 6.65 + 0.11 * w + 0.027 * k3 + 0.074 * mk;
-  }
+  if (other == kTcOtherRing && M == 2 && w <= 2.0) return false;
+  if (other == kTcOtherMany && M >= 5 && M <= 8 && N <= 512) return false;
   TcPlan pl;
-  return tc_plan(M, N, K, sm_count, 0, 0, &pl) && 1.02 * pl.us < us;
+  if (!tc_plan(M, N, K, sm_count, 0, 0, &pl)) return false;
+  if (other == kTcOtherRing) return true;
+  if (other == kTcOtherStream)
+    return M == 2 ? K >= 3840 && N <= 128 * sm_count : w >= 80.0 && 1.02 * pl.us < 2.6 + 0.094 * w + 0.011 * k3 + 1.75 * mk;
+  if (M <= 4) return 1.02 * pl.us < 6.65 + 0.11 * w + 0.027 * k3 + 0.074 * mk;
+  const double us = pl.us + (pl.form       ? 2.03 * pl.busy * pl.busy
+                             : pl.several ? 0.5
+                                          : 0.025 * w + 0.7 * pl.busy - (pl.ks > 1 ? 0.34 : 0.0));
+  return 1.02 * us < gemv_mid_us(M, N, K, sm_count, partial_cap);
 }
 
 int gemv_tc_describe(int M, int N, int K, int flags, int sm_count, bool many, char* buf, int buflen) {

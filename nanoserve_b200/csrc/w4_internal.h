@@ -134,7 +134,7 @@ int gemv_tc_describe(int M, int N, int K, int flags, int sm_count, bool many, ch
 // Whether the tcgen05 GEMV is shorter for a plain call than the kernel that the GEMV's own rules give it.
 enum TcOther { kTcOtherMany, kTcOtherStream, kTcOtherRing };
 bool gemv_tc_shorter(const void* X, const void* Wq, const void* S, const void* Y, int M, int N, int K, int G, int flags,
-                     int sm_count, TcOther other);
+                     int sm_count, size_t partial_cap, TcOther other);
 bool gemv_tc_applies(const void* X, const void* Wq, const void* S, const void* Y, int M, int N, int K, int G, int flags,
                      int sm_count);
 int gemv_tc_launch(const void* X, const void* Wq, const void* S, void* Y, int M, int N, int K, const Workspace& ws,
@@ -172,6 +172,7 @@ size_t gemv_stream_scratch_bytes(int M, int N, int K, int G, int flags, int sm_c
 // (no prologue, epilogue or tensor-parallel form).
 bool gemv_mid_applies(const void* X, const void* Wq, const void* S, int M, int N, int K, int G, int flags,
                       int sm_count, size_t partial_cap);
+double gemv_mid_us(int M, int N, int K, int sm_count, size_t partial_cap);
 int gemv_mid_launch(const void* X, const void* Wq, const void* S, void* Y, int M, int N, int K, const Workspace& ws,
                     int flags, int sm_count, cudaStream_t stream);
 int gemv_mid_describe(int M, int N, int K, int flags, int sm_count, size_t partial_cap, char* buf, int buflen);

@@ -85,3 +85,18 @@ def test_rule_on_layer_shapes(kernels, M, N, K):
 ])
 def test_rule_takes_the_shorter_kernel(kernels, M, N, K, here):
     assert ("tcgen05" in kernels.gemv_describe(M, N, K, 128)) == here
+
+
+# us of the kernel that keeps the call and of this one
+@pytest.mark.parametrize("M,N,K", [
+    (10, 178, 26112),   # 9.4, 14.5
+    (9, 440, 27648),    # 11.1, 15.5
+    (16, 144, 19456),   # 9.0, 11.4
+    (16, 290, 22784),   # 10.7, 12.0
+    (12, 84, 13824),    # 7.6, 8.3
+    (7, 54677, 256),    # 6.3, 7.6
+    (2, 29616, 5632),   # 19.3, 21.7
+    (2, 37888, 3584),   # 14.6, 15.5
+])
+def test_rule_leaves_calls_where_they_are_shorter(kernels, M, N, K):
+    assert "tcgen05" not in kernels.gemv_describe(M, N, K, 128)
