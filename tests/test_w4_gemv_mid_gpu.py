@@ -34,17 +34,17 @@ def served(k, M, N, K, flags=ops.FLAG_MID_KERNEL):
 
 def test_dispatch(kernels):
     assert served(kernels, 8, 18944, 3584) and served(kernels, 16, 18944, 3584) and served(kernels, 5, 2368, 256)
-    assert served(kernels, 8, 28672, 8192, 0) and served(kernels, 16, 18944, 3584, 0) and served(kernels, 16, 28672, 8192, 0)
+    assert served(kernels, 8, 28672, 8192) and served(kernels, 16, 28672, 8192)
     # nine to sixteen tokens: the tcgen05 GEMV where its estimate is lower
     for M, N, K in [(9, 37888, 3584), (16, 3584, 18944)]:
         assert kernels.gemv_describe(M, N, K, 128, 0).startswith("tcgen05 GEMV")
         assert kernels.gemv_scratch_bytes(M, N, K) == 0
         assert served(kernels, M, N, K, ops.FLAG_MID_KERNEL)
-    assert served(kernels, 8, 37888, 3584, 0) and served(kernels, 5, 3584, 3584, 0)
+    assert served(kernels, 8, 37888, 3584) and served(kernels, 5, 3584, 3584)
     assert not served(kernels, 4, 18944, 3584, 0)
-    plan = kernels.gemv_describe(8, 512, 3584, 128, 0)  # few rows: K in slices that fill the SMs
+    plan = kernels.gemv_describe(8, 512, 3584, 128, ops.FLAG_MID_KERNEL)  # few rows: K in slices that fill the SMs
     assert plan.startswith("many-token kernel") and "K slices across CTAs 4 (sum kernel)" in plan
-    assert served(kernels, 2, 3584, 18944, 0) and served(kernels, 4, 28672, 8192, 0) and not served(kernels, 1, 3584, 18944)
+    assert served(kernels, 2, 3584, 18944) and served(kernels, 4, 28672, 8192) and not served(kernels, 1, 3584, 18944)
     plan = kernels.gemv_describe(16, 3584, 18944, 128, ops.FLAG_MID_KERNEL)  # the converted X fits in slices of K only
     assert plan.startswith("many-token kernel") and "K slices across CTAs 5 (sum kernel)" in plan
     assert "K slices across CTAs 1," in kernels.gemv_describe(16, 18944, 3584, 128, ops.FLAG_MID_KERNEL)

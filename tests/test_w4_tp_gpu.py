@@ -72,7 +72,7 @@ def test_consumer_waits_on_the_counter_and_reads_the_gathered_row(kernels):
     wa, sa, wb, sb = u32_to_torch(Wa), bits_to_torch(Sa), u32_to_torch(Wb), bits_to_torch(Sb)
     g = torch.Generator(device="cuda").manual_seed(5)
     x = torch.randn(M, K1, device="cuda", generator=g).to(torch.bfloat16)
-    gu = kernels.w4_linear(x, wa, sa, G)
+    gu = kernels.w4_linear(x, wa, sa, G, flags=ops.FLAG_RING_KERNEL)  # the kernel that has a tensor-parallel form: its bits
     want = kernels.w4_linear_fused(gu, wb, sb, G, prologue=2)
 
     buf = torch.zeros(M, 2 * I, dtype=torch.bfloat16, device="cuda")
