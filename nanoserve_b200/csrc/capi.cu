@@ -77,19 +77,18 @@ int* device_status_word(int* rc) {
 namespace {
 
 // Which launcher takes a plain call.  (Pointers: null = "assume aligned", for the queries that have no operands.)
-// kRouteManyTc: a call of the many-token kernel that runs on tcgen05, a name of its own for gemv_describe only.
-enum Route { kRouteGemv, kRouteGemvTc, kRouteManyTc, kRouteGemm };
+enum Route { kRouteGemv, kRouteGemvTc, kRouteGemm };
 Route plain_route(const DeviceState& st, const void* X, const void* Wq, const void* S, const void* Y, int M, int N, int K,
                   int G, int flags) {
   if (M > 16) return kRouteGemm;
-  if (b2::gemv_tc_applies(X, Wq, S, Y, M, N, K, G, flags, st.sm_count)) return kRouteGemvTc;
+  if (flags < 0 && b2::gemv_tc_serves(X, Wq, S, Y, M, N, K, G, flags, st.sm_count)) return kRouteGemvTc;
   if (flags == 0 || flags == b2::kFlagNoPdl) {
     const bool many = b2::gemv_mid_applies(X, Wq, S, M, N, K, G, flags, st.sm_count, st.ws.partial_bytes);
     const b2::TcOther other = many                                             ? b2::kTcOtherMany
                               : b2::gemv_stream_applies(Wq, M, N, K, G, flags) ? b2::kTcOtherStream
                                                                                : b2::kTcOtherRing;
     if (b2::gemv_tc_shorter(X, Wq, S, Y, M, N, K, G, flags, st.sm_count, st.ws.partial_bytes, other))
-      return many ? kRouteManyTc : kRouteGemvTc;
+      return kRouteGemvTc;
   }
   return b2::gemm_narrow_takes_decode(X, Wq, S, Y, M, N, K, G, flags, st.sm_count) ? kRouteGemm : kRouteGemv;
 }
@@ -104,7 +103,7 @@ int linear_dispatch(const void* X, const void* Wq, const void* S, void* Y, int M
   // (a null operand is answered by the checks of the GEMV and the GEMM)
   const bool operands = X && Wq && S && Y;
   const Route route = operands || M > 16 ? plain_route(*st, X, Wq, S, Y, M, N, K, G, flags) : kRouteGemv;
-  if (route == kRouteGemvTc || route == kRouteManyTc)
+  if (route == kRouteGemvTc)
     return b2::gemv_tc_launch(X, Wq, S, Y, M, N, K, st->ws, flags, st->sm_count, s);
   if (route == kRouteGemv) return b2::gemv_launch(X, Wq, S, Y, M, N, K, G, st->ws, flags, st->sm_count, s);
   return b2::gemm_launch(X, Wq, S, Y, M, N, K, G, st->ws, flags, st->sm_count, s);
@@ -205,9 +204,7 @@ int b2_w4_gemv_describe(int M, int N, int K, int G, int flags, char* buf, int bu
   if (!buf || buflen < 1) return b2::kErrBadPointer;
   const Route route =
       M < 1 ? kRouteGemv : plain_route(*st, nullptr, nullptr, nullptr, nullptr, M, N, K, G, flags);
-  if ((route == kRouteGemvTc || route == kRouteManyTc) &&
-      b2::gemv_tc_describe(M, N, K, flags, st->sm_count, route == kRouteManyTc, buf, buflen) > 0)
-    return 0;
+  if (route == kRouteGemvTc && b2::gemv_tc_describe(M, N, K, flags, st->sm_count, buf, buflen) > 0) return 0;
   if (route == kRouteGemm && b2::gemm_describe(M, N, K, G, st->ws, flags, st->sm_count, buf, buflen) > 0) return 0;
   return b2::gemv_describe(M, N, K, G, flags, st->sm_count, st->ws.partial_bytes, st->ws.n_counters - 1, buf, buflen);
 }

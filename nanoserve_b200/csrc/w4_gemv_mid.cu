@@ -1,6 +1,6 @@
 // W4A16 decode GEMV for sm_100a, several tokens (five to sixteen; two to four where K is long):
-// Y[M,N] (bf16) = X[M,K] (bf16) . dequant(Wq, S)^T.  (Plain calls it serves run on tcgen05 instead where gemv_tc_shorter says so,
-// which is most of them: w4_gemv_tc.cu.)
+// Y[M,N] (bf16) = X[M,K] (bf16) . dequant(Wq, S)^T.  (Of plain calls only those are left to it that gemv_tc_shorter,
+// w4_gemv_tc.cu, estimates to be shorter here: a few rows with a long K, many rows with a K of a few hundred.)
 //
 // Replaces the reference's w4a16_gemv_kernel / w4a16_gemv (kernels/quant/w4a16.cuh:42-115) for the token counts at
 // which its own analysis (README.md:137-146) finds it compute-bound.  G == 128, K % 256 == 0, a staged X that fits in

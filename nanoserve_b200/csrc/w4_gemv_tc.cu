@@ -639,34 +639,11 @@ bool tc_operands(const void* X, const void* Wq, const void* S, const void* Y, in
 
 }  // namespace
 
-// The calls that come here by name: flags that ask for this kernel, and nine to sixteen tokens on the shapes below (a line
-// through steps of 256 rows and of 128, drawn when a step took 0.62 and 0.5 to 1.0 us, against 6 + 0.145 w + 3 K / 1e4 us of the
-// mma.sync kernel, w = millions of weights).  What the line leaves to the other kernels comes here from there where it is the
-// shorter way (gemv_tc_shorter).
 // (Pointers: null = "assume aligned", for the queries that have no operands.)
-bool gemv_tc_applies(const void* X, const void* Wq, const void* S, const void* Y, int M, int N, int K, int G, int flags,
-                     int sm_count) {
-  if (!tc_operands(X, Wq, S, Y, M, N, K, G)) return false;
-  if (flags < 0) {
-    TcPlan pl;
-    return tc_plan(M, N, K, sm_count, (flags >> 24) & 3, (flags >> 20) & 15, &pl);
-  }
-  if ((flags & ~kFlagNoPdl) != 0 || M <= 8 || (K <= 256 && N < 5000)) return false;
-  const int nkb = K / kStepK;
-  double best = 1e30;
-  for (int ks = 1; ks <= 8 && ks <= nkb; ++ks) {
-    const int steps = (nkb + ks - 1) / ks;
-    for (int form = 0; form < 2; ++form) {
-      if (steps > (form ? 39 : 19)) continue;  // (the converted X of a CTA's steps was held in shared memory)
-      const double cap = (form ? 1 : 2) * sm_count * (ks == 1 ? 1.0 : ks == 7 ? 0.7 : ks == 8 ? 0.8 : 0.87);
-      const long ctas = (long)((N + (form ? 255 : 127)) / (form ? 256 : 128)) * ks, waves = (long)std::ceil(ctas / (double)(long)cap);
-      const double busy = std::min(1.0, (double)ctas / waves / (2.0 * sm_count));
-      const double us =
-          waves * (form ? 4.6 + 0.62 * steps : 3.8 + (0.5 + 0.5 * busy) * steps + (steps == 1 ? 2.0 * busy : 0.0));
-      best = std::min(best, us * (form == 0 && steps >= 9 ? 1.1 : 1.04));
-    }
-  }
-  return best < 6.0 + 0.145e-6 * ((double)N * K) + 3e-4 * K;
+bool gemv_tc_serves(const void* X, const void* Wq, const void* S, const void* Y, int M, int N, int K, int G, int flags,
+                    int sm_count) {
+  TcPlan pl;
+  return tc_operands(X, Wq, S, Y, M, N, K, G) && tc_plan(M, N, K, sm_count, (flags >> 24) & 3, (flags >> 20) & 15, &pl);
 }
 
 // Whether this kernel is shorter than the GEMV that would take a plain call of 2 to 16 tokens, `other` one of kTcOther*.  Lines drawn
@@ -704,7 +681,7 @@ bool gemv_tc_shorter(const void* X, const void* Wq, const void* S, const void* Y
   return 1.02 * us < gemv_mid_us(M, N, K, sm_count, partial_cap);
 }
 
-int gemv_tc_describe(int M, int N, int K, int flags, int sm_count, bool many, char* buf, int buflen) {
+int gemv_tc_describe(int M, int N, int K, int flags, int sm_count, char* buf, int buflen) {
   const bool forced = flags < 0;
   TcPlan pl;
   if (!tc_plan(M, N, K, sm_count, forced ? (flags >> 24) & 3 : 0, forced ? (flags >> 20) & 15 : 0, &pl)) return 0;
@@ -712,9 +689,9 @@ int gemv_tc_describe(int M, int N, int K, int flags, int sm_count, bool many, ch
   TcParams p{};
   tc_layout(pl, M, &p);
   return snprintf(buf, buflen,
-                  "%s: %d CTAs (%d per SM), tiles of %d rows x %d tokens, clusters of %d along K, %d planes (%d-bit X), "
-                  "%d ring slots",
-                  many ? "many-token kernel on tcgen05" : "tcgen05 GEMV", (N + rows - 1) / rows * pl.ks, pl.form ? 1 : 2, rows,
+                  "tcgen05 GEMV: %d CTAs (%d per SM), tiles of %d rows x %d tokens, clusters of %d along K, %d planes (%d-bit "
+                  "X), %d ring slots",
+                  (N + rows - 1) / rows * pl.ks, pl.form ? 1 : 2, rows,
                   tc_tokens(M), pl.ks, M <= 4 ? 4 : 2, M <= 4 ? 32 : 16, p.sw);
 }
 

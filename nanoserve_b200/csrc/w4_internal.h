@@ -130,12 +130,13 @@ int gemm_narrow_launch(const void* X, const void* Wq, const void* S, void* Y, in
                        const Workspace& ws, int flags, int sm_count, cudaStream_t stream);
 int gemm_describe(int M, int N, int K, int G, const Workspace& ws, int flags, int sm_count, char* buf, int buflen);
 int gemm_narrow_describe(int M, int N, int K, int G, int flags, int sm_count, char* buf, int buflen);
-int gemv_tc_describe(int M, int N, int K, int flags, int sm_count, bool many, char* buf, int buflen);
+int gemv_tc_describe(int M, int N, int K, int flags, int sm_count, char* buf, int buflen);
 // Whether the tcgen05 GEMV is shorter for a plain call than the kernel that the GEMV's own rules give it.
 enum TcOther { kTcOtherMany, kTcOtherStream, kTcOtherRing };
 bool gemv_tc_shorter(const void* X, const void* Wq, const void* S, const void* Y, int M, int N, int K, int G, int flags,
                      int sm_count, size_t partial_cap, TcOther other);
-bool gemv_tc_applies(const void* X, const void* Wq, const void* S, const void* Y, int M, int N, int K, int G, int flags,
+// Whether it can serve a call that asks for it by kFlagDecodeNarrow.
+bool gemv_tc_serves(const void* X, const void* Wq, const void* S, const void* Y, int M, int N, int K, int G, int flags,
                      int sm_count);
 int gemv_tc_launch(const void* X, const void* Wq, const void* S, void* Y, int M, int N, int K, const Workspace& ws,
                    int flags, int sm_count, cudaStream_t stream);

@@ -1,5 +1,5 @@
 """GPU parity tests of the many-token decode GEMV (2 <= M <= 16 -- by default from five tokens, from two where K is
-long, nine to sixteen only where the tcgen05 kernel is not estimated shorter --, G == 128, K % 256 == 0; plain launches), through the C ABI, against the CPU oracle.
+long, and only where the tcgen05 kernel is not estimated shorter --, G == 128, K % 256 == 0; plain launches), through the C ABI, against the CPU oracle.
 
 The kernel carries X as 16-bit block fixed point per (token, 128-chunk), like the ring kernel: the int4 unpack must be
 bit-exact; bf16 outputs are within one correct rounding plus 2e-5 of the largest output on N(0,1) inputs (each element

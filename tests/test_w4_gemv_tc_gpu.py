@@ -81,19 +81,20 @@ def test_alignments(kernels, y_off, s_off):
         assert np.array_equal(torch_to_bits(y), run(kernels, X, Wq, S, FLAG_DECODE_NARROW))
 
 
-# tokens, rows, columns, the kernel that was the shorter one, us of the many-token and of this kernel
+# tokens, rows, columns, the shorter kernel, us of the many-token and of this kernel
 @pytest.mark.parametrize("M,N,K,kernel", [
-    (10, 1500, 11008, "many-token kernel"),  # 11.0, 13.9
-    (11, 1444, 9472, "many-token kernel"),  # 10.6, 12.8
-    (16, 57344, 8192, "many-token kernel"),  # 88, 96
-    (16, 700, 256, "many-token kernel"),  # 3.3, 4.1
-    (13, 512, 3584, "tcgen05 GEMV"),
-    (9, 545, 768, "tcgen05 GEMV"),  # 5.7, 4.2
-    (13, 3584, 3584, "tcgen05 GEMV"),  # 9.4, 7.8
-    (13, 10240, 8192, "tcgen05 GEMV"),  # 24.6, 19.2
-    (13, 14336, 4096, "tcgen05 GEMV"),  # 17.6, 14.6
-    (13, 37888, 3584, "tcgen05 GEMV"),  # 25.9, 21.7
-    (16, 3584, 18944, "tcgen05 GEMV"),  # 20.8, 18.1
+    (10, 1500, 11008, "tcgen05 GEMV"),  # 10.8, 10.2
+    (11, 1444, 9472, "tcgen05 GEMV"),  # 10.4, 9.2
+    (16, 57344, 8192, "tcgen05 GEMV"),  # 93, 74
+    (16, 700, 256, "tcgen05 GEMV"),  # 3.3, 3.2
+    (16, 144, 19456, "many-token kernel"),  # 9.0, 11.4
+    (13, 512, 3584, "tcgen05 GEMV"),  # 7.3, 4.5
+    (9, 545, 768, "tcgen05 GEMV"),  # 5.7, 3.5
+    (13, 3584, 3584, "tcgen05 GEMV"),  # 9.5, 6.7
+    (13, 10240, 8192, "tcgen05 GEMV"),  # 24.2, 15.8
+    (13, 14336, 4096, "tcgen05 GEMV"),  # 17.3, 12.2
+    (13, 37888, 3584, "tcgen05 GEMV"),  # 26.0, 18.1
+    (16, 3584, 18944, "tcgen05 GEMV"),  # 20.6, 14.8
 ])
 def test_rule_takes_the_shorter_kernel(kernels, M, N, K, kernel):
     assert kernels.gemv_describe(M, N, K, 128).startswith(kernel)

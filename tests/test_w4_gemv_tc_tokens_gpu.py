@@ -5,7 +5,7 @@ import pytest
 import torch
 
 import oracle
-from nanoserve_b200.ops import FLAG_DECODE_NARROW, FLAG_NO_PDL, narrow_flags
+from nanoserve_b200.ops import FLAG_DECODE_NARROW, FLAG_MID_KERNEL, FLAG_NO_PDL, FLAG_RING_KERNEL, narrow_flags
 from tests.util import bits_to_torch, check_bf16_output, torch_to_bits, u32_to_torch
 
 pytestmark = pytest.mark.gpu
@@ -100,3 +100,13 @@ def test_rule_takes_the_shorter_kernel(kernels, M, N, K, here):
 ])
 def test_rule_leaves_calls_where_they_are_shorter(kernels, M, N, K):
     assert "tcgen05" not in kernels.gemv_describe(M, N, K, 128)
+
+
+@pytest.mark.parametrize("M,N,K", [(5, 2300, 2048), (8, 700, 256), (16, 1500, 11008), (10, 178, 26112), (2, 900, 2560)])
+def test_a_plain_call_runs_the_kernel_it_is_described_as(kernels, M, N, K):
+    """The kernels differ in the order of their fp32 sums: the call's bits are those of the kernel with its name."""
+    flags = {"tcgen05 GEMV": FLAG_DECODE_NARROW, "many-token kernel": FLAG_MID_KERNEL, "ring kernel": FLAG_RING_KERNEL}
+    name = kernels.gemv_describe(M, N, K, 128).split(":")[0]
+    assert kernels.gemv_describe(M, N, K, 128, flags[name]) == kernels.gemv_describe(M, N, K, 128)
+    X, Wq, S = oracle.synth_inputs(M, N, K, 128, seed=8)
+    assert np.array_equal(run(kernels, X, Wq, S, 0), run(kernels, X, Wq, S, flags[name]))
