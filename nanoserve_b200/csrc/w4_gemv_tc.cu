@@ -660,15 +660,10 @@ bool gemv_tc_serves(const void* X, const void* Wq, const void* S, const void* Y,
 //     20.0 against 14.6): 32 of 303 calls run here, none lost.  At three and four tokens X has 32 bits here and 16 there: level
 //     above eighty million weights (2 of 11 lost, 6 %), shorter there below.
 //   * Ring kernel: never shorter (1840 calls, 1.65 times as fast here, one lost).
-// Two tokens on up to two million weights stay with the ring kernel: the tensor-parallel form of such a call gives its bits.
-// Up to 512 rows at five to eight tokens stay with the many-token kernel's slices of K, 6.6 us against 3.9 at 512 x 3584: callers
-// rely on the plan that gemv_describe names there.
 bool gemv_tc_shorter(const void* X, const void* Wq, const void* S, const void* Y, int M, int N, int K, int G, int flags,
                      int sm_count, size_t partial_cap, TcOther other) {
   if (M < 2 || (flags & ~kFlagNoPdl) != 0 || !tc_operands(X, Wq, S, Y, M, N, K, G)) return false;
   const double w = 1e-6 * N * K, k3 = 1e-3 * K, mk = 1e-4 * M * K;
-  if (other == kTcOtherRing && M == 2 && w <= 2.0) return false;
-  if (other == kTcOtherMany && M >= 5 && M <= 8 && N <= 512) return false;
   TcPlan pl;
   if (!tc_plan(M, N, K, sm_count, 0, 0, &pl)) return false;
   if (other == kTcOtherRing) return true;

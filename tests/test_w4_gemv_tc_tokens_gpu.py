@@ -76,7 +76,8 @@ def test_rule_on_layer_shapes(kernels, M, N, K):
 @pytest.mark.parametrize("M,N,K,here", [
     (2, 18944, 3584, False),  # 8.9 and 10.0
     (4, 22705, 1024, False),  # 4.8, 5.4
-    (8, 512, 3584, False),    # (6.6, 3.9: stays, see the rule)
+    (8, 512, 3584, True),     # 6.6, 3.9
+    (2, 512, 3584, True),     # 6.7, 3.6
     (1, 37888, 3584, False),  # 13.7, 15.7
     (4, 3584, 3584, True),    # 7.5, 5.6
     (8, 700, 256, True),      # 3.1, 2.5
