@@ -655,9 +655,9 @@ bool gemv_tc_serves(const void* X, const void* Wq, const void* S, const void* Y,
 //     lost, up to 55 %, small matrices of long K most: 10 x 178 x 26112 14.5 us against 9.4, 16 x 290 x 22784 12.0 against 10.7.)
 //   * Many-token kernel, two to four tokens (K >= 8192): X has 32 bits here and 16 there, so what a line in w (millions of weights),
 //     M and K brought here stays.  1.19 times as fast in the geometric mean, 18 of 801 calls lost (15 %).
-//   * Streaming kernel at two tokens: shorter (18944 x 3584 9.2 us against 11.4, 37888 x 3584 14.6 against 15.5) except where one
-//     CTA to an SM is all it has and K is longer than its ring and X leave room for (17570 x 4096 13.4 against 11.3, 14739 x 6912
-//     20.0 against 14.6): 32 of 303 calls run here, none lost.  At three and four tokens X has 32 bits here and 16 there: level
+//   * Streaming kernel at two tokens: shorter (18944 x 3584 9.2 us against 11.4, 37888 x 3584 14.6 against 15.5, 18928 x 4096 10.2
+//     against 11.9) except where its CTAs of 128 rows leave SMs over, which it fills by twice the warps per tile, and K is long
+//     (17570 x 4096 13.4 against 11.3, 14739 x 6912 20.0 against 14.6): of 106 calls that this takes 2 are lost (10 %).  At three and four tokens X has 32 bits here and 16 there: level
 //     above eighty million weights (2 of 11 lost, 6 %), shorter there below.
 //   * Ring kernel: never shorter (1840 calls, 1.65 times as fast here, one lost).
 bool gemv_tc_shorter(const void* X, const void* Wq, const void* S, const void* Y, int M, int N, int K, int G, int flags,
@@ -668,7 +668,7 @@ bool gemv_tc_shorter(const void* X, const void* Wq, const void* S, const void* Y
   if (!tc_plan(M, N, K, sm_count, 0, 0, &pl)) return false;
   if (other == kTcOtherRing) return true;
   if (other == kTcOtherStream)
-    return M == 2 ? K >= 3840 && N <= 128 * sm_count : w >= 80.0 && 1.02 * pl.us < 2.6 + 0.094 * w + 0.011 * k3 + 1.75 * mk;
+    return M == 2 ? K >= 3840 && N <= 128 * (sm_count - 1) : w >= 80.0 && 1.02 * pl.us < 2.6 + 0.094 * w + 0.011 * k3 + 1.75 * mk;
   if (M <= 4) return 1.02 * pl.us < 6.65 + 0.11 * w + 0.027 * k3 + 0.074 * mk;
   const double us = pl.us + (pl.form       ? 2.03 * pl.busy * pl.busy
                              : pl.several ? 0.5

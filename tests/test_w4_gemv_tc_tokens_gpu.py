@@ -98,6 +98,7 @@ def test_rule_takes_the_shorter_kernel(kernels, M, N, K, here):
     (7, 54677, 256),    # 6.3, 7.6
     (2, 29616, 5632),   # 19.3, 21.7
     (2, 37888, 3584),   # 14.6, 15.5
+    (2, 18928, 4096),   # 10.2, 11.9
 ])
 def test_rule_leaves_calls_where_they_are_shorter(kernels, M, N, K):
     assert "tcgen05" not in kernels.gemv_describe(M, N, K, 128)
