@@ -633,7 +633,7 @@ bool tc_plan(int M, int N, int K, int sm_count, int wanted_form, int wanted_ks, 
 
 bool tc_operands(const void* X, const void* Wq, const void* S, const void* Y, int M, int N, int K, int G) {
   if (G != kStepK || K < 2 * kStepK || K % (2 * kStepK) || N < 1 || M < 1 || M > kTokens) return false;
-  return !(((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(Wq)) & 15) || (reinterpret_cast<uintptr_t>(Y) & 7) ||
+  return !(((reinterpret_cast<uintptr_t>(X) | reinterpret_cast<uintptr_t>(Wq)) & 15) || (reinterpret_cast<uintptr_t>(Y) & 1) ||
            (reinterpret_cast<uintptr_t>(S) & 3));
 }
 

@@ -65,7 +65,7 @@ def test_extreme_inputs(kernels):
 
 @pytest.mark.parametrize("y_off,s_off", [(4, 0), (2, 0), (0, 2), (0, 1), (1, 1)])
 def test_alignments(kernels, y_off, s_off):
-    """Y from 8 bytes and S from 4 run this kernel, anything less the kernel that serves it: within the same bounds."""
+    """S from 4 bytes and any Y run this kernel, anything less the kernel that serves it: within the same bounds."""
     M, N, K = 13, 1000, 1536
     X, Wq, S = oracle.synth_inputs(M, N, K, 128, seed=6)
     out = torch.zeros(M * N + 8, dtype=torch.bfloat16, device="cuda")
@@ -77,7 +77,7 @@ def test_alignments(kernels, y_off, s_off):
     assert kernels.device_status() == 0
     check_bf16_output(torch_to_bits(y), oracle.w4_linear_f32(X, Wq, S, 128), SLACK)
     assert not out[:y_off].any() and not out[y_off + M * N:].any()
-    if y_off % 4 == 0 and s_off % 2 == 0:
+    if s_off % 2 == 0:
         assert np.array_equal(torch_to_bits(y), run(kernels, X, Wq, S, FLAG_DECODE_NARROW))
 
 

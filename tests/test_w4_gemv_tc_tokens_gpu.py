@@ -37,6 +37,26 @@ def test_tiles_and_splits(kernels, tile, split):
         assert np.array_equal(y, run(kernels, X, Wq, S, flags | FLAG_NO_PDL))
 
 
+@pytest.mark.parametrize("M,K", [(2, 1024), (3, 1536), (8, 768)])  # scales by four, by four and by two
+@pytest.mark.parametrize("y_off,s_off", [(0, 0), (1, 0), (2, 2), (3, 4), (0, 1), (1, 3)])
+def test_alignments(kernels, M, K, y_off, s_off):
+    """The outputs are stored one by one, wherever they start; scales are loaded in pairs or fours, and where S starts at an odd
+    one another kernel runs, within the 16-bit form's bound."""
+    N = 1000
+    X, Wq, S = oracle.synth_inputs(M, N, K, 128, seed=6)
+    out = torch.full((M * N + 8,), 7.0, dtype=torch.bfloat16, device="cuda")
+    y = out[y_off:y_off + M * N].view(M, N)
+    s = torch.empty(S.size + 8, dtype=torch.bfloat16, device="cuda")[s_off:s_off + S.size].view(*S.shape)
+    s.copy_(bits_to_torch(S))
+    kernels.w4_linear(bits_to_torch(X), u32_to_torch(Wq), s, 128, out=y)
+    torch.cuda.synchronize()
+    assert kernels.device_status() == 0
+    check_bf16_output(torch_to_bits(y), oracle.w4_linear_f32(X, Wq, S, 128), slack(M) if s_off % 2 == 0 else 2e-5)
+    assert bool((out[:y_off] == 7.0).all()) and bool((out[y_off + M * N:] == 7.0).all())
+    if s_off % 2 == 0:
+        assert np.array_equal(torch_to_bits(y), run(kernels, X, Wq, S, FLAG_DECODE_NARROW))
+
+
 @pytest.mark.parametrize("M", [4, 8, 16])
 def test_longest_k_of_a_cta(kernels, M):
     N, K = 130, 28672  # 112 pairs in one CTA
