@@ -4,6 +4,10 @@ import shutil
 
 import pytest
 import torch
+import torch.autograd.forward_ad as fwAD
+from torch._subclasses.fake_tensor import FakeTensorMode
+from torch.overrides import TorchFunctionMode
+from torch.utils._python_dispatch import TorchDispatchMode
 
 from nanoserve_b200 import ops
 
@@ -80,3 +84,81 @@ def test_errors_and_streams(kernels, call):
     graph.replay()
     torch.cuda.synchronize()
     assert torch.equal(y, kernels.w4_linear(x, wq, s))
+
+
+@pytest.mark.gpu
+def test_hands_back_cuda_calls_that_are_not_plain(kernels, call):
+    """On CUDA tensors, so that nothing but the subclass, the mode or the transform is the reason; the call through ctypes then
+    answers or refuses as it does without the extension."""
+    g = torch.Generator(device="cuda").manual_seed(2)
+    N, K = 96, 512
+    wq = torch.randint(-2**31, 2**31 - 1, (N, K // 8), dtype=torch.int32, device="cuda", generator=g)
+    s = torch.rand(N, K // 128, device="cuda", generator=g).to(torch.bfloat16)
+    x = torch.randn(3, K, device="cuda", generator=g).to(torch.bfloat16)
+    out = torch.empty(3, N, dtype=torch.bfloat16, device="cuda")
+    linear = lambda *a: ops._call_linear(kernels._linear, *a[:3], 128, 0, a[3] if len(a) > 3 else None)
+    quantize = lambda w: ops._call_quantize(kernels._quantize, w, 128)
+    want, want_q = linear(x, wq, s), quantize(x)
+    assert isinstance(want, torch.Tensor) and torch.equal(want_q[0], kernels.w4_quantize(x)[0])
+    assert linear(x[0], wq, s) is NotImplemented and quantize(x[0]) is NotImplemented
+
+    class Sub(torch.Tensor):
+        pass
+
+    for i in range(4):
+        args = [x, wq, s, out]
+        args[i] = args[i].as_subclass(Sub)
+        assert linear(*args) is NotImplemented
+        assert torch.equal(kernels.w4_linear(*args[:3], out=args[3]), want)
+    assert quantize(x.as_subclass(Sub)) is NotImplemented
+
+    seen = []
+
+    class Dispatch(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            seen.append(str(func))
+            return func(*args, **(kwargs or {}))
+
+    class Function(TorchFunctionMode):
+        def __torch_function__(self, func, types, args=(), kwargs=None):
+            seen.append(getattr(func, "__name__", str(func)))
+            return func(*args, **(kwargs or {}))
+
+    for mode in (Dispatch(), Function(), torch.device("cpu")):
+        seen.clear()
+        with mode:
+            assert linear(x, wq, s) is NotImplemented and quantize(x) is NotImplemented
+            got = kernels.w4_linear(x, wq, s)
+        assert got.is_cuda and torch.equal(got, want)
+        assert isinstance(mode, torch.device) or any("empty" in name for name in seen)  # the mode sees the allocation
+    with FakeTensorMode(allow_non_fake_inputs=True):
+        assert linear(x, wq, s) is NotImplemented
+
+    def mapped(v):
+        assert linear(v, wq, s) is NotImplemented and linear(x, wq, s) is NotImplemented
+        assert quantize(v) is NotImplemented
+        with pytest.raises(RuntimeError):  # a batched tensor has no data pointer
+            kernels.w4_linear(v, wq, s)
+        return v
+
+    torch.func.vmap(mapped)(torch.stack([x, x]))
+    assert torch.equal(linear(x, wq, s), want)
+
+
+@pytest.mark.gpu
+def test_grad_modes(kernels, call):
+    """Calls under inference mode or with a tangent are taken: the outputs are what the call through ctypes makes of them."""
+    wq = torch.full((64, 32), 0x12345678, dtype=torch.int32, device="cuda")
+    s = torch.ones(64, 2, dtype=torch.bfloat16, device="cuda")
+    x = torch.ones(1, 256, dtype=torch.bfloat16, device="cuda", requires_grad=True)
+    slow = ops.Kernels()
+    slow._linear = slow._quantize = None
+    assert ops._call_linear(kernels._linear, x, wq, s, 128, 0, None) is not NotImplemented
+    with torch.inference_mode():
+        a, b = kernels.w4_linear(x, wq, s), slow.w4_linear(x, wq, s)
+        assert a.is_inference() and b.is_inference() and torch.equal(a, b)
+    with fwAD.dual_level():
+        dual = fwAD.make_dual(x.detach(), torch.ones_like(x))
+        a, b = kernels.w4_linear(dual, wq, s), slow.w4_linear(dual, wq, s)
+        assert fwAD.unpack_dual(a).tangent is None and fwAD.unpack_dual(b).tangent is None and torch.equal(a, b)
+    assert not kernels.w4_linear(x, wq, s).requires_grad

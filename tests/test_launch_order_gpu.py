@@ -18,8 +18,8 @@ def rand_x(M, K, gen):
     return torch.randn(M, K, device="cuda", generator=gen).to(torch.bfloat16)
 
 
-@pytest.mark.parametrize("M,G,flags", [(13, 128, FLAG_DECODE_NARROW), (4, 64, FLAG_DECODE_NARROW), (48, 128, FLAG_GEMM_NARROW),
-                                       (48, 32, FLAG_GEMM_NARROW), (300, 128, 0)])
+@pytest.mark.parametrize("M,G,flags", [(3, 128, FLAG_DECODE_NARROW), (8, 128, FLAG_DECODE_NARROW), (13, 128, FLAG_DECODE_NARROW),
+                                       (4, 64, FLAG_DECODE_NARROW), (48, 128, FLAG_GEMM_NARROW), (48, 32, FLAG_GEMM_NARROW), (300, 128, 0)])
 def test_weights_written_by_the_kernel_in_front(kernels, M, G, flags):
     """The kernel in front lets its dependents start at once and stores at its end: a linear whose output is the next one's
     scales, or its packed words.  The result is that of the same launches with a synchronisation in between."""
@@ -53,7 +53,7 @@ def test_weights_written_by_the_kernel_in_front(kernels, M, G, flags):
     assert kernels.device_status() == 0
 
 
-@pytest.mark.parametrize("M", [13, 48])
+@pytest.mark.parametrize("M", [3, 8, 13, 48])
 def test_linear_behind_its_quantizer(kernels, M):
     gen = torch.Generator(device="cuda").manual_seed(M)
     W, x = rand_x(5000, 3584, gen), rand_x(M, 3584, gen)
@@ -88,7 +88,8 @@ def long_launch(kernels):
     return go
 
 
-@pytest.mark.parametrize("M,G,flags", [(13, 128, FLAG_DECODE_NARROW), (4, 64, FLAG_DECODE_NARROW), (48, 128, FLAG_GEMM_NARROW)])
+@pytest.mark.parametrize("M,G,flags", [(3, 128, FLAG_DECODE_NARROW), (8, 128, FLAG_DECODE_NARROW), (13, 128, FLAG_DECODE_NARROW),
+                                       (4, 64, FLAG_DECODE_NARROW), (48, 128, FLAG_GEMM_NARROW)])
 def test_wait_for_a_long_launch_is_no_time_out(kernels, long_launch, M, G, flags):
     gen = torch.Generator(device="cuda").manual_seed(M)
     x, (Wq, S) = rand_x(M, 1024, gen), rand_w4(1024, 1024, G, gen)
@@ -100,7 +101,7 @@ def test_wait_for_a_long_launch_is_no_time_out(kernels, long_launch, M, G, flags
 
 
 @pytest.mark.parametrize("M,N,K,G", [(1, 3584, 3584, 128), (4, 1000, 2048, 64), (8, 3584, 18944, 128), (13, 3584, 3584, 128),
-                                     (16, 3584, 18944, 32), (48, 4608, 3584, 128), (2, 1000, 2048, 32)])
+                                     (16, 3584, 18944, 32), (48, 4608, 3584, 128), (2, 1000, 2048, 32), (2, 512, 3584, 128), (3, 3584, 3584, 128)])
 def test_a_plain_launch_runs_the_same_kernel(kernels, M, N, K, G):
     assert kernels.gemv_describe(M, N, K, G, FLAG_NO_PDL) == kernels.gemv_describe(M, N, K, G)
     gen = torch.Generator(device="cuda").manual_seed(N)
@@ -109,7 +110,7 @@ def test_a_plain_launch_runs_the_same_kernel(kernels, M, N, K, G):
     assert kernels.device_status() == 0
 
 
-@pytest.mark.parametrize("M,G", [(1, 128), (4, 128), (13, 128), (16, 128), (4, 64), (16, 32), (48, 128), (300, 64)])
+@pytest.mark.parametrize("M,G", [(1, 128), (3, 128), (4, 128), (8, 128), (13, 128), (16, 128), (4, 64), (16, 32), (48, 128), (300, 64)])
 def test_chain_of_dependent_launches(kernels, M, G):
     """Linears that read one another's outputs and write into buffers that are still being read, eager and captured: bit for
     bit the chain with a synchronisation after each launch."""
