@@ -366,15 +366,17 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         const uint32_t s2 = s2_next;
         if (i + 1 < nkb) s2_next = load_scale(kb0 + i + 1);
 
-        // Asking a barrier takes some 100 cycles, complete or not: both questions of the block go ahead of the conversion, and
-        // the next block's words are loaded behind it.  (With one arrival per warp instead of per thread and 17 instead of 19
-        // instructions per word: 18944 x 3584 at 300 / 512 tokens 52.2 / 54.3 -> 51.1 / 53.5 us, 37888 x 3584 at 512 118 -> 116.)
-        const bool free = mbar_try_wait(bar_bd_empty + 8 * b, bph ^ 1);
+        // An answer takes some 100 cycles: both questions of the block go ahead of the conversion, and the next block's words
+        // are loaded behind it.  They do not wait (a try_wait may, ahead of a conversion that needs neither answer: 28672 x
+        // 8192 at 200 tokens 130.0 -> 128.5 us).  With one arrival per warp instead of per thread and 17 instead of 19
+        // instructions per word, 18944 x 3584 at 300 / 512 / 1024 tokens 52.6 / 53.8 / 105.8 -> 51.5 / 52.9 / 104.1 us, 37888 x
+        // 3584 at 512 108.3 -> 106.8; tiles of 128 tokens, which wait for HBM, 1 % longer (28672 x 8192 at 200 126.5).
+        const bool free = mbar_test_wait(bar_bd_empty + 8 * b, bph ^ 1);
         const int s_this = s;
         if (++s == geo::kStages) { s = 0; ph ^= 1; }
         const bool more = i + 1 < nkb;
         bool there = more;
-        if (more) there = mbar_try_wait(w_full + 8 * s, ph);
+        if (more) there = mbar_test_wait(w_full + 8 * s, ph);
         uint4 o[kWords];
 #pragma unroll
         for (int c = 0; c < kWords; ++c) {

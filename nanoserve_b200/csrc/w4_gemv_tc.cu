@@ -15,7 +15,7 @@
 //     groups (no second launch, one cluster barrier behind the sums).
 // What bounds it: from the wait for the kernel in front to the last pair it runs at HBM's rate (37888 x 3584 at four tokens: 10.4
 // of 15.9 us for 70 MB); the rest is the boundary between launches (1.7 us), barriers and tensor memory before it (0.7), the
-// last sums and stores (1.3).  What the pairs are for: asking a barrier takes a warp some 130 cycles even where the answer is
+// last sums and stores (1.3).  What the pairs are for: an answer of a barrier takes a warp some 130 cycles even where it is
 // yes, an arrival with its fence 100, and a chunk at a time with one group (0.55 us per chunk of 256 rows, HBM 0.37) these were
 // most of a step.  Measured, weights from HBM, us at 4 / 8 / 13 tokens, in brackets the shortest of the mma.sync kernels and, at
 // 13, this kernel before (a chunk per step, X converted first): 37888 x 3584 15.9 / 16.5 / 18.1 (15.8 / 19.3 / 21.5), 3584 x
@@ -106,8 +106,7 @@ __device__ __forceinline__ void tmem_ld_sums(uint32_t taddr, uint32_t (&d)[16]) 
   }
 }
 
-// All questions of a pair of steps in one go: asking a barrier takes some 100 cycles, complete or not, and one after the
-// other they add up.
+// All questions of a pair of steps in one go: an answer takes some 100 cycles, and one after the other they add up.
 __device__ __forceinline__ bool mbar_try_wait2(uint32_t bar0, uint32_t parity0, uint32_t bar1, uint32_t parity1) {
   uint32_t ok;
   asm volatile(
@@ -360,7 +359,7 @@ __global__ void __launch_bounds__(MB == 2 ? 896 : 512, MB == 2 ? 1 : 2)
           vb[u] = vb[u + 1];
         }
         load(step + kXAhead * kStride, va[kXAhead - 1], vb[kXAhead - 1]);
-        const bool room = mbar_try_wait(bar_x_empty + 8 * sl, xph);
+        const bool room = mbar_test_wait(bar_x_empty + 8 * sl, xph);
         uint32_t mx2 = 0;
 #pragma unroll
         for (int i = 0; i < 8; ++i) mx2 = __vmaxu2(mx2, w[i] & 0x7FFF7FFFu);

@@ -40,3 +40,10 @@ def test_scale_prefetches_are_bounded():
     assert len(found) == sum(s.count("prefetch_l2(s_row") for s in SOURCES.values()) >= 2
     for cond, at in found:
         assert re.search(r"\b%s < p\.KG" % at, cond), (cond, at)
+
+
+def test_questions_ahead_of_work_do_not_wait():
+    """A try_wait may suspend the warp for a while: an answer that is only used behind a block's conversion is asked for by
+    test_wait, and try_wait stands where nothing else is left to do (in the waits of ptx.cuh and in pairs of questions)."""
+    for name, s in SOURCES.items():
+        assert not re.search(r"= mbar_try_wait\(", s), name
