@@ -25,9 +25,11 @@ def test_named_barriers_and_the_status_word(name):
         assert body.startswith("const bool poisoned = *status_seen != 0;", decision)
     else:
         assert body.startswith("const bool poisoned = __any_sync(", decision)
-        barriers = re.findall(r'(if \([^;{}]*\)[^;{}]*)?asm volatile\("(bar\.sync[^"]*)"', body[decision:])
-        met = sorted(b for skipped, b in barriers if skipped.startswith("if (poisoned && "))
-        assert met and met == sorted(b for skipped, b in barriers if not skipped.startswith("if (poisoned && "))
+        work, skipped = body[decision:].split("\n  } else if (p.ks == 1 && warp < kMain) {", 1)
+        skipped = skipped[:skipped.index("\n  }\n")]
+        assert "\n  if (!poisoned) {\n" in work and "bar.sync" not in body[decision + len(work) + len(skipped) + 60:]
+        barriers = [re.findall(r'asm volatile\("(bar\.sync[^;]*);', part) for part in (work, skipped)]
+        assert len(barriers[0]) == 1 == len(barriers[1])
 
 
 def test_scale_prefetches_are_bounded():
