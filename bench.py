@@ -44,8 +44,8 @@ from nanoserve_b200 import synth  # noqa: E402
 
 METRIC = "W4A16 GEMV HBM GB/s at M=1 (Qwen2.5-7B-shaped layer, int4 g128)"
 METRIC_70B = "W4A16 GEMV HBM GB/s at M=1 (70B-class layer: hidden 8192, intermediate 28672, int4 g128)"
-DTYPE = ("int4 weights x bf16 activations; X as block fixed point per (token, 128-chunk) -- 32-bit for one token, 15-bit + "
-         "sign above -- on 8-bit integer mma, s32 accumulation per chunk, fp32 across chunks, bf16 output")
+DTYPE = ("int4 weights x bf16 activations; X as block fixed point per (token, 128-chunk) -- 32-bit for one token, and up to "
+         "four on tcgen05, else 15-bit + sign -- on 8-bit integer mma, s32 accumulation per chunk, fp32 across chunks, bf16 output")
 UNIT = "GB/s"
 G = 128
 M_DECODE = 1
@@ -655,7 +655,7 @@ def main():
         t_e2e_eager = time.perf_counter() - t0
     # the same step as a serving loop would issue it: ShardedLayer.host_step, one CUDA graph per step with the two
     # copies inside (one graph launch + one stream synchronisation per step)
-    t_e2e_wall, e2e_path = t_e2e_eager, "Kernels.w4_linear per launch (ctypes -> C ABI), pinned host X in, all outputs out"
+    t_e2e_wall, e2e_path = t_e2e_eager, "Kernels.w4_linear per launch (C ABI), pinned host X in, all outputs out"
     if not seven:
         host_steps = [l.host_step(M, stream, zero_copy_out=(world == 1)) for l in lb.layers]
         for hs in host_steps:
@@ -836,7 +836,7 @@ def main():
                     "d2h_bytes_per_step": d2h, "ms_per_step": t_e2e_wall / args.steps * 1e3, "path": e2e_path,
                     "per_launch_api": {"value": nbytes * args.steps / t_e2e_eager / 1e9,
                                        "ms_per_step": t_e2e_eager / args.steps * 1e3,
-                                       "path": "Kernels.w4_linear per launch (ctypes -> C ABI), same copies, no graph"}},
+                                       "path": "Kernels.w4_linear per launch (C ABI), same copies, no graph"}},
             "gpu_launches": lb.launches_per_step() * args.steps * (blocks[0] + 1),
             "clocks": clocks,
         }

@@ -589,8 +589,9 @@ int tc_capacity(int form, int ks, int sm_count, int dev) {
 // exchange through the cluster, waves of CTAs that take their pairs of steps at the rate of a warp group's chain or of HBM.  The
 // 128-row form shares an SM with a second CTA where K is cut or there are more CTAs than SMs.  Several waves with K whole have
 // a line of their own (26 shapes of 38000 to 60000 rows): the 256-row form takes whole waves, the 128-row one lets a CTA start
-// wherever one ends (53886 x 5632 at three tokens 35 us against 41; 57344 x 8192 60 against 58).  What it picks takes 1.016 times
-// the best plan's time in the geometric mean; its own time is 2 % short there.
+// wherever one ends (53886 x 5632 at three tokens 35 us against 41; 57344 x 8192 60 against 58).  Over 6472 calls on 1627 shapes what
+// it picks takes 1.016 times the best plan's time in the geometric mean, 1.11 times in one of twenty; its own time is 6 % short there
+// (12 % in the standard deviation), most where the chip is full: gemv_tc_shorter adds that.
 bool tc_plan(int M, int N, int K, int sm_count, int wanted_form, int wanted_ks, TcPlan* out) {
   static constexpr double kChain[2][3] = {{0.541, 0.582, 0.879}, {0.734, 0.775, 0.913}}, kShared[3] = {1.042, 1.121, 1.593};
   static constexpr double kToken[3] = {0.0, 0.141, 0.359}, kWave[3] = {0.84, 0.84, 1.04}, kFluid[3] = {0.87, 0.93, 1.35};
@@ -650,7 +651,7 @@ bool gemv_tc_serves(const void* X, const void* Wq, const void* S, const void* Y,
 // one timed, and 4308 more of the many-token kernel's; "lost" is a call that takes 5 % more time than with the other kernel.
 //   * Many-token kernel, five and more tokens: by the estimates of both, this one's with what plans have in common (they come out
 //     short where the chip is full).  Of 4127 calls at five to eight tokens 44 are lost (at most 20 %), of 3439 above 34 (19 %); the
-//     time is 1.003 and 1.002 times the shorter kernel's in the geometric mean.  (With a line in M, N and K alone 134 and 498 were
+//     time is 1.003 and 1.002 times the shorter kernel's in the geometric mean.  (With a line in M, N and K alone 113 and 496 were
 //     lost, up to 55 %, small matrices of long K most: 10 x 178 x 26112 14.5 us against 9.4, 16 x 290 x 22784 12.0 against 10.7.)
 //   * Many-token kernel, two to four tokens (K >= 8192): X has 32 bits here and 16 there, so what a line in w (millions of weights),
 //     M and K brought here stays.  1.19 times as fast in the geometric mean, 18 of 801 calls lost (15 %).
