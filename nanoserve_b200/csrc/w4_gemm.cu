@@ -370,7 +370,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         // are loaded behind it.  They do not wait (a try_wait may, ahead of a conversion that needs neither answer: 28672 x
         // 8192 at 200 tokens 130.0 -> 128.5 us).  With one arrival per warp instead of per thread and 17 instead of 19
         // instructions per word, 18944 x 3584 at 300 / 512 / 1024 tokens 52.6 / 53.8 / 105.8 -> 51.5 / 52.9 / 104.1 us, 37888 x
-        // 3584 at 512 108.3 -> 106.8; tiles of 128 tokens, which wait for HBM, 1 % longer (28672 x 8192 at 200 126.5).
+        // 3584 at 512 108.3 -> 106.8; tiles of 128 tokens alone 5 to 9 % shorter (37888 x 3584 at 100 54.1 -> 49.2), in pairs
+        // level to 3 % longer (18944 x 3648 at 200 49.7 -> 51.2), with or without the questions.
         const bool free = mbar_test_wait(bar_bd_empty + 8 * b, bph ^ 1);
         const int s_this = s;
         if (++s == geo::kStages) { s = 0; ph ^= 1; }
