@@ -22,8 +22,8 @@
 //            rank-0 CTA, each CTA holding and unpacking half of the weight tile
 //   warps 2-17 dequant: two threads per weight row of the tile, each owning a 32-wide half of the K block (pairs:
 //            four threads per row of the CTA's 128 rows, a 16-wide quarter each):
-//            one 16-byte (8-byte) shared load of packed nibbles, LOP3 unpack to bf16 pairs, exact -8 (bf16x2
-//            subtract), one bf16x2 multiply by the group scale, and four 16-byte stores into a K-major,
+//            one 16-byte (8-byte) shared load of packed nibbles, one bf16x2 fused multiply-add per pair of them with the
+//            group scale (w4_common.cuh; 28672 x 8192 at 4096 tokens 1596 -> 1564 us), and four 16-byte stores into a K-major,
 //            128-byte-swizzled bf16 tile (three buffers in rotation, four for pairs) that the MMA reads through the async
 //            proxy (fence.proxy.async before the arrive)
 //   epilogue the same sixteen warps read the accumulators with tcgen05.ld (32 lanes x 32 columns), convert to
@@ -331,9 +331,6 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
       const int n = n0 + wr0 + r;               // the weight row
       const uint32_t bd_off = geo::kBdOffset + r * 128;  // its place in this CTA's dequantised buffer
       const uint32_t sw = (uint32_t)(r & 7);
-      // unpack constants pinned in registers: each (x & mask) | magic is then a single LOP3
-      uint32_t k_mask = kNibblePairMask, k_magic = kMagic128x2;
-      asm volatile("" : "+r"(k_mask), "+r"(k_magic));
       const __nv_bfloat16* s_row = p.S + (size_t)(n < p.N ? n : 0) * p.KG;
       int s = 0, b = 0;
       uint32_t ph = 0, bph = 0;
@@ -379,11 +376,21 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         bool there = more;
         if (more) there = mbar_test_wait(w_full + 8 * s, ph);
         uint4 o[kWords];
+        if (__all_sync(0xffffffffu, dequant_scale_plain(s2))) {
+          const DequantScale ds = dequant_scale(s2);
 #pragma unroll
-        for (int c = 0; c < kWords; ++c) {
-          uint32_t v[4];
-          dequant_word(words[c], s2, k_mask, k_magic, v);
-          o[c] = make_uint4(v[0], v[1], v[2], v[3]);
+          for (int c = 0; c < kWords; ++c) {
+            uint32_t v[4];
+            dequant_word(words[c], ds, v);
+            o[c] = make_uint4(v[0], v[1], v[2], v[3]);
+          }
+        } else {
+#pragma unroll
+          for (int c = 0; c < kWords; ++c) {
+            uint32_t v[4];
+            dequant_word_any(words[c], s2, v);
+            o[c] = make_uint4(v[0], v[1], v[2], v[3]);
+          }
         }
         if (!__all_sync(0xffffffffu, free)) {
           if (lane == 0) mbar_wait(bar_bd_empty + 8 * b, bph ^ 1, abort_flag);
@@ -446,8 +453,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
               uint32_t* ow = reinterpret_cast<uint32_t*>(&o);
 #pragma unroll
               for (int e = 0; e < 4; ++e) {
-                const __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(v[8 * q + 2 * e]),
-                                                               __uint_as_float(v[8 * q + 2 * e + 1]));
+                const __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(v[8 * q + 2 * e]) * (1.f / kDequantUnit),
+                                                               __uint_as_float(v[8 * q + 2 * e + 1]) * (1.f / kDequantUnit));
                 ow[e] = *reinterpret_cast<const uint32_t*>(&h);
               }
               *reinterpret_cast<uint4*>(yrow + 8 * q) = o;
@@ -455,7 +462,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
           } else {
 #pragma unroll
             for (int e = 0; e < 32; ++e)
-              if (n0 + c0 + e < p.N) yrow[e] = __float2bfloat16(__uint_as_float(v[e]));
+              if (n0 + c0 + e < p.N) yrow[e] = __float2bfloat16(__uint_as_float(v[e]) * (1.f / kDequantUnit));
           }
         }
       }
@@ -485,6 +492,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
 #pragma unroll
               for (int e = 0; e < 32; ++e) sum[e] += __ldcg(pt + e * 128);
             }
+#pragma unroll
+            for (int e = 0; e < 32; ++e) sum[e] *= 1.f / kDequantUnit;
             if (m < p.M) {
               __nv_bfloat16* yrow = p.Y + (size_t)m * p.N + n0 + c0;
               if (vec_ok && n0 + c0 + 32 <= p.N) {

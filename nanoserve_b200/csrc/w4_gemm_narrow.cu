@@ -4,7 +4,7 @@
 // products accumulate in fp32, one rounding at the store.
 //
 // What bounds it: the packed weights' way from HBM (0.5 bytes per weight), and next to it the conversion of every
-// weight (17 instructions per eight).  w4_gemm.cu gives the tokens the 128-row side of the MMA and writes the converted
+// weight (ten instructions per eight, six of them on the ALU pipe at two cycles).  w4_gemm.cu gives the tokens the 128-row side of the MMA and writes the converted
 // weights to shared memory: with 48 tokens it pads the MMA to 128, sends every weight through shared memory twice and
 // has one CTA per 256 weight rows with no way to fill the chip but fp32 part-tiles in global memory.  Here
 //   * the WEIGHTS are the M side of tcgen05.mma (128 rows per block) and the tokens its N side (16 to 128 columns, a
@@ -18,8 +18,10 @@
 //     a decoder stack at 48 tokens, us: ring filled before the wait 233, nothing 248, the whole ring into L2 251, its first
 //     slot 243.)
 // Measured, weights from HBM, against w4_gemm.cu at 48 tokens: 4608 x 3584 7.9 us (25), 37888 x 3584 22.7 (46), 3584 x
-// 18944 17.8 (51), 8192 x 28672 39.5 (113).  Of the 22.7 us, 11 are the weights' way from HBM; with the conversion taken
-// out (a copy of the raw words) it takes 17.5: a step's chain of waits, then the conversion's issue slots (60 % taken).
+// 18944 17.8 (51), 8192 x 28672 39.5 (113), all with 17 instructions per eight weights; with ten, sixteen such launches (four
+// 7B-shaped layers) take 228 us instead of 241, 777 x 5000 x 4096 in groups of 64 34.1 instead of 35.7, 512 x 3584 x 18944 73.2
+// instead of 77.2.  Of the 22.7 us, 11 are the weights' way from HBM; with the conversion taken out (a copy of the raw
+// words) it took 17.5: a step's chain of waits, then the conversion's issue slots.
 // Warps: 0 packed words (TMA), 1 MMA issue and TMEM, 2 X tiles (TMA), 3 idle, then DW conversion warps, which also do
 // the epilogue.  All rings run on mbarriers with bounded waits; a CTA that gives up records a status, still takes part in
 // the cluster barriers, frees its TMEM and returns.
@@ -199,8 +201,6 @@ __global__ void __launch_bounds__(128 + DW * 32, MINB)
     if (!poisoned) {
       const int n = n0 + row;
       const bool live = n < p.N;
-      uint32_t k_mask = kNibblePairMask, k_magic = kMagic128x2;
-      asm volatile("" : "+r"(k_mask), "+r"(k_magic));
       const __nv_bfloat16* s_row = p.S + (size_t)(live ? n : 0) * p.KG;
       // Scales, p.sv of them per load (a thread reads along its own row, so every load touches 32 lines), the next load
       // in flight while one is used.  General groups: (g, kin) is the group of the current K position and the position
@@ -271,6 +271,12 @@ __global__ void __launch_bounds__(128 + DW * 32, MINB)
           }
           k += 2 * kKB;
         }
+        bool plain = dequant_scale_plain(sc[0]);
+        if constexpr (!G128) {
+#pragma unroll
+          for (int j = 1; j < 4; ++j) plain = plain && dequant_scale_plain(sc[j]);
+        }
+        plain = __all_sync(0xffffffffu, plain);
         mbar_wait(bar_w_full + 8 * s, ph, abort_flag);
         uint4 w[4];
 #pragma unroll
@@ -278,13 +284,25 @@ __global__ void __launch_bounds__(128 + DW * 32, MINB)
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
           uint32_t v[32];
+          if (plain) {
 #pragma unroll
-          for (int j = 0; j < 2; ++j) {
-            const uint4 q = w[2 * half + j];
-            dequant_word(q.x, sc[2 * half + j], k_mask, k_magic, v + 16 * j);
-            dequant_word(q.y, sc[2 * half + j], k_mask, k_magic, v + 16 * j + 4);
-            dequant_word(q.z, sc[2 * half + j], k_mask, k_magic, v + 16 * j + 8);
-            dequant_word(q.w, sc[2 * half + j], k_mask, k_magic, v + 16 * j + 12);
+            for (int j = 0; j < 2; ++j) {
+              const uint4 q = w[2 * half + j];
+              const DequantScale ds = dequant_scale(sc[2 * half + j]);
+              dequant_word(q.x, ds, v + 16 * j);
+              dequant_word(q.y, ds, v + 16 * j + 4);
+              dequant_word(q.z, ds, v + 16 * j + 8);
+              dequant_word(q.w, ds, v + 16 * j + 12);
+            }
+          } else {
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+              const uint4 q = w[2 * half + j];
+              dequant_word_any(q.x, sc[2 * half + j], v + 16 * j);
+              dequant_word_any(q.y, sc[2 * half + j], v + 16 * j + 4);
+              dequant_word_any(q.z, sc[2 * half + j], v + 16 * j + 8);
+              dequant_word_any(q.w, sc[2 * half + j], v + 16 * j + 12);
+            }
           }
           if (half == 0) {
             mbar_wait(bar_a_empty + 8 * grp, aph, abort_flag);
@@ -317,7 +335,7 @@ __global__ void __launch_bounds__(128 + DW * 32, MINB)
           __nv_bfloat16* y = p.Y + (size_t)(m0 + c0) * p.N + n;
 #pragma unroll
           for (int e = 0; e < 16; ++e)
-            if (live && c0 + e < rt) y[(size_t)e * p.N] = __float2bfloat16(__uint_as_float(v[e]));
+            if (live && c0 + e < rt) y[(size_t)e * p.N] = __float2bfloat16(__uint_as_float(v[e]) * (1.f / kDequantUnit));
         } else {  // [token][row], over the rings: every copy has landed and every MMA has read its operands
 #pragma unroll
           for (int e = 0; e < 16; ++e)
@@ -344,6 +362,7 @@ __global__ void __launch_bounds__(128 + DW * 32, MINB)
             const float4 b = ld_cluster_f4(at, z);
             a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
           }
+        a.x *= 1.f / kDequantUnit; a.y *= 1.f / kDequantUnit; a.z *= 1.f / kDequantUnit; a.w *= 1.f / kDequantUnit;
         __nv_bfloat16* y = p.Y + (size_t)(m0 + tok) * p.N + n;
         if (n + 4 <= p.N && (p.N & 3) == 0) {
           const __nv_bfloat162 lo = __floats2bfloat162_rn(a.x, a.y), hi = __floats2bfloat162_rn(a.z, a.w);

@@ -72,8 +72,10 @@ def test_linear_behind_its_quantizer(kernels, M):
 @pytest.fixture(scope="module")
 def long_launch(kernels):
     """A launch that lets its dependents start at once and then runs longer than any bounded wait of the library (10^9
-    cycles, 0.51 s at 1.965 GHz): one CTA walks a K of 2^28."""
-    K, G = 2**28, 64
+    cycles, 0.51 s at 1.965 GHz): one CTA walks a K of 2^29, 2^22 steps.  A step cannot take less than 300 cycles (two hand-overs
+    through barriers of some 100 each, a store to tensor memory and eight products that each add to the one before), 0.64 s
+    in all; it takes 560."""
+    K, G = 2**29, 64
     x = torch.zeros(1, K, dtype=torch.bfloat16, device="cuda")
     Wq = torch.zeros(1, K // 8, dtype=torch.int32, device="cuda")
     S = torch.ones(1, K // G, dtype=torch.bfloat16, device="cuda")

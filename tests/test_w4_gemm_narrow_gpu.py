@@ -5,7 +5,7 @@ import pytest
 import torch
 
 import oracle
-from nanoserve_b200.ops import FLAG_DECODE_NARROW, FLAG_GEMM_WIDE, narrow_flags
+from nanoserve_b200.ops import FLAG_DECODE_NARROW, FLAG_GEMM_NO_PAIRS, FLAG_GEMM_WIDE, narrow_flags
 from tests.test_w4_gemm_gpu import rounded_weight_reference
 from tests.util import bits_to_torch, check_bf16_output, torch_to_bits, u32_to_torch
 
@@ -113,3 +113,29 @@ def test_rule_takes_the_shorter_kernel(kernels, M, N, K, G, kernel):
 ])
 def test_rule_at_decode_tokens(kernels, M, N, K, G, kernel):
     assert kernels.gemv_describe(M, N, K, G).startswith(kernel)
+
+
+@pytest.mark.parametrize("M,flags", [(32, narrow_flags(1, 1)), (32, narrow_flags(2, 2)), (32, FLAG_GEMM_WIDE), (300, FLAG_GEMM_NO_PAIRS | FLAG_GEMM_WIDE),
+                                     (300, FLAG_GEMM_WIDE)])
+@pytest.mark.parametrize("G", [32, 64, 128])
+def test_scales_of_any_size(kernels, M, flags, G):
+    """Tokens that pick one k each give back single weights, which are RN_bf16((q - 8) * s) to the bit: scales on either side of
+    the line below which a weight is one fused multiply-add, rows that cross it and rows beside them that do not."""
+    N, K = 200, 512
+    gen = torch.Generator(device="cuda").manual_seed(G)
+    Wq = torch.randint(-2**31, 2**31 - 1, (N, K // 8), dtype=torch.int32, device="cuda", generator=gen)
+    sizes = torch.tensor([1.0, 7.96875, 8.0, -7.96875, -8.0, 0.0133, 1e4, 3e37, 1e-30, 0.0], device="cuda")
+    S = sizes[torch.randint(0, 10, (N, K // G), device="cuda", generator=gen)].to(torch.bfloat16)
+    S[:N // 2, 1:] = 0.02  # warps whose rows leave the line for a group only
+    ks = torch.randint(0, K, (M,), device="cuda", generator=gen)
+    x = torch.zeros(M, K, dtype=torch.bfloat16, device="cuda")
+    x[torch.arange(M, device="cuda"), ks] = 1.0
+    shifts = torch.arange(0, 32, 4, device="cuda", dtype=torch.int32)
+    w = (((Wq[:, :, None] >> shifts) & 15).flatten(1) - 8).float() * S.float().repeat_interleave(G, dim=1)
+    y = kernels.w4_linear(x, Wq, S, G, flags=flags)
+    assert kernels.device_status() == 0
+    assert torch.equal(y.float(), w.to(torch.bfloat16)[:, ks].T.float())
+    S[3, 0] = float("inf")
+    y = kernels.w4_linear(x, Wq, S, G, flags=flags)
+    assert bool(y[:, 3].isnan().any()) and bool(y[:, :3].isfinite().all()) and bool(y[:, 4:].isfinite().all())
+    assert kernels.device_status() == 0
