@@ -72,9 +72,9 @@ int ns_flash_fwd(const void* q, const void* k, const void* v, void* o, int N, in
  * carries X as block fixed point per (token, 128-wide chunk of K) -- 32 bits for M <= 2 (exact to fp32 summation
  * order), 15 bits + sign above -- on an 8-bit integer mma.  The many-token kernel (G == 128, K % 256 == 0, plain
  * launches) runs five to sixteen tokens, and two to four where K >= 8192, with X as 16-bit block
- * fixed point.  The tcgen05 kernel takes plain calls of two to sixteen tokens (G == 128, K % 256 == 0, X and Wq 16-byte, S
- * 4-byte aligned) from these kernels where that is estimated shorter, which is most of them: the same arithmetic, with 32 bits for
- * M <= 4.  The ring kernel runs everything else, with X as 16-bit block fixed point (every element off by at most
+ * fixed point.  The tcgen05 kernel takes plain calls of up to sixteen tokens (G == 128, K % 256 == 0, X and Wq 16-byte, S
+ * 4-byte aligned) from these kernels where that is estimated shorter, which is most of them from two tokens on and small matrices at
+ * one: the same arithmetic, with 32 bits for M <= 4.  The ring kernel runs everything else, with X as 16-bit block fixed point (every element off by at most
  * 2^-16 of its chunk's largest magnitude) or as the flags below say.  No kernel measures anything or synchronises:
  * every call is asynchronous.  Groups finer than 128, whose weights the ring kernel rounds to bf16, run the few-token GEMM
  * instead where that is estimated shorter (X, Wq, Y 16-byte aligned).  More than 16 tokens run the few-token GEMM or the

@@ -1,4 +1,4 @@
-// W4A16 decode GEMV on the fifth-generation tensor cores, two to sixteen tokens, groups of 128:
+// W4A16 decode GEMV on the fifth-generation tensor cores, up to sixteen tokens, groups of 128:
 // Y[M,N] (bf16) = X[M,K] (bf16) . dequant(Wq, S)^T with exact weights.
 //
 // The arithmetic is that of the mma.sync kernels: nibbles as signed bytes 16 (q - 8), X as block fixed point per (token,
@@ -12,15 +12,19 @@
 //   * a hand-over is a pair of chunks, K = 256.  Two groups of warps take the pairs in turn: while one group's products run the
 //     other converts words, and each reads and scales its sums when it comes back for its buffer;
 //   * K is cut over a cluster.  A CTA sends its sums into the shared memory of the CTA that adds them, in the order of ranks and
-//     groups (no second launch, one cluster barrier behind the sums).
-// What bounds it: from the wait for the kernel in front to the last pair it runs at HBM's rate (37888 x 3584 at four tokens: 10.4
-// of 15.9 us for 70 MB); the rest is the boundary between launches (1.7 us), barriers and tensor memory before it (0.7), the
-// last sums and stores (1.3).  What the pairs are for: an answer of a barrier takes a warp some 130 cycles even where it is
-// yes, an arrival with its fence 100, and a chunk at a time with one group (0.55 us per chunk of 256 rows, HBM 0.37) these were
-// most of a step.  Measured, weights from HBM, us at 4 / 8 / 13 tokens, in brackets the shortest of the mma.sync kernels and, at
-// 13, this kernel before (a chunk per step, X converted first): 37888 x 3584 15.9 / 16.5 / 18.1 (15.8 / 19.3 / 21.5), 3584 x
-// 18944 12.9 / 13.4 / 14.7 (15.0 / 16.2 / 18.2), 3584 x 3584 5.6 / 5.8 / 6.5 (7.5 / 6.8 / 8.2), 8192 x 28672 28 / 30 / 34 (41 / 42
-// / 50), 57344 x 8192 56 / 59 / 68 (59 / 60 / 89).
+//     groups (no second launch; st.async counted on a barrier of that CTA).
+// What bounds it: HBM's rate once it runs (37888 x 3584 at four tokens: 7.5 TB/s from the seventh pair on, 70 MB in 11 of 15.4
+// us), the issue slots above eight tokens (1540 of the 1550 cycles of a pair at 13: the words' bytes 96 instructions per row and
+// pair, the sums 7 per token, the conversion of X a sixth of all), and around that the boundary between launches: the wait for the kernel
+// in front returns 0.9 us after its last CTA has left, a CTA starts 0.9 us after the one before it on the SM has (0.3 where
+// neither uses tensor memory), first words and X 0.7 later, first products 0.5, the exchange of parts 0.9.
+// The chain of a group is what the order in the loop is for: half of a pair's words are converted while the products of the group's last
+// pair run, and the sums of that one are added while this pair's do (2530 -> 2300 cycles per pair of a group; 8192 x 28672 at
+// eight tokens 30.7 -> 28.6 us).  The status word is asked for at the start and answered behind the set-up, the parts of a cut K go
+// to the CTA that adds them with a barrier of their own instead of the cluster's (4608 x 3584 6.65 -> 5.8 us), tensor memory
+// is freed beside the last sums.  Measured, weights from HBM, us at 4 / 8 / 13 tokens, in brackets before that: 37888 x
+// 3584 15.2 / 15.4 / 16.9 (15.4 / 16.1 / 17.8), 3584 x 18944 12.4 / 12.6 / 14.7 (13.2 / 13.5 / 15.2), 4608 x 3584 at 4 and 13 5.8 and
+// 6.8 (6.65 and 7.2), 57344 x 8192 at 8 57.9 (61.0).
 // Every wait is bounded; a CTA that gives up records a status, still takes part in the cluster barriers and frees its TMEM.
 #include <cuda.h>
 
@@ -56,6 +60,7 @@ struct TcParams {
   int ks;       // CTAs of a cluster, each with its share of the pairs
   int sw, sx;   // ring slots of a pair: packed words (per block of 128 rows), X
   int ahead;    // slots of packed words that are brought into L2 ahead of the ring
+  int x_first;  // the ring's further slots are not asked for before the first X is there
   int off_w, off_x, off_info, off_red;
 };
 
@@ -75,11 +80,14 @@ __host__ __device__ constexpr uint32_t umma_idesc_s8(int b_signed, int M, int N)
 }
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-__device__ __forceinline__ void st_cluster_f32(uint32_t addr, uint32_t rank, float v) {
+// 16 bytes into the shared memory of CTA `rank` of the cluster, counted on its barrier at the same address as `bar` here.
+__device__ __forceinline__ void st_async_f4(uint32_t addr, uint32_t bar, uint32_t rank, float a, float b, float c, float d) {
   asm volatile(
-      "{\n\t.reg .u32 a;\n\t"
-      "mapa.shared::cluster.u32 a, %0, %1;\n\t"
-      "st.shared::cluster.f32 [a], %2;\n\t}" ::"r"(addr), "r"(rank), "f"(v)
+      "{\n\t.reg .u32 a, m;\n\t"
+      "mapa.shared::cluster.u32 a, %0, %2;\n\t"
+      "mapa.shared::cluster.u32 m, %1, %2;\n\t"
+      "st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [a], {%3, %4, %5, %6}, [m];\n\t}" ::"r"(addr),
+      "r"(bar), "r"(rank), "f"(a), "f"(b), "f"(c), "f"(d)
       : "memory");
 }
 template <int N>
@@ -106,21 +114,6 @@ __device__ __forceinline__ void tmem_ld_sums(uint32_t taddr, uint32_t (&d)[16]) 
   }
 }
 
-// All questions of a pair of steps in one go: an answer takes some 100 cycles, and one after the other they add up.
-__device__ __forceinline__ bool mbar_try_wait2(uint32_t bar0, uint32_t parity0, uint32_t bar1, uint32_t parity1) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p, q;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 q, [%3], %4;\n\t"
-      "and.pred p, p, q;\n\t"
-      "selp.b32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(bar0), "r"(parity0), "r"(bar1), "r"(parity1)
-      : "memory");
-  return ok != 0;
-}
-
 // MT: token columns (4, 8 or 16).  Four and fewer tokens keep X in 32 bits (three unsigned planes and a signed one), more
 // in 16 (one and one).  MB: blocks of 128 weight rows.  SV: scales per load.
 template <int MB, int MT, int SV>
@@ -140,18 +133,29 @@ __global__ void __launch_bounds__(MB == 2 ? 896 : 512, MB == 2 ? 1 : 2)
   const uint32_t bar_a_full = bar_w_empty + 8 * 8, bar_a_empty = bar_a_full + 8 * 4;  // [block][group]
   const uint32_t bar_x_empty = bar_a_empty + 8 * 4;                                   // [slot], at most 16
   const uint32_t bar_x_full = base + kSlotBars;                                       // [pair]
+  const uint32_t bar_red = base + 16;                                                 // the parts of a cut K
   const uint32_t ring_w = base + p.off_w, ring_x = base + p.off_x, info = base + p.off_info, red = base + p.off_red;
 
+  // (Read by every warp for itself, and answered behind the set-up: another CTA may set it in between.)
+  const int status_seen = *reinterpret_cast<volatile int*>(p.status);
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const int crank = p.ks > 1 ? (int)cluster_rank() : 0;
   const int n0 = (blockIdx.x / p.ks) * kRows;
   const int pr0 = (int)((long)crank * p.pairs / p.ks), np = (int)((long)(crank + 1) * p.pairs / p.ks) - pr0;
   const int groups = (p.M + 3) >> 2;  // of four tokens: one warp's piece of a step's X
+  // the blocks of 32 rows that this CTA of a cluster adds up
+  const int first_blk = (crank * kBlocks + p.ks - 1) / p.ks, blks = ((crank + 1) * kBlocks + p.ks - 1) / p.ks - first_blk;
 
   for (int i = tid; i < np; i += kWarps * 32) mbar_init(bar_x_full + 8 * i, 2 * groups);
   // (the barriers of the rings lie one behind the other: 8 + 8 + 4 + 4 + 16)
   if (tid < 40) mbar_init(base + kBarOffset + 8 * tid, tid < 8 ? 1 : tid < 20 ? 4 : tid < 24 ? 1 : MB);
-  if (tid == 0) *abort_flag = 0;
+  if (tid == 0) {
+    *abort_flag = 0;
+    if (p.ks > 1) {
+      mbar_init(bar_red, 1);
+      mbar_arrive_expect_tx(bar_red, (uint32_t)(blks * p.ks * 2 * groups) * 512);
+    }
+  }
   fence_mbar_init();
   if (warp == kWarpW && lane == 0) tma_prefetch_desc(&tmap_w);
   if (warp == kWarpMma) {
@@ -162,17 +166,19 @@ __global__ void __launch_bounds__(MB == 2 ? 896 : 512, MB == 2 ? 1 : 2)
   __syncthreads();
   tc_fence_after_sync();
   pdl_launch_dependents();
-  if (p.ks > 1) cluster_arrive();  // (waited for before the first store into a peer: it runs by then)
+  if (p.ks > 1) cluster_arrive();  // (waited for before the first store into a peer: it runs by then, its barrier is set up)
   const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);  // [block][group]: 64 columns of sums, 64 of bytes
-  // (Read by every warp for itself: another CTA may set it in between, so the named barrier below is met either way.  One read
-  // per CTA ahead of the __syncthreads cost four layers at 13 tokens 2.0 us of 184.)
-  const bool poisoned = __any_sync(0xffffffffu, *reinterpret_cast<volatile int*>(p.status) != 0);
+  const bool poisoned = __any_sync(0xffffffffu, status_seen != 0);
+  if (poisoned && lane == 0) *abort_flag = 1;  // the CTA's other warps may have read zero: their waits end
 
   // The rows' warps need more registers than an even share.  256 rows, 896 threads of 72: 4 x 88 + 2 x 48 + 56 = 7 x 72 by
   // warpgroup; 128 rows, 512 of 64: 2 x 80 + 2 x 48 = 4 x 64.
   if (warp < kMain) regs_up<MB == 2 ? 88 : 80>();
   else if (warp < kWarpW) regs_down<48>();
   else regs_down<MB == 2 ? 56 : 48>();
+  // Behind this the rows' warps leave tensor memory alone: the warp that allocated it frees it while they add up and store.
+  // (A kernel that frees it last ends 0.14 us later.)
+  auto rows_done = [&] { asm volatile("bar.arrive 3, %0;" ::"n"(kMain * 32 + 32) : "memory"); };
   if (!poisoned) {
     if (warp < kMain) {
       // ---- the rows: words -> bytes in TMEM; sums of a step -> registers.  Two groups of warps take the pairs in turn.
@@ -201,14 +207,20 @@ __global__ void __launch_bounds__(MB == 2 ? 896 : 512, MB == 2 ? 1 : 2)
       const uint32_t d_src = tmem + ((uint32_t)(quad * 32) << 16) + (mb * 2 + grp) * 128, a_dst = d_src + 64;
       const uint32_t b_wf = bar_w_full + 32 * mb, b_we = bar_w_empty + 32 * mb;
       const uint32_t b_af = bar_a_full + 8 * (mb * 2 + grp), b_ae = bar_a_empty + 8 * (mb * 2 + grp);
+      if (p.ks > 1) cluster_wait();
       float acc[MT];
 #pragma unroll
       for (int e = 0; e < MT; ++e) acc[e] = 0.f;
-      // the sums of a step: planes joined as integers, one conversion per pair, then scale times the token's factor
-      auto add_step = [&](int step, float scale) {
-        uint32_t d[kCols];
-        tmem_ld_sums<kLo>(d_src + (step & 1) * 32, d);
-        tmem_ld_wait();
+      // the sums of a step: planes joined as integers, ...
+      auto join = [&](const uint32_t (&d)[kCols], int (&j)[kCols / 2]) {
+#pragma unroll
+        for (int t = 0; t < MT; ++t) {
+          j[t] = (int)d[t] + ((int)d[MT + t] << 8);
+          if constexpr (P == 4) j[MT + t] = (int)d[2 * MT + t] + ((int)d[3 * MT + t] << 8);
+        }
+      };
+      // ... one conversion per pair, then scale times the token's factor
+      auto add_step = [&](int step, float scale, const int (&j)[kCols / 2]) {
         const float2 scale2 = make_float2(scale, scale);
 #pragma unroll
         for (int q = 0; q < MT / 4; ++q) {
@@ -221,9 +233,8 @@ __global__ void __launch_bounds__(MB == 2 ? 896 : 512, MB == 2 ? 1 : 2)
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
               const int t = q * 4 + h * 2 + e;
-              v[e] = (float)((int)d[t] + ((int)d[MT + t] << 8));
-              if constexpr (P == 4)
-                v[e] = fmaf((float)((int)d[2 * MT + t] + ((int)d[3 * MT + t] << 8)), 65536.f, v[e]);
+              v[e] = (float)j[t];
+              if constexpr (P == 4) v[e] = fmaf((float)j[MT + t], 65536.f, v[e]);
             }
             float2 a = make_float2(acc[q * 4 + h * 2], acc[q * 4 + h * 2 + 1]);
             a = fma_f32x2(mul_f32x2(scale2, ff[h]), make_float2(v[0], v[1]), a);
@@ -232,23 +243,32 @@ __global__ void __launch_bounds__(MB == 2 ? 896 : 512, MB == 2 ? 1 : 2)
           }
         }
       };
-      auto add_pair = [&](int i) {
-        add_step(2 * i, __uint_as_float(cur << 16));
-        add_step(2 * i + 1, __uint_as_float(cur & 0xFFFF0000u));
+      // Takes the sums of pair i out of tensor memory; `then` runs as soon as the products may write there again.
+      auto add_pair = [&](int i, auto&& then) {
+        uint32_t d0[kCols], d1[kCols];
+        int j[kCols / 2];
+        tmem_ld_sums<kLo>(d_src, d0);
+        if constexpr (MT == 16) {  // (no registers for 64 sums)
+          tmem_ld_wait();
+          join(d0, j);
+        }
+        tmem_ld_sums<kLo>(d_src + 32, d1);
+        tmem_ld_wait();
+        then();
+        if constexpr (MT != 16) join(d0, j);
+        add_step(2 * i, __uint_as_float(cur << 16), j);
+        join(d1, j);
+        add_step(2 * i + 1, __uint_as_float(cur & 0xFFFF0000u), j);
         cur = nxt;
         g += 4;
         nxt = pair_scales(g + 4);
       };
-      uint4 w[4];  // the packed words of a step
-      auto load_words = [&](uint32_t slot, int half) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) w[j] = lds128(slot + (((uint32_t)(half * 4 + j) ^ swz) << 4));
-      };
-      auto put_words = [&](int half) {
-        uint32_t v[32];
+      uint32_t v[32];  // a step's bytes
+      auto convert = [&](uint32_t slot, int half) {
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          const uint32_t ww[4] = {w[j].x, w[j].y, w[j].z, w[j].w};
+          const uint4 w = lds128(slot + (((uint32_t)(half * 4 + j) ^ swz) << 4));
+          const uint32_t ww[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
           for (int h = 0; h < 2; ++h) {  // two words: their even nibbles, their odd nibbles
             v[8 * j + 4 * h] = ((ww[2 * h] << 4) & 0xF0F0F0F0u) ^ 0x80808080u;
@@ -257,50 +277,62 @@ __global__ void __launch_bounds__(MB == 2 ? 896 : 512, MB == 2 ? 1 : 2)
             v[8 * j + 4 * h + 3] = (ww[2 * h + 1] & 0xF0F0F0F0u) ^ 0x80808080u;
           }
         }
-        tmem_st_32x32(a_dst + half * 32, v);
       };
       int s = grp;  // (the ring has an even number of slots: a group's slots are its own)
-      uint32_t wph = 0, aph = 1;
+      uint32_t wph = 0, aph = 0;
+      bool there = false;
       for (int i = grp; i < np; i += 2) {
-        const uint32_t slot = slot0 + s * kWSlot;
-        // the bytes of the group's last pair have been read and its sums are complete; this pair's words are there
-        const bool ready = mbar_try_wait2(b_ae, aph, b_wf + 8 * s, wph);
-        if (!__all_sync(0xffffffffu, ready)) {
-          mbar_wait(b_ae, aph, abort_flag);
+        // Half of the words are converted while the products of the group's last pair may still run; its sums are added while
+        // those of this pair do.
+        const uint32_t slot = slot0 + s * kWSlot, b_we_this = b_we + 8 * s;
+        if (!__all_sync(0xffffffffu, there)) {
           mbar_wait(b_wf + 8 * s, wph, abort_flag);
           __syncwarp();
         }
-        tc_fence_after_sync();
-        load_words(slot, 0);
-        if (i >= 2) {
-          mbar_wait(bar_x_full + 8 * (i - 2), 0, abort_flag);  // (complete: its factors were written before it)
-          __syncwarp();
-          add_pair(i - 2);
-        }
-        put_words(0);
-        load_words(slot, 1);
-        put_words(1);
-        tmem_st_wait();
-        tc_fence_before_sync();
-        __syncwarp();
-        mbar_arrive_if(b_af, lane == 0);
-        mbar_arrive_if(b_we + 8 * s, lane == 0);
-        aph ^= 1;
         s += 2;
         if (s >= p.sw) {
           s -= p.sw;
           wph ^= 1;
         }
+        convert(slot, 0);
+        if (i >= 2) {
+          // the bytes of the group's last pair have been read and its sums are complete; so is that pair's X, whose factors
+          // were written before it
+          if (!__all_sync(0xffffffffu, mbar_try_wait2(b_ae, aph, bar_x_full + 8 * (i - 2), 0))) {
+            mbar_wait(b_ae, aph, abort_flag);
+            mbar_wait(bar_x_full + 8 * (i - 2), 0, abort_flag);
+            __syncwarp();
+          }
+          aph ^= 1;
+          tc_fence_after_sync();
+        }
+        tmem_st_32x32(a_dst, v);
+        convert(slot, 1);
+        tmem_st_32x32(a_dst + 32, v);
+        auto hand_over = [&] {
+          tmem_st_wait();
+          tc_fence_before_sync();
+          __syncwarp();
+          mbar_arrive_if(b_af, lane == 0);
+          mbar_arrive_if(b_we_this, lane == 0);
+          if (i + 2 < np) there = mbar_test_wait(b_wf + 8 * s, wph);
+        };
+        if (i >= 2)
+          add_pair(i - 2, hand_over);
+        else
+          hand_over();
       }
       if (const int last = np - 1 - ((np - 1 - grp) & 1); last >= 0) {  // the group's last pair
         mbar_wait(b_ae, aph, abort_flag);
         mbar_wait(bar_x_full + 8 * last, 0, abort_flag);
         __syncwarp();
         tc_fence_after_sync();
-        add_pair(last);
+        add_pair(last, [&] {
+          tc_fence_before_sync();
+          __syncwarp();
+        });
       }
-      tc_fence_before_sync();
-      __syncwarp();
+      rows_done();
       if (p.ks == 1) {  // the second group's sums through shared memory
         float* part = reinterpret_cast<float*>(gen + p.off_red) + (row >> 5) * (MT * 32) + lane;
         if (grp == 1) {
@@ -317,13 +349,32 @@ __global__ void __launch_bounds__(MB == 2 ? 896 : 512, MB == 2 ? 1 : 2)
         }
       } else {
         // Every part goes to the CTA that sums its block of 32 rows, block * ks / kBlocks of the cluster, which adds the parts
-        // in the order of ranks and groups: [block][rank][group][token][32 rows]
+        // in the order of ranks and groups: [block][rank][group][four tokens][32 rows]
         const int blk = row >> 5, owner = blk * p.ks / kBlocks, first = (owner * kBlocks + p.ks - 1) / p.ks;
-        const uint32_t at = red + (uint32_t)((((blk - first) * p.ks + crank) * 2 + grp) * MT * 32 + lane) * 4;
-        cluster_wait();
+        const uint32_t at = red + (uint32_t)((((blk - first) * p.ks + crank) * 2 + grp) * (MT / 4) * 32 + lane) * 16;
 #pragma unroll
-        for (int e = 0; e < MT; ++e)
-          if (e < p.M) st_cluster_f32(at + e * 128, owner, acc[e]);
+        for (int q = 0; q < MT / 4; ++q)
+          if (q < groups) st_async_f4(at + q * 512, bar_red, owner, acc[4 * q], acc[4 * q + 1], acc[4 * q + 2], acc[4 * q + 3]);
+        if (warp < blks * groups) {
+          mbar_wait(bar_red, 0, abort_flag);
+          __syncwarp();
+        }
+        for (int item = warp; item < blks * groups; item += kMain) {
+          const int b = item / groups, q = item - b * groups, ny = n0 + (first_blk + b) * 32 + lane;
+          const uint32_t part = red + (uint32_t)((b * p.ks * 2 * (MT / 4) + q) * 32 + lane) * 16;
+          float sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+          for (int z = 0; z < 2 * p.ks; ++z) {
+            const uint4 f = lds128(part + z * (MT / 4) * 512);
+            sum[0] += __uint_as_float(f.x);
+            sum[1] += __uint_as_float(f.y);
+            sum[2] += __uint_as_float(f.z);
+            sum[3] += __uint_as_float(f.w);
+          }
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+            if (ny < p.N && q * 4 + e < p.M) p.Y[(size_t)(q * 4 + e) * p.N + ny] = __float2bfloat16(sum[e]);
+        }
       }
     } else if (warp < kWarpW) {
       // ---- X: a warp takes four tokens of a step, a lane 16 consecutive k of a token, the eight lanes of a token side by
@@ -424,12 +475,13 @@ __global__ void __launch_bounds__(MB == 2 ? 896 : 512, MB == 2 ? 1 : 2)
         for (int i = 0; i < np; ++i) {
 #pragma unroll
           for (int mb = 0; mb < MB; ++mb) {
-            mbar_wait(bar_w_empty + 32 * mb + 8 * s, ph, abort_flag);
+            if (i >= p.sw) mbar_wait(bar_w_empty + 32 * mb + 8 * s, ph, abort_flag);
             mbar_arrive_expect_tx(bar_w_full + 32 * mb + 8 * s, kWSlot);
             tma_load_2d(ring_w + (mb * p.sw + s) * kWSlot, &tmap_w, (pr0 + i) * 32, n0 + mb * 128,
                         bar_w_full + 32 * mb + 8 * s);
           }
           if (++s == p.sw) { s = 0; ph ^= 1; }
+          if (i == 0 && p.x_first) mbar_wait(bar_x_full, 0, abort_flag);
         }
       }
       __syncwarp();
@@ -469,33 +521,32 @@ __global__ void __launch_bounds__(MB == 2 ? 896 : 512, MB == 2 ? 1 : 2)
         if (++xs == p.sx) xs = 0;
       }
     }
-  } else if (p.ks == 1 && warp < kMain) {  // the block's other warps may be there, and this barrier has no limit
-    asm volatile("bar.sync %0, 256;" ::"r"(1 + (warp >> 2) % MB) : "memory");
+  } else if (warp < kMain) {  // the CTA's other warps may be there, and these barriers have no limit
+    rows_done();
+    if (p.ks == 1) asm volatile("bar.sync %0, 256;" ::"r"(1 + (warp >> 2) % MB) : "memory");
   }
   __syncwarp();
-  if (p.ks > 1) {
-    if (warp >= kMain || poisoned) cluster_wait();
-    __syncwarp();
-    cluster_arrive();
-    cluster_wait();
-    const int first = (crank * kBlocks + p.ks - 1) / p.ks, count = ((crank + 1) * kBlocks + p.ks - 1) / p.ks - first;
-    for (int blk = 0; blk < count && !poisoned; ++blk)
-      for (int tok = warp; tok < p.M; tok += kWarps) {
-        const float* part = reinterpret_cast<const float*>(gen + p.off_red) + (blk * p.ks * 2 * MT + tok) * 32 + lane;
-        const int n = n0 + (first + blk) * 32 + lane;
-        float sum = 0.f;
-#pragma unroll 4
-        for (int z = 0; z < 2 * p.ks; ++z) sum += part[z * MT * 32];
-        if (n < p.N) p.Y[(size_t)tok * p.N + n] = __float2bfloat16(sum);
-      }
+  bool freed = false;
+  if (warp == kWarpMma) {
+    asm volatile("bar.sync 3, %0;" ::"n"(kMain * 32 + 32) : "memory");
+    if (!__any_sync(0xffffffffu, *abort_flag != 0)) {  // (every product has been waited for)
+      tc_fence_after_sync();
+      tmem_dealloc(tmem, kTmemCols);
+      freed = true;
+    }
   }
+  if (p.ks > 1 && (warp >= kMain || poisoned)) cluster_wait();
   __syncthreads();
   if (*abort_flag) {
+    if (p.ks > 1) {  // peers that have not given up may send parts here until they leave
+      cluster_arrive();
+      cluster_wait();
+    }
     if (tid == 0) atomicCAS(p.status, kStatusOk, kStatusGemvTimeout);
     for (int i = 0; i < 64; ++i) __nanosleep(2000);  // copies in flight land before the shared memory is released
     __syncthreads();
   }
-  if (warp == kWarpMma) {
+  if (warp == kWarpMma && !freed) {
     tc_fence_after_sync();
     tmem_dealloc(tmem, kTmemCols);
   }
@@ -646,29 +697,36 @@ bool gemv_tc_serves(const void* X, const void* Wq, const void* S, const void* Y,
   return tc_operands(X, Wq, S, Y, M, N, K, G) && tc_plan(M, N, K, sm_count, (flags >> 24) & 3, (flags >> 20) & 15, &pl);
 }
 
-// Whether this kernel is shorter than the GEMV that would take a plain call of 2 to 16 tokens, `other` one of kTcOther*.  Lines drawn
-// through 6472 calls on 1627 random shapes (48 to 60000 rows, K 256 to 28672, weights from HBM), every kernel and every plan of this
-// one timed, and 4308 more of the many-token kernel's; "lost" is a call that takes 5 % more time than with the other kernel.
+// Whether this kernel is shorter than the GEMV that would take a plain call of 1 to 16 tokens, `other` one of kTcOther*.  Lines
+// drawn through 2044 calls on random shapes (128 to 60000 rows, K 512 to 28672, weights from HBM, one launch behind the other), every
+// kernel and every plan of this one timed, and earlier through 6472 more.
+//   * One token (streaming kernel): both hold X in 32 bits.  From K = 1024 and up to twelve million weights a launch is its latencies, and the
+//     other converts the whole of X before its first product (512 x 3584 3.4 us against 4.5, 1909 x 4352 3.8 against 5.2); between K of
+//     9728 and 16384 it does so several times per thread (4980 x 14080 12.8 against 15.0), above 22000 it cuts K through memory
+//     (8192 x 28672 26.6 against 29.2).  Of 335 calls those that come here take 0.83 of their time there, three of them 3 % more (at
+//     most 5); the others, at HBM's rate, are shorter there (37888 x 3584 14.3 against 15.6).
+//   * Two to four tokens (streaming kernel; X has 15 bits there at three and four): shorter here but for many rows of a short K (21667 x
+//     1024 at four tokens 4.8 us there, 5.5 here; 18944 x 3584 at two 9.6 and 10.7).  Of 150 calls five lose 3 % (at most 6).
 //   * Many-token kernel, five and more tokens: by the estimates of both, this one's with what plans have in common (they come out
-//     short where the chip is full).  Of 4127 calls at five to eight tokens 44 are lost (at most 20 %), of 3439 above 34 (19 %); the
-//     time is 1.003 and 1.002 times the shorter kernel's in the geometric mean.  (With a line in M, N and K alone 113 and 496 were
-//     lost, up to 55 %, small matrices of long K most: 10 x 178 x 26112 14.5 us against 9.4, 16 x 290 x 22784 12.0 against 10.7.)
+//     short where the chip is full): 1.008 and 1.003 times the shortest kernel's time up to eight tokens and above.
 //   * Many-token kernel, two to four tokens (K >= 8192): X has 32 bits here and 16 there, so what a line in w (millions of weights),
-//     M and K brought here stays.  1.19 times as fast in the geometric mean, 18 of 801 calls lost (15 %).
-//   * Streaming kernel at two tokens: shorter (18944 x 3584 9.2 us against 11.4, 37888 x 3584 14.6 against 15.5, 18928 x 4096 10.2
-//     against 11.9) except where its CTAs of 128 rows leave SMs over, which it fills by twice the warps per tile, and K is long
-//     (17570 x 4096 13.4 against 11.3, 14739 x 6912 20.0 against 14.6): of 106 calls that this takes 2 are lost (10 %).  At three and four tokens X has 32 bits here and 16 there: level
-//     above eighty million weights (2 of 11 lost, 6 %), shorter there below.
-//   * Ring kernel: never shorter (1840 calls, 1.65 times as fast here, one lost).
+//     M and K brought here stays.
+//   * Ring kernel: never shorter.
 bool gemv_tc_shorter(const void* X, const void* Wq, const void* S, const void* Y, int M, int N, int K, int G, int flags,
                      int sm_count, size_t partial_cap, TcOther other) {
-  if (M < 2 || (flags & ~kFlagNoPdl) != 0 || !tc_operands(X, Wq, S, Y, M, N, K, G)) return false;
+  if (M < 1 || (flags & ~kFlagNoPdl) != 0 || !tc_operands(X, Wq, S, Y, M, N, K, G)) return false;
   const double w = 1e-6 * N * K, k3 = 1e-3 * K, mk = 1e-4 * M * K;
   TcPlan pl;
   if (!tc_plan(M, N, K, sm_count, 0, 0, &pl)) return false;
+  if (M == 1) {
+    if (w <= 12.0) return K >= 1024 && (N <= 5776 ? pl.us <= 8.5 : pl.us <= 3.5);
+    return (K >= 9728 && K <= 16384 && N <= 4992) || (K >= 22016 && N >= 7424);
+  }
   if (other == kTcOtherRing) return true;
   if (other == kTcOtherStream)
-    return M == 2 ? K >= 3840 && N <= 128 * (sm_count - 1) : w >= 80.0 && 1.02 * pl.us < 2.6 + 0.094 * w + 0.011 * k3 + 1.75 * mk;
+    return M > 2       ? K >= 2304 || N <= 12000
+           : K >= 3840 ? N <= 128 * (sm_count - 1)  // (above, that kernel's CTAs of 128 rows leave no SM over)
+                       : N <= (K <= 1536 ? 5800 : 11000);
   if (M <= 4) return 1.02 * pl.us < 6.65 + 0.11 * w + 0.027 * k3 + 0.074 * mk;
   const double us = pl.us + (pl.form       ? 2.03 * pl.busy * pl.busy
                              : pl.several ? 0.5
@@ -708,6 +766,12 @@ int gemv_tc_launch(const void* X, const void* Wq, const void* S, void* Y, int M,
   p.ks = pl.ks;
   tc_layout(pl, M, &p);
   p.ahead = 3;
+  // Where the rings of nearly all SMs fill at once X waits behind them for two microseconds: then only the first slot goes ahead
+  // of it (8192 x 28672 at 8 tokens 30.2 -> 29.3 us, 37888 x 3584 at 13 17.4 -> 16.9).  Elsewhere it is X that is waited for (4608 x
+  // 3584 at 4 tokens 5.8 against 6.1), and with a short K and few tokens it is there soon enough between other launches (four
+  // 7B-shaped layers at 4 tokens 154.1 against 157.0, at 13 185.9 against 184.5).
+  const long ctas = (long)((N + rows - 1) / rows) * p.ks;
+  p.x_first = (mt == 16 || p.pairs > 16) && p.pairs / p.ks > 4 && ctas * 10 >= (form ? 8 : 9) * (long)sm_count;
   CUtensorMap tw;
   if (!make_tensor_map_2d(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, Wq, (uint64_t)N, (uint64_t)K / 8, 128, 32,
                           CU_TENSOR_MAP_SWIZZLE_128B))

@@ -132,3 +132,26 @@ def test_a_plain_call_runs_the_kernel_it_is_described_as(kernels, M, N, K):
     assert kernels.gemv_describe(M, N, K, 128, flags[name]) == kernels.gemv_describe(M, N, K, 128)
     X, Wq, S = oracle.synth_inputs(M, N, K, 128, seed=8)
     assert np.array_equal(run(kernels, X, Wq, S, 0), run(kernels, X, Wq, S, flags[name]))
+
+
+# us of the streaming kernel and of this one
+@pytest.mark.parametrize("N,K,here", [
+    (512, 3584, True),      # 4.5, 3.4
+    (130, 1024, True),      # 3.5, 2.7
+    (130, 768, False),
+    (5776, 2048, True),     # 4.5, 4.4
+    (4980, 14080, True),    # 15.0, 12.8
+    (8192, 28672, True),    # 29.2, 26.6
+    (3584, 3584, False),    # 5.0, 5.1
+    (8430, 1024, False),    # 4.1, 4.8
+    (6308, 5632, False),    # 7.8, 8.4
+])
+def test_one_token_runs_the_shorter_kernel(kernels, N, K, here):
+    assert ("tcgen05" in kernels.gemv_describe(1, N, K, 128)) == here
+    X, Wq, S = oracle.synth_inputs(1, N, K, 128, seed=7)
+    f = oracle.bf16_bits_to_f32(X).copy()
+    f[0, ::97] *= np.float32(1000.0)  # X has 32 bits in either kernel: outliers cost the others nothing
+    X = oracle.f32_to_bf16_bits(f)
+    rows = np.unique(np.concatenate([[0, N - 1], np.random.default_rng(0).integers(0, N, 60)]))
+    ref = oracle.w4_linear_f32(X, Wq[rows], S[rows], 128, threads=oracle.max_threads())
+    check_bf16_output(run(kernels, X, Wq, S, 0)[:, rows], ref, slack(1))
