@@ -13,15 +13,17 @@
 //     the MMA takes its A operand from there.  Shared memory carries the packed words once and the X tile;
 //   * K is cut over the CTAs of a CLUSTER (up to eight), which add their fp32 accumulators up through distributed shared
 //     memory in rank order: no scratch in global memory, no counters, the result does not depend on timing;
-//   * launched programmatically: while the previous kernel finishes, the first packed words and scales are brought into
-//     L2.  All reads and writes come after it has, so it may be the kernel that writes the weights.  (Sixteen launches of
-//     a decoder stack at 48 tokens, us: ring filled before the wait 233, nothing 248, the whole ring into L2 251, its first
-//     slot 243.)
-// Measured, weights from HBM, against w4_gemm.cu at 48 tokens: 4608 x 3584 7.9 us (25), 37888 x 3584 22.7 (46), 3584 x
-// 18944 17.8 (51), 8192 x 28672 39.5 (113), all with 17 instructions per eight weights; with ten, sixteen such launches (four
-// 7B-shaped layers) take 228 us instead of 241, 777 x 5000 x 4096 in groups of 64 34.1 instead of 35.7, 512 x 3584 x 18944 73.2
-// instead of 77.2.  Of the 22.7 us, 11 are the weights' way from HBM; with the conversion taken out (a copy of the raw
-// words) it took 17.5: a step's chain of waits, then the conversion's issue slots.
+//   * launched programmatically: the first slots of packed words are brought into L2 ahead of everything else, the first scales
+//     before the wait for the kernel in front.  All reads and writes come after it has finished, so it may be the kernel that
+//     writes the weights.
+// Measured, weights from HBM, us at 48 tokens, in brackets w4_gemm.cu: 4608 x 3584 8.8 (25), 37888 x 3584 23.3 (46), 3584 x 18944 16.7
+// (51), 8192 x 28672 42 (113).  What moved them: weights converted in ten instructions instead of 17 per eight (sixteen such launches,
+// four 7B-shaped layers, 241 -> 228 us), then the questions to the barriers ahead of the last products of a step, parts of a
+// cut K sent instead of fetched and tensor memory freed beside the last sums (224; 777 x 5000 x 4096 in groups of 64 34.1 -> 33.2,
+// 512 x 3584 x 18944 73 -> 69, 128 x 37888 x 3584 37.1 -> 34.7).  What bounds it: at 48 tokens the sixteen products of a step
+// take 590 cycles (37 each, whatever the tokens up to 64: the weights' way out of tensor memory) and the conversion 980 per step
+// of either group, neither hidden whole by the other; 11 of the 23.3 us are HBM's; from 112 token columns the products (57 cycles
+// each).  A third group of conversion warps (24 in all, three buffers) changed nothing.
 // Warps: 0 packed words (TMA), 1 MMA issue and TMEM, 2 X tiles (TMA), 3 idle, then DW conversion warps, which also do
 // the epilogue.  All rings run on mbarriers with bounded waits; a CTA that gives up records a status, still takes part in
 // the cluster barriers, frees its TMEM and returns.
@@ -44,6 +46,9 @@ constexpr int kMaxSlots = 10;
 constexpr int kHeaderBytes = 1024;    // barriers and flags
 constexpr int kSmemHalf = 115712;     // two CTAs per SM: (228 KB / 2) - 1 KB
 constexpr int kSmemFull = 232448;
+constexpr uint32_t kUnitBytes = 16 * 32 * 4;  // fp32 sums of 16 tokens x 32 rows
+constexpr int kMinSlots = 3;                  // slots of packed words that a CTA with work for them keeps
+constexpr int kAhead = 3;  // slots of packed words brought into L2 ahead of the wait for the kernel in front
 
 struct NarrowParams {
   const __nv_bfloat16* S;
@@ -57,6 +62,7 @@ struct NarrowParams {
   int sw, sx;     // ring slots of packed words, of X
   int sv;         // scales per load: 4, 2 or 1, by the alignment of a row of S
   int tmem_cols;  // power of two
+  int red;        // offset of the parts of a cut K, sent there as they are ready; 0: none, they lie over the rings and are fetched
 };
 
 // D[tmem] (+)= A[tmem] * B[smem desc]: A is 128 lanes x 8 columns of bf16 pairs per K = 16.
@@ -86,7 +92,7 @@ __global__ void __launch_bounds__(128 + DW * 32, MINB)
   const uint32_t bar_w_full = base, bar_w_empty = base + 8 * kMaxSlots;
   const uint32_t bar_x_full = base + 16 * kMaxSlots, bar_x_empty = base + 24 * kMaxSlots;
   const uint32_t bar_a_full = base + 32 * kMaxSlots, bar_a_empty = bar_a_full + 16;
-  const uint32_t bar_acc = bar_a_empty + 16;
+  const uint32_t bar_acc = bar_a_empty + 16, bar_red = bar_acc + 8;
   volatile int* abort_flag = reinterpret_cast<volatile int*>(gen + 512);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(gen + 516);
   volatile int* status_seen = reinterpret_cast<volatile int*>(gen + 520);
@@ -99,6 +105,14 @@ __global__ void __launch_bounds__(128 + DW * 32, MINB)
   const int m0 = (tile % p.t_tiles) * p.nt, n0 = (tile / p.t_tiles) * kRows;
   const int kb0 = (int)((long)crank * p.nkb / p.ks), nkb = (int)((long)(crank + 1) * p.nkb / p.ks) - kb0;
 
+  // Units of 16 tokens x 32 rows, in the order (tokens, rows): the parts of a cut K are added by unit, and these are this CTA's.
+  const int rt = min(p.nt, p.M - m0), units = (rt + 15) / 16 * (kRows / 32);
+  const int first_unit = (crank * units + p.ks - 1) / p.ks, n_units = ((crank + 1) * units + p.ks - 1) / p.ks - first_unit;
+  const uint32_t red = base + p.red;
+
+  // (only brought into L2: the kernel in front may be the one that writes them)
+  if (tid == 64)
+    for (int i = 0; i < nkb && i < 2 * kAhead; i += 2) tma_prefetch_2d(&tmap_w, (kb0 + i) * (kKB / 8), n0);
   if (tid == 0) {
     *abort_flag = 0;
     for (int s = 0; s < kMaxSlots; ++s) {
@@ -112,6 +126,8 @@ __global__ void __launch_bounds__(128 + DW * 32, MINB)
       mbar_init(bar_a_empty + 8 * b, 1);
     }
     mbar_init(bar_acc, 1);
+    mbar_init(bar_red, 1);
+    if (p.red) mbar_arrive_expect_tx(bar_red, (uint32_t)(n_units * p.ks) * kUnitBytes);
     fence_mbar_init();
     tma_prefetch_desc(&tmap_w);
     tma_prefetch_desc(&tmap_x);
@@ -125,14 +141,16 @@ __global__ void __launch_bounds__(128 + DW * 32, MINB)
   __syncthreads();
   tc_fence_after_sync();
   pdl_launch_dependents();
+  if (p.red) cluster_arrive();  // (waited for before the first store into a peer: its barrier is set up)
   const uint32_t tmem_d = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   const uint32_t tmem_a = tmem_d + ((MB * p.nt + 31) & ~31);
   const bool poisoned = *status_seen != 0;
+  // Behind this the conversion warps leave tensor memory alone: the warp that allocated it frees it while they add up and store.
+  auto rows_done = [&] { asm volatile("bar.arrive 1, %0;" ::"n"(DW * 32 + 32) : "memory"); };
 
   if (!poisoned) {
     if (warp == 0) {
       if (lane == 0) {
-        tma_prefetch_2d(&tmap_w, kb0 * (kKB / 8), n0);
         pdl_wait_prior_grid();  // it may be the kernel that writes the weights
         int s = 0;
         uint32_t ph = 1;
@@ -168,28 +186,39 @@ __global__ void __launch_bounds__(128 + DW * 32, MINB)
       int xs = 0;
       uint32_t xph = 0;
       pdl_wait_prior_grid();  // the kernel in front may run longer than a bounded wait for X
+      // An answer of a barrier takes some 130 cycles: the questions of the next step go in ahead of the last products of this one,
+      // which the tensor core takes as long to get through (128 tokens, 37888 x 3584: 37.1 -> 36.2 us; 48: 24.7 -> 24.1).
+      bool ready = false;
       for (int i = 0; i < nkb; ++i) {
-        const int buf = i & 1;
-        mbar_wait(bar_x_full + 8 * xs, xph, abort_flag);
-        mbar_wait(bar_a_full + 8 * buf, (i >> 1) & 1, abort_flag);
-        __syncwarp();
+        const int buf = i & 1, xs_this = xs;
+        if (!ready) {
+          if (!__all_sync(0xffffffffu, mbar_try_wait2(bar_x_full + 8 * xs, xph, bar_a_full + 8 * buf, (i >> 1) & 1))) {
+            mbar_wait(bar_x_full + 8 * xs, xph, abort_flag);
+            mbar_wait(bar_a_full + 8 * buf, (i >> 1) & 1, abort_flag);
+            __syncwarp();
+          }
+        }
         tc_fence_after_sync();
         const uint64_t db = desc0 + ((xs * x_slot) >> 4);
         const uint32_t a = tmem_a + buf * MB * 64;
+        if (++xs == p.sx) { xs = 0; xph ^= 1; }
+        bool next = false;
         if (elect_one()) {
 #pragma unroll
           for (int kk = 0; kk < 8; ++kk) {
+            if (kk == 7)  // (of no meaning behind the last step)
+              next = mbar_test_wait2(bar_x_full + 8 * xs, xph, bar_a_full + 8 * (buf ^ 1), ((i + 1) >> 1) & 1);
             const uint64_t d = db + (kk & 3) * 2 + (kk >> 2) * (x_slot >> 5);
 #pragma unroll
             for (int mb = 0; mb < MB; ++mb)
               umma_f16_ts(tmem_d + mb * p.nt, a + mb * 64 + kk * 8, d, idesc, (i > 0 || kk > 0) ? 1u : 0u);
           }
           umma_commit(bar_a_empty + 8 * buf);
-          umma_commit(bar_x_empty + 8 * xs);
+          umma_commit(bar_x_empty + 8 * xs_this);
           if (i + 1 == nkb) umma_commit(bar_acc);
         }
+        ready = __any_sync(0xffffffffu, next);
         __syncwarp();
-        if (++xs == p.sx) { xs = 0; xph ^= 1; }
       }
     }
   }
@@ -326,7 +355,7 @@ __global__ void __launch_bounds__(128 + DW * 32, MINB)
       tc_fence_after_sync();
 
       // ---- the accumulator columns (tokens) of the warp's 32 rows; two groups of warps take alternate 16 columns
-      const int rt = min(p.nt, p.M - m0);  // tokens of the tile
+      if (p.red) cluster_wait();
       for (int c0 = 16 * grp; c0 < rt; c0 += 16 * kGroups) {
         uint32_t v[16];
         tmem_ld_32x16(tmem_d + lane_off + mb * p.nt + c0, v);
@@ -336,6 +365,14 @@ __global__ void __launch_bounds__(128 + DW * 32, MINB)
 #pragma unroll
           for (int e = 0; e < 16; ++e)
             if (live && c0 + e < rt) y[(size_t)e * p.N] = __float2bfloat16(__uint_as_float(v[e]) * (1.f / kDequantUnit));
+        } else if (p.red) {
+          // a unit's parts go to the CTA that adds them, in the order of ranks: [unit][rank][four tokens][row]
+          const int u = c0 / 16 * (kRows / 32) + (row >> 5), owner = u * p.ks / units;
+          const uint32_t at = red + (uint32_t)((u - (owner * units + p.ks - 1) / p.ks) * p.ks + crank) * kUnitBytes + lane * 16;
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            st_async_f4(at + q * 512, bar_red, owner, __uint_as_float(v[4 * q]), __uint_as_float(v[4 * q + 1]),
+                        __uint_as_float(v[4 * q + 2]), __uint_as_float(v[4 * q + 3]));
         } else {  // [token][row], over the rings: every copy has landed and every MMA has read its operands
 #pragma unroll
           for (int e = 0; e < 16; ++e)
@@ -343,16 +380,58 @@ __global__ void __launch_bounds__(128 + DW * 32, MINB)
                          : "memory");
         }
       }
+      tc_fence_before_sync();
+      __syncwarp();
+      rows_done();
+      if (p.red && dw < n_units) {
+        mbar_wait(bar_red, 0, abort_flag);
+        __syncwarp();
+        for (int b = dw; b < n_units; b += DW) {
+          const int u = first_unit + b, c0 = u / (kRows / 32) * 16, ny = n0 + u % (kRows / 32) * 32 + lane;
+          const uint32_t part = red + (uint32_t)(b * p.ks) * kUnitBytes + lane * 16;
+          __nv_bfloat16* y = p.Y + (size_t)(m0 + c0) * p.N + ny;
+#pragma unroll 1
+          for (int q = 0; q < 4; ++q) {
+            float sum[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int z = 0; z < 8; ++z)
+              if (z < p.ks) {
+                const uint4 f = lds128(part + z * kUnitBytes + q * 512);
+                sum[0] += __uint_as_float(f.x);
+                sum[1] += __uint_as_float(f.y);
+                sum[2] += __uint_as_float(f.z);
+                sum[3] += __uint_as_float(f.w);
+              }
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              if (ny < p.N && c0 + 4 * q + e < rt)
+                y[(size_t)(4 * q + e) * p.N] = __float2bfloat16(sum[e] * (1.f / kDequantUnit));
+          }
+        }
+      }
+    } else {  // (this barrier has no limit)
+      rows_done();
     }
   }
-  tc_fence_before_sync();
-  if (p.ks > 1) {
+  __syncwarp();
+  bool freed = false;
+  if (warp == 1) {
+    asm volatile("bar.sync 1, %0;" ::"n"(DW * 32 + 32) : "memory");
+    if (!poisoned && !__any_sync(0xffffffffu, *abort_flag != 0)) {  // (every product has been waited for)
+      tc_fence_after_sync();
+      tmem_dealloc(tmem_d, p.tmem_cols);
+      freed = true;
+    }
+  }
+  if (p.red) {
+    if (warp < 4 || poisoned) cluster_wait();
+  } else if (p.ks > 1) {
     cluster_barrier();
     // every CTA adds up its share of the tile, four rows of a token per thread, in rank order
     if (warp >= 4 && !poisoned) {
-      const int rt = min(p.nt, p.M - m0), units = rt * (kRows / 4);
-      const int u1 = (int)((long)(crank + 1) * units / p.ks);
-      for (int u = (int)((long)crank * units / p.ks) + tid - 128; u < u1; u += DW * 32) {
+      const int quads = rt * (kRows / 4);
+      const int u1 = (int)((long)(crank + 1) * quads / p.ks);
+      for (int u = (int)((long)crank * quads / p.ks) + tid - 128; u < u1; u += DW * 32) {
         const int tok = u / (kRows / 4), r = (u % (kRows / 4)) * 4, n = n0 + r;
         const uint32_t at = ring_w + (uint32_t)(tok * kRows + r) * 4;
         float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -380,12 +459,16 @@ __global__ void __launch_bounds__(128 + DW * 32, MINB)
     cluster_barrier();  // the peers have read this CTA's part
   }
   __syncthreads();
-  if (*abort_flag) {
+  if (*abort_flag || (poisoned && p.red)) {
+    if (p.red) {  // peers that have not given up may send parts here until they leave
+      cluster_arrive();
+      cluster_wait();
+    }
     if (tid == 0) atomicCAS(p.status, kStatusOk, kStatusGemmTimeout);
     for (int i = 0; i < 64; ++i) __nanosleep(2000);  // copies in flight land before the shared memory is released
     __syncthreads();
   }
-  if (warp == 1) {
+  if (warp == 1 && !freed) {
     tc_fence_after_sync();
     tmem_dealloc(tmem_d, p.tmem_cols);
   }
@@ -598,8 +681,18 @@ int gemm_narrow_launch(const void* X, const void* Wq, const void* S, void* Y, in
   const NarrowForm f = narrow_form(pl.form, narrow_variant(S, K, G));
   const int slot_w = f.rows * 128, slot_x = p.nt * 256, room = f.smem - kHeaderBytes - 1024;
   const int x_bytes = pl.form ? 128 << 10 : p.nt > 64 ? 72 << 10 : 48 << 10;  // the rest holds packed words
-  p.sx = std::max(2, std::min(6, x_bytes / slot_x));
+  const int blocks = (p.nkb + p.ks - 1) / p.ks;
+  p.sx = std::max(2, std::min({6, x_bytes / slot_x, blocks}));
   p.sw = std::min(kMaxSlots, (room - p.sx * slot_x) / slot_w);
+  // Up to 64 token columns the parts of a cut K have a place of their own where the rings can spare it: every CTA then sends them
+  // as soon as it has them and leaves (3584 x 3584 at 48 tokens 8.1 -> 7.2 us).  More columns are fetched from the rings' place
+  // behind a cluster barrier: sixteen bytes at a time, each counted, are slower from there (512 tokens 17.3 against 20.3).
+  const int units = p.nt / 16 * (f.rows / 32), parts = (units + p.ks - 1) / p.ks * p.ks * (int)kUnitBytes;
+  const int spare = (room - p.sx * slot_x - parts) / slot_w;
+  if (p.ks > 1 && p.nt <= 64 && spare >= std::min(kMinSlots, (blocks + 1) / 2)) {
+    p.sw = std::min(kMaxSlots, spare);
+    p.red = kHeaderBytes + p.sw * slot_w + p.sx * slot_x;
+  }
   p.tmem_cols = pl.form ? 512 : 256;
   CUtensorMap tx, tw;
   if (!make_tensor_map_2d(&tx, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, X, (uint64_t)M, (uint64_t)K, p.nt, 64,

@@ -78,18 +78,6 @@ __host__ __device__ constexpr uint32_t umma_idesc_s8(int b_signed, int M, int N)
   return (2u << 4) | (1u << 7) | (static_cast<uint32_t>(b_signed) << 10) | (static_cast<uint32_t>(N >> 3) << 17) |
          (static_cast<uint32_t>(M >> 4) << 24);
 }
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-// 16 bytes into the shared memory of CTA `rank` of the cluster, counted on its barrier at the same address as `bar` here.
-__device__ __forceinline__ void st_async_f4(uint32_t addr, uint32_t bar, uint32_t rank, float a, float b, float c, float d) {
-  asm volatile(
-      "{\n\t.reg .u32 a, m;\n\t"
-      "mapa.shared::cluster.u32 a, %0, %2;\n\t"
-      "mapa.shared::cluster.u32 m, %1, %2;\n\t"
-      "st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.f32 [a], {%3, %4, %5, %6}, [m];\n\t}" ::"r"(addr),
-      "r"(bar), "r"(rank), "f"(a), "f"(b), "f"(c), "f"(d)
-      : "memory");
-}
 template <int N>
 __device__ __forceinline__ void regs_up() {
   asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N));
@@ -169,8 +157,6 @@ __global__ void __launch_bounds__(MB == 2 ? 896 : 512, MB == 2 ? 1 : 2)
   if (p.ks > 1) cluster_arrive();  // (waited for before the first store into a peer: it runs by then, its barrier is set up)
   const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);  // [block][group]: 64 columns of sums, 64 of bytes
   const bool poisoned = __any_sync(0xffffffffu, status_seen != 0);
-  if (poisoned && lane == 0) *abort_flag = 1;  // the CTA's other warps may have read zero: their waits end
-
   // The rows' warps need more registers than an even share.  256 rows, 896 threads of 72: 4 x 88 + 2 x 48 + 56 = 7 x 72 by
   // warpgroup; 128 rows, 512 of 64: 2 x 80 + 2 x 48 = 4 x 64.
   if (warp < kMain) regs_up<MB == 2 ? 88 : 80>();
@@ -521,9 +507,12 @@ __global__ void __launch_bounds__(MB == 2 ? 896 : 512, MB == 2 ? 1 : 2)
         if (++xs == p.sx) xs = 0;
       }
     }
-  } else if (warp < kMain) {  // the CTA's other warps may be there, and these barriers have no limit
-    rows_done();
-    if (p.ks == 1) asm volatile("bar.sync %0, 256;" ::"r"(1 + (warp >> 2) % MB) : "memory");
+  } else {  // the CTA's other warps may have read zero: their waits end, and these barriers, which have no limit, are met
+    if (lane == 0) *abort_flag = 1;
+    if (warp < kMain) {
+      rows_done();
+      if (p.ks == 1) asm volatile("bar.sync %0, 256;" ::"r"(1 + (warp >> 2) % MB) : "memory");
+    }
   }
   __syncwarp();
   bool freed = false;
