@@ -64,8 +64,10 @@ __device__ __forceinline__ uint32_t abs_max_bits(const uint4& v) {
   return max(m & 0xFFFFu, m >> 16);
 }
 
-// LPG lanes per group (G = 8 LPG).  Groups tile W without gaps (K % G == 0), so W is one run of 8-weight words: a warp
-// takes kUnroll blocks of 32 consecutive words, all their loads in flight before the first is used.
+// LPG lanes per group, a lane two of its words (G = 16 LPG), half a group apart: a warp's load covers whole lines or sectors.  Groups
+// tile W without gaps (K % G == 0): a warp takes kUnroll times 32 / LPG consecutive groups, all their loads in flight before
+// the first is used.  The scale and its reciprocal are then computed once for sixteen weights of a lane, and the arithmetic takes
+// two weights per instruction: with one word per lane the kernel was bound by its 75 instructions per word as much as by memory.
 //
 // The division is replaced without changing a bit.  w and s have 8-bit significands, so w / s is either exactly halfway
 // between two integers or at least 2^-10 from it (the numerator of w / s - (k + 1/2) is a multiple of the smaller unit
@@ -74,70 +76,90 @@ __device__ __forceinline__ uint32_t abs_max_bits(const uint4& v) {
 // rint, and leaves q = rint(w / s) + 8 in the low mantissa bits; |w / s| <= 7.03, so no clamp.  This needs a finite,
 // normal s with a normal reciprocal; a group that has none, or an inf or a nan, is divided as before.
 //
-// 18944 x 3584 at G = 128: 34.8 us (4.9 TB/s of bf16 in, words and scales out), where a division per weight with half
-// of the lanes idle took 162 us (1.05 TB/s).
-constexpr int kUnroll = 4;  // 1, 2, 4, 8 loads in flight per lane: 45.1, 36.4, 35.0, 37.2 us
+// 18944 x 3584 at G = 128: 27.0 us (6.3 TB/s of bf16 in, words and scales out; a copy's rate), one word per lane 35.0, with a
+// division per weight and half of the lanes idle 162.
+constexpr int kUnroll = 2, kThreads = 128;  // 1, 2, 3, 4 at 256 threads: 30.4, 27.3, 27.8, 28.8 us; 2 at 128 and 512: 27.0, 28.8
 template <int LPG>
-__global__ void __launch_bounds__(256) w4_quantize_fast_kernel(const uint4* __restrict__ W, uint32_t* __restrict__ Wq,
-                                                               __nv_bfloat16* __restrict__ S, size_t words) {
-  const int lane = threadIdx.x & 31;
-  const size_t base = (((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * (32 * kUnroll) + lane;
-  uint4 v[kUnroll];
+__global__ void __launch_bounds__(kThreads) w4_quantize_fast_kernel(const uint4* __restrict__ W, uint32_t* __restrict__ Wq,
+                                                               __nv_bfloat16* __restrict__ S, size_t groups) {
+  constexpr int kGroups = 32 / LPG;  // of a warp at a time
+  const int lane = threadIdx.x & 31, r = lane % LPG;
+  const size_t g0 = (((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * (kGroups * kUnroll) + lane / LPG;
+  uint4 v[kUnroll][2];
 #pragma unroll
   for (int u = 0; u < kUnroll; ++u) {
-    v[u] = make_uint4(0u, 0u, 0u, 0u);
-    if (base + u * 32 < words) v[u] = __ldcs(W + base + u * 32);
+    const size_t g = g0 + u * kGroups;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      v[u][h] = make_uint4(0u, 0u, 0u, 0u);
+      if (g < groups) v[u][h] = __ldcs(W + g * (2 * LPG) + h * LPG + r);
+    }
   }
 #pragma unroll
   for (int u = 0; u < kUnroll; ++u) {
-    uint32_t mx = abs_max_bits(v[u]);
+    uint32_t mx = max(abs_max_bits(v[u][0]), abs_max_bits(v[u][1]));
 #pragma unroll
     for (int o = LPG / 2; o > 0; o >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    const uint32_t e[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
     __nv_bfloat16 sb = __float2bfloat16(mx ? __fdiv_rn(__uint_as_float(mx << 16), 7.f) : 1.f);
     float sf = __bfloat162float(sb);
-    uint32_t word = 0;
+    uint32_t word[2] = {0u, 0u};
     // s outside [2^-100, 2^100] (or of an infinite or nan maximum): the quotient itself
     const bool plain = mx < 0x7F80u && sf >= 0x1p-100f && sf <= 0x1p100f;
     if (__all_sync(0xffffffffu, plain)) {
-      const float r = __frcp_rn(sf);
+      const float rc = __frcp_rn(sf);
+      const float2 rc2 = make_float2(rc, rc), half2 = make_float2(1536.f, 1536.f);
       const float to_int = 12582912.f - 1536.f + 8.f;  // 1.5 * 2^23 + 8: q in the low mantissa bits
+      const float2 to_int2 = make_float2(to_int, to_int);
 #pragma unroll
-      for (int i = 3; i >= 0; --i) {
-        const float hi = __fadd_rn(fmaf(__uint_as_float(e[i] & 0xFFFF0000u), r, 1536.f), to_int);
-        const float lo = __fadd_rn(fmaf(__uint_as_float(e[i] << 16), r, 1536.f), to_int);
-        word = word * 16u + __float_as_uint(hi);
-        word = word * 16u + __float_as_uint(lo);
+      for (int h = 0; h < 2; ++h) {
+        const uint32_t e[4] = {v[u][h].x, v[u][h].y, v[u][h].z, v[u][h].w};
+#pragma unroll
+        for (int i = 3; i >= 0; --i) {
+          const float2 w2 = make_float2(__uint_as_float(e[i] << 16), __uint_as_float(e[i] & 0xFFFF0000u));
+          const float2 q = add_f32x2(fma_f32x2(w2, rc2, half2), to_int2);
+          word[h] = word[h] * 16u + __float_as_uint(q.y);
+          word[h] = word[h] * 16u + __float_as_uint(q.x);
+        }
+        word[h] -= 0x4B400000u * 0x11111111u;  // what the eight exponents left (modulo 2^32)
       }
-      word -= 0x4B400000u * 0x11111111u;  // what the eight exponents left (modulo 2^32)
     } else {
       float m = 0.f;  // the maximum leaves nans out, like fmaxf
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
-        m = fmaxf(m, fmaxf(fabsf(__uint_as_float(e[i] << 16)), fabsf(__uint_as_float(e[i] & 0xFFFF0000u))));
+      for (int h = 0; h < 2; ++h) {
+        const uint32_t e[4] = {v[u][h].x, v[u][h].y, v[u][h].z, v[u][h].w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          m = fmaxf(m, fmaxf(fabsf(__uint_as_float(e[i] << 16)), fabsf(__uint_as_float(e[i] & 0xFFFF0000u))));
+      }
 #pragma unroll
       for (int o = LPG / 2; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
       sb = __float2bfloat16(m > 0.f ? __fdiv_rn(m, 7.f) : 1.f);
       sf = __bfloat162float(sb);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const float w = __uint_as_float(i & 1 ? e[i >> 1] & 0xFFFF0000u : e[i >> 1] << 16);
-        word |= static_cast<uint32_t>(min(15, max(0, __float2int_rn(__fdiv_rn(w, sf)) + 8))) << (4 * i);
+      for (int h = 0; h < 2; ++h) {
+        const uint32_t e[4] = {v[u][h].x, v[u][h].y, v[u][h].z, v[u][h].w};
+#pragma unroll 1
+        for (int i = 0; i < 8; ++i) {
+          const uint32_t pair = i < 2 ? e[0] : i < 4 ? e[1] : i < 6 ? e[2] : e[3];
+          const float w = __uint_as_float(i & 1 ? pair & 0xFFFF0000u : pair << 16);
+          word[h] |= static_cast<uint32_t>(min(15, max(0, __float2int_rn(__fdiv_rn(w, sf)) + 8))) << (4 * i);
+        }
       }
     }
-    const size_t at = base + u * 32;
-    if (at < words) {
-      Wq[at] = word;
-      if (lane % LPG == 0) S[at / LPG] = sb;
+    const size_t g = g0 + u * kGroups;
+    if (g < groups) {
+      __stcs(Wq + g * (2 * LPG) + r, word[0]);
+      __stcs(Wq + g * (2 * LPG) + LPG + r, word[1]);
+      if (r == 0) S[g] = sb;
     }
   }
 }
 
 template <int LPG>
-void launch_fast(const void* W, void* Wq, void* S, size_t words, cudaStream_t stream) {
-  const size_t per_cta = 8 * 32 * kUnroll;
-  w4_quantize_fast_kernel<LPG><<<(unsigned)((words + per_cta - 1) / per_cta), 256, 0, stream>>>(
-      static_cast<const uint4*>(W), static_cast<uint32_t*>(Wq), static_cast<__nv_bfloat16*>(S), words);
+void launch_fast(const void* W, void* Wq, void* S, size_t groups, cudaStream_t stream) {
+  const size_t per_cta = (kThreads / 32) * (32 / LPG) * kUnroll;
+  w4_quantize_fast_kernel<LPG><<<(unsigned)((groups + per_cta - 1) / per_cta), kThreads, 0, stream>>>(
+      static_cast<const uint4*>(W), static_cast<uint32_t*>(Wq), static_cast<__nv_bfloat16*>(S), groups);
 }
 
 }  // namespace
@@ -147,13 +169,13 @@ int quantize_launch(const void* W, void* Wq, void* S, int N, int K, int G, cudaS
   if (!W || !Wq || !S) return kErrBadPointer;
   // 16-byte loads of W need 16-byte aligned rows and groups: K % 8 == 0 follows from G % 32 == 0
   if (reinterpret_cast<uintptr_t>(W) & 15) return kErrBadPointer;
-  const size_t groups = (size_t)N * (K / G), words = groups * (G / 8);
+  const size_t groups = (size_t)N * (K / G);
   if (G == 32 || G == 64 || G == 128 || G == 256) {
     switch (G) {
-      case 32: launch_fast<4>(W, Wq, S, words, stream); break;
-      case 64: launch_fast<8>(W, Wq, S, words, stream); break;
-      case 128: launch_fast<16>(W, Wq, S, words, stream); break;
-      default: launch_fast<32>(W, Wq, S, words, stream); break;
+      case 32: launch_fast<2>(W, Wq, S, groups, stream); break;
+      case 64: launch_fast<4>(W, Wq, S, groups, stream); break;
+      case 128: launch_fast<8>(W, Wq, S, groups, stream); break;
+      default: launch_fast<16>(W, Wq, S, groups, stream); break;
     }
     return (int)cudaGetLastError();
   }
