@@ -201,10 +201,10 @@ int b2_w4_gemv_noalloc(const void* X, const void* Wq, const void* S, void* Y, in
  *   b2_decode_attention_fused: both of the above with the RoPE / KV-store launch folded into the attention pass.
  *     qkv is read, not modified: every CTA rotates the query heads it serves in registers; the CTA whose key slice
  *     holds position *pos builds the new k and v rows, stores them to the caches and uses them from shared memory.
- *     flags 0: the merge of the key slices is a second launch (two launches in all; the faster form: 9.0 -> about
- *     7 us per layer at 600 positions).  flags 1: ONE launch; the last CTA of a KV head to finish merges the slices
- *     (an arrival counter per KV head; nobody waits), which puts a fence, an atomic and the merge's two L2 round
- *     trips behind the slowest CTA.  flags 2 (may be added to either): the caller promises that the kernel launched
+ *     flags 0: without tp ONE launch, a cluster of sixteen CTAs per KV head that exchange the key slices' results (the
+ *     fastest form); with tp the merge of the key slices is a second launch.  flags 1: one launch in which the last CTA of a
+ *     KV head to finish merges the slices (an arrival counter per KV head; nobody waits), which puts a fence, an atomic and
+ *     the merge's two L2 round trips behind the slowest CTA.  flags 2 (may be added to either): the caller promises that the kernel launched
  *     in front of this one on the stream writes neither *pos nor cached rows below *pos (true for a decode step, where
  *     that kernel is the q|k|v projection); the first tile of cached rows is then requested before that kernel has
  *     completed.  Results are bit-identical to the two calls above in every form.

@@ -72,6 +72,11 @@ int* device_status_word(int* rc) {
   DeviceState* st = device_state(rc);
   return st ? st->ws.status : nullptr;
 }
+int* device_status_word_if_ready() {
+  int dev = -1;
+  DeviceState* st = device_state_if_ready(&dev);
+  return st ? st->ws.status : nullptr;
+}
 }  // namespace b2
 
 namespace {

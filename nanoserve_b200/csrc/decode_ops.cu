@@ -7,11 +7,14 @@
 // 147-151, 174-177: bias add, rope, _store_kv, SDPA over the cache, argmax); a host-side position would force one
 // graph per step.  Arithmetic follows the reference's conventions: bf16 storage, fp32 math, rotate-half RoPE with
 // angle = pos * inv_freq[i] (kernels/fused/rope.cuh:14-43), softmax scale 1/sqrt(D).
+#include <atomic>
 #include <cfloat>
 #include <cstdint>
 #include <cuda_bf16.h>
 
 #include "../../include/nanoserve_b200.h"
+#include "ptx.cuh"
+#include "w4_common.cuh"
 #include "w4_internal.h"
 
 namespace {
@@ -454,6 +457,268 @@ __global__ void __launch_bounds__(256) decode_attention_fused_kernel(
   }
 }
 
+// The same in one launch without a last CTA to wait for: the sixteen CTAs of a KV head are a cluster and send their partials to
+// the CTA that merges them (st.async, counted on a barrier of that CTA; CTA r merges dimensions [r D/16, (r + 1) D/16) of every
+// head).  A CTA holds two of the 32 slices, a warp one (query head, slice); every sum is taken over the same values in the same
+// order as in the two kernels above, so the results are theirs to the bit.
+// What bounds it is latency: 0.6 us until the kernel in front is seen complete, 0.6 for q's load and the rotation, 2 for the rows of a
+// slice, one way through the cluster 0.5, the merge 0.5.  A layer's attention at 560 positions, alone in a chain: 8.6 us in two
+// launches, 5.6 in this one; a decode step of 28 layers 1.567 -> 1.490 ms.  On the way: eight CTAs of 28 warps found no place beside a
+// GEMV's CTA and started late (1.620 ms); a butterfly per row and an exponential per row and warp took 270 cycles a row.
+constexpr int kAttnCtas = 16, kSlicesPerCta = kSplits / kAttnCtas;
+template <int D>
+struct AttnSmem {  // offsets of the dynamic shared memory
+  static constexpr int kTile = kSlicesPerCta * kTileRows * D * 2;  // K or V rows of a pass
+  static constexpr int kNew = 2 * kTile;                           // the new k and v row
+  static constexpr int kMaxSum = kNew + 4 * D;                     // [head][slice] maximum and sum
+  static constexpr int kPart = kMaxSum + 8 * kSplits * 8;          // [head][slice][D / 8] un-normalised
+  static constexpr int kRot = kPart + 8 * kSplits * (D / kAttnCtas) * 4;  // sine and cosine of the new position
+  // More than half of an SM, so that no SM takes two of these CTAs while others have none, and less than what a GEMV's CTA (112
+  // KB) leaves: it is there early, and the next kernel's beside it.  (1.513 -> 1.490 ms per token.)
+  static constexpr int kBytes = 116224;
+  static_assert(kRot + D / 2 * 8 <= kBytes, "shared memory");
+};
+// E (2 or 4) consecutive bf16 of shared memory as floats.
+template <int E>
+__device__ __forceinline__ void lds_row(const bf16* p, float (&f)[E]) {
+  if constexpr (E == 4) {
+    const uint2 v = *reinterpret_cast<const uint2*>(p);
+    f[0] = __uint_as_float(v.x << 16);
+    f[1] = __uint_as_float(v.x & 0xFFFF0000u);
+    f[2] = __uint_as_float(v.y << 16);
+    f[3] = __uint_as_float(v.y & 0xFFFF0000u);
+  } else {
+    const unsigned v = *reinterpret_cast<const unsigned*>(p);
+    f[0] = __uint_as_float(v << 16);
+    f[1] = __uint_as_float(v & 0xFFFF0000u);
+  }
+}
+template <int E>
+__device__ __forceinline__ void send_part(uint32_t addr, uint32_t bar, uint32_t rank, const float (&a)[E]) {
+  if constexpr (E == 4) b2::st_async_f4(addr, bar, rank, a[0], a[1], a[2], a[3]);
+  else b2::st_async_f2(addr, bar, rank, a[0], a[1]);
+}
+
+template <int D>
+__global__ void __launch_bounds__(512, 2) decode_attention_cluster_kernel(
+    const bf16* qkv, const bf16* __restrict__ bias, const float* __restrict__ inv_freq, const int* pos_ptr,
+    bf16* cache_k, bf16* cache_v, bf16* out, int Hq, int Hk, int max_len, float scale, int early, int* status) {
+  constexpr int E = D / 32;        // elements per lane
+  constexpr int kRowU4 = D / 8;    // 16-byte units per row
+  constexpr int half = D / 2, kMine = D / kAttnCtas;
+  using S = AttnSmem<D>;
+  extern __shared__ __align__(16) unsigned char sm[];
+  __shared__ __align__(8) unsigned long long s_bar;
+  __shared__ int s_abort;
+  const uint32_t base = b2::smem_u32(sm), bar = b2::smem_u32(&s_bar);
+  bf16* s_k = reinterpret_cast<bf16*>(sm);
+  bf16* s_v = reinterpret_cast<bf16*>(sm + S::kTile);
+  bf16* s_newk = reinterpret_cast<bf16*>(sm + S::kNew);
+  bf16* s_newv = s_newk + D;
+  const int crank = (int)b2::cluster_rank(), kh = blockIdx.x / kAttnCtas;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, rep = Hq / Hk;
+  const int slice = warp / rep, w = warp - slice * rep, sp = crank * kSlicesPerCta + slice;
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (tid == 0) {
+    s_abort = 0;
+    b2::mbar_init(bar, 1);
+    b2::mbar_arrive_expect_tx(bar, (uint32_t)(rep * kSplits) * (kMine * 4 + 8));
+    b2::fence_mbar_init();
+  }
+  __syncthreads();
+  b2::cluster_arrive();  // (waited for before the first store into a peer: its barrier is set up)
+
+  const uint4* kbase = reinterpret_cast<const uint4*>(cache_k + (size_t)kh * max_len * D);
+  const uint4* vbase = reinterpret_cast<const uint4*>(cache_v + (size_t)kh * max_len * D);
+  int pos = 0, n = 0, per = 0;
+  auto find = [&]() {
+    pos = __ldcg(pos_ptr);
+    n = min(pos + 1, max_len);
+    per = (n + kSplits - 1) / kSplits;
+  };
+  // rows [t0, t0 + kTileRows) of each of the CTA's slices, copied past the registers; the row that this launch appends is not in
+  // the cache yet
+  auto request = [&](int t0) {
+    const int rows = min(kTileRows, per - t0), units = kSlicesPerCta * rows * kRowU4;
+    for (int u = tid; u < units; u += blockDim.x) {
+      const int c = u % kRowU4, r = u / kRowU4, sl = r / rows, j = (crank * kSlicesPerCta + sl) * per + t0 + (r - sl * rows);
+      if (j < n && j != pos) {
+        const uint32_t dst = base + ((sl * kTileRows + (r - sl * rows)) * kRowU4 + c) * 16;
+        b2::cp_async_cg16(dst, kbase + (size_t)j * kRowU4 + c);
+        b2::cp_async_cg16(dst + S::kTile, vbase + (size_t)j * kRowU4 + c);
+      }
+    }
+  };
+  // `early`: the position and the cached rows below it were written by earlier steps, not by the kernel in front of this one
+  if (early) {
+    find();
+    request(0);
+  }
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (!early) {
+    find();
+    request(0);
+  }
+  const int j0 = sp * per, j1 = min(n, j0 + per);
+
+  // ---- this warp's query head; the rotation's sines and cosines once per CTA
+  const int h = kh * rep + w;
+  float2* s_rot = reinterpret_cast<float2*>(sm + S::kRot);
+  float qf[E], qb[E];
+  ld_row<E>(qkv + (size_t)h * D + lane * E, qf);
+#pragma unroll
+  for (int e = 0; e < E; ++e) qb[e] = bias != nullptr ? __bfloat162float(bias[(size_t)h * D + lane * E + e]) : 0.f;
+  for (int i = tid; i < half; i += blockDim.x) {
+    float sn, cs;
+    sincosf((float)pos * inv_freq[i], &sn, &cs);
+    s_rot[i] = make_float2(sn, cs);
+  }
+  __syncthreads();
+  // ---- the new k and v rows, in the CTA whose slices hold the new position: i < D/2 rotates the pair (i, i + D/2) of k, the
+  // next D/2 add the bias to a pair of v
+  for (int t = tid; pos < max_len && pos / per / kSlicesPerCta == crank && t < D; t += blockDim.x) {
+    const bool is_v = t >= half;
+    const int i = is_v ? t - half : t;
+    const int hh = Hq + (is_v ? Hk : 0) + kh;
+    const bf16* x = qkv + (size_t)hh * D;
+    float a = ld_bf16(x + i), b = ld_bf16(x + i + half);
+    if (bias != nullptr) {
+      a = __bfloat162float(__float2bfloat16(a + __bfloat162float(bias[(size_t)hh * D + i])));
+      b = __bfloat162float(__float2bfloat16(b + __bfloat162float(bias[(size_t)hh * D + i + half])));
+    }
+    if (!is_v) {
+      const float sn = s_rot[i].x, cs = s_rot[i].y;
+      const float ra = a * cs - b * sn, rb = b * cs + a * sn;
+      a = ra;
+      b = rb;
+    }
+    const bf16 oa = __float2bfloat16(a), ob = __float2bfloat16(b);
+    bf16* row = is_v ? s_newv : s_newk;
+    row[i] = oa;
+    row[i + half] = ob;
+    bf16* dst = (is_v ? cache_v : cache_k) + ((size_t)kh * max_len + pos) * D;
+    dst[i] = oa;
+    dst[i + half] = ob;
+  }
+  // ---- bias, rotation, bf16 rounding, softmax scale
+  if (bias != nullptr) {
+#pragma unroll
+    for (int e = 0; e < E; ++e) qf[e] = __bfloat162float(__float2bfloat16(qf[e] + qb[e]));
+  }
+#pragma unroll
+  for (int e = 0; e < E; ++e) {
+    const float other = __shfl_xor_sync(0xffffffffu, qf[e], 16);  // the element D/2 away
+    const float2 rot = s_rot[(lane * E + e) % half];
+    const float sn = rot.x, cs = rot.y;
+    const float r = lane < 16 ? qf[e] * cs - other * sn : qf[e] * cs + other * sn;
+    qf[e] = __bfloat162float(__float2bfloat16(r)) * scale;
+  }
+
+  float m = -FLT_MAX, l = 0.f, acc[E];
+#pragma unroll
+  for (int e = 0; e < E; ++e) acc[e] = 0.f;
+  for (int t0 = 0; t0 < per; t0 += kTileRows) {
+    if (t0 > 0) {
+      __syncthreads();  // everybody is done with the rows of the last pass
+      request(t0);
+    }
+    b2::cp_async_wait_all();
+    __syncthreads();
+    // the new row into its place in the pass that holds it
+    if (const int r = pos - t0 - (crank * kSlicesPerCta + pos / per % kSlicesPerCta) * per;
+        pos < max_len && pos / per / kSlicesPerCta == crank && r >= 0 && r < kTileRows) {
+      const int at = (pos / per % kSlicesPerCta * kTileRows + r) * kRowU4;
+      for (int u = tid; u < 2 * kRowU4; u += blockDim.x)
+        *reinterpret_cast<uint4*>(sm + (u < kRowU4 ? 0 : S::kTile) + (at + u % kRowU4) * 16) =
+            reinterpret_cast<const uint4*>(s_newk)[u];
+      __syncthreads();
+    }
+    const int rows = min(kTileRows, j1 - j0 - t0);
+    const bf16* tk = s_k + slice * kTileRows * D + lane * E;
+    const bf16* tv = s_v + slice * kTileRows * D + lane * E;
+    // Eight rows at a time.  A row's parts are added over the lanes as one tree, as a butterfly would; each of its first three steps
+    // halves the rows that a lane goes on with (9 exchanges for the 40 of eight butterflies), and row q ends in lanes 4 q to
+    // 4 q + 3.  There the running maxima are a scan and the exponentials of all rows one instruction; only the products and sums
+    // that depend on one another go row by row.
+    for (int r0 = 0; r0 < rows; r0 += 8, tk += 8 * D, tv += 8 * D) {
+      float x[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {  // (what rows behind the slice's end hold is not used)
+        float kf[E];
+        lds_row<E>(tk + q * D, kf);
+        x[q] = 0.f;
+#pragma unroll
+        for (int e = 0; e < E; ++e) x[q] += qf[e] * kf[e];
+      }
+#pragma unroll
+      for (int o = 16, k = 4; o >= 4; o >>= 1, k >>= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int q = 0; q < k; ++q) {
+          const float give = up ? x[q] : x[q + k], keep = up ? x[q + k] : x[q];
+          x[q] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+      }
+      float sq = x[0];
+      sq += __shfl_xor_sync(0xffffffffu, sq, 2);
+      sq += __shfl_xor_sync(0xffffffffu, sq, 1);
+      float mn = sq;
+#pragma unroll
+      for (int o = 4; o < 32; o <<= 1) {
+        const float before = __shfl_up_sync(0xffffffffu, mn, o);
+        if (lane >= o) mn = fmaxf(before, mn);
+      }
+      mn = fmaxf(m, mn);
+      const float last = __shfl_up_sync(0xffffffffu, mn, 4), mp = lane < 4 ? m : last;
+      const float corr = __expf(mp - mn), pj = __expf(sq - mn);
+      const int count = min(8, rows - r0);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        if (q >= count) break;
+        const float c = __shfl_sync(0xffffffffu, corr, q * 4), pq = __shfl_sync(0xffffffffu, pj, q * 4);
+        float vf[E];
+        lds_row<E>(tv + q * D, vf);
+        l = l * c + pq;
+#pragma unroll
+        for (int e = 0; e < E; ++e) acc[e] = acc[e] * c + pq * vf[e];
+      }
+      m = __shfl_sync(0xffffffffu, mn, (count - 1) * 4);
+    }
+  }
+
+  // ---- partials to the CTAs that merge them: lanes 4 r .. 4 r + 3 hold the dimensions of CTA r
+  b2::cluster_wait();
+  send_part<E>(base + S::kPart + ((w * kSplits + sp) * kMine + lane % (32 / kAttnCtas) * E) * 4, bar, lane / (32 / kAttnCtas), acc);
+  if (lane < kAttnCtas) b2::st_async_f2(base + S::kMaxSum + (w * kSplits + sp) * 8, bar, lane, m, l);
+  if (warp < rep) {  // a warp merges a head: a lane a slice's weight, then a lane a dimension
+    b2::mbar_wait(bar, 0, &s_abort);
+    __syncwarp();
+    float2* ml = reinterpret_cast<float2*>(sm + S::kMaxSum) + warp * kSplits;
+    const float* as = reinterpret_cast<const float*>(sm + S::kPart) + warp * kSplits * kMine + lane % kMine;
+    const float2 mine = ml[lane];
+    float mm = mine.x;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) mm = fmaxf(mm, __shfl_xor_sync(0xffffffffu, mm, o));
+    ml[lane].x = mine.x == -FLT_MAX ? 0.f : __expf(mine.x - mm);
+    __syncwarp();
+    float num = 0.f, den = 0.f;
+#pragma unroll 16
+    for (int z = 0; z < kSplits; ++z) {
+      const float2 f = ml[z];
+      num += f.x * as[z * kMine];
+      den += f.x * f.y;
+    }
+    if (lane < kMine) out[(size_t)(kh * rep + warp) * D + crank * kMine + lane] = __float2bfloat16(den > 0.f ? num / den : 0.f);
+  }
+  __syncthreads();
+  if (s_abort) {  // a peer never sent: nothing may come in after this CTA has left
+    b2::cluster_arrive();
+    b2::cluster_wait();
+    if (tid == 0 && status != nullptr) atomicCAS(status, 0, b2::kStatusGemvTimeout);
+    for (int i = 0; i < 64; ++i) __nanosleep(2000);
+  }
+}
+
 // Greedy choice in two launches.  Pass 1, kArgBlocks CTAs: each scans a slice of the logits and writes its best
 // (value, index).  Pass 2, one CTA: picks the best of those (lowest index on ties, as torch.argmax returns the
 // first occurrence), records the token, advances step and position, and copies the token's embedding row.
@@ -607,6 +872,42 @@ int decode_attention_fused_launch(const void* qkv, const void* bias, const void*
   const bool one_launch = (flags & 1) != 0;
   int* counters = one_launch ? reinterpret_cast<int*>(part + (size_t)Hq * kSplits * (D + 2)) : nullptr;
   const dim3 grid(Hk, kSplits);
+  if (!one_launch && tp == nullptr) {
+    auto cluster = [&](auto kernel, int smem, std::atomic<bool>* done) {
+      int dev = -1;
+      cudaError_t e = cudaGetDevice(&dev);
+      if (e != cudaSuccess) return e;
+      const bool cached = dev >= 0 && dev < 64;
+      if (!cached || !done[dev].load(std::memory_order_acquire)) {
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) return e;
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        if (e != cudaSuccess) return e;
+        if (cached) done[dev].store(true, std::memory_order_release);
+      }
+      cudaLaunchConfig_t cfg{};
+      cfg.gridDim = dim3(Hk * kAttnCtas);
+      cfg.blockDim = dim3(Hq / Hk * kSlicesPerCta * 32);
+      cfg.dynamicSmemBytes = smem;
+      cfg.stream = stream;
+      cudaLaunchAttribute attr[2];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = kAttnCtas;
+      attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+      attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      attr[1].val.programmaticStreamSerializationAllowed = 1;
+      cfg.attrs = attr;
+      cfg.numAttrs = 2;
+      return cudaLaunchKernelEx(&cfg, kernel, static_cast<const bf16*>(qkv), static_cast<const bf16*>(bias),
+                                static_cast<const float*>(inv_freq), static_cast<const int*>(pos),
+                                static_cast<bf16*>(cache_k), static_cast<bf16*>(cache_v), static_cast<bf16*>(out), Hq, Hk,
+                                max_len, scale, (flags & 2) ? 1 : 0, device_status_word_if_ready());
+    };
+    static std::atomic<bool> done[2][64];
+    const cudaError_t e = D == 128 ? cluster(decode_attention_cluster_kernel<128>, AttnSmem<128>::kBytes, done[0])
+                                   : cluster(decode_attention_cluster_kernel<64>, AttnSmem<64>::kBytes, done[1]);
+    return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
+  }
   auto go = [&](auto kernel) {
     return launch_pdl(kernel, grid, dim3(256), stream, static_cast<const bf16*>(qkv),
                       static_cast<const bf16*>(bias), static_cast<const float*>(inv_freq),

@@ -374,7 +374,7 @@ __device__ __forceinline__ void cluster_barrier() {
 // The barrier's halves.  A thread that has left the kernel counts as arrived.
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
-// 16 bytes into the shared memory of CTA `rank` of the cluster, counted on its barrier at the same address as `bar` here.
+// 16 (8) bytes into the shared memory of CTA `rank` of the cluster, counted on its barrier at the same address as `bar` here.
 __device__ __forceinline__ void st_async_f4(uint32_t addr, uint32_t bar, uint32_t rank, float a, float b, float c, float d) {
   asm volatile(
       "{\n\t.reg .u32 a, m;\n\t"
@@ -385,6 +385,15 @@ __device__ __forceinline__ void st_async_f4(uint32_t addr, uint32_t bar, uint32_
       : "memory");
 }
 
+__device__ __forceinline__ void st_async_f2(uint32_t addr, uint32_t bar, uint32_t rank, float a, float b) {
+  asm volatile(
+      "{\n\t.reg .u32 a, m;\n\t"
+      "mapa.shared::cluster.u32 a, %0, %2;\n\t"
+      "mapa.shared::cluster.u32 m, %1, %2;\n\t"
+      "st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.f32 [a], {%3, %4}, [m];\n\t}" ::"r"(addr),
+      "r"(bar), "r"(rank), "f"(a), "f"(b)
+      : "memory");
+}
 __device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr, uint32_t rank) {
   float4 v;
   asm volatile(

@@ -147,6 +147,7 @@ int decode_attention_fused_launch(const void* qkv, const void* bias, const void*
                                   int max_len, const GemvTp* tp, int flags, int* status, cudaStream_t stream);
 // The status word of the current device's scratch (created on first use); rc receives 0 or an error code.
 int* device_status_word(int* rc);
+int* device_status_word_if_ready();  // null where the device has no state yet: never creates it
 int tp_wait_launch(const void* wait_sig, const void* epoch, unsigned wait_per_epoch, int* status, cudaStream_t stream,
                    const GemvTp* announce = nullptr, int advance_epoch = 0);
 int rope_kv_store_launch(void* qkv, const void* bias, const void* inv_freq, const void* pos, void* cache_k,

@@ -271,9 +271,9 @@ class Qwen2Runner:
 
     @torch.no_grad()
     def decode_step(self):
-        """One token.  Six launches per layer on one GPU: qkv GEMV (residual add + RMSNorm folded in), attention
-        (bias, RoPE, KV store and the pass over the cache in one kernel, then the merge), o GEMV, gate|up GEMV (add + norm
-        in its prologue, SwiGLU in its epilogue), down GEMV.
+        """One token.  Five launches per layer on one GPU: qkv GEMV (residual add + RMSNorm folded in), attention
+        (bias, RoPE, KV store, the pass over the cache and the merge in one kernel), o GEMV, gate|up GEMV (add + norm in its
+        prologue, SwiGLU in its epilogue), down GEMV.
         The residual stream alternates between two buffers because a fused GEMV may not overwrite the X other CTAs
         are still reading; every step starts again from `self.x`, where b2_greedy_next puts the next embedding."""
         if self.peer is not None:
@@ -473,7 +473,7 @@ def decode_rate(kernels: Kernels, device, rank: int = 0, world: int = 1, cfg: Op
     return {"tp_check": tp_check, "tokens_sha1": sha, "distinct_tokens": len(set(tokens)), "tok_s": (n_new - 1) / t_decode, "ms_per_token": t_decode / (n_new - 1) * 1e3,
             "prefill_tok_s": prompt_len / t_prefill, "prompt_len": prompt_len, "n_new": n_new,
             "weight_bytes_per_token_per_rank": r.weight_bytes_per_token(), "first_tokens": tokens[:8],
-            "launches_per_token": "6 per layer + lm_head (final norm and block argmax folded in) + the pick, one CUDA graph; " +
+            "launches_per_token": f"{5 if r.peer is None else 6} per layer + lm_head (final norm and block argmax folded in) + the pick, one CUDA graph; " +
                                   ("all-gathers fused into the GEMVs" if r.peer is not None else
                                    "NCCL all-gathers at the layer boundaries" if world > 1 else "one GPU")}
 
