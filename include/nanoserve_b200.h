@@ -238,6 +238,13 @@ int b2_greedy_next(const void* logits, int V, const void* embed, int H, void* po
 int b2_qkv_prefill(void* qkv, const void* bias, const void* inv_freq, void* cache_k, void* cache_v, int T, int Hq,
                    int Hk, int D, int max_len, void* stream);
 int b2_swiglu_blocks(const void* gu, void* out, int T, int I, int block, void* stream);
+/*
+ * Y [M, N/2] = SwiGLU of the projection X . dequant(Wq, S)^T whose rows alternate in blocks of 16 gate and 16 up rows (N % 32 ==
+ * 0): ns_w4_linear and b2_swiglu_blocks with block 16, to the bit, in one launch where the prefill GEMM runs the projection.  tmp:
+ * room for it, M * N bf16, left undefined.  tmp and Y 16-byte aligned.
+ */
+int b2_w4_linear_swiglu(const void* X, const void* Wq, const void* S, void* tmp, void* Y, int M, int N, int K, int G, int flags,
+                        void* stream);
 
 /*
  * The bf16 vocabulary projection of a decode step with the greedy argmax in its epilogue.  No counterpart in the

@@ -259,6 +259,20 @@ int b2_decode_attention_fused(const void* qkv, const void* bias, const void* inv
                                            static_cast<cudaStream_t>(stream));
 }
 
+int b2_w4_linear_swiglu(const void* X, const void* Wq, const void* S, void* tmp, void* Y, int M, int N, int K, int G, int flags,
+                        void* stream) {
+  if (N < 32 || N % 32) return b2::kErrBadShape;
+  if (!tmp || !Y || ((reinterpret_cast<uintptr_t>(tmp) | reinterpret_cast<uintptr_t>(Y)) & 15)) return b2::kErrBadPointer;
+  if (M <= 16) {
+    const int rc = linear_dispatch(X, Wq, S, tmp, M, N, K, G, flags, stream);
+    return rc != 0 ? rc : b2::swiglu_blocks_launch(tmp, Y, M, N / 2, 16, static_cast<cudaStream_t>(stream));
+  }
+  int rc = 0;
+  DeviceState* st = device_state(&rc);
+  if (!st) return rc;
+  return b2::gemm_launch(X, Wq, S, tmp, M, N, K, G, st->ws, flags, st->sm_count, static_cast<cudaStream_t>(stream), Y);
+}
+
 int ns_w4_quantize(const void* W, void* Wq, void* S, int N, int K, int G, void* stream) {
   return b2::quantize_launch(W, Wq, S, N, K, G, static_cast<cudaStream_t>(stream));
 }

@@ -36,7 +36,9 @@
 #include <algorithm>
 #include <cstdio>
 #include <mutex>
+#include <type_traits>
 
+#include "fused_ops.h"
 #include "ptx.cuh"
 #include "tensor_map.h"
 #include "w4_common.cuh"
@@ -55,6 +57,7 @@ constexpr int kDequantThreads = 512;        // two threads per weight row of the
 constexpr int kDequantWarps = kDequantThreads / 32;
 constexpr int kGemmThreads = 32 * 2 + kDequantThreads;
 constexpr int kGemmSmemLimit = 232448;
+constexpr int kPairBlock = 16;              // SwiGLU in the epilogue: rows of gate, then as many of up, alternate
 
 struct GemmParams {
   const __nv_bfloat16* S;
@@ -149,7 +152,50 @@ struct GemmGeo {
   static constexpr int kTmemCols = MI * kBN;                  // 256 or 512: powers of two
 };
 
-template <int MI, bool PAIR>
+// 32 sums of a token as outputs: rounded to bf16 and stored, or, SWIGLU, as 16 gate values and their 16 up values, each rounded to
+// bf16 first, silu(gate) * up (the bits of a plain launch and b2_swiglu_blocks: 13.4 us and a launch less per layer of 512 x 37888,
+// and half of what is stored).  `n`: the first of them among the matrix's rows.
+template <bool SWIGLU>
+__device__ __forceinline__ void store_outputs(__nv_bfloat16* Y, int m, int n, int N, bool vec_ok, const float (&v)[32]) {
+  if constexpr (SWIGLU) {
+    if (n >= N) return;  // (N is a multiple of 32)
+    uint32_t o[8];
+#pragma unroll
+    for (int e = 0; e < 16; e += 2) {
+      float r[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const float g = __bfloat162float(__float2bfloat16(v[e + h])), u = __bfloat162float(__float2bfloat16(v[16 + e + h]));
+        r[h] = g / (1.f + __expf(-g)) * u;
+      }
+      const __nv_bfloat162 p = __floats2bfloat162_rn(r[0], r[1]);
+      o[e / 2] = *reinterpret_cast<const uint32_t*>(&p);
+    }
+    uint4* y = reinterpret_cast<uint4*>(Y + (size_t)m * (N / 2) + n / 2);
+    y[0] = make_uint4(o[0], o[1], o[2], o[3]);
+    y[1] = make_uint4(o[4], o[5], o[6], o[7]);
+  } else {
+    __nv_bfloat16* y = Y + (size_t)m * N + n;
+    if (vec_ok && n + 32 <= N) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        uint32_t o[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const __nv_bfloat162 h = __floats2bfloat162_rn(v[8 * q + 2 * e], v[8 * q + 2 * e + 1]);
+          o[e] = *reinterpret_cast<const uint32_t*>(&h);
+        }
+        *reinterpret_cast<uint4*>(y + 8 * q) = make_uint4(o[0], o[1], o[2], o[3]);
+      }
+    } else {
+#pragma unroll
+      for (int e = 0; e < 32; ++e)
+        if (n + e < N) y[e] = __float2bfloat16(v[e]);
+    }
+  }
+}
+
+template <int MI, bool PAIR, bool SWIGLU>
 __global__ void __launch_bounds__(kGemmThreads, 1)
     w4_gemm_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
                    const GemmParams p) {
@@ -445,25 +491,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
           continue;
         }
         if (m < p.M) {
-          __nv_bfloat16* yrow = p.Y + (size_t)m * p.N + n0 + c0;
-          if (vec_ok && n0 + c0 + 32 <= p.N) {
+          float out[32];
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              uint4 o;
-              uint32_t* ow = reinterpret_cast<uint32_t*>(&o);
-#pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                const __nv_bfloat162 h = __floats2bfloat162_rn(__uint_as_float(v[8 * q + 2 * e]) * (1.f / kDequantUnit),
-                                                               __uint_as_float(v[8 * q + 2 * e + 1]) * (1.f / kDequantUnit));
-                ow[e] = *reinterpret_cast<const uint32_t*>(&h);
-              }
-              *reinterpret_cast<uint4*>(yrow + 8 * q) = o;
-            }
-          } else {
-#pragma unroll
-            for (int e = 0; e < 32; ++e)
-              if (n0 + c0 + e < p.N) yrow[e] = __float2bfloat16(__uint_as_float(v[e]) * (1.f / kDequantUnit));
-          }
+          for (int e = 0; e < 32; ++e) out[e] = __uint_as_float(v[e]) * (1.f / kDequantUnit);
+          store_outputs<SWIGLU>(p.Y, m, n0 + c0, p.N, vec_ok, out);
         }
       }
       if (parts) {
@@ -494,26 +525,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
             }
 #pragma unroll
             for (int e = 0; e < 32; ++e) sum[e] *= 1.f / kDequantUnit;
-            if (m < p.M) {
-              __nv_bfloat16* yrow = p.Y + (size_t)m * p.N + n0 + c0;
-              if (vec_ok && n0 + c0 + 32 <= p.N) {
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                  uint4 o;
-                  uint32_t* ow = reinterpret_cast<uint32_t*>(&o);
-#pragma unroll
-                  for (int e = 0; e < 4; ++e) {
-                    const __nv_bfloat162 h = __floats2bfloat162_rn(sum[8 * q + 2 * e], sum[8 * q + 2 * e + 1]);
-                    ow[e] = *reinterpret_cast<const uint32_t*>(&h);
-                  }
-                  *reinterpret_cast<uint4*>(yrow + 8 * q) = o;
-                }
-              } else {
-#pragma unroll
-                for (int e = 0; e < 32; ++e)
-                  if (n0 + c0 + e < p.N) yrow[e] = __float2bfloat16(sum[e]);
-              }
-            }
+            if (m < p.M) store_outputs<SWIGLU>(p.Y, m, n0 + c0, p.N, vec_ok, sum);
           }
         }
       }
@@ -540,9 +552,9 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
 }
 
 // ------------------------------------------------------------------ host side
-template <int MI, bool PAIR>
+template <int MI, bool PAIR, bool SWIGLU>
 int launch_gemm(const CUtensorMap& tx, const CUtensorMap& tw, const GemmParams& p, cudaStream_t stream) {
-  auto kernel = w4_gemm_kernel<MI, PAIR>;
+  auto kernel = w4_gemm_kernel<MI, PAIR, SWIGLU>;
   cudaError_t e =
       cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmGeo<MI, PAIR>::kSmemBytes);
   if (e != cudaSuccess) return (int)e;
@@ -632,7 +644,7 @@ int gemm_plan(int M, int N, int K, const Workspace& ws, int flags, int sm_count,
 }  // namespace
 
 int gemm_launch(const void* X, const void* Wq, const void* S, void* Y, int M, int N, int K, int G,
-                const Workspace& ws, int flags, int sm_count, cudaStream_t stream) {
+                const Workspace& ws, int flags, int sm_count, cudaStream_t stream, void* act) {
   static_assert(GemmGeo<2>::kSmemBytes <= kGemmSmemLimit && GemmGeo<1>::kSmemBytes <= kGemmSmemLimit &&
                     GemmGeo<2, true>::kSmemBytes <= kGemmSmemLimit,
                 "smem");
@@ -646,11 +658,13 @@ int gemm_launch(const void* X, const void* Wq, const void* S, void* Y, int M, in
 
   GemmPlan pl;
   if (const int rc = gemm_plan(M, N, K, ws, flags, sm_count, &pl)) return rc;
-  if (gemm_narrow_applies(S, M, N, K, G, flags, pl.us, std::max(1, sm_count)))
-    return gemm_narrow_launch(X, Wq, S, Y, M, N, K, G, ws, flags, std::max(1, sm_count), stream);
+  if (gemm_narrow_applies(S, M, N, K, G, flags, pl.us, std::max(1, sm_count))) {
+    const int rc = gemm_narrow_launch(X, Wq, S, Y, M, N, K, G, ws, flags, std::max(1, sm_count), stream);
+    return rc != 0 || act == nullptr ? rc : swiglu_blocks_launch(Y, act, M, N / 2, kPairBlock, stream);
+  }
   GemmParams p{};
   p.S = static_cast<const __nv_bfloat16*>(S);
-  p.Y = static_cast<__nv_bfloat16*>(Y);
+  p.Y = static_cast<__nv_bfloat16*>(act != nullptr ? act : Y);
   p.M = M; p.N = N; p.K = K; p.G = G;
   p.KG = K / G;
   p.nkb = pl.nkb;
@@ -669,8 +683,12 @@ int gemm_launch(const void* X, const void* Wq, const void* S, void* Y, int M, in
       !make_tensor_map_2d(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, Wq, (uint64_t)N, (uint64_t)K / 8, pl.pair ? kBN / 2 : kBN,
                  kBK / 8, CU_TENSOR_MAP_SWIZZLE_NONE))
     return kErrDevice;
-  if (pl.pair) return launch_gemm<2, true>(tx, tw, p, stream);
-  return pl.mi == 1 ? launch_gemm<1, false>(tx, tw, p, stream) : launch_gemm<2, false>(tx, tw, p, stream);
+  auto launch = [&](auto swiglu) {
+    constexpr bool kSwiglu = decltype(swiglu)::value;
+    if (pl.pair) return launch_gemm<2, true, kSwiglu>(tx, tw, p, stream);
+    return pl.mi == 1 ? launch_gemm<1, false, kSwiglu>(tx, tw, p, stream) : launch_gemm<2, false, kSwiglu>(tx, tw, p, stream);
+  };
+  return act != nullptr ? launch(std::true_type{}) : launch(std::false_type{});
 }
 
 int gemm_describe(int M, int N, int K, int G, const Workspace& ws, int flags, int sm_count, char* buf, int buflen) {

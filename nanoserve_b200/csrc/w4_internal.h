@@ -120,8 +120,10 @@ int gemv_launch_ex(const void* X, const void* Wq, const void* S, void* Y, int M,
 size_t gemv_grid(int M, int N, int K, int G, int flags, int sm_count, size_t partial_cap, int counters_cap);
 int gemv_launch(const void* X, const void* Wq, const void* S, void* Y, int M, int N, int K, int G,
                 const Workspace& ws, int flags, int sm_count, cudaStream_t stream);
+// act: null, or the [M, N / 2] output of SwiGLU over alternating blocks of 16 gate and 16 up rows (N % 32 == 0, 16-byte aligned);
+// Y is then room for the projection, which a kernel that applies it to its own sums does not use.
 int gemm_launch(const void* X, const void* Wq, const void* S, void* Y, int M, int N, int K, int G,
-                const Workspace& ws, int flags, int sm_count, cudaStream_t stream);
+                const Workspace& ws, int flags, int sm_count, cudaStream_t stream, void* act = nullptr);
 // Whether the few-token GEMM takes a call of at most 16 tokens from the GEMVs (gemm_launch then runs it).
 bool gemm_narrow_takes_decode(const void* X, const void* Wq, const void* S, const void* Y, int M, int N, int K, int G,
                               int flags, int sm_count);

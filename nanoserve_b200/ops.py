@@ -70,6 +70,7 @@ SIGNATURES = {
     "b2_w4_gemv_noalloc": ([_vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _vp], _i32),
     "b2_rope_kv_store": ([_vp, _vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _vp], _i32),
     "b2_qkv_prefill": ([_vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _vp], _i32),
+    "b2_w4_linear_swiglu": ([_vp] * 5 + [_i32] * 5 + [_vp], _i32),
     "b2_swiglu_blocks": ([_vp, _vp, _i32, _i32, _i32, _vp], _i32),
     "b2_decode_attention": ([_vp, _vp, _vp, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _vp], _i32),
     "b2_greedy_next": ([_vp, _i32, _vp, _i32, _vp, _vp, _vp, _vp, _vp, _vp], _i32),
@@ -306,6 +307,20 @@ class Kernels:
         out = torch.empty((T, I), dtype=gu.dtype, device=gu.device)
         self._check(self.lib.b2_swiglu_blocks(gu.data_ptr(), out.data_ptr(), T, I, block, self._stream()),
                     "b2_swiglu_blocks")
+        return out
+
+    def w4_linear_swiglu(self, x, Wq, S, group=128, flags=0):
+        """x [M, K], rows of Wq in alternating blocks of 16 gate and 16 up rows -> silu(gate) * up, [M, N / 2]: the bits of
+        `swiglu_blocks(w4_linear(x, Wq, S, group), 16)`."""
+        self._cuda(x, Wq, S)
+        assert x.is_contiguous() and x.dtype == torch.bfloat16 and Wq.is_contiguous() and S.is_contiguous()
+        M, K, N = x.shape[0], x.shape[1], Wq.shape[0]
+        assert Wq.shape[1] * 8 == K and tuple(S.shape) == (N, K // group)
+        tmp = torch.empty((M, N), dtype=x.dtype, device=x.device)
+        out = torch.empty((M, N // 2), dtype=x.dtype, device=x.device)
+        rc = self.lib.b2_w4_linear_swiglu(x.data_ptr(), Wq.data_ptr(), S.data_ptr(), tmp.data_ptr(), out.data_ptr(), M, N, K,
+                                          group, flags, self._stream())
+        self._check(rc, "b2_w4_linear_swiglu")
         return out
 
     def w4_linear_fused(self, x, Wq, S, group=128, prologue=0, r=None, wn=None, eps=0.0, x_out=None, flags=0,

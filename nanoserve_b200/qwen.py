@@ -230,8 +230,10 @@ class Qwen2Runner:
             a = F.scaled_dot_product_attention(qh, kh, vh, is_causal=True, enable_gqa=True)
             a = a[0].transpose(0, 1).reshape(T, self.nq).contiguous()
             h = k.rmsnorm(x, self._gather(self.linear(a, L["o"])), L["ln_post"], cfg.rms_eps)
-            gu = self.linear(h, L["gu"])
-            act = self._gather(k.swiglu_blocks(gu, self.gu_block))  # gate and up row blocks alternate (see __init__)
+            if self.gu_block == 16:  # gate and up row blocks alternate (see __init__)
+                act = self._gather(k.w4_linear_swiglu(h, L["gu"][0], L["gu"][1], cfg.group))
+            else:
+                act = self._gather(k.swiglu_blocks(self.linear(h, L["gu"]), self.gu_block))
             nxt = self.layers[li + 1]["ln_in"] if li + 1 < cfg.n_layers else self.final_norm
             h = k.rmsnorm(x, self._gather(self.linear(act, L["d"])), nxt, cfg.rms_eps)
         self.pos.fill_(T - 1)  # the pick advances it to T, the position of the first generated token

@@ -8,6 +8,8 @@ import pytest
 import torch
 import torch.nn.functional as F
 
+from nanoserve_b200.ops import FLAG_GEMM_NO_PAIRS, FLAG_GEMM_WIDE
+
 pytestmark = pytest.mark.gpu
 
 
@@ -263,3 +265,19 @@ def test_greedy_next(kernels):
                               step.data_ptr(), x.data_ptr(), ws.data_ptr(), st) == 0
     torch.cuda.synchronize()
     assert int(toks[2]) == 777 and int(pos) == 12 and int(step) == 3 and torch.equal(x, embed[777])
+
+
+# one CTA per tile and pairs of them, tiles cut along K with ragged tokens, the few-token kernel, a GEMV; a tile of rows less a block
+@pytest.mark.parametrize("M,N,K,flags", [(100, 512, 1024, FLAG_GEMM_WIDE), (300, 1504, 2048, FLAG_GEMM_WIDE),
+                                         (300, 736, 8192, FLAG_GEMM_WIDE | FLAG_GEMM_NO_PAIRS), (513, 32, 512, FLAG_GEMM_WIDE),
+                                         (700, 4096, 1024, 0), (48, 1024, 1024, 0), (5, 1024, 1024, 0)])
+def test_linear_swiglu_equals_its_parts(kernels, M, N, K, flags):
+    gen = torch.Generator(device="cuda").manual_seed(M)
+    x = torch.randn(M, K, device="cuda", generator=gen).to(torch.bfloat16)
+    Wq = torch.randint(-2**31, 2**31 - 1, (N, K // 8), dtype=torch.int32, device="cuda", generator=gen)
+    S = (0.005 + (torch.randn(N, K // 128, device="cuda", generator=gen) * 0.01).abs()).to(torch.bfloat16)
+    want = kernels.swiglu_blocks(kernels.w4_linear(x, Wq, S, flags=flags), 16)
+    assert torch.equal(kernels.w4_linear_swiglu(x, Wq, S, flags=flags), want)
+    with pytest.raises(RuntimeError, match="b2_w4_linear_swiglu failed with code -1"):
+        kernels.w4_linear_swiglu(x, Wq[:N - 16].contiguous(), S[:N - 16].contiguous(), flags=flags)
+    assert kernels.device_status() == 0
