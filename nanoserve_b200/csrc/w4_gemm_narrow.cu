@@ -47,7 +47,6 @@ constexpr int kHeaderBytes = 1024;    // barriers and flags
 constexpr int kSmemHalf = 115712;     // two CTAs per SM: (228 KB / 2) - 1 KB
 constexpr int kSmemFull = 232448;
 constexpr uint32_t kUnitBytes = 16 * 32 * 4;  // fp32 sums of 16 tokens x 32 rows
-constexpr int kMinSlots = 3;                  // slots of packed words that a CTA with work for them keeps
 constexpr int kAhead = 3;  // slots of packed words brought into L2 ahead of the wait for the kernel in front
 
 struct NarrowParams {
@@ -78,8 +77,9 @@ __device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, ui
 // MB: blocks of 128 weight rows per tile (each X tile is then read by MB MMAs).  DW: conversion warps, in DW / (4 MB)
 // groups that take the K blocks in turn; the converted weights of two K blocks fit in TMEM.  MINB: CTAs per SM.
 // MODE: 4 or 2: groups of 128 (a scale per row and step), read that many at a time; 64, 32: groups of 64 or 32 and whole
-// steps, a step's two or four scales per read; 0: any group, any K.
-template <int MB, int DW, int MINB, int MODE>
+// steps, a step's two or four scales per read; 0: any group, any K.  RED: the parts of a cut K are sent (p.red); a kernel of its
+// own, since its code made short launches of the others up to 6 % longer.
+template <int MB, int DW, int MINB, int MODE, bool RED>
 __global__ void __launch_bounds__(128 + DW * 32, MINB)
     w4_gemm_narrow_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
                           const NarrowParams p) {
@@ -105,10 +105,10 @@ __global__ void __launch_bounds__(128 + DW * 32, MINB)
   const int m0 = (tile % p.t_tiles) * p.nt, n0 = (tile / p.t_tiles) * kRows;
   const int kb0 = (int)((long)crank * p.nkb / p.ks), nkb = (int)((long)(crank + 1) * p.nkb / p.ks) - kb0;
 
-  // Units of 16 tokens x 32 rows, in the order (tokens, rows): the parts of a cut K are added by unit, and these are this CTA's.
+  // Units of 16 tokens x 32 rows, in the order (tokens, rows): the parts of a cut K are added by unit, and this CTA adds those from
+  // first_unit(crank) to first_unit(crank + 1).
   const int rt = min(p.nt, p.M - m0), units = (rt + 15) / 16 * (kRows / 32);
-  const int first_unit = (crank * units + p.ks - 1) / p.ks, n_units = ((crank + 1) * units + p.ks - 1) / p.ks - first_unit;
-  const uint32_t red = base + p.red;
+  auto first_unit = [&](int rank) { return (rank * units + p.ks - 1) / p.ks; };
 
   // (only brought into L2: the kernel in front may be the one that writes them)
   if (tid == 64)
@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(128 + DW * 32, MINB)
     }
     mbar_init(bar_acc, 1);
     mbar_init(bar_red, 1);
-    if (p.red) mbar_arrive_expect_tx(bar_red, (uint32_t)(n_units * p.ks) * kUnitBytes);
+    if constexpr (RED) mbar_arrive_expect_tx(bar_red, (uint32_t)((first_unit(crank + 1) - first_unit(crank)) * p.ks) * kUnitBytes);
     fence_mbar_init();
     tma_prefetch_desc(&tmap_w);
     tma_prefetch_desc(&tmap_x);
@@ -141,12 +141,16 @@ __global__ void __launch_bounds__(128 + DW * 32, MINB)
   __syncthreads();
   tc_fence_after_sync();
   pdl_launch_dependents();
-  if (p.red) cluster_arrive();  // (waited for before the first store into a peer: its barrier is set up)
+  if constexpr (RED) cluster_arrive();  // (waited for before the first store into a peer: its barrier is set up)
   const uint32_t tmem_d = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   const uint32_t tmem_a = tmem_d + ((MB * p.nt + 31) & ~31);
   const bool poisoned = *status_seen != 0;
   // Behind this the conversion warps leave tensor memory alone: the warp that allocated it frees it while they add up and store.
-  auto rows_done = [&] { asm volatile("bar.arrive 1, %0;" ::"n"(DW * 32 + 32) : "memory"); };
+  // (Where the parts are fetched it does so behind the cluster barrier: ahead of it all would wait.)
+  const bool fetched = !RED && p.ks > 1;
+  auto rows_done = [&] {
+    if (!fetched) asm volatile("bar.arrive 1, %0;" ::"n"(DW * 32 + 32) : "memory");
+  };
 
   if (!poisoned) {
     if (warp == 0) {
@@ -355,24 +359,24 @@ __global__ void __launch_bounds__(128 + DW * 32, MINB)
       tc_fence_after_sync();
 
       // ---- the accumulator columns (tokens) of the warp's 32 rows; two groups of warps take alternate 16 columns
-      if (p.red) cluster_wait();
+      if constexpr (RED) cluster_wait();
       for (int c0 = 16 * grp; c0 < rt; c0 += 16 * kGroups) {
         uint32_t v[16];
         tmem_ld_32x16(tmem_d + lane_off + mb * p.nt + c0, v);
         tmem_ld_wait();
-        if (p.ks == 1) {
-          __nv_bfloat16* y = p.Y + (size_t)(m0 + c0) * p.N + n;
-#pragma unroll
-          for (int e = 0; e < 16; ++e)
-            if (live && c0 + e < rt) y[(size_t)e * p.N] = __float2bfloat16(__uint_as_float(v[e]) * (1.f / kDequantUnit));
-        } else if (p.red) {
+        if constexpr (RED) {
           // a unit's parts go to the CTA that adds them, in the order of ranks: [unit][rank][four tokens][row]
           const int u = c0 / 16 * (kRows / 32) + (row >> 5), owner = u * p.ks / units;
-          const uint32_t at = red + (uint32_t)((u - (owner * units + p.ks - 1) / p.ks) * p.ks + crank) * kUnitBytes + lane * 16;
+          const uint32_t at = base + p.red + (uint32_t)((u - first_unit(owner)) * p.ks + crank) * kUnitBytes + lane * 16;
 #pragma unroll
           for (int q = 0; q < 4; ++q)
             st_async_f4(at + q * 512, bar_red, owner, __uint_as_float(v[4 * q]), __uint_as_float(v[4 * q + 1]),
                         __uint_as_float(v[4 * q + 2]), __uint_as_float(v[4 * q + 3]));
+        } else if (p.ks == 1) {
+          __nv_bfloat16* y = p.Y + (size_t)(m0 + c0) * p.N + n;
+#pragma unroll
+          for (int e = 0; e < 16; ++e)
+            if (live && c0 + e < rt) y[(size_t)e * p.N] = __float2bfloat16(__uint_as_float(v[e]) * (1.f / kDequantUnit));
         } else {  // [token][row], over the rings: every copy has landed and every MMA has read its operands
 #pragma unroll
           for (int e = 0; e < 16; ++e)
@@ -383,29 +387,32 @@ __global__ void __launch_bounds__(128 + DW * 32, MINB)
       tc_fence_before_sync();
       __syncwarp();
       rows_done();
-      if (p.red && dw < n_units) {
-        mbar_wait(bar_red, 0, abort_flag);
-        __syncwarp();
-        for (int b = dw; b < n_units; b += DW) {
-          const int u = first_unit + b, c0 = u / (kRows / 32) * 16, ny = n0 + u % (kRows / 32) * 32 + lane;
-          const uint32_t part = red + (uint32_t)(b * p.ks) * kUnitBytes + lane * 16;
-          __nv_bfloat16* y = p.Y + (size_t)(m0 + c0) * p.N + ny;
+      if constexpr (RED) {
+        const int u0 = first_unit(crank), n_units = first_unit(crank + 1) - u0;
+        if (dw < n_units) {
+          mbar_wait(bar_red, 0, abort_flag);
+          __syncwarp();
+          for (int b = dw; b < n_units; b += DW) {
+            const int u = u0 + b, c0 = u / (kRows / 32) * 16, ny = n0 + u % (kRows / 32) * 32 + lane;
+            const uint32_t part = base + p.red + (uint32_t)(b * p.ks) * kUnitBytes + lane * 16;
+            __nv_bfloat16* y = p.Y + (size_t)(m0 + c0) * p.N + ny;
 #pragma unroll 1
-          for (int q = 0; q < 4; ++q) {
-            float sum[4] = {0.f, 0.f, 0.f, 0.f};
+            for (int q = 0; q < 4; ++q) {
+              float sum[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-            for (int z = 0; z < 8; ++z)
-              if (z < p.ks) {
-                const uint4 f = lds128(part + z * kUnitBytes + q * 512);
-                sum[0] += __uint_as_float(f.x);
-                sum[1] += __uint_as_float(f.y);
-                sum[2] += __uint_as_float(f.z);
-                sum[3] += __uint_as_float(f.w);
-              }
+              for (int z = 0; z < 8; ++z)
+                if (z < p.ks) {
+                  const uint4 f = lds128(part + z * kUnitBytes + q * 512);
+                  sum[0] += __uint_as_float(f.x);
+                  sum[1] += __uint_as_float(f.y);
+                  sum[2] += __uint_as_float(f.z);
+                  sum[3] += __uint_as_float(f.w);
+                }
 #pragma unroll
-            for (int e = 0; e < 4; ++e)
-              if (ny < p.N && c0 + 4 * q + e < rt)
-                y[(size_t)(4 * q + e) * p.N] = __float2bfloat16(sum[e] * (1.f / kDequantUnit));
+              for (int e = 0; e < 4; ++e)
+                if (ny < p.N && c0 + 4 * q + e < rt)
+                  y[(size_t)(4 * q + e) * p.N] = __float2bfloat16(sum[e] * (1.f / kDequantUnit));
+            }
           }
         }
       }
@@ -415,18 +422,22 @@ __global__ void __launch_bounds__(128 + DW * 32, MINB)
   }
   __syncwarp();
   bool freed = false;
-  if (warp == 1) {
-    asm volatile("bar.sync 1, %0;" ::"n"(DW * 32 + 32) : "memory");
+  auto free_early = [&] {
     if (!poisoned && !__any_sync(0xffffffffu, *abort_flag != 0)) {  // (every product has been waited for)
       tc_fence_after_sync();
       tmem_dealloc(tmem_d, p.tmem_cols);
       freed = true;
     }
+  };
+  if (warp == 1 && !fetched) {
+    asm volatile("bar.sync 1, %0;" ::"n"(DW * 32 + 32) : "memory");
+    free_early();
   }
-  if (p.red) {
+  if constexpr (RED) {
     if (warp < 4 || poisoned) cluster_wait();
-  } else if (p.ks > 1) {
+  } else if (fetched) {
     cluster_barrier();
+    if (warp == 1) free_early();
     // every CTA adds up its share of the tile, four rows of a token per thread, in rank order
     if (warp >= 4 && !poisoned) {
       const int quads = rt * (kRows / 4);
@@ -459,8 +470,8 @@ __global__ void __launch_bounds__(128 + DW * 32, MINB)
     cluster_barrier();  // the peers have read this CTA's part
   }
   __syncthreads();
-  if (*abort_flag || (poisoned && p.red)) {
-    if (p.red) {  // peers that have not given up may send parts here until they leave
+  if (*abort_flag || (RED && poisoned)) {
+    if constexpr (RED) {  // peers that have not given up may send parts here until they leave
       cluster_arrive();
       cluster_wait();
     }
@@ -478,20 +489,23 @@ using NarrowKernel = void (*)(const CUtensorMap, const CUtensorMap, const Narrow
 struct NarrowForm {
   NarrowKernel kernel;
   int variant, rows, warps, per_sm, smem;
+  bool red;
 };
 // form 0: 128 weight rows, two CTAs per SM; form 1: 256 rows, one CTA.  All of an SM's (or half an SM's) shared memory
 // is asked for, needed or not: at most 512 columns' worth of CTAs then fit on an SM, whatever mix of these launches
 // overlaps, and no CTA of a cluster waits for tensor memory that a CTA at a cluster barrier holds.
 // variant: 0 any group, 1 and 2 groups of 128 by two and by four scales, 3 groups of 64, 4 groups of 32
-NarrowForm narrow_form(int form, int variant) {
-  static constexpr NarrowKernel kHalf[5] = {w4_gemm_narrow_kernel<1, 8, 2, 0>, w4_gemm_narrow_kernel<1, 8, 2, 2>,
-                                            w4_gemm_narrow_kernel<1, 8, 2, 4>, w4_gemm_narrow_kernel<1, 8, 2, 64>,
-                                            w4_gemm_narrow_kernel<1, 8, 2, 32>};
-  static constexpr NarrowKernel kFull[5] = {w4_gemm_narrow_kernel<2, 16, 1, 0>, w4_gemm_narrow_kernel<2, 16, 1, 2>,
-                                            w4_gemm_narrow_kernel<2, 16, 1, 4>, w4_gemm_narrow_kernel<2, 16, 1, 64>,
-                                            w4_gemm_narrow_kernel<2, 16, 1, 32>};
-  if (form == 0) return {kHalf[variant], variant, 128, 8, 2, kSmemHalf};
-  return {kFull[variant], variant, 256, 16, 1, kSmemFull};
+template <int MB, int DW, int MINB, bool RED>
+NarrowKernel narrow_kernel(int variant) {
+  static constexpr NarrowKernel kKernels[5] = {w4_gemm_narrow_kernel<MB, DW, MINB, 0, RED>, w4_gemm_narrow_kernel<MB, DW, MINB, 2, RED>,
+                                               w4_gemm_narrow_kernel<MB, DW, MINB, 4, RED>, w4_gemm_narrow_kernel<MB, DW, MINB, 64, RED>,
+                                               w4_gemm_narrow_kernel<MB, DW, MINB, 32, RED>};
+  return kKernels[variant];
+}
+NarrowForm narrow_form(int form, int variant, bool red) {
+  if (form == 0)
+    return {red ? narrow_kernel<1, 8, 2, true>(variant) : narrow_kernel<1, 8, 2, false>(variant), variant, 128, 8, 2, kSmemHalf, red};
+  return {red ? narrow_kernel<2, 16, 1, true>(variant) : narrow_kernel<2, 16, 1, false>(variant), variant, 256, 16, 1, kSmemFull, red};
 }
 int narrow_scales_per_load(const void* S, int K, int G) {
   const uintptr_t sa = reinterpret_cast<uintptr_t>(S);
@@ -507,10 +521,10 @@ int narrow_variant(const void* S, int K, int G) {
 }
 
 int narrow_attributes(const NarrowForm& f, int form, int dev) {
-  static std::atomic<bool> done[64][2][5];
-  if (dev >= 0 && dev < 64 && done[dev][form][f.variant].load(std::memory_order_acquire)) return 0;
+  static std::atomic<bool> done[64][2][5][2];
+  if (dev >= 0 && dev < 64 && done[dev][form][f.variant][f.red].load(std::memory_order_acquire)) return 0;
   const cudaError_t e = cudaFuncSetAttribute(f.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, f.smem);
-  if (e == cudaSuccess && dev >= 0 && dev < 64) done[dev][form][f.variant].store(true, std::memory_order_release);
+  if (e == cudaSuccess && dev >= 0 && dev < 64) done[dev][form][f.variant][f.red].store(true, std::memory_order_release);
   return (int)e;
 }
 
@@ -543,7 +557,7 @@ int narrow_clusters(int ks, int sm_count, int dev) {
   const bool cached = dev >= 0 && dev < 64;
   if (cached)
     if (const int v = known[dev][ks].load(std::memory_order_relaxed)) return v;
-  const NarrowForm f = narrow_form(1, 2);
+  const NarrowForm f = narrow_form(1, 2, false);
   int clusters = 0;
   cudaLaunchConfig_t cfg{};
   cudaLaunchAttribute attr[2];
@@ -678,20 +692,23 @@ int gemm_narrow_launch(const void* X, const void* Wq, const void* S, void* Y, in
   p.nt = pl.nt;
   p.ks = pl.ks;
   p.sv = narrow_scales_per_load(S, K, G);
-  const NarrowForm f = narrow_form(pl.form, narrow_variant(S, K, G));
+  const int variant = narrow_variant(S, K, G);
+  NarrowForm f = narrow_form(pl.form, variant, false);
   const int slot_w = f.rows * 128, slot_x = p.nt * 256, room = f.smem - kHeaderBytes - 1024;
   const int x_bytes = pl.form ? 128 << 10 : p.nt > 64 ? 72 << 10 : 48 << 10;  // the rest holds packed words
   const int blocks = (p.nkb + p.ks - 1) / p.ks;
   p.sx = std::max(2, std::min({6, x_bytes / slot_x, blocks}));
   p.sw = std::min(kMaxSlots, (room - p.sx * slot_x) / slot_w);
-  // Up to 64 token columns the parts of a cut K have a place of their own where the rings can spare it: every CTA then sends them
-  // as soon as it has them and leaves (3584 x 3584 at 48 tokens 8.1 -> 7.2 us).  More columns are fetched from the rings' place
+  // Up to 64 token columns the parts of a cut K have a place of their own where the rings can spare it without a slot that the CTA has
+  // work for (39 x 11469 x 9984 with three slots of four 28.7 us, so 25.0): every CTA then sends them as soon as it has them and
+  // leaves (3584 x 3584 at 48 tokens 8.1 -> 7.0 us).  More columns are fetched from the rings' place
   // behind a cluster barrier: sixteen bytes at a time, each counted, are slower from there (512 tokens 17.3 against 20.3).
   const int units = p.nt / 16 * (f.rows / 32), parts = (units + p.ks - 1) / p.ks * p.ks * (int)kUnitBytes;
   const int spare = (room - p.sx * slot_x - parts) / slot_w;
-  if (p.ks > 1 && p.nt <= 64 && spare >= std::min(kMinSlots, (blocks + 1) / 2)) {
+  if (p.ks > 1 && p.nt <= 64 && spare >= std::min(p.sw, (blocks + 1) / 2)) {
     p.sw = std::min(kMaxSlots, spare);
     p.red = kHeaderBytes + p.sw * slot_w + p.sx * slot_x;
+    f = narrow_form(pl.form, variant, true);
   }
   p.tmem_cols = pl.form ? 512 : 256;
   CUtensorMap tx, tw;

@@ -705,12 +705,12 @@ bool gemv_tc_shorter(const void* X, const void* Wq, const void* S, const void* Y
   TcPlan pl;
   if (!tc_plan(M, N, K, sm_count, 0, 0, &pl)) return false;
   if (M == 1) {
-    if (w <= 12.0) return K >= 1024 && (N <= 5776 ? pl.us <= 8.5 : pl.us <= 3.5);
+    if (w <= 12.0) return K >= 1024 && (N <= 4096 ? pl.us <= 8.5 : pl.us <= 3.5);
     return (K >= 9728 && K <= 16384 && N <= 4992) || (K >= 22016 && N >= 7424);
   }
   if (other == kTcOtherRing) return true;
   if (other == kTcOtherStream)
-    return M > 2       ? K >= 2304 || N <= 12000
+    return M > 2       ? K >= 2304 || N <= 8000
            : K >= 3840 ? N <= 128 * (sm_count - 1)  // (above, that kernel's CTAs of 128 rows leave no SM over)
                        : N <= (K <= 1536 ? 5800 : 11000);
   if (M <= 4) return 1.02 * pl.us < 6.65 + 0.11 * w + 0.027 * k3 + 0.074 * mk;

@@ -139,7 +139,8 @@ def test_a_plain_call_runs_the_kernel_it_is_described_as(kernels, M, N, K):
     (512, 3584, True),      # 4.5, 3.4
     (130, 1024, True),      # 3.5, 2.7
     (130, 768, False),
-    (5776, 2048, True),     # 4.5, 4.4
+    (4096, 2048, True),     # 4.4, 4.1
+    (4997, 1536, False),    # 4.2, 4.8
     (4980, 14080, True),    # 15.0, 12.8
     (8192, 28672, True),    # 29.2, 26.6
     (3584, 3584, False),    # 5.0, 5.1
