@@ -240,7 +240,7 @@ __global__ void decode_attention_merge_kernel(const float* part, bf16* out) {
 // b2_rope_kv_store stores it).  The CTA whose slice holds the new position computes the new k and v rows, stores them
 // to the cache and serves them to its own tile loop from shared memory.  The last CTA of a KV head to have written
 // its partials (an arrival counter per KV head; nobody waits) merges the splits of that head's query heads.
-// Launches per layer of a decode step: 5 instead of 7.
+// (Tensor-parallel calls and the form with a counter; the others run decode_attention_cluster_kernel below.)
 template <int D>
 __global__ void __launch_bounds__(256) decode_attention_fused_kernel(
     const bf16* qkv, const bf16* __restrict__ bias, const float* __restrict__ inv_freq, const int* pos_ptr,
@@ -895,18 +895,11 @@ int decode_attention_fused_launch(const void* qkv, const void* bias, const void*
   int* counters = one_launch ? reinterpret_cast<int*>(part + (size_t)Hq * kSplits * (D + 2)) : nullptr;
   const dim3 grid(Hk, kSplits);
   if (!one_launch && tp == nullptr) {
-    auto cluster = [&](auto kernel, int smem, std::atomic<bool>* done) {
-      int dev = -1;
-      cudaError_t e = cudaGetDevice(&dev);
-      if (e != cudaSuccess) return e;
-      const bool cached = dev >= 0 && dev < 64;
-      if (!cached || !done[dev].load(std::memory_order_acquire)) {
-        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess) return e;
-        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-        if (e != cudaSuccess) return e;
-        if (cached) done[dev].store(true, std::memory_order_release);
-      }
+    // (A device that cannot hold a cluster of sixteen, a slice of one for instance, keeps the two launches: asked once.)
+    static std::atomic<int> fits_on[2][64];  // 1: yes, 2: no
+    int dev = -1;
+    if (const cudaError_t e = cudaGetDevice(&dev); e != cudaSuccess) return (int)e;
+    auto cluster = [&](auto kernel, int smem, bool* fits) {
       cudaLaunchConfig_t cfg{};
       cfg.gridDim = dim3(Hk * kAttnCtas);
       cfg.blockDim = dim3(Hq / Hk * kSlicesPerCta * 32);
@@ -919,16 +912,35 @@ int decode_attention_fused_launch(const void* qkv, const void* bias, const void*
       attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
       attr[1].val.programmaticStreamSerializationAllowed = 1;
       cfg.attrs = attr;
+      const bool cached = dev >= 0 && dev < 64;
+      int known = cached ? fits_on[D == 128][dev].load(std::memory_order_acquire) : 0;
+      if (known == 0) {
+        int clusters = 0;
+        cfg.numAttrs = 1;
+        cfg.gridDim = dim3(kAttnCtas);
+        cfg.blockDim = dim3(8 * kSlicesPerCta * 32);  // the most heads that share a KV head
+        known = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess &&
+                        cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                        cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess && clusters > 0
+                    ? 1
+                    : 2;
+        if (known == 2) (void)cudaGetLastError();
+        if (cached) fits_on[D == 128][dev].store(known, std::memory_order_release);
+        cfg.gridDim = dim3(Hk * kAttnCtas);
+        cfg.blockDim = dim3(Hq / Hk * kSlicesPerCta * 32);
+      }
+      *fits = known == 1;
+      if (!*fits) return cudaSuccess;
       cfg.numAttrs = 2;
       return cudaLaunchKernelEx(&cfg, kernel, static_cast<const bf16*>(qkv), static_cast<const bf16*>(bias),
                                 static_cast<const float*>(inv_freq), static_cast<const int*>(pos),
                                 static_cast<bf16*>(cache_k), static_cast<bf16*>(cache_v), static_cast<bf16*>(out), Hq, Hk,
                                 max_len, scale, (flags & 2) ? 1 : 0, device_status_word_if_ready());
     };
-    static std::atomic<bool> done[2][64];
-    const cudaError_t e = D == 128 ? cluster(decode_attention_cluster_kernel<128>, AttnSmem<128>::kBytes, done[0])
-                                   : cluster(decode_attention_cluster_kernel<64>, AttnSmem<64>::kBytes, done[1]);
-    return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
+    bool fits = false;
+    const cudaError_t e = D == 128 ? cluster(decode_attention_cluster_kernel<128>, AttnSmem<128>::kBytes, &fits)
+                                   : cluster(decode_attention_cluster_kernel<64>, AttnSmem<64>::kBytes, &fits);
+    if (e != cudaSuccess || fits) return e != cudaSuccess ? (int)e : (int)cudaGetLastError();
   }
   auto go = [&](auto kernel) {
     return launch_pdl(kernel, grid, dim3(256), stream, static_cast<const bf16*>(qkv),

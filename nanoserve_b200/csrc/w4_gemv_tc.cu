@@ -20,9 +20,8 @@
 // neither uses tensor memory), first words and X 0.7 later, first products 0.5, the exchange of parts 0.9.
 // The chain of a group is what the order in the loop is for: half of a pair's words are converted while the products of the group's last
 // pair run, and the sums of that one are added while this pair's do (2530 -> 2300 cycles per pair of a group; 8192 x 28672 at
-// eight tokens 30.7 -> 28.6 us).  The status word is asked for at the start and answered behind the set-up, the parts of a cut K go
-// to the CTA that adds them with a barrier of their own instead of the cluster's (4608 x 3584 6.65 -> 5.8 us), tensor memory
-// is freed beside the last sums.  Measured, weights from HBM, us at 4 / 8 / 13 tokens, in brackets before that: 37888 x
+// eight tokens 30.7 -> 28.6 us).  The parts of a cut K go to the CTA that adds them with a barrier of their own instead of the
+// cluster's (4608 x 3584 6.65 -> 5.8 us), tensor memory is freed beside the last sums.  Measured, weights from HBM, us at 4 / 8 / 13 tokens, in brackets before that: 37888 x
 // 3584 15.2 / 15.4 / 16.9 (15.4 / 16.1 / 17.8), 3584 x 18944 12.4 / 12.6 / 14.7 (13.2 / 13.5 / 15.2), 4608 x 3584 at 4 and 13 5.8 and
 // 6.8 (6.65 and 7.2), 57344 x 8192 at 8 57.9 (61.0).
 // Every wait is bounded; a CTA that gives up records a status, still takes part in the cluster barriers and frees its TMEM.
@@ -122,10 +121,9 @@ __global__ void __launch_bounds__(MB == 2 ? 896 : 512, MB == 2 ? 1 : 2)
   const uint32_t bar_x_empty = bar_a_empty + 8 * 4;                                   // [slot], at most 16
   const uint32_t bar_x_full = base + kSlotBars;                                       // [pair]
   const uint32_t bar_red = base + 16;                                                 // the parts of a cut K
+  const uint32_t bar_done = base + 24;                                                // tensor memory has been read
   const uint32_t ring_w = base + p.off_w, ring_x = base + p.off_x, info = base + p.off_info, red = base + p.off_red;
 
-  // (Read by every warp for itself, and answered behind the set-up: another CTA may set it in between.)
-  const int status_seen = *reinterpret_cast<volatile int*>(p.status);
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   const int crank = p.ks > 1 ? (int)cluster_rank() : 0;
   const int n0 = (blockIdx.x / p.ks) * kRows;
@@ -139,6 +137,7 @@ __global__ void __launch_bounds__(MB == 2 ? 896 : 512, MB == 2 ? 1 : 2)
   if (tid < 40) mbar_init(base + kBarOffset + 8 * tid, tid < 8 ? 1 : tid < 20 ? 4 : tid < 24 ? 1 : MB);
   if (tid == 0) {
     *abort_flag = 0;
+    mbar_init(bar_done, kMain);
     if (p.ks > 1) {
       mbar_init(bar_red, 1);
       mbar_arrive_expect_tx(bar_red, (uint32_t)(blks * p.ks * 2 * groups) * 512);
@@ -156,7 +155,9 @@ __global__ void __launch_bounds__(MB == 2 ? 896 : 512, MB == 2 ? 1 : 2)
   pdl_launch_dependents();
   if (p.ks > 1) cluster_arrive();  // (waited for before the first store into a peer: it runs by then, its barrier is set up)
   const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);  // [block][group]: 64 columns of sums, 64 of bytes
-  const bool poisoned = __any_sync(0xffffffffu, status_seen != 0);
+  // (Read by every warp for itself: another CTA may set it in between, so the named barrier below is met either way.  Asked for ahead
+  // of the __syncthreads it cost four layers at 4 tokens 155.4 us for 153.6 and at 13 187.3 for 182.4, since all then wait for it.)
+  const bool poisoned = __any_sync(0xffffffffu, *reinterpret_cast<volatile int*>(p.status) != 0);
   // The rows' warps need more registers than an even share.  256 rows, 896 threads of 72: 4 x 88 + 2 x 48 + 56 = 7 x 72 by
   // warpgroup; 128 rows, 512 of 64: 2 x 80 + 2 x 48 = 4 x 64.
   if (warp < kMain) regs_up<MB == 2 ? 88 : 80>();
@@ -164,7 +165,7 @@ __global__ void __launch_bounds__(MB == 2 ? 896 : 512, MB == 2 ? 1 : 2)
   else regs_down<MB == 2 ? 56 : 48>();
   // Behind this the rows' warps leave tensor memory alone: the warp that allocated it frees it while they add up and store.
   // (A kernel that frees it last ends 0.14 us later.)
-  auto rows_done = [&] { asm volatile("bar.arrive 3, %0;" ::"n"(kMain * 32 + 32) : "memory"); };
+  auto rows_done = [&] { mbar_arrive_if(bar_done, lane == 0); };
   if (!poisoned) {
     if (warp < kMain) {
       // ---- the rows: words -> bytes in TMEM; sums of a step -> registers.  Two groups of warps take the pairs in turn.
@@ -504,17 +505,14 @@ __global__ void __launch_bounds__(MB == 2 ? 896 : 512, MB == 2 ? 1 : 2)
         if (++xs == p.sx) xs = 0;
       }
     }
-  } else {  // the CTA's other warps may have read zero: their waits end, and these barriers, which have no limit, are met
-    if (lane == 0) *abort_flag = 1;
-    if (warp < kMain) {
-      rows_done();
-      if (p.ks == 1) asm volatile("bar.sync %0, 256;" ::"r"(1 + (warp >> 2) % MB) : "memory");
-    }
+  } else if (p.ks == 1 && warp < kMain) {  // the block's other warps may be there, and this barrier has no limit
+    asm volatile("bar.sync %0, 256;" ::"r"(1 + (warp >> 2) % MB) : "memory");
   }
   __syncwarp();
+  if (poisoned && lane == 0) *abort_flag = 1;  // the CTA's other warps may have read zero: their waits end
   bool freed = false;
-  if (warp == kWarpMma) {
-    asm volatile("bar.sync 3, %0;" ::"n"(kMain * 32 + 32) : "memory");
+  if (warp == kWarpMma && !poisoned) {
+    mbar_wait(bar_done, 0, abort_flag);
     if (!__any_sync(0xffffffffu, *abort_flag != 0)) {  // (every product has been waited for)
       tc_fence_after_sync();
       tmem_dealloc(tmem, kTmemCols);
