@@ -207,7 +207,9 @@ int b2_w4_gemv_noalloc(const void* X, const void* Wq, const void* S, void* Y, in
  *     the merge's two L2 round trips behind the slowest CTA.  flags 2 (may be added to either): the caller promises that the kernel launched
  *     in front of this one on the stream writes neither *pos nor cached rows below *pos (true for a decode step, where
  *     that kernel is the q|k|v projection); the first tile of cached rows is then requested before that kernel has
- *     completed.  Results are bit-identical to the two calls above in every form.
+ *     completed.  The appended rows are those of b2_rope_kv_store to the bit in every form, the outputs the same with flags 0
+ *     and 2; the two calls above round a query's rotation, and flags 1 adds the denominators up, in another order (one output
+ *     in 10^4 to 10^5 by one bf16 step).
  *     workspace: b2_decode_attention_fused_workspace_bytes(Hq, Hk, D) bytes, ZEROED once by the caller (the counters
  *     at its end return to zero after every launch).  tp: NULL, or the consumer side (wait_sig, epoch,
  *     wait_per_epoch, announce_peer) of the tensor-parallel GEMV that produced qkv (see b2_tp_desc).

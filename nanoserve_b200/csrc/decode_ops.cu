@@ -49,6 +49,17 @@ __device__ __forceinline__ void ld_row(const bf16* p, float (&f)[E]) {
     f[1] = __uint_as_float(v & 0xFFFF0000u);
   }
 }
+// The rotation of the pair (a, b) of a key, and of the element x of a query whose partner D/2 away is `other`.  Which product is
+// rounded before the addition is written out: left to the compiler it differed between kernels, and one in 2 * 10^5 of the
+// appended key elements with it (one in 250 where the products cancel).
+__device__ __forceinline__ void rotate_pair(float& a, float& b, float sn, float cs) {
+  const float ra = __fmaf_rn(a, cs, -__fmul_rn(b, sn)), rb = __fmaf_rn(b, cs, __fmul_rn(a, sn));
+  a = ra;
+  b = rb;
+}
+__device__ __forceinline__ float rotate_query(float x, float other, float sn, float cs, bool first_half) {
+  return first_half ? __fmaf_rn(x, cs, -__fmul_rn(other, sn)) : __fmaf_rn(other, sn, __fmul_rn(x, cs));
+}
 template <typename... Args>
 cudaError_t launch_pdl(void (*kernel)(Args...), dim3 grid, dim3 block, cudaStream_t stream, Args... args) {
   cudaLaunchConfig_t cfg{};
@@ -102,9 +113,7 @@ __global__ void rope_kv_store_kernel(bf16* qkv, const bf16* __restrict__ bias,
   if (h < Hq + Hk) {  // q and k heads rotate, v heads do not
     float sn, cs;
     sincosf((float)pos * inv_freq[i], &sn, &cs);
-    const float ra = a * cs - b * sn, rb = b * cs + a * sn;
-    a = ra;
-    b = rb;
+    rotate_pair(a, b, sn, cs);
   }
   const bf16 oa = __float2bfloat16(a), ob = __float2bfloat16(b);
   x[i] = oa;
@@ -331,9 +340,7 @@ __global__ void __launch_bounds__(256) decode_attention_fused_kernel(
     if (!is_v) {
       float sn, cs;
       sincosf((float)pos * inv_freq[i], &sn, &cs);
-      const float ra = a * cs - b * sn, rb = b * cs + a * sn;
-      a = ra;
-      b = rb;
+      rotate_pair(a, b, sn, cs);
     }
     const bf16 oa = __float2bfloat16(a), ob = __float2bfloat16(b);
     bf16* sm = is_v ? s_newv : s_newk;
@@ -359,8 +366,7 @@ __global__ void __launch_bounds__(256) decode_attention_fused_kernel(
       const float other = __shfl_xor_sync(0xffffffffu, qf[e], 16);  // the element D/2 away
       float sn, cs;
       sincosf((float)pos * inv_freq[(lane * E + e) % half], &sn, &cs);
-      const float r = lane < 16 ? qf[e] * cs - other * sn : qf[e] * cs + other * sn;
-      qf[e] = __bfloat162float(__float2bfloat16(r)) * scale;
+      qf[e] = __bfloat162float(__float2bfloat16(rotate_query(qf[e], other, sn, cs, lane < 16))) * scale;
     }
   }
 
@@ -460,7 +466,7 @@ __global__ void __launch_bounds__(256) decode_attention_fused_kernel(
 // The same in one launch without a last CTA to wait for: the sixteen CTAs of a KV head are a cluster and send their partials to
 // the CTA that merges them (st.async, counted on a barrier of that CTA; CTA r merges dimensions [r D/16, (r + 1) D/16) of every
 // head).  A CTA holds two of the 32 slices, a warp one (query head, slice); every sum is taken over the same values in the same
-// order as in the two kernels above, so the results are theirs to the bit.
+// order as in the pass and the merge launch of the two-launch form, so the results are that form's to the bit.
 // What bounds it is latency: 0.6 us until the kernel in front is seen complete, 0.6 for q's load and the rotation, 2 for the rows of a
 // slice, one way through the cluster 0.5, the merge 0.5.  A layer's attention at 560 positions, alone in a chain: 8.6 us in two
 // launches, 5.6 in this one; a decode step of 28 layers 1.567 -> 1.490 ms.  On the way: eight CTAs of 28 warps found no place beside a
@@ -587,10 +593,7 @@ __global__ void __launch_bounds__(512, 2) decode_attention_cluster_kernel(
       b = __bfloat162float(__float2bfloat16(b + __bfloat162float(bias[(size_t)hh * D + i + half])));
     }
     if (!is_v) {
-      const float sn = s_rot[i].x, cs = s_rot[i].y;
-      const float ra = a * cs - b * sn, rb = b * cs + a * sn;
-      a = ra;
-      b = rb;
+      rotate_pair(a, b, s_rot[i].x, s_rot[i].y);
     }
     const bf16 oa = __float2bfloat16(a), ob = __float2bfloat16(b);
     bf16* row = is_v ? s_newv : s_newk;
@@ -609,9 +612,7 @@ __global__ void __launch_bounds__(512, 2) decode_attention_cluster_kernel(
   for (int e = 0; e < E; ++e) {
     const float other = __shfl_xor_sync(0xffffffffu, qf[e], 16);  // the element D/2 away
     const float2 rot = s_rot[(lane * E + e) % half];
-    const float sn = rot.x, cs = rot.y;
-    const float r = lane < 16 ? qf[e] * cs - other * sn : qf[e] * cs + other * sn;
-    qf[e] = __bfloat162float(__float2bfloat16(r)) * scale;
+    qf[e] = __bfloat162float(__float2bfloat16(rotate_query(qf[e], other, rot.x, rot.y, lane < 16))) * scale;
   }
 
   float m = -FLT_MAX, l = 0.f, acc[E];

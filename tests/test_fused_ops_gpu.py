@@ -254,6 +254,33 @@ def test_fused_attention_in_several_passes(kernels, Hq, Hk, D, L, pos):
     test_fused_attention_equals_the_two_calls(kernels, Hq, Hk, D, L, pos)
 
 
+@pytest.mark.parametrize("Hq,Hk,D,flags", [(28, 7, 128, 0), (28, 7, 128, 1), (28, 7, 128, 2), (16, 2, 64, 0), (16, 2, 64, 1)])
+def test_fused_attention_appends_the_rows_of_rope_kv_store(kernels, Hq, Hk, D, flags):
+    """Key pairs (a, b) whose products cancel in the rotation: which of them is rounded first then shows in one of some 250
+    elements, where it shows in one of 2 * 10^5 of ordinary ones."""
+    lib, L, half = kernels.lib, 1100, D // 2
+    g = torch.Generator(device="cuda").manual_seed(D)
+    st = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    inv = 1.0 / (1e6 ** (torch.arange(0, D, 2, device="cuda").float() / D))
+    ck = torch.zeros(2, Hk, L, D, dtype=torch.bfloat16, device="cuda")
+    cv = torch.zeros_like(ck)
+    out = torch.empty(Hq * D, dtype=torch.bfloat16, device="cuda")
+    ws = torch.zeros(int(lib.b2_decode_attention_fused_workspace_bytes(Hq, Hk, D)), dtype=torch.uint8, device="cuda")
+    for pos in range(1, L, 5):
+        p = torch.tensor([pos], dtype=torch.int32, device="cuda")
+        sn, cs = (pos * inv).double().sin(), (pos * inv).double().cos()
+        qkv = torch.randn(Hq + 2 * Hk, D, device="cuda", generator=g).to(torch.bfloat16)
+        a = qkv[Hq:Hq + Hk, :half].double()
+        first = torch.rand(Hk, half, device="cuda", generator=g) < 0.5  # a cos - b sin vanishes, or b cos + a sin
+        qkv[Hq:Hq + Hk, half:] = torch.where(first, a * cs / sn, -a * sn / cs).clamp(-1e4, 1e4).to(torch.bfloat16)
+        assert lib.b2_decode_attention_fused(qkv.data_ptr(), None, inv.data_ptr(), p.data_ptr(), ck[0].data_ptr(),
+                                             cv[0].data_ptr(), out.data_ptr(), ws.data_ptr(), Hq, Hk, D, L, None, flags, st) == 0
+        assert lib.b2_rope_kv_store(qkv.data_ptr(), None, inv.data_ptr(), p.data_ptr(), ck[1].data_ptr(), cv[1].data_ptr(),
+                                    Hq, Hk, D, L, st) == 0
+    assert torch.equal(ck[0], ck[1]) and torch.equal(cv[0], cv[1]) and bool(ck[0].any())
+    assert kernels.device_status() == 0
+
+
 def test_greedy_next(kernels):
     lib = kernels.lib
     V, H = 152064, 64
