@@ -201,14 +201,16 @@ int b2_w4_gemv_noalloc(const void* X, const void* Wq, const void* S, void* Y, in
  *   b2_decode_attention_fused: both of the above with the RoPE / KV-store launch folded into the attention pass.
  *     qkv is read, not modified: every CTA rotates the query heads it serves in registers; the CTA whose key slice
  *     holds position *pos builds the new k and v rows, stores them to the caches and uses them from shared memory.
- *     flags 0: without tp ONE launch, a cluster of sixteen CTAs per KV head that exchange the key slices' results (the
- *     fastest form); with tp the merge of the key slices is a second launch.  flags 1: one launch in which the last CTA of a
+ *     flags 0: without tp, and where the device holds a cluster of sixteen CTAs per KV head at once (up to seven KV heads on a
+ *     B200), ONE launch, in which the CTAs exchange the key slices' results (28 query and 4 KV heads of 128 at 512 positions, in a
+ *     chain: 5.8 us a layer, in two launches 8.2); else the merge of the key slices is a second launch.  flags 4 (may be
+ *     added): two launches wherever flags 0 would take one.  flags 1: one launch in which the last CTA of a
  *     KV head to finish merges the slices (an arrival counter per KV head; nobody waits), which puts a fence, an atomic and
- *     the merge's two L2 round trips behind the slowest CTA.  flags 2 (may be added to either): the caller promises that the kernel launched
+ *     the merge's two L2 round trips behind the slowest CTA.  flags 2 (may be added to any): the caller promises that the kernel launched
  *     in front of this one on the stream writes neither *pos nor cached rows below *pos (true for a decode step, where
  *     that kernel is the q|k|v projection); the first tile of cached rows is then requested before that kernel has
- *     completed.  The appended rows are those of b2_rope_kv_store to the bit in every form, the outputs the same with flags 0
- *     and 2; the two calls above round a query's rotation, and flags 1 adds the denominators up, in another order (one output
+ *     completed.  The appended rows are those of b2_rope_kv_store to the bit in every form, the outputs the same with flags 0,
+ *     2, 4 and 6; the two calls above round a query's rotation, and flags 1 adds the denominators up, in another order (one output
  *     in 10^4 to 10^5 by one bf16 step).
  *     workspace: b2_decode_attention_fused_workspace_bytes(Hq, Hk, D) bytes, ZEROED once by the caller (the counters
  *     at its end return to zero after every launch).  tp: NULL, or the consumer side (wait_sig, epoch,

@@ -895,15 +895,17 @@ int decode_attention_fused_launch(const void* qkv, const void* bias, const void*
   const bool one_launch = (flags & 1) != 0;
   int* counters = one_launch ? reinterpret_cast<int*>(part + (size_t)Hq * kSplits * (D + 2)) : nullptr;
   const dim3 grid(Hk, kSplits);
-  if (!one_launch && tp == nullptr) {
-    // (A device that cannot hold a cluster of sixteen, a slice of one for instance, keeps the two launches: asked once.)
-    static std::atomic<int> fits_on[2][64];  // 1: yes, 2: no
+  // The cluster form where all of the call's clusters run at once: a CTA takes an SM, so that a second wave costs as much as the
+  // first, where the two launches keep several small CTAs to an SM.  The line is the device's count of clusters of sixteen (seven on
+  // a B200; none on a slice of one).  us per layer in a chain, this form and in brackets the two launches, 512 / 4096 positions, heads of
+  // 128: 28 query and 4 KV heads 5.8 / 21.6 (8.2 / 34.9), 28 and 7 5.8 / 19.0 (7.4 / 24.8), 32 and 8, with two waves, 10.1 / 36.4 (7.2 /
+  // 23.5), 64 and 8 12.3 / 44.3 (10.1 / 40.1), 32 and 32 27.7 / 108 (11.9 / 41.0).
+  if (!one_launch && tp == nullptr && (flags & 4) == 0) {
+    static std::atomic<int> clusters_on[2][64];  // one more than their number: asked once
     int dev = -1;
     if (const cudaError_t e = cudaGetDevice(&dev); e != cudaSuccess) return (int)e;
     auto cluster = [&](auto kernel, int smem, bool* fits) {
       cudaLaunchConfig_t cfg{};
-      cfg.gridDim = dim3(Hk * kAttnCtas);
-      cfg.blockDim = dim3(Hq / Hk * kSlicesPerCta * 32);
       cfg.dynamicSmemBytes = smem;
       cfg.stream = stream;
       cudaLaunchAttribute attr[2];
@@ -914,24 +916,23 @@ int decode_attention_fused_launch(const void* qkv, const void* bias, const void*
       attr[1].val.programmaticStreamSerializationAllowed = 1;
       cfg.attrs = attr;
       const bool cached = dev >= 0 && dev < 64;
-      int known = cached ? fits_on[D == 128][dev].load(std::memory_order_acquire) : 0;
+      int known = cached ? clusters_on[D == 128][dev].load(std::memory_order_acquire) : 0;
       if (known == 0) {
         int clusters = 0;
         cfg.numAttrs = 1;
         cfg.gridDim = dim3(kAttnCtas);
         cfg.blockDim = dim3(8 * kSlicesPerCta * 32);  // the most heads that share a KV head
-        known = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess &&
-                        cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-                        cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess && clusters > 0
-                    ? 1
-                    : 2;
-        if (known == 2) (void)cudaGetLastError();
-        if (cached) fits_on[D == 128][dev].store(known, std::memory_order_release);
-        cfg.gridDim = dim3(Hk * kAttnCtas);
-        cfg.blockDim = dim3(Hq / Hk * kSlicesPerCta * 32);
+        const bool asked = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) == cudaSuccess &&
+                           cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                           cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess;
+        if (!asked) (void)cudaGetLastError();
+        known = asked ? clusters + 1 : 1;
+        if (cached) clusters_on[D == 128][dev].store(known, std::memory_order_release);
       }
-      *fits = known == 1;
+      *fits = Hk < known;
       if (!*fits) return cudaSuccess;
+      cfg.gridDim = dim3(Hk * kAttnCtas);
+      cfg.blockDim = dim3(Hq / Hk * kSlicesPerCta * 32);
       cfg.numAttrs = 2;
       return cudaLaunchKernelEx(&cfg, kernel, static_cast<const bf16*>(qkv), static_cast<const bf16*>(bias),
                                 static_cast<const float*>(inv_freq), static_cast<const int*>(pos),

@@ -233,7 +233,7 @@ def test_fused_attention_equals_the_two_calls(kernels, Hq, Hk, D, L, pos):
     # the fused form, twice
     ws = torch.zeros(int(lib.b2_decode_attention_fused_workspace_bytes(Hq, Hk, D)), dtype=torch.uint8, device="cuda")
     keep = qkv.clone()
-    for flags in (1, 1, 0, 2, 3):
+    for flags in (1, 1, 0, 2, 3, 4, 6):
         ck1, cv1 = ck.clone(), cv.clone()
         out = torch.full((Hq * D,), 7.0, dtype=torch.bfloat16, device="cuda")
         assert lib.b2_decode_attention_fused(qkv.data_ptr(), bias.data_ptr(), inv.data_ptr(), p.data_ptr(),
@@ -278,6 +278,33 @@ def test_fused_attention_appends_the_rows_of_rope_kv_store(kernels, Hq, Hk, D, f
         assert lib.b2_rope_kv_store(qkv.data_ptr(), None, inv.data_ptr(), p.data_ptr(), ck[1].data_ptr(), cv[1].data_ptr(),
                                     Hq, Hk, D, L, st) == 0
     assert torch.equal(ck[0], ck[1]) and torch.equal(cv[0], cv[1]) and bool(ck[0].any())
+    assert kernels.device_status() == 0
+
+
+@pytest.mark.parametrize("Hq,Hk,D,one", [(28, 4, 128, True), (7, 1, 64, True), (64, 32, 128, False), (40, 40, 64, False),
+                                         (32, 8, 128, None), (28, 7, 128, None)])
+def test_attention_in_one_launch_equals_two(kernels, Hq, Hk, D, one):
+    """The form that plain flags take against the two launches, to the bit, over a thousand positions; it is the one in clusters,
+    which leaves the workspace alone, only where all its clusters run at once (32 clusters of sixteen never do)."""
+    lib, L = kernels.lib, 1000
+    g = torch.Generator(device="cuda").manual_seed(Hq)
+    st = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    rand = lambda *shape: torch.randn(*shape, device="cuda", generator=g).to(torch.bfloat16)
+    inv = 1.0 / (1e6 ** (torch.arange(0, D, 2, device="cuda").float() / D))
+    caches = rand(2, Hk, L, D)[None].repeat(2, 1, 1, 1, 1)
+    bias, outs = 0.1 * rand((Hq + 2 * Hk) * D), torch.empty(2, Hq * D, dtype=torch.bfloat16, device="cuda")
+    ws = torch.zeros(int(lib.b2_decode_attention_fused_workspace_bytes(Hq, Hk, D)), dtype=torch.uint8, device="cuda")
+    for pos in range(0, L, 7):
+        p, qkv = torch.tensor([pos], dtype=torch.int32, device="cuda"), rand((Hq + 2 * Hk) * D)
+        for i, flags in enumerate((2 * (pos & 1), 4 + 2 * (pos & 1))):
+            ws[:-4 * Hk] = 0xA5
+            assert lib.b2_decode_attention_fused(qkv.data_ptr(), bias.data_ptr(), inv.data_ptr(), p.data_ptr(),
+                                                 caches[i, 0].data_ptr(), caches[i, 1].data_ptr(), outs[i].data_ptr(),
+                                                 ws.data_ptr(), Hq, Hk, D, L, None, flags, st) == 0
+            untouched = bool((ws[:-4 * Hk] == 0xA5).all())
+            assert untouched == (one if i == 0 and one is not None else untouched and i == 0)
+        assert torch.equal(outs[0], outs[1])
+    assert torch.equal(caches[0], caches[1])
     assert kernels.device_status() == 0
 
 
