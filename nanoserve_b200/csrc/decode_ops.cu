@@ -471,16 +471,21 @@ __global__ void __launch_bounds__(256) decode_attention_fused_kernel(
 // slice, one way through the cluster 0.5, the merge 0.5.  A layer's attention at 560 positions, alone in a chain: 8.6 us in two
 // launches, 5.6 in this one; a decode step of 28 layers 1.567 -> 1.490 ms.  On the way: eight CTAs of 28 warps found no place beside a
 // GEMV's CTA and started late (1.620 ms); a butterfly per row and an exponential per row and warp took 270 cycles a row.
+// With many positions it is a warp's chain over its rows, 32 to a pass: the next pass's rows are on their way meanwhile, into a second
+// stage (loaded behind the pass they cost 28 query and 4 KV heads 21.6 us at 4096 positions, now 19.0, and made long contexts of
+// few heads slower than the two launches: 7 and 1 head at 32768 154 us, now 126, there 141; 1 and 1 152, now 121, there 129).
 constexpr int kAttnCtas = 16, kSlicesPerCta = kSplits / kAttnCtas;
 template <int D>
 struct AttnSmem {  // offsets of the dynamic shared memory
   static constexpr int kTile = kSlicesPerCta * kTileRows * D * 2;  // K or V rows of a pass
-  static constexpr int kNew = 2 * kTile;                           // the new k and v row
+  static constexpr int kStage = 2 * kTile;                         // both; the next pass's are loaded beside them
+  static constexpr int kNew = 2 * kStage;                          // the new k and v row
   static constexpr int kMaxSum = kNew + 4 * D;                     // [head][slice] maximum and sum
-  static constexpr int kPart = kMaxSum + 8 * kSplits * 8;          // [head][slice][D / 8] un-normalised
+  static constexpr int kPart = kMaxSum + 8 * kSplits * 8;          // [head][slice][D / 16] un-normalised
   static constexpr int kRot = kPart + 8 * kSplits * (D / kAttnCtas) * 4;  // sine and cosine of the new position
-  // More than half of an SM, so that no SM takes two of these CTAs while others have none, and less than what a GEMV's CTA (112
-  // KB) leaves: it is there early, and the next kernel's beside it.  (1.513 -> 1.490 ms per token.)
+  // More than half of an SM, so that no SM takes two of these CTAs while others have none, and less than a CTA of the streaming
+  // GEMV, a decode step's other kernel (112 KB), leaves: it is there early, and the next kernel's beside it.  (1.513 -> 1.490 ms per
+  // token.  The half-SM CTAs of the other GEMVs, 113 KB, find no place beside it: two halves and no more make a whole.)
   static constexpr int kBytes = 116224;
   static_assert(kRot + D / 2 * 8 <= kBytes, "shared memory");
 };
@@ -517,8 +522,6 @@ __global__ void __launch_bounds__(512, 2) decode_attention_cluster_kernel(
   __shared__ __align__(8) unsigned long long s_bar;
   __shared__ int s_abort;
   const uint32_t base = b2::smem_u32(sm), bar = b2::smem_u32(&s_bar);
-  bf16* s_k = reinterpret_cast<bf16*>(sm);
-  bf16* s_v = reinterpret_cast<bf16*>(sm + S::kTile);
   bf16* s_newk = reinterpret_cast<bf16*>(sm + S::kNew);
   bf16* s_newv = s_newk + D;
   const int crank = (int)b2::cluster_rank(), kh = blockIdx.x / kAttnCtas;
@@ -544,12 +547,13 @@ __global__ void __launch_bounds__(512, 2) decode_attention_cluster_kernel(
   };
   // rows [t0, t0 + kTileRows) of each of the CTA's slices, copied past the registers; the row that this launch appends is not in
   // the cache yet
-  auto request = [&](int t0) {
+  auto request = [&](int t0, int stage) {
     const int rows = min(kTileRows, per - t0), units = kSlicesPerCta * rows * kRowU4;
     for (int u = tid; u < units; u += blockDim.x) {
-      const int c = u % kRowU4, r = u / kRowU4, sl = r / rows, j = (crank * kSlicesPerCta + sl) * per + t0 + (r - sl * rows);
+      static_assert(kSlicesPerCta == 2, "no division");
+      const int c = u % kRowU4, r = u / kRowU4, sl = r >= rows, j = (crank * kSlicesPerCta + sl) * per + t0 + (r - sl * rows);
       if (j < n && j != pos) {
-        const uint32_t dst = base + ((sl * kTileRows + (r - sl * rows)) * kRowU4 + c) * 16;
+        const uint32_t dst = base + stage * S::kStage + ((sl * kTileRows + (r - sl * rows)) * kRowU4 + c) * 16;
         b2::cp_async_cg16(dst, kbase + (size_t)j * kRowU4 + c);
         b2::cp_async_cg16(dst + S::kTile, vbase + (size_t)j * kRowU4 + c);
       }
@@ -558,12 +562,12 @@ __global__ void __launch_bounds__(512, 2) decode_attention_cluster_kernel(
   // `early`: the position and the cached rows below it were written by earlier steps, not by the kernel in front of this one
   if (early) {
     find();
-    request(0);
+    request(0, 0);
   }
   asm volatile("griddepcontrol.wait;" ::: "memory");
   if (!early) {
     find();
-    request(0);
+    request(0, 0);
   }
   const int j0 = sp * per, j1 = min(n, j0 + per);
 
@@ -618,25 +622,23 @@ __global__ void __launch_bounds__(512, 2) decode_attention_cluster_kernel(
   float m = -FLT_MAX, l = 0.f, acc[E];
 #pragma unroll
   for (int e = 0; e < E; ++e) acc[e] = 0.f;
-  for (int t0 = 0; t0 < per; t0 += kTileRows) {
-    if (t0 > 0) {
-      __syncthreads();  // everybody is done with the rows of the last pass
-      request(t0);
-    }
+  for (int t0 = 0, stage = 0; t0 < per; t0 += kTileRows, stage ^= 1) {
     b2::cp_async_wait_all();
-    __syncthreads();
+    __syncthreads();  // the pass's rows are there, and everybody is done with those of the last one
+    if (t0 + kTileRows < per) request(t0 + kTileRows, stage ^ 1);
+    unsigned char* tile = sm + stage * S::kStage;
     // the new row into its place in the pass that holds it
     if (const int r = pos - t0 - (crank * kSlicesPerCta + pos / per % kSlicesPerCta) * per;
         pos < max_len && pos / per / kSlicesPerCta == crank && r >= 0 && r < kTileRows) {
       const int at = (pos / per % kSlicesPerCta * kTileRows + r) * kRowU4;
       for (int u = tid; u < 2 * kRowU4; u += blockDim.x)
-        *reinterpret_cast<uint4*>(sm + (u < kRowU4 ? 0 : S::kTile) + (at + u % kRowU4) * 16) =
+        *reinterpret_cast<uint4*>(tile + (u < kRowU4 ? 0 : S::kTile) + (at + u % kRowU4) * 16) =
             reinterpret_cast<const uint4*>(s_newk)[u];
       __syncthreads();
     }
     const int rows = min(kTileRows, j1 - j0 - t0);
-    const bf16* tk = s_k + slice * kTileRows * D + lane * E;
-    const bf16* tv = s_v + slice * kTileRows * D + lane * E;
+    const bf16* tk = reinterpret_cast<const bf16*>(tile) + slice * kTileRows * D + lane * E;
+    const bf16* tv = tk + S::kTile / 2;
     // Eight rows at a time.  A row's parts are added over the lanes as one tree, as a butterfly would; each of its first three steps
     // halves the rows that a lane goes on with (9 exchanges for the 40 of eight butterflies), and row q ends in lanes 4 q to
     // 4 q + 3.  There the running maxima are a scan and the exponentials of all rows one instruction; only the products and sums
@@ -687,7 +689,7 @@ __global__ void __launch_bounds__(512, 2) decode_attention_cluster_kernel(
     }
   }
 
-  // ---- partials to the CTAs that merge them: lanes 4 r .. 4 r + 3 hold the dimensions of CTA r
+  // ---- partials to the CTAs that merge them: lanes 2 r and 2 r + 1 hold the dimensions of CTA r
   b2::cluster_wait();
   send_part<E>(base + S::kPart + ((w * kSplits + sp) * kMine + lane % (32 / kAttnCtas) * E) * 4, bar, lane / (32 / kAttnCtas), acc);
   if (lane < kAttnCtas) b2::st_async_f2(base + S::kMaxSum + (w * kSplits + sp) * 8, bar, lane, m, l);
@@ -897,9 +899,9 @@ int decode_attention_fused_launch(const void* qkv, const void* bias, const void*
   const dim3 grid(Hk, kSplits);
   // The cluster form where all of the call's clusters run at once: a CTA takes an SM, so that a second wave costs as much as the
   // first, where the two launches keep several small CTAs to an SM.  The line is the device's count of clusters of sixteen (seven on
-  // a B200; none on a slice of one).  us per layer in a chain, this form and in brackets the two launches, 512 / 4096 positions, heads of
-  // 128: 28 query and 4 KV heads 5.8 / 21.6 (8.2 / 34.9), 28 and 7 5.8 / 19.0 (7.4 / 24.8), 32 and 8, with two waves, 10.1 / 36.4 (7.2 /
-  // 23.5), 64 and 8 12.3 / 44.3 (10.1 / 40.1), 32 and 32 27.7 / 108 (11.9 / 41.0).
+  // a B200; none on a slice of one).  us per layer in a chain, this form and in brackets the two launches, 512 / 4096 positions,
+  // heads of 128: 28 query and 4 KV heads 5.8 / 19.0 (8.2 / 34.7), 28 and 7 5.7 / 16.5 (7.4 / 24.7); with two waves and more, a
+  // pass's rows loaded behind the last pass, 32 and 8 10.1 / 36.4 (7.2 / 23.5), 32 and 32 27.7 / 108 (11.9 / 41.0).
   if (!one_launch && tp == nullptr && (flags & 4) == 0) {
     static std::atomic<int> clusters_on[2][64];  // one more than their number: asked once
     int dev = -1;

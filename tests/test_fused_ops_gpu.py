@@ -249,7 +249,7 @@ def test_fused_attention_equals_the_two_calls(kernels, Hq, Hk, D, L, pos):
 
 # slices of more rows than are staged at a time, the new row in the first and in the last pass; one head to a KV head and eight
 @pytest.mark.parametrize("Hq,Hk,D,L,pos", [(8, 2, 128, 2100, 2050), (28, 4, 128, 1100, 1055), (8, 1, 64, 3000, 2999),
-                                            (3, 3, 128, 1300, 1024), (16, 2, 64, 1040, 1039)])
+                                            (3, 3, 128, 1300, 1024), (16, 2, 64, 1040, 1039), (28, 7, 128, 7000, 6600), (4, 4, 64, 9000, 8800)])
 def test_fused_attention_in_several_passes(kernels, Hq, Hk, D, L, pos):
     test_fused_attention_equals_the_two_calls(kernels, Hq, Hk, D, L, pos)
 
