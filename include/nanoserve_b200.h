@@ -202,7 +202,7 @@ int b2_w4_gemv_noalloc(const void* X, const void* Wq, const void* S, void* Y, in
  *     qkv is read, not modified: every CTA rotates the query heads it serves in registers; the CTA whose key slice
  *     holds position *pos builds the new k and v rows, stores them to the caches and uses them from shared memory.
  *     flags 0: without tp, and where the device holds a cluster of sixteen CTAs per KV head at once (up to seven KV heads on a
- *     B200), ONE launch, in which the CTAs exchange the key slices' results (28 query and 4 KV heads of 128 at 512 positions, in a
+ *     B200) and the library's state exists (b2_init, or any linear before), ONE launch, in which the CTAs exchange the key slices' results (28 query and 4 KV heads of 128 at 512 positions, in a
  *     chain: 5.8 us a layer, in two launches 8.2); else the merge of the key slices is a second launch.  flags 4 (may be
  *     added): two launches wherever flags 0 would take one.  flags 1: one launch in which the last CTA of a
  *     KV head to finish merges the slices (an arrival counter per KV head; nobody waits), which puts a fence, an atomic and

@@ -247,7 +247,7 @@ int b2_decode_attention_fused(const void* qkv, const void* bias, const void* inv
                               const b2_tp_desc* tp, int flags, void* stream) {
   int* status = nullptr;
   b2::GemvTp t;
-  if (tp != nullptr) {  // only a wait can time out
+  if (tp != nullptr) {  // its waits can time out (the cluster form, without tp, asks for the status word itself)
     int rc = 0;
     DeviceState* st = device_state(&rc);
     if (!st) return rc;

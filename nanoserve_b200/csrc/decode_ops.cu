@@ -717,7 +717,7 @@ __global__ void __launch_bounds__(512, 2) decode_attention_cluster_kernel(
   if (s_abort) {  // a peer never sent: nothing may come in after this CTA has left
     b2::cluster_arrive();
     b2::cluster_wait();
-    if (tid == 0 && status != nullptr) atomicCAS(status, 0, b2::kStatusGemvTimeout);
+    if (tid == 0) atomicCAS(status, 0, b2::kStatusGemvTimeout);
     for (int i = 0; i < 64; ++i) __nanosleep(2000);
   }
 }
@@ -902,7 +902,10 @@ int decode_attention_fused_launch(const void* qkv, const void* bias, const void*
   // a B200; none on a slice of one).  us per layer in a chain, this form and in brackets the two launches, 512 / 4096 positions,
   // heads of 128: 28 query and 4 KV heads 5.8 / 19.0 (8.2 / 34.7), 28 and 7 5.7 / 16.5 (7.4 / 24.7); with two waves and more, a
   // pass's rows loaded behind the last pass, 32 and 8 10.1 / 36.4 (7.2 / 23.5), 32 and 32 27.7 / 108 (11.9 / 41.0).
-  if (!one_launch && tp == nullptr && (flags & 4) == 0) {
+  // Its waits for the peers are bounded, so it needs the device's status word; the two launches wait for nobody, and run where the
+  // word does not exist yet (a first call, under capture perhaps, where it could not be made).
+  int* const word = tp == nullptr ? device_status_word_if_ready() : nullptr;
+  if (!one_launch && word != nullptr && (flags & 4) == 0) {
     static std::atomic<int> clusters_on[2][64];  // one more than their number: asked once
     int dev = -1;
     if (const cudaError_t e = cudaGetDevice(&dev); e != cudaSuccess) return (int)e;
@@ -939,7 +942,7 @@ int decode_attention_fused_launch(const void* qkv, const void* bias, const void*
       return cudaLaunchKernelEx(&cfg, kernel, static_cast<const bf16*>(qkv), static_cast<const bf16*>(bias),
                                 static_cast<const float*>(inv_freq), static_cast<const int*>(pos),
                                 static_cast<bf16*>(cache_k), static_cast<bf16*>(cache_v), static_cast<bf16*>(out), Hq, Hk,
-                                max_len, scale, (flags & 2) ? 1 : 0, device_status_word_if_ready());
+                                max_len, scale, (flags & 2) ? 1 : 0, word);
     };
     bool fits = false;
     const cudaError_t e = D == 128 ? cluster(decode_attention_cluster_kernel<128>, AttnSmem<128>::kBytes, &fits)

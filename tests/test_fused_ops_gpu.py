@@ -3,6 +3,9 @@ helpers, against plain PyTorch fp32 references of the same ops (the reference pr
 same formulas, python/nanoserve/ops.py:101-142).  Bound: 3e-2 relative to |ref| + 1, the reference's fused-op gate
 (bench/bench_fused.cu:70-77)."""
 import ctypes
+import os
+import subprocess
+import sys
 
 import pytest
 import torch
@@ -306,6 +309,39 @@ def test_attention_in_one_launch_equals_two(kernels, Hq, Hk, D, one):
         assert torch.equal(outs[0], outs[1])
     assert torch.equal(caches[0], caches[1])
     assert kernels.device_status() == 0
+
+
+FIRST_CALL = """
+import sys, torch
+from nanoserve_b200.ops import Kernels
+lib = (k := Kernels(sys.argv[1])).lib
+Hq, Hk, D, L = 28, 4, 128, 64
+z = lambda *shape, t=torch.bfloat16: torch.zeros(*shape, dtype=t, device="cuda")
+qkv, ck, cv, out, inv, p = z((Hq + 2 * Hk) * D), z(Hk, L, D), z(Hk, L, D), z(Hq * D), z(D // 2, t=torch.float32), z(1, t=torch.int32)
+ws = z(lib.b2_decode_attention_fused_workspace_bytes(Hq, Hk, D), t=torch.uint8)
+def run():
+    assert lib.b2_decode_attention_fused(qkv.data_ptr(), None, inv.data_ptr(), p.data_ptr(), ck.data_ptr(), cv.data_ptr(),
+                                         out.data_ptr(), ws.data_ptr(), Hq, Hk, D, L, None, 0, k._stream()) == 0
+def untouched(go):
+    ws[:-4 * Hk] = 0xA5
+    go()
+    return bool((ws[:-4 * Hk] == 0xA5).all())
+graph = torch.cuda.CUDAGraph()
+torch.cuda.synchronize()
+with torch.cuda.graph(graph):
+    run()
+assert not untouched(graph.replay) and not untouched(run)
+k.init()
+assert untouched(run) and not untouched(graph.replay) and lib.b2_device_status() == 0
+"""
+
+
+def test_attention_as_the_first_call(lib_path):
+    """The form whose waits may give up runs only where the status word that records it exists: a first call, captured or not,
+    takes the two launches, which write to the workspace."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    res = subprocess.run([sys.executable, "-c", FIRST_CALL, lib_path], cwd=root, capture_output=True, text=True, timeout=300)
+    assert res.returncode == 0, res.stderr
 
 
 def test_greedy_next(kernels):
