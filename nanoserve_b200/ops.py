@@ -207,10 +207,11 @@ class Kernels:
                 raise RuntimeError("nanoserve_b200 operators take CUDA tensors only (no CPU path)")
 
     # x: [T, H] residual stream, updated in place when r is given. Returns rmsnorm(x) * w.
-    def rmsnorm(self, x, r, w, eps):
-        self._cuda(x, r, w)
+    def rmsnorm(self, x, r, w, eps, out=None):
+        self._cuda(x, r, w, out)
         assert x.is_contiguous() and x.dtype == torch.bfloat16
-        y = torch.empty_like(x)
+        y = torch.empty_like(x) if out is None else out
+        assert out is None or out.is_contiguous() and out.dtype == x.dtype and out.shape == x.shape
         rc = self.lib.ns_rmsnorm(x.data_ptr(), None if r is None else r.data_ptr(), w.data_ptr(),
                                  y.data_ptr(), x.shape[0], x.shape[1], eps, self._stream())
         self._check(rc, "ns_rmsnorm")
@@ -309,15 +310,17 @@ class Kernels:
                     "b2_swiglu_blocks")
         return out
 
-    def w4_linear_swiglu(self, x, Wq, S, group=128, flags=0):
+    def w4_linear_swiglu(self, x, Wq, S, group=128, flags=0, tmp=None, out=None):
         """x [M, K], rows of Wq in alternating blocks of 16 gate and 16 up rows -> silu(gate) * up, [M, N / 2]: the bits of
-        `swiglu_blocks(w4_linear(x, Wq, S, group), 16)`."""
-        self._cuda(x, Wq, S)
+        `swiglu_blocks(w4_linear(x, Wq, S, group), 16)`.  tmp [M, N], left undefined, and out: buffers of the caller's."""
+        self._cuda(x, Wq, S, tmp, out)
         assert x.is_contiguous() and x.dtype == torch.bfloat16 and Wq.is_contiguous() and S.is_contiguous()
         M, K, N = x.shape[0], x.shape[1], Wq.shape[0]
         assert Wq.shape[1] * 8 == K and tuple(S.shape) == (N, K // group)
-        tmp = torch.empty((M, N), dtype=x.dtype, device=x.device)
-        out = torch.empty((M, N // 2), dtype=x.dtype, device=x.device)
+        tmp = torch.empty((M, N), dtype=x.dtype, device=x.device) if tmp is None else tmp
+        out = torch.empty((M, N // 2), dtype=x.dtype, device=x.device) if out is None else out
+        assert tmp.is_contiguous() and out.is_contiguous() and tmp.dtype == out.dtype == x.dtype
+        assert tmp.shape == (M, N) and out.shape == (M, N // 2)
         rc = self.lib.b2_w4_linear_swiglu(x.data_ptr(), Wq.data_ptr(), S.data_ptr(), tmp.data_ptr(), out.data_ptr(), M, N, K,
                                           group, flags, self._stream())
         self._check(rc, "b2_w4_linear_swiglu")

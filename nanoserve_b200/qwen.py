@@ -209,19 +209,19 @@ class Qwen2Runner:
             off += wl
         return torch.cat(parts, dim=1)
 
-    def linear(self, x, wt):
-        return self.k.w4_linear(x, wt[0], wt[1], self.cfg.group)
+    def linear(self, x, wt, out=None):
+        assert out is None or out.shape[1] == wt[0].shape[0]  # (w4_linear takes the rows from the weights alone)
+        return self.k.w4_linear(x, wt[0], wt[1], self.cfg.group, out=out)
 
     # ------------------------------------------------------------------ prompt (eager, GEMM path)
     @torch.no_grad()
     def prefill(self, ids: torch.Tensor) -> torch.Tensor:
         """Runs the prompt, fills the KV cache, leaves the device state ready for decoding.  Returns the first
         generated token (tensor on the device)."""
-        cfg, k = self.cfg, self.k
-        T, D = ids.shape[0], cfg.head_dim
+        T = ids.shape[0]
         assert T < self.max_len
         x = F.embedding(ids, self.embed).contiguous()
-        h = self._prompt_layers_one_gpu(x) if self.world == 1 and self.gu_block == 16 else self._prompt_layers(x)
+        h = self._prompt_layers(x)
         self.pos.fill_(T - 1)  # the pick advances it to T, the position of the first generated token
         self.step.zero_()
         if self.peer is not None:
@@ -230,55 +230,31 @@ class Qwen2Runner:
         return self.tokens[0]
 
     def _prompt_layers(self, x):
-        """The decoder layers over a prompt's residual stream x [T, H]; returns the final norm of it."""
-        cfg, k, T, D = self.cfg, self.k, x.shape[0], self.cfg.head_dim
-        h = k.rmsnorm(x, None, self.layers[0]["ln_in"], cfg.rms_eps)
-        for li, L in enumerate(self.layers):
-            qkv = self._gather_parts(self.linear(h, L["qkv"]), [self.nq, self.nkv, self.nkv])
-            k.qkv_prefill(qkv, L["bias"], self.inv_freq, self.cache_k[li], self.cache_v[li], cfg.n_heads, cfg.n_kv_heads, D)
-            qh = qkv[:, :self.nq].view(T, cfg.n_heads, D).transpose(0, 1)[None]
-            kh, vh = self.cache_k[li, :, :T][None], self.cache_v[li, :, :T][None]
-            a = F.scaled_dot_product_attention(qh, kh, vh, is_causal=True, enable_gqa=True)
-            a = a[0].transpose(0, 1).reshape(T, self.nq).contiguous()
-            h = k.rmsnorm(x, self._gather(self.linear(a, L["o"])), L["ln_post"], cfg.rms_eps)
-            if self.gu_block == 16:  # gate and up row blocks alternate (see __init__)
-                act = self._gather(k.w4_linear_swiglu(h, L["gu"][0], L["gu"][1], cfg.group))
-            else:
-                act = self._gather(k.swiglu_blocks(self.linear(h, L["gu"]), self.gu_block))
-            nxt = self.layers[li + 1]["ln_in"] if li + 1 < cfg.n_layers else self.final_norm
-            h = k.rmsnorm(x, self._gather(self.linear(act, L["d"])), nxt, cfg.rms_eps)
-        return h
-
-    def _prompt_layers_one_gpu(self, x):
-        """The same launches with what a layer writes in buffers that all layers share and with their addresses at hand: up to
-        some 150 tokens a layer's kernels are shorter than 117 us of Python, of which this leaves half."""
-        cfg, k, lib, T, D = self.cfg, self.k, self.k.lib, x.shape[0], self.cfg.head_dim
-        H, I, nq, G, st = cfg.hidden, self.I, self.nq, cfg.group, self._st()
-        h, qkv, proj, gu, act = (torch.empty(T, n, dtype=torch.bfloat16, device=self.dev)
-                                 for n in (H, nq + 2 * self.nkv, H, 2 * I, I))
-        xp, hp, qkvp, projp, gup, actp, invp = (t.data_ptr() for t in (x, h, qkv, proj, gu, act, self.inv_freq))
-        qh = qkv[:, :nq].view(T, cfg.n_heads, D).transpose(0, 1)[None]
+        """The decoder layers over a prompt's residual stream x [T, H]; returns the final norm of it.  On one GPU all layers write
+        into the same buffers: up to some 150 tokens a layer's kernels are shorter than its calls, and allocations and views were
+        half of these."""
+        cfg, k, T, D, nq, I = self.cfg, self.k, x.shape[0], self.cfg.head_dim, self.nq, self.I
+        one = self.world == 1
+        buf = lambda n: torch.empty(T, n, dtype=torch.bfloat16, device=self.dev) if one else None
+        h_buf, qkv_buf, proj, gu, act_buf = (buf(n) for n in (cfg.hidden, nq + 2 * self.nkv, cfg.hidden, 2 * I, I))
+        cache_k, cache_v = self.cache_k.unbind(0), self.cache_v.unbind(0)
         keys, values = (c[:, None, :, :T].unbind(0) for c in (self.cache_k, self.cache_v))
-
-        def norm(r, w):
-            rc = lib.ns_rmsnorm(xp, r, w.data_ptr(), hp, T, H, cfg.rms_eps, st)
-            k._check(rc, "ns_rmsnorm")
-
-        norm(None, self.layers[0]["ln_in"])
+        qh = None
+        h = k.rmsnorm(x, None, self.layers[0]["ln_in"], cfg.rms_eps, out=h_buf)
         for li, L in enumerate(self.layers):
-            k.w4_linear(h, L["qkv"][0], L["qkv"][1], G, out=qkv)
-            rc = lib.b2_qkv_prefill(qkvp, L["bias"].data_ptr(), invp, keys[li].data_ptr(), values[li].data_ptr(), T, cfg.n_heads,
-                                    cfg.n_kv_heads, D, self.max_len, st)
-            k._check(rc, "b2_qkv_prefill")
+            qkv = self._gather_parts(self.linear(h, L["qkv"], qkv_buf), [nq, self.nkv, self.nkv])
+            k.qkv_prefill(qkv, L["bias"], self.inv_freq, cache_k[li], cache_v[li], cfg.n_heads, cfg.n_kv_heads, D)
+            if qh is None or not one:
+                qh = qkv[:, :nq].view(T, cfg.n_heads, D).transpose(0, 1)[None]
             a = F.scaled_dot_product_attention(qh, keys[li], values[li], is_causal=True, enable_gqa=True)
             a = a[0].transpose(0, 1).reshape(T, nq).contiguous()
-            k.w4_linear(a, L["o"][0], L["o"][1], G, out=proj)
-            norm(projp, L["ln_post"])
-            wq, sc = L["gu"]
-            rc = lib.b2_w4_linear_swiglu(hp, wq.data_ptr(), sc.data_ptr(), gup, actp, T, 2 * I, H, G, 0, st)
-            k._check(rc, "b2_w4_linear_swiglu")
-            k.w4_linear(act, L["d"][0], L["d"][1], G, out=proj)
-            norm(projp, self.layers[li + 1]["ln_in"] if li + 1 < cfg.n_layers else self.final_norm)
+            h = k.rmsnorm(x, self._gather(self.linear(a, L["o"], proj)), L["ln_post"], cfg.rms_eps, out=h_buf)
+            if self.gu_block == 16:  # gate and up row blocks alternate (see __init__)
+                act = self._gather(k.w4_linear_swiglu(h, L["gu"][0], L["gu"][1], cfg.group, tmp=gu, out=act_buf))
+            else:
+                act = self._gather(k.swiglu_blocks(self.linear(h, L["gu"], gu), self.gu_block))
+            nxt = self.layers[li + 1]["ln_in"] if li + 1 < cfg.n_layers else self.final_norm
+            h = k.rmsnorm(x, self._gather(self.linear(act, L["d"], proj)), nxt, cfg.rms_eps, out=h_buf)
         return h
 
     def _lm_head_and_pick(self, x, r, wn):

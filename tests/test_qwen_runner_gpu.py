@@ -86,3 +86,37 @@ def test_decode_logits_and_graph(kernels):
     assert eager == graphed
     assert eager[0] == first and len(eager) == 12
     assert kernels.device_status() == 0
+
+
+def test_prompt_without_a_bias(kernels):
+    r = Qwen2Runner(CFG, kernels, torch.device("cuda"), seed=3, max_len=96, norm_gain=1.0)
+    prompt = torch.arange(40, device="cuda")
+    for L in r.layers:
+        L["bias"] = torch.zeros_like(L["bias"])
+    want, keys = int(r.prefill(prompt)), r.cache_k.clone()
+    for L in r.layers:
+        L["bias"] = None
+    assert int(r.prefill(prompt)) == want and torch.equal(r.cache_k, keys) and bool(keys.any())
+
+
+def test_prompt_refuses_operands_that_its_kernels_do_not_take(kernels):
+    """A layer's tensors are looked at in every prompt: the library sees addresses only."""
+    r = Qwen2Runner(CFG, kernels, torch.device("cuda"), seed=3, max_len=96, norm_gain=1.0)
+    prompt = torch.arange(40, device="cuda")
+    good = dict(r.layers[1])
+    (gq, gs), (qq, qs) = good["gu"], good["qkv"]
+    strided = lambda t: t.repeat_interleave(2, dim=-1)[..., ::2]
+    for name, bad in [("bias", good["bias"].float()), ("bias", strided(good["bias"])), ("bias", good["bias"][:-8]),
+                      ("gu", (strided(gq), gs)), ("gu", (gq, strided(gs))), ("gu", (gq, gs[:, :1])), ("qkv", (qq[:-8], qs[:-8]))]:
+        r.layers[1] = {**good, name: bad}
+        with pytest.raises(AssertionError):
+            r.prefill(prompt)
+    r.layers[1] = good
+    whole = r.cache_k
+    r.cache_k = strided(whole)
+    with pytest.raises(AssertionError):
+        r.prefill(prompt)
+    r.cache_k = whole
+    r.prefill(prompt)
+    torch.cuda.synchronize()
+    assert kernels.device_status() == 0
