@@ -43,23 +43,22 @@ __device__ __forceinline__ uint32_t bf16_dup(__nv_bfloat16 s) {
   return b | (b << 16);
 }
 
-// One packed word -> four bf16 pairs of (q - 8) * s * kDequantUnit in their natural order {w0,w1} {w2,w3} {w4,w5} {w6,w7}.
+// One packed word -> four bf16 pairs of (q - 8) * s in their natural order {w0,w1} {w2,w3} {w4,w5} {w6,w7}, each rounded once.
 // A byte b in the low half of a bf16 is the number b * 2^-133 (up to 127 a subnormal, above it a normal, on one line), so
-// the even nibbles of the word, as bytes, are q * 2^-133, the odd ones, left where they are, 16 q * 2^-133; the byte above
+// the even nibbles of the word, as 8 q, are q * 2^-130, the odd ones, left where they are as 16 q, q * 2^-129; the byte above
 // is zero, the sign of an even nibble's byte.  The rest is one fused multiply-add per pair: q * s - 8 s, whose addend is exact
-// (8 is a power of two, the 136 of a biased nibble is not), is rounded once, as the product (q - 8) * s is.  Ten
+// (8 is a power of two, the 136 of a biased nibble is not), is rounded once, as the product (q - 8) * s is.  Eleven
 // instructions per eight weights, six of them on the ALU pipe that bounds the conversion (two cycles each); unpacked to 128 + q,
-// 136 subtracted and multiplied it took 17 and nine.
-// The unit keeps the multiplier s * 2^125 finite for scales below 8, and the sums are multiplied by its inverse at the end
-// (exact both ways, but for weights below 2^-118).  Other scales, infinities and nans among them: dequant_word_any.
-constexpr float kDequantUnit = 0x1p-8f;
+// 136 subtracted and multiplied it took 17 and nine.  (Even nibbles as q, a shift less, leave s * 2^133 finite only below 1/32; weights
+// carried at 2^-8 of their size to make up for that lost bits below 2^-118.)
+// The multiplier s * 2^130 is finite for scales below a quarter.  Other scales, infinities and nans among them: dequant_word_any.
 struct DequantScale {
   uint32_t mul, add;
 };
 __device__ __forceinline__ DequantScale dequant_scale(uint32_t s2) {
-  return {mul_bf16x2(s2, 0x7C007E00u), mul_bf16x2(s2, 0xBD00BD00u)};  // s * {2^125, 2^121}, -s * 2^-5
+  return {mul_bf16x2(mul_bf16x2(s2, 0x7E807F00u), 0x41004100u), mul_bf16x2(s2, 0xC100C100u)};  // s * {2^127, 2^126} * 8, -s * 8
 }
-__device__ __forceinline__ bool dequant_scale_plain(uint32_t s2) { return (s2 & 0x7FFFu) < 0x4100u; }
+__device__ __forceinline__ bool dequant_scale_plain(uint32_t s2) { return (s2 & 0x7FFFu) < 0x3E80u; }
 __device__ __forceinline__ uint32_t fma_bf16x2(uint32_t a, uint32_t b, uint32_t c) {
   uint32_t d;
   asm("fma.rn.bf16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
@@ -72,18 +71,18 @@ __device__ __forceinline__ uint32_t nibble_pair(uint32_t even, uint32_t odd) {
   return d;
 }
 __device__ __forceinline__ void dequant_word(uint32_t w, const DequantScale& sc, uint32_t* o) {
-  const uint32_t even = w & 0x0F0F0F0Fu, odd = w & 0xF0F0F0F0u;
+  const uint32_t even = (w << 3) & 0x78787878u, odd = w & 0xF0F0F0F0u;
   o[0] = fma_bf16x2(nibble_pair<0>(even, odd), sc.mul, sc.add);
   o[1] = fma_bf16x2(nibble_pair<1>(even, odd), sc.mul, sc.add);
   o[2] = fma_bf16x2(nibble_pair<2>(even, odd), sc.mul, sc.add);
   o[3] = fma_bf16x2(nibble_pair<3>(even, odd), sc.mul, sc.add);
 }
-// Any scale: (q - 8) * 2^-6 exactly, then times s * 2^-2.
+// Any scale: (q - 8) / 8 and q - 8 exactly, then the product.
 __device__ __forceinline__ void dequant_word_any(uint32_t w, uint32_t s2, uint32_t* o) {
-  const DequantScale whole = {0x7D007F00u, 0xBE00BE00u};  // {2^127, 2^123}, -2^-3
-  dequant_word(w, whole, o);
+  const DequantScale eighth = {0x7E807F00u, 0xBF80BF80u};  // {2^127, 2^126}, -1
+  dequant_word(w, eighth, o);
 #pragma unroll
-  for (int i = 0; i < 4; ++i) o[i] = mul_bf16x2(o[i], mul_bf16x2(s2, 0x3E803E80u));
+  for (int i = 0; i < 4; ++i) o[i] = mul_bf16x2(mul_bf16x2(o[i], 0x41004100u), s2);
 }
 
 // 16-byte shared-memory accesses by 32-bit shared address.

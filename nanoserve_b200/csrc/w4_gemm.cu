@@ -493,7 +493,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         if (m < p.M) {
           float out[32];
 #pragma unroll
-          for (int e = 0; e < 32; ++e) out[e] = __uint_as_float(v[e]) * (1.f / kDequantUnit);
+          for (int e = 0; e < 32; ++e) out[e] = __uint_as_float(v[e]);
           store_outputs<SWIGLU>(p.Y, m, n0 + c0, p.N, vec_ok, out);
         }
       }
@@ -523,8 +523,6 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
 #pragma unroll
               for (int e = 0; e < 32; ++e) sum[e] += __ldcg(pt + e * 128);
             }
-#pragma unroll
-            for (int e = 0; e < 32; ++e) sum[e] *= 1.f / kDequantUnit;
             if (m < p.M) store_outputs<SWIGLU>(p.Y, m, n0 + c0, p.N, vec_ok, sum);
           }
         }

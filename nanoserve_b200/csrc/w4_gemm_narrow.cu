@@ -4,7 +4,7 @@
 // products accumulate in fp32, one rounding at the store.
 //
 // What bounds it: the packed weights' way from HBM (0.5 bytes per weight), and next to it the conversion of every
-// weight (ten instructions per eight, six of them on the ALU pipe at two cycles).  w4_gemm.cu gives the tokens the 128-row side of the MMA and writes the converted
+// weight (eleven instructions per eight, six of them on the ALU pipe at two cycles).  w4_gemm.cu gives the tokens the 128-row side of the MMA and writes the converted
 // weights to shared memory: with 48 tokens it pads the MMA to 128, sends every weight through shared memory twice and
 // has one CTA per 256 weight rows with no way to fill the chip but fp32 part-tiles in global memory.  Here
 //   * the WEIGHTS are the M side of tcgen05.mma (128 rows per block) and the tokens its N side (16 to 128 columns, a
@@ -17,7 +17,7 @@
 //     before the wait for the kernel in front.  All reads and writes come after it has finished, so it may be the kernel that
 //     writes the weights.
 // Measured, weights from HBM, us at 48 tokens, in brackets w4_gemm.cu: 4608 x 3584 8.8 (25), 37888 x 3584 23.3 (46), 3584 x 18944 16.7
-// (51), 8192 x 28672 42 (113).  What moved them: weights converted in ten instructions instead of 17 per eight (sixteen such launches,
+// (51), 8192 x 28672 42 (113).  What moved them: weights converted in eleven instructions instead of 17 per eight (sixteen such launches,
 // four 7B-shaped layers, 241 -> 228 us), then the questions to the barriers ahead of the last products of a step, parts of a
 // cut K sent instead of fetched and tensor memory freed beside the last sums (224; 777 x 5000 x 4096 in groups of 64 34.1 -> 33.2,
 // 512 x 3584 x 18944 73 -> 69, 128 x 37888 x 3584 37.1 -> 34.7).  What bounds it: at 48 tokens the sixteen products of a step
@@ -376,7 +376,7 @@ __global__ void __launch_bounds__(128 + DW * 32, MINB)
           __nv_bfloat16* y = p.Y + (size_t)(m0 + c0) * p.N + n;
 #pragma unroll
           for (int e = 0; e < 16; ++e)
-            if (live && c0 + e < rt) y[(size_t)e * p.N] = __float2bfloat16(__uint_as_float(v[e]) * (1.f / kDequantUnit));
+            if (live && c0 + e < rt) y[(size_t)e * p.N] = __float2bfloat16(__uint_as_float(v[e]));
         } else {  // [token][row], over the rings: every copy has landed and every MMA has read its operands
 #pragma unroll
           for (int e = 0; e < 16; ++e)
@@ -411,7 +411,7 @@ __global__ void __launch_bounds__(128 + DW * 32, MINB)
 #pragma unroll
               for (int e = 0; e < 4; ++e)
                 if (ny < p.N && c0 + 4 * q + e < rt)
-                  y[(size_t)(4 * q + e) * p.N] = __float2bfloat16(sum[e] * (1.f / kDequantUnit));
+                  y[(size_t)(4 * q + e) * p.N] = __float2bfloat16(sum[e]);
             }
           }
         }
@@ -452,7 +452,6 @@ __global__ void __launch_bounds__(128 + DW * 32, MINB)
             const float4 b = ld_cluster_f4(at, z);
             a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
           }
-        a.x *= 1.f / kDequantUnit; a.y *= 1.f / kDequantUnit; a.z *= 1.f / kDequantUnit; a.w *= 1.f / kDequantUnit;
         __nv_bfloat16* y = p.Y + (size_t)(m0 + tok) * p.N + n;
         if (n + 4 <= p.N && (p.N & 3) == 0) {
           const __nv_bfloat162 lo = __floats2bfloat162_rn(a.x, a.y), hi = __floats2bfloat162_rn(a.z, a.w);

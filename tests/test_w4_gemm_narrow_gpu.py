@@ -139,3 +139,33 @@ def test_scales_of_any_size(kernels, M, flags, G):
     y = kernels.w4_linear(x, Wq, S, G, flags=flags)
     assert bool(y[:, 3].isnan().any()) and bool(y[:, :3].isfinite().all()) and bool(y[:, 4:].isfinite().all())
     assert kernels.device_status() == 0
+
+
+@pytest.mark.parametrize("M,flags", [(32, narrow_flags(1, 1)), (32, narrow_flags(2, 2)), (32, FLAG_GEMM_WIDE), (300, FLAG_GEMM_NO_PAIRS | FLAG_GEMM_WIDE),
+                                     (300, FLAG_GEMM_WIDE)])
+@pytest.mark.parametrize("G", [32, 64, 128])
+@pytest.mark.parametrize("up", [2.0**100, 1.0])
+def test_scales_at_the_ends_of_their_range(kernels, M, flags, G, up):
+    """Weights down to the smallest bf16 and up to the largest, picked out one by one: RN_bf16((q - 8) * s) to the bit.  Small ones
+    are picked with 2^100 and come out as normal numbers."""
+    N, K = 200, 512
+    gen = torch.Generator(device="cuda").manual_seed(G)
+    Wq = torch.randint(-2**31, 2**31 - 1, (N, K // 8), dtype=torch.int32, device="cuda", generator=gen)
+    below = [2.0**-133, 3 * 2.0**-133, 1.3e-39, 2.0**-126, 1.9e-38, 2.0**-122, 1.1e-37, 2.0**-121, 3.1e-36, 2.0**-118, 5e-36, 1e-33]
+    above = [0.2490234375, 0.25, -0.25, 0.49, 0.5, 1.3, 2.0**100, 2.0**124, -1.1 * 2.0**124]
+    sizes = torch.tensor(below if up > 1 else above, device="cuda", dtype=torch.float64).float().to(torch.bfloat16)
+    S = sizes[torch.randint(0, len(sizes), (N, K // G), device="cuda", generator=gen)]
+    S[:N // 2, 1:] = sizes[0]  # warps whose rows leave a range for a group only
+    S[N // 2:N // 2 + 32] = below[4] if up > 1 else 2.0  # a warp of one size
+    if up > 1:
+        S[1] = 0.3  # small scales beside one above the line
+    ks = torch.randint(0, K, (M,), device="cuda", generator=gen)
+    x = torch.zeros(M, K, dtype=torch.bfloat16, device="cuda")
+    x[torch.arange(M, device="cuda"), ks] = up
+    shifts = torch.arange(0, 32, 4, device="cuda", dtype=torch.int32)
+    w = (((Wq[:, :, None] >> shifts) & 15).flatten(1) - 8).double() * S.double().repeat_interleave(G, dim=1)
+    q = torch.exp2(torch.clamp(torch.floor(torch.log2(w.abs())) - 7, min=-133.0))  # a bf16's last place
+    want = torch.where(w == 0, w, torch.round(w / q) * q)[:, ks].T * up
+    y = kernels.w4_linear(x, Wq, S, G, flags=flags).double()
+    assert kernels.device_status() == 0
+    assert bool(want.isfinite().all()) and torch.equal(y, want)
