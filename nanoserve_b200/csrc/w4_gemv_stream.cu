@@ -1246,6 +1246,21 @@ bool gemv_stream_applies(const void* Wq, int M, int N, int K, int G, int flags) 
   return false;
 }
 
+// Estimated time (us) of a plain launch at one token in groups of 128, for the choice between this kernel and the tcgen05 one: a fit
+// to 4000 shapes (128 to 60000 x 512 to 28672, chained launches, weights from HBM; standard deviation 5 %) by what a plan has in
+// common: super-chunks of X that a thread converts, weights, super-chunks that a warp walks.  CTAs that take an SM each are not
+// estimated: in one wave nothing beats them, a second, mostly empty one always loses (13819 x 25856: 216 CTAs 53.8 us, there 43.0).
+double gemv_stream_us(int N, int K, int sm_count, size_t partial_cap) {
+  StreamPlan pl;
+  if (!make_stream_plan(1, N, K, 128, nullptr, 0, sm_count, partial_cap, &pl)) return 1e30;
+  const double w = 1e-6 * N * K;
+  if (pl.nslices > 1) return 5.7 + 0.32 * pl.scps + 0.0526 * w;
+  if (pl.smem > kSmemTwoPerSm) return pl.grid_x > sm_count ? 1e30 : 0.0;
+  if (pl.RB > 1) return 0.0;  // (never longer)
+  const int waves = pl.q.n_tiles ? 1 : (pl.grid_x + 2 * sm_count - 1) / (2 * sm_count);
+  return 3.0 + 0.074 * pl.scps + 0.067 * w + 0.135 * waves * pl.scps / pl.ks;
+}
+
 size_t gemv_stream_grid(int M, int N, int K, int G, int flags, int sm_count, size_t partial_cap) {
   StreamPlan pl;
   if (!make_stream_plan(M, N, K, G, nullptr, flags, sm_count, partial_cap, &pl)) return 0;

@@ -684,11 +684,14 @@ bool gemv_tc_serves(const void* X, const void* Wq, const void* S, const void* Y,
 // Whether this kernel is shorter than the GEMV that would take a plain call of 1 to 16 tokens, `other` one of kTcOther*.  Lines
 // drawn through 2044 calls on random shapes (128 to 60000 rows, K 512 to 28672, weights from HBM, one launch behind the other), every
 // kernel and every plan of this one timed, and earlier through 6472 more.
-//   * One token (streaming kernel): both hold X in 32 bits.  From K = 1024 and up to twelve million weights a launch is its latencies, and the
-//     other converts the whole of X before its first product (512 x 3584 3.4 us against 4.5, 1909 x 4352 3.8 against 5.2); between K of
+//   * One token (streaming kernel): both hold X in 32 bits.  Only where that kernel has a weakness: up to twelve million weights a
+//     launch is its latencies, and it converts the whole of X before its first product (512 x 3584 3.4 us against 4.5); between K of
 //     9728 and 16384 it does so several times per thread (4980 x 14080 12.8 against 15.0), above 22000 it cuts K through memory
-//     (8192 x 28672 26.6 against 29.2).  Of 335 calls those that come here take 0.83 of their time there, three of them 3 % more (at
-//     most 5); the others, at HBM's rate, are shorter there (37888 x 3584 14.3 against 15.6).
+//     (8192 x 28672 26.6 against 29.2).  Within these lines, which cost a call's host side next to nothing, tiles of 128 rows as they
+//     are and tiles of 256 by the estimates of both kernels: by the lines alone these took 3500 x 2048 (5.3 us for 4.4), 2861 x 3584
+//     (5.6 for 5.1), 11771 x 28160 (54 for 39, 92 CTAs).  A full house of clusters of three and more is left out: a few SMs that the
+//     kernel in front still holds cost it a wave (11343 x 26624, 135 CTAs, 38.4 for 36.4).  Of 4000 calls on shapes like these 1464 come here,
+//     0.837 of their time there in the geometric mean; eight lose 3 % (at most 9), with the lines alone 157 (at most 41).
 //   * Two to four tokens (streaming kernel; X has 15 bits there at three and four): shorter here but for many rows of a short K (21667 x
 //     1024 at four tokens 4.8 us there, 5.5 here; 18944 x 3584 at two 9.6 and 10.7).  Of 150 calls five lose 3 % (at most 6).
 //   * Many-token kernel, five and more tokens: by the estimates of both, this one's with what plans have in common (they come out
@@ -700,17 +703,21 @@ bool gemv_tc_shorter(const void* X, const void* Wq, const void* S, const void* Y
                      int sm_count, size_t partial_cap, TcOther other) {
   if (M < 1 || (flags & ~kFlagNoPdl) != 0 || !tc_operands(X, Wq, S, Y, M, N, K, G)) return false;
   const double w = 1e-6 * N * K, k3 = 1e-3 * K, mk = 1e-4 * M * K;
+  // the lines in N and K first: a call of few tokens is bound by its host side, and most need no plan
+  if (M == 1 && !(w <= 12.0 ? K >= 1024 : (K >= 9728 && K <= 16384 && N <= 4992) || (K >= 22016 && N >= 7424))) return false;
+  if (M > 1 && other == kTcOtherStream &&
+      !(M > 2       ? K >= 2304 || N <= 8000
+        : K >= 3840 ? N <= 128 * (sm_count - 1)  // (above, that kernel's CTAs of 128 rows leave no SM over)
+                    : N <= (K <= 1536 ? 5800 : 11000)))
+    return false;
   TcPlan pl;
   if (!tc_plan(M, N, K, sm_count, 0, 0, &pl)) return false;
   if (M == 1) {
-    if (w <= 12.0) return K >= 1024 && (N <= 4096 ? pl.us <= 8.5 : pl.us <= 3.5);
-    return (K >= 9728 && K <= 16384 && N <= 4992) || (K >= 22016 && N >= 7424);
+    if (!pl.form) return w > 12.0 || pl.us <= (N <= 4096 ? 8.5 : 3.5);
+    if (pl.several || (pl.ks > 2 && pl.busy > 0.985)) return false;
+    return 1.04 * (0.862 * pl.us + 0.009 * w + 3.44 * pl.busy - 0.88) < gemv_stream_us(N, K, sm_count, partial_cap);
   }
-  if (other == kTcOtherRing) return true;
-  if (other == kTcOtherStream)
-    return M > 2       ? K >= 2304 || N <= 8000
-           : K >= 3840 ? N <= 128 * (sm_count - 1)  // (above, that kernel's CTAs of 128 rows leave no SM over)
-                       : N <= (K <= 1536 ? 5800 : 11000);
+  if (other != kTcOtherMany) return true;
   if (M <= 4) return 1.02 * pl.us < 6.65 + 0.11 * w + 0.027 * k3 + 0.074 * mk;
   const double us = pl.us + (pl.form       ? 2.03 * pl.busy * pl.busy
                              : pl.several ? 0.5

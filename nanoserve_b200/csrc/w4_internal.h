@@ -164,6 +164,7 @@ bool gemv_stream_applies(const void* Wq, int M, int N, int K, int G, int flags);
 int gemv_stream_launch(const void* X, const void* Wq, const void* S, void* Y, int M, int N, int K, int G,
                        const GemvPrologue& pro, const Workspace& ws, int flags, int sm_count, cudaStream_t stream,
                        const GemvTp* tp);
+double gemv_stream_us(int N, int K, int sm_count, size_t partial_cap);
 size_t gemv_stream_grid(int M, int N, int K, int G, int flags, int sm_count, size_t partial_cap);
 int gemv_stream_describe(int M, int N, int K, int G, int flags, int sm_count, size_t partial_cap, int counters_cap,
                          char* buf, int buflen);

@@ -156,3 +156,23 @@ def test_one_token_runs_the_shorter_kernel(kernels, N, K, here):
     rows = np.unique(np.concatenate([[0, N - 1], np.random.default_rng(0).integers(0, N, 60)]))
     ref = oracle.w4_linear_f32(X, Wq[rows], S[rows], 128, threads=oracle.max_threads())
     check_bf16_output(run(kernels, X, Wq, S, 0)[:, rows], ref, slack(1))
+
+
+# both sides of every line, us of the streaming kernel and of this one
+@pytest.mark.parametrize("N,K,here", [
+    (3500, 2048, False),    # 4.4, 5.3: tiles of 256 rows
+    (4096, 1024, True),     # 4.1, 3.2
+    (2861, 3584, False),    # 5.1, 5.6
+    (1909, 4352, True),     # 5.5, 4.1
+    (11771, 28160, False),  # 38.9, 54.3: 92 CTAs
+    (10140, 26880, True),   # 31.4, 29.0: 120
+    (11343, 26624, False),  # 36.4, 38.4: a full house of clusters of three
+    (13819, 25856, True),   # 53.8, 43.0: the other kernel's 216 CTAs take an SM each
+    (14651, 27136, False),  # 48.1, 54.8: its 115 CTAs do
+    (7300, 24064, False),   # outside the lines in N and K
+    (4992, 12544, True),    # 13.5, 11.4
+    (5100, 12544, False),
+    (256, 896, False),      # K is no multiple of 256
+])
+def test_one_token_on_both_sides_of_the_lines(kernels, N, K, here):
+    assert ("tcgen05" in kernels.gemv_describe(1, N, K, 128)) == here
