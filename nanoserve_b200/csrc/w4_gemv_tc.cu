@@ -242,13 +242,14 @@ __global__ void __launch_bounds__(MB == 2 ? 896 : 512, MB == 2 ? 1 : 2)
         tmem_ld_sums<kLo>(d_src + 32, d1);
         tmem_ld_wait();
         then();
+        const uint32_t far = pair_scales(g + 8);  // (asked for ahead of the sums: behind them short launches were up to 2 % longer)
         if constexpr (MT != 16) join(d0, j);
         add_step(2 * i, __uint_as_float(cur << 16), j);
         join(d1, j);
         add_step(2 * i + 1, __uint_as_float(cur & 0xFFFF0000u), j);
         cur = nxt;
         g += 4;
-        nxt = pair_scales(g + 4);
+        nxt = far;
       };
       uint32_t v[32];  // a step's bytes
       auto convert = [&](uint32_t slot, int half) {
@@ -502,6 +503,18 @@ __global__ void __launch_bounds__(MB == 2 ? 896 : 512, MB == 2 ? 1 : 2)
           umma_commit(bar_x_empty + 8 * xs);
         }
         __syncwarp();
+        // With rows of S that start anywhere in a sector (K / 256 odd) some lane's next scales come from HBM in every pair, which
+        // takes longer than a group's turn: the sector of eight pairs ahead is brought into L2.  26965 x 12544 at 5 tokens 43.0 -> 40.4
+        // us, 14289 x 25856 at 6 47.1 -> 43.5.  Here, since the same in the rows' warps cost short launches 1 %.
+        if constexpr (SV == 2) {
+          if ((i & 7) == 0 && i + 8 < np) {
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+              const int n = n0 + mb * 128 + r * 32 + lane;
+              if (n < p.N) prefetch_l2(p.S + (size_t)n * p.KG + 2 * (pr0 + i) + 16);
+            }
+          }
+        }
         if (++xs == p.sx) xs = 0;
       }
     }

@@ -176,3 +176,13 @@ def test_one_token_runs_the_shorter_kernel(kernels, N, K, here):
 ])
 def test_one_token_on_both_sides_of_the_lines(kernels, N, K, here):
     assert ("tcgen05" in kernels.gemv_describe(1, N, K, 128)) == here
+
+
+# K / 256 odd and more than eight pairs per CTA: scales that are brought into L2 ahead; tiles cut off, one CTA, K cut
+@pytest.mark.parametrize("M,N,K,form,split", [(1, 300, 2816, 2, 1), (4, 129, 4352, 1, 1), (8, 700, 12544, 2, 1), (13, 257, 5888, 2, 2),
+                                              (16, 64, 8448, 1, 3), (5, 513, 2304, 2, 1)])
+def test_scales_ahead(kernels, M, N, K, form, split):
+    flags = FLAG_DECODE_NARROW | narrow_flags(split, form)
+    X, Wq, S = oracle.synth_inputs(M, N, K, 128, seed=N)
+    ref = oracle.w4_linear_f32(X, Wq, S, 128, threads=oracle.max_threads())
+    check_bf16_output(run(kernels, X, Wq, S, flags), ref, slack(M))
