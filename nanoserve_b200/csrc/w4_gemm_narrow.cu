@@ -78,13 +78,15 @@ __device__ __forceinline__ void umma_f16_ts(uint32_t tmem_d, uint32_t tmem_a, ui
 // groups that take the K blocks in turn; the converted weights of two K blocks fit in TMEM.  MINB: CTAs per SM.
 // MODE: 4 or 2: groups of 128 (a scale per row and step), read that many at a time; 64, 32: groups of 64 or 32 and whole
 // steps, a step's two or four scales per read; 0: any group, any K.  RED: the parts of a cut K are sent (p.red); a kernel of its
-// own, since its code made short launches of the others up to 6 % longer.
-template <int MB, int DW, int MINB, int MODE, bool RED>
+// own, since its code made short launches of the others up to 6 % longer.  AHEAD: scales are brought into L2 a sector ahead, by the rows'
+// warps (1) or the one that issues the products (2), see narrow_form_ahead.
+template <int MB, int DW, int MINB, int MODE, bool RED, int AHEAD = 0>
 __global__ void __launch_bounds__(128 + DW * 32, MINB)
     w4_gemm_narrow_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
                           const NarrowParams p) {
   constexpr int kRows = MB * 128, kGroups = DW / (4 * MB), kWSlot = kRows * 128;  // a slot of packed words: K = 256
   static_assert(kGroups == 2, "a slot of packed words holds a step for either group");
+  [[maybe_unused]] constexpr int kSectorSteps = 16 * MODE / 128;  // steps whose scales fill a sector of 32 bytes (MODE 64, 32)
   constexpr bool G128 = MODE == 2 || MODE == 4;
   extern __shared__ unsigned char smem_raw[];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;  // swizzled tiles
@@ -223,6 +225,15 @@ __global__ void __launch_bounds__(128 + DW * 32, MINB)
         }
         ready = __any_sync(0xffffffffu, next);
         __syncwarp();
+        if constexpr (AHEAD == 2) {
+          if (i % kSectorSteps == 0 && i + kSectorSteps < nkb) {
+#pragma unroll
+            for (int r = 0; r < 4 * MB; ++r) {
+              const int n = n0 + r * 32 + lane;
+              if (n < p.N) prefetch_l2(p.S + (size_t)n * p.KG + (kb0 + i + kSectorSteps) * (128 / MODE));
+            }
+          }
+        }
       }
     }
   }
@@ -303,6 +314,9 @@ __global__ void __launch_bounds__(128 + DW * 32, MINB)
             advance(j < 3 ? 32 : 32 + kKB);
           }
           k += 2 * kKB;
+        }
+        if constexpr (AHEAD == 1) {
+          if (i % kSectorSteps == 0 && i + kSectorSteps < nkb && live) prefetch_l2(s_row + (kb0 + i + kSectorSteps) * (128 / MODE));
         }
         bool plain = dequant_scale_plain(sc[0]);
         if constexpr (!G128) {
@@ -506,6 +520,20 @@ NarrowForm narrow_form(int form, int variant, bool red) {
     return {red ? narrow_kernel<1, 8, 2, true>(variant) : narrow_kernel<1, 8, 2, false>(variant), variant, 128, 8, 2, kSmemHalf, red};
   return {red ? narrow_kernel<2, 16, 1, true>(variant) : narrow_kernel<2, 16, 1, false>(variant), variant, 256, 16, 1, kSmemFull, red};
 }
+// Long shares of K in groups of 64 and 32, K a multiple of 256 and not of 512 (variants 5 and 6): there the next scales of some lane
+// come from HBM in most steps, later than the one step ahead that they are asked for, and the faster conversion lost by it (31604 x 9984
+// at 24 tokens, groups of 64 and of 32: 52.8 and 57 us with the old one, 57 and 63 with the new).  With the sector ahead brought into
+// L2 50 and 56 (6400: 30 and 40 for 31 and 44 at 4 tokens).  Not below 48 steps to a CTA (5376 level, 2816 in groups of 32 4 % longer) nor
+// for other K, which have no such loss, and kernels of their own, since the code alone costs short launches 1 to 3 %.  Groups of 32 have
+// the warp that issues the products ask (5 % shorter), but for parts that are sent (2 % longer).
+NarrowForm narrow_form_ahead(int variant, bool red) {
+  static constexpr NarrowKernel k64[2] = {w4_gemm_narrow_kernel<2, 16, 1, 64, false, 1>, w4_gemm_narrow_kernel<2, 16, 1, 64, true, 1>};
+  static constexpr NarrowKernel k32[2] = {w4_gemm_narrow_kernel<2, 16, 1, 32, false, 2>, w4_gemm_narrow_kernel<2, 16, 1, 32, true, 1>};
+  return {variant == 3 ? k64[red] : k32[red], variant + 2, 256, 16, 1, kSmemFull, red};
+}
+bool narrow_ahead(int form, int variant, int nt, int K, int blocks) {
+  return form == 1 && variant >= 3 && nt <= 64 && K % 512 == 256 && blocks >= 48;
+}
 int narrow_scales_per_load(const void* S, int K, int G) {
   const uintptr_t sa = reinterpret_cast<uintptr_t>(S);
   const int kg = K / G;
@@ -520,7 +548,7 @@ int narrow_variant(const void* S, int K, int G) {
 }
 
 int narrow_attributes(const NarrowForm& f, int form, int dev) {
-  static std::atomic<bool> done[64][2][5][2];
+  static std::atomic<bool> done[64][2][7][2];
   if (dev >= 0 && dev < 64 && done[dev][form][f.variant][f.red].load(std::memory_order_acquire)) return 0;
   const cudaError_t e = cudaFuncSetAttribute(f.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, f.smem);
   if (e == cudaSuccess && dev >= 0 && dev < 64) done[dev][form][f.variant][f.red].store(true, std::memory_order_release);
@@ -709,6 +737,7 @@ int gemm_narrow_launch(const void* X, const void* Wq, const void* S, void* Y, in
     p.red = kHeaderBytes + p.sw * slot_w + p.sx * slot_x;
     f = narrow_form(pl.form, variant, true);
   }
+  if (narrow_ahead(pl.form, variant, p.nt, K, blocks)) f = narrow_form_ahead(variant, f.red);
   p.tmem_cols = pl.form ? 512 : 256;
   CUtensorMap tx, tw;
   if (!make_tensor_map_2d(&tx, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, X, (uint64_t)M, (uint64_t)K, p.nt, 64,

@@ -169,3 +169,14 @@ def test_scales_at_the_ends_of_their_range(kernels, M, flags, G, up):
     y = kernels.w4_linear(x, Wq, S, G, flags=flags).double()
     assert kernels.device_status() == 0
     assert bool(want.isfinite().all()) and torch.equal(y, want)
+
+
+@pytest.mark.parametrize("G", [64, 32])
+@pytest.mark.parametrize("M,N,K,split", [(3, 300, 6400, 1), (48, 257, 6400, 1), (64, 31, 6912, 1), (20, 513, 12544, 2), (20, 256, 6144, 1),
+                                         (70, 256, 6400, 1)])
+def test_scales_ahead(kernels, M, N, K, split, G):
+    """Shares of K around the line from which scales are brought into L2 ahead: above it with rows cut off, parts that are sent, and on
+    the other side (K a multiple of 512, more than 64 token columns)."""
+    X, Wq, S = oracle.synth_inputs(M, N, K, G, seed=N)
+    flags = narrow_flags(split, 2) | (FLAG_DECODE_NARROW if M <= 16 else 0)
+    check_bf16_output(run(kernels, X, Wq, S, G, flags), rounded_weight_reference(X, Wq, S, G), 6e-5)
