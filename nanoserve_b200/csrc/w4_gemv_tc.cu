@@ -183,6 +183,9 @@ __global__ void __launch_bounds__(MB == 2 ? 896 : 512, MB == 2 ? 1 : 2)
       };
       int g = 2 * (pr0 + grp);  // the pair's first step: even
       if (live && g < p.KG) prefetch_l2(s_row + g);  // (the second group has none where the CTA's share is one pair)
+      // (with rows of S that start anywhere in a sector the share's next two; 755 x 18688 at three tokens 8.0 -> 7.7 us.  Tiles of 256 rows
+      // lost 1 % by it.)
+      if (SV == 2 && MB == 1 && live && np > 2) prefetch_l2(s_row + 2 * pr0 + min(2 * np - 2, 14 + 2 * grp));
       pdl_wait_prior_grid();
       // SV == 4: two pairs, this group's one of them; SV == 2: one
       auto pair_scales = [&](int step) {
