@@ -14,8 +14,10 @@
 //   * K is cut over a cluster.  A CTA sends its sums into the shared memory of the CTA that adds them, in the order of ranks and
 //     groups (no second launch; st.async counted on a barrier of that CTA).
 // What bounds it: HBM's rate once it runs (37888 x 3584 at four tokens: 7.5 TB/s from the seventh pair on, 70 MB in 11 of 15.4
-// us), the issue slots above eight tokens (1540 of the 1550 cycles of a pair at 13: the words' bytes 96 instructions per row and
-// pair, the sums 7 per token, the conversion of X a sixth of all), and around that the boundary between launches: the wait for the kernel
+// us; a pair 0.89 us, 5.6 TB/s); above eight tokens no unit alone (a pair at 13 tokens takes 1.09 us by 37888 x 14336 less 37888 x 3584,
+// 2150 cycles at 1965 MHz: the issue slots are taken for 1140 of them, the words' bytes 96 instructions per row and pair, the sums 7
+// per token, the conversion of X a sixth of all, and HBM runs at 4.6 TB/s; the rest are waits between a group's steps); and around
+// that the boundary between launches: the wait for the kernel
 // in front returns 0.9 us after its last CTA has left, a CTA starts 0.9 us after the one before it on the SM has (0.3 where
 // neither uses tensor memory), first words and X 0.7 later, first products 0.5, the exchange of parts 0.9.
 // The chain of a group is what the order in the loop is for: half of a pair's words are converted while the products of the group's last
@@ -59,6 +61,7 @@ struct TcParams {
   int ks;       // CTAs of a cluster, each with its share of the pairs
   int sw, sx;   // ring slots of a pair: packed words (per block of 128 rows), X
   int ahead;    // slots of packed words that are brought into L2 ahead of the ring
+  int together; // a cluster's CTAs leave as one
   int x_first;  // the ring's further slots are not asked for before the first X is there
   int off_w, off_x, off_info, off_red;
 };
@@ -537,11 +540,11 @@ __global__ void __launch_bounds__(MB == 2 ? 896 : 512, MB == 2 ? 1 : 2)
   }
   if (p.ks > 1 && (warp >= kMain || poisoned)) cluster_wait();
   __syncthreads();
+  if (p.ks > 1 && (p.together || *abort_flag)) {  // (aborted: peers that have not given up may send parts here until they leave)
+    cluster_arrive();
+    cluster_wait();
+  }
   if (*abort_flag) {
-    if (p.ks > 1) {  // peers that have not given up may send parts here until they leave
-      cluster_arrive();
-      cluster_wait();
-    }
     if (tid == 0) atomicCAS(p.status, kStatusOk, kStatusGemvTimeout);
     for (int i = 0; i < 64; ++i) __nanosleep(2000);  // copies in flight land before the shared memory is released
     __syncthreads();
@@ -722,9 +725,8 @@ bool gemv_tc_serves(const void* X, const void* Wq, const void* S, const void* Y,
 //     9728 and 16384 it does so several times per thread (4980 x 14080 12.8 against 15.0), above 22000 it cuts K through memory
 //     (8192 x 28672 26.6 against 29.2).  Within these lines, which cost a call's host side next to nothing, tiles of 128 rows as they
 //     are and tiles of 256 by the estimates of both kernels: by the lines alone these took 3500 x 2048 (5.3 us for 4.4), 2861 x 3584
-//     (5.6 for 5.1), 11771 x 28160 (54 for 39, 92 CTAs).  A full house of clusters of three and more is left out: a few SMs that the
-//     kernel in front still holds cost it a wave (11343 x 26624, 135 CTAs, 38.4 for 36.4).  Of 4000 calls on shapes like these 1464 come here,
-//     0.837 of their time there in the geometric mean; eight lose 3 % (at most 9), with the lines alone 157 (at most 41).
+//     (5.6 for 5.1), 11771 x 28160 (54 for 39, 92 CTAs).  Of 3000 shapes like these 935 come here, 0.843 of their time there in
+//     the geometric mean, and 20 lose 3 % (at most 11); by the lines alone 1052, of which 96 (at most 41).
 //   * Two to four tokens (streaming kernel; X has 15 bits there at three and four): shorter here but for many rows of a short K (21667 x
 //     1024 at four tokens 4.8 us there, 5.5 here; 18944 x 3584 at two 9.6 and 10.7).  Of 150 calls five lose 3 % (at most 6).
 //   * Many-token kernel, five and more tokens: by the estimates of both, this one's with what plans have in common (they come out
@@ -747,7 +749,7 @@ bool gemv_tc_shorter(const void* X, const void* Wq, const void* S, const void* Y
   if (!tc_plan(M, N, K, sm_count, 0, 0, &pl)) return false;
   if (M == 1) {
     if (!pl.form) return w > 12.0 || pl.us <= (N <= 4096 ? 8.5 : 3.5);
-    if (pl.several || (pl.ks > 2 && pl.busy > 0.985)) return false;
+    if (pl.several) return false;
     return 1.04 * (0.862 * pl.us + 0.009 * w + 3.44 * pl.busy - 0.88) < gemv_stream_us(N, K, sm_count, partial_cap);
   }
   if (other != kTcOtherMany) return true;
@@ -790,6 +792,11 @@ int gemv_tc_launch(const void* X, const void* Wq, const void* S, void* Y, int M,
   p.ks = pl.ks;
   tc_layout(pl, M, &p);
   p.ahead = 3;
+  // Clusters of three that take every place the device has for them (45 on 148 SMs): where their CTAs leave one by one the next
+  // launch's clusters start in other places and some find none, a wave of their own (11300 x 27392 at 4 tokens 32.8 us for 44 then;
+  // 11500 x 14336 20.5 for 24.8).  Not below eight pairs to a CTA (11400 x 4096 9.1, together 9.7), nor for other sizes of clusters,
+  // full or not: leaving together costs up to 0.7 us there (3800 x 14336 in clusters of eight 10.9 and 11.6).
+  p.together = form && pl.ks == 3 && pl.pairs >= 8 && pl.busy > 0.97;
   // Where the rings of nearly all SMs fill at once X waits behind them for two microseconds: then only the first slot goes ahead
   // of it (8192 x 28672 at 8 tokens 30.2 -> 29.3 us, 37888 x 3584 at 13 17.4 -> 16.9).  Elsewhere it is X that is waited for (4608 x
   // 3584 at 4 tokens 5.8 against 6.1), and with a short K and few tokens it is there soon enough between other launches (four

@@ -166,7 +166,8 @@ def test_one_token_runs_the_shorter_kernel(kernels, N, K, here):
     (1909, 4352, True),     # 5.5, 4.1
     (11771, 28160, False),  # 38.9, 54.3: 92 CTAs
     (10140, 26880, True),   # 31.4, 29.0: 120
-    (11343, 26624, False),  # 36.4, 38.4: a full house of clusters of three
+    (8264, 25088, True),    # 24.1, 22.7: clusters of four in all their places
+    (11343, 26624, True),   # 36.4, 34: clusters of three in all their places
     (13819, 25856, True),   # 53.8, 43.0: the other kernel's 216 CTAs take an SM each
     (14651, 27136, False),  # 48.1, 54.8: its 115 CTAs do
     (7300, 24064, False),   # outside the lines in N and K
@@ -186,3 +187,16 @@ def test_scales_ahead(kernels, M, N, K, form, split):
     X, Wq, S = oracle.synth_inputs(M, N, K, 128, seed=N)
     ref = oracle.w4_linear_f32(X, Wq, S, 128, threads=oracle.max_threads())
     check_bf16_output(run(kernels, X, Wq, S, flags), ref, slack(M))
+
+
+# clusters of three in nearly all places of the device (44 and 45 of 45 on 148 SMs), one after the other: their CTAs leave together
+@pytest.mark.parametrize("M,N,K", [(4, 11500, 5632), (13, 11300, 6144), (8, 11200, 5888), (4, 11500, 5120)])
+def test_clusters_of_three_in_a_chain(kernels, M, N, K):
+    flags = FLAG_DECODE_NARROW | narrow_flags(3, 2)
+    X, Wq, S = oracle.synth_inputs(M, N, K, 128, seed=M)
+    x, wq, s = bits_to_torch(X), u32_to_torch(Wq), bits_to_torch(S)
+    outs = [kernels.w4_linear(x, wq, s, 128, flags=flags) for _ in range(8)]
+    torch.cuda.synchronize()
+    assert kernels.device_status() == 0 and all(torch.equal(o, outs[0]) for o in outs)
+    rows = np.random.default_rng(M).integers(0, N, 40)
+    check_bf16_output(torch_to_bits(outs[0])[:, rows], oracle.w4_linear_f32(X, Wq[rows], S[rows], 128, threads=oracle.max_threads()), slack(M))
