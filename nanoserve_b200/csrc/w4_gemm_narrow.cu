@@ -16,14 +16,15 @@
 //   * launched programmatically: the first slots of packed words are brought into L2 ahead of everything else, the first scales
 //     before the wait for the kernel in front.  All reads and writes come after it has finished, so it may be the kernel that
 //     writes the weights.
-// Measured, weights from HBM, us at 48 tokens, in brackets w4_gemm.cu: 4608 x 3584 8.8 (25), 37888 x 3584 23.3 (46), 3584 x 18944 16.7
-// (51), 8192 x 28672 42 (113).  What moved them: weights converted in eleven instructions instead of 17 per eight (sixteen such launches,
-// four 7B-shaped layers, 241 -> 228 us), then the questions to the barriers ahead of the last products of a step, parts of a
-// cut K sent instead of fetched and tensor memory freed beside the last sums (224; 777 x 5000 x 4096 in groups of 64 34.1 -> 33.2,
-// 512 x 3584 x 18944 73 -> 69, 128 x 37888 x 3584 37.1 -> 34.7).  What bounds it: at 48 tokens the sixteen products of a step
-// take 590 cycles (37 each, whatever the tokens up to 64: the weights' way out of tensor memory) and the conversion 980 per step
-// of either group, neither hidden whole by the other; 11 of the 23.3 us are HBM's; from 112 token columns the products (57 cycles
-// each).  A third group of conversion warps (24 in all, three buffers) changed nothing.
+// Measured, weights from HBM, one launch behind the other on one card, us at 48 tokens, in brackets this kernel with 17 instructions
+// per eight weights and fetched parts, and w4_gemm.cu: 4608 x 3584 8.8 (9.5, 24), 37888 x 3584 21.7 (24.9, 45), 3584 x 18944 16.3 (18.4, 49),
+// 8192 x 28672 40.0 (44.8, 103), 3584 x 3584 6.9 (8.8, 23.5); 128 x 37888 x 3584 35.0 (39.2, 51), 777 x 5000 x 4096 in groups of 64 30.9
+// (33.6), 512 x 3584 x 18944 71.9 (77.4).  What moved them: weights converted in eleven instructions, the questions to the
+// barriers ahead of the last products of a step, parts of a cut K sent instead of fetched, tensor memory freed beside the last
+// sums.  What bounds it: at 48 tokens the sixteen products of a step take 590 cycles (37 each, whatever the tokens up to 64: the
+// weights' way out of tensor memory) and the conversion 980 per step of either group; a step takes 0.60 us (37888 x 14336 less
+// 37888 x 3584), 1170 cycles at 1965 MHz, so neither hides the other whole; 11 of the 21.7 us are HBM's.  At 112 columns the products take
+// 57 cycles each, 912 a step, and a step 0.82 us, 1610 cycles: nearly one behind the other.  A third group of conversion warps (24 in all, three buffers) changed nothing.
 // Warps: 0 packed words (TMA), 1 MMA issue and TMEM, 2 X tiles (TMA), 3 idle, then DW conversion warps, which also do
 // the epilogue.  All rings run on mbarriers with bounded waits; a CTA that gives up records a status, still takes part in
 // the cluster barriers, frees its TMEM and returns.

@@ -1258,7 +1258,8 @@ double gemv_stream_us(int N, int K, int sm_count, size_t partial_cap) {
   if (pl.smem > kSmemTwoPerSm) return pl.grid_x > sm_count ? 1e30 : 0.0;
   if (pl.RB > 1) return 0.0;  // (never longer)
   const int waves = pl.q.n_tiles ? 1 : (pl.grid_x + 2 * sm_count - 1) / (2 * sm_count);
-  return 3.0 + 0.074 * pl.scps + 0.067 * w + 0.135 * waves * pl.scps / pl.ks;
+  const double us = 3.0 + 0.074 * pl.scps + 0.067 * w + 0.135 * waves * pl.scps / pl.ks;
+  return pl.grid_x == sm_count && pl.scps >= 30 ? 0.88 * us : us;  // (one CTA to every SM: 2364 x 11520 7.9 us, 149 for 2372 x 12032 9.4)
 }
 
 size_t gemv_stream_grid(int M, int N, int K, int G, int flags, int sm_count, size_t partial_cap) {

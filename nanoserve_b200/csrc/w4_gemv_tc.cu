@@ -725,8 +725,8 @@ bool gemv_tc_serves(const void* X, const void* Wq, const void* S, const void* Y,
 //     9728 and 16384 it does so several times per thread (4980 x 14080 12.8 against 15.0), above 22000 it cuts K through memory
 //     (8192 x 28672 26.6 against 29.2).  Within these lines, which cost a call's host side next to nothing, tiles of 128 rows as they
 //     are and tiles of 256 by the estimates of both kernels: by the lines alone these took 3500 x 2048 (5.3 us for 4.4), 2861 x 3584
-//     (5.6 for 5.1), 11771 x 28160 (54 for 39, 92 CTAs).  Of 3000 shapes like these 935 come here, 0.843 of their time there in
-//     the geometric mean, and 20 lose 3 % (at most 11); by the lines alone 1052, of which 96 (at most 41).
+//     (5.6 for 5.1), 11771 x 28160 (54 for 39, 92 CTAs).  Of 3000 shapes like these 926 come here, 0.843 of their time there in
+//     the geometric mean; of all 3000 22 lose 3 % and one 6, with the lines alone 98 and 49 (at most 41).
 //   * Two to four tokens (streaming kernel; X has 15 bits there at three and four): shorter here but for many rows of a short K (21667 x
 //     1024 at four tokens 4.8 us there, 5.5 here; 18944 x 3584 at two 9.6 and 10.7).  Of 150 calls five lose 3 % (at most 6).
 //   * Many-token kernel, five and more tokens: by the estimates of both, this one's with what plans have in common (they come out
