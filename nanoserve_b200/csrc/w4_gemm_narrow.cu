@@ -317,7 +317,8 @@ __global__ void __launch_bounds__(128 + DW * 32, MINB)
           k += 2 * kKB;
         }
         if constexpr (AHEAD == 1) {
-          if (i % kSectorSteps == 0 && i + kSectorSteps < nkb && live) prefetch_l2(s_row + (kb0 + i + kSectorSteps) * (128 / MODE));
+          const int ahead = (kb0 + i + kSectorSteps) * (128 / MODE);
+          if (i % kSectorSteps == 0 && i + kSectorSteps < nkb && live && ahead < p.KG) prefetch_l2(s_row + ahead);
         }
         bool plain = dequant_scale_plain(sc[0]);
         if constexpr (!G128) {

@@ -61,7 +61,6 @@ struct TcParams {
   int ks;       // CTAs of a cluster, each with its share of the pairs
   int sw, sx;   // ring slots of a pair: packed words (per block of 128 rows), X
   int ahead;    // slots of packed words that are brought into L2 ahead of the ring
-  int together; // a cluster's CTAs leave as one
   int x_first;  // the ring's further slots are not asked for before the first X is there
   int off_w, off_x, off_info, off_red;
 };
@@ -106,7 +105,7 @@ __device__ __forceinline__ void tmem_ld_sums(uint32_t taddr, uint32_t (&d)[16]) 
 
 // MT: token columns (4, 8 or 16).  Four and fewer tokens keep X in 32 bits (three unsigned planes and a signed one), more
 // in 16 (one and one).  MB: blocks of 128 weight rows.  SV: scales per load.
-template <int MB, int MT, int SV>
+template <int MB, int MT, int SV, bool TOGETHER = false>
 __global__ void __launch_bounds__(MB == 2 ? 896 : 512, MB == 2 ? 1 : 2)
     w4_gemv_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const TcParams p) {
   constexpr int P = MT == 4 ? 4 : 2;
@@ -188,7 +187,7 @@ __global__ void __launch_bounds__(MB == 2 ? 896 : 512, MB == 2 ? 1 : 2)
       if (live && g < p.KG) prefetch_l2(s_row + g);  // (the second group has none where the CTA's share is one pair)
       // (with rows of S that start anywhere in a sector the share's next two; 755 x 18688 at three tokens 8.0 -> 7.7 us.  Tiles of 256 rows
       // lost 1 % by it.)
-      if (SV == 2 && MB == 1 && live && np > 2) prefetch_l2(s_row + 2 * pr0 + min(2 * np - 2, 14 + 2 * grp));
+      if (const int next = 2 * pr0 + min(2 * np - 2, 14 + 2 * grp); SV == 2 && MB == 1 && MT < 16 && np > 2 && live && next < p.KG) prefetch_l2(s_row + next);
       pdl_wait_prior_grid();
       // SV == 4: two pairs, this group's one of them; SV == 2: one
       auto pair_scales = [&](int step) {
@@ -512,7 +511,7 @@ __global__ void __launch_bounds__(MB == 2 ? 896 : 512, MB == 2 ? 1 : 2)
         // With rows of S that start anywhere in a sector (K / 256 odd) some lane's next scales come from HBM in every pair, which
         // takes longer than a group's turn: the sector of eight pairs ahead is brought into L2.  26965 x 12544 at 5 tokens 43.0 -> 40.4
         // us, 14289 x 25856 at 6 47.1 -> 43.5.  Here, since the same in the rows' warps cost short launches 1 %.
-        if constexpr (SV == 2) {
+        if constexpr (SV == 2 && (MB == 2 || MT < 16)) {
           if ((i & 7) == 0 && i + 8 < np) {
 #pragma unroll
             for (int r = 0; r < 4; ++r) {
@@ -540,11 +539,15 @@ __global__ void __launch_bounds__(MB == 2 ? 896 : 512, MB == 2 ? 1 : 2)
   }
   if (p.ks > 1 && (warp >= kMain || poisoned)) cluster_wait();
   __syncthreads();
-  if (p.ks > 1 && (p.together || *abort_flag)) {  // (aborted: peers that have not given up may send parts here until they leave)
+  if constexpr (TOGETHER) {  // (p.ks > 1)
     cluster_arrive();
     cluster_wait();
   }
   if (*abort_flag) {
+    if (!TOGETHER && p.ks > 1) {  // peers that have not given up may send parts here until they leave
+      cluster_arrive();
+      cluster_wait();
+    }
     if (tid == 0) atomicCAS(p.status, kStatusOk, kStatusGemvTimeout);
     for (int i = 0; i < 64; ++i) __nanosleep(2000);  // copies in flight land before the shared memory is released
     __syncthreads();
@@ -584,16 +587,24 @@ template <int MB, int SV>
 TcKernel tc_kernel_mt(int mt) {
   return mt == 4 ? w4_gemv_tc_kernel<MB, 4, SV> : mt == 8 ? w4_gemv_tc_kernel<MB, 8, SV> : w4_gemv_tc_kernel<MB, 16, SV>;
 }
-TcKernel tc_kernel(int form, int mt, bool sv4) {
-  return form ? (sv4 ? tc_kernel_mt<2, 4>(mt) : tc_kernel_mt<2, 2>(mt)) : (sv4 ? tc_kernel_mt<1, 4>(mt) : tc_kernel_mt<1, 2>(mt));
+template <int SV>
+TcKernel tc_kernel_together(int mt) {
+  return mt == 4   ? w4_gemv_tc_kernel<2, 4, SV, true>
+         : mt == 8 ? w4_gemv_tc_kernel<2, 8, SV, true>
+                   : w4_gemv_tc_kernel<2, 16, SV, true>;
 }
-int tc_attributes(TcKernel kernel, int form, int mt, bool sv4, int dev) {
-  static std::atomic<bool> done[64][2][2][3];
+// kind: a form, or 2: 256 rows, a cluster's CTAs leave together
+TcKernel tc_kernel(int kind, int mt, bool sv4) {
+  if (kind == 2) return sv4 ? tc_kernel_together<4>(mt) : tc_kernel_together<2>(mt);
+  return kind ? (sv4 ? tc_kernel_mt<2, 4>(mt) : tc_kernel_mt<2, 2>(mt)) : (sv4 ? tc_kernel_mt<1, 4>(mt) : tc_kernel_mt<1, 2>(mt));
+}
+int tc_attributes(TcKernel kernel, int kind, int mt, bool sv4, int dev) {
+  static std::atomic<bool> done[64][3][2][3];
   const bool cached = dev >= 0 && dev < 64;
-  if (cached && done[dev][form][sv4][mt / 8].load(std::memory_order_acquire)) return 0;
+  if (cached && done[dev][kind][sv4][mt / 8].load(std::memory_order_acquire)) return 0;
   const cudaError_t e =
-      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, form ? kSmemFull : kSmemHalf);
-  if (e == cudaSuccess && cached) done[dev][form][sv4][mt / 8].store(true, std::memory_order_release);
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kind ? kSmemFull : kSmemHalf);
+  if (e == cudaSuccess && cached) done[dev][kind][sv4][mt / 8].store(true, std::memory_order_release);
   return (int)e;
 }
 void tc_config(int form, int grid, int ks, bool pdl, cudaLaunchConfig_t* cfg, cudaLaunchAttribute (&attr)[2]) {
@@ -795,8 +806,9 @@ int gemv_tc_launch(const void* X, const void* Wq, const void* S, void* Y, int M,
   // Clusters of three that take every place the device has for them (45 on 148 SMs): where their CTAs leave one by one the next
   // launch's clusters start in other places and some find none, a wave of their own (11300 x 27392 at 4 tokens 32.8 us for 44 then;
   // 11500 x 14336 20.5 for 24.8).  Not below eight pairs to a CTA (11400 x 4096 9.1, together 9.7), nor for other sizes of clusters,
-  // full or not: leaving together costs up to 0.7 us there (3800 x 14336 in clusters of eight 10.9 and 11.6).
-  p.together = form && pl.ks == 3 && pl.pairs >= 8 && pl.busy > 0.97;
+  // full or not: leaving together costs up to 0.7 us there (3800 x 14336 in clusters of eight 10.9 and 11.6).  A kernel of its own: asking
+  // at the end cost short launches 2 %.
+  const int kind = form && pl.ks == 3 && pl.pairs >= 8 && pl.busy > 0.97 ? 2 : form;
   // Where the rings of nearly all SMs fill at once X waits behind them for two microseconds: then only the first slot goes ahead
   // of it (8192 x 28672 at 8 tokens 30.2 -> 29.3 us, 37888 x 3584 at 13 17.4 -> 16.9).  Elsewhere it is X that is waited for (4608 x
   // 3584 at 4 tokens 5.8 against 6.1), and with a short K and few tokens it is there soon enough between other launches (four
@@ -808,11 +820,11 @@ int gemv_tc_launch(const void* X, const void* Wq, const void* S, void* Y, int M,
                           CU_TENSOR_MAP_SWIZZLE_128B))
     return kErrDevice;
   const bool sv4 = p.KG % 4 == 0 && reinterpret_cast<uintptr_t>(S) % 8 == 0;
-  const TcKernel kernel = tc_kernel(form, mt, sv4);
+  const TcKernel kernel = tc_kernel(kind, mt, sv4);
   int dev = -1;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return (int)e;
-  if (const int rc = tc_attributes(kernel, form, mt, sv4, dev)) return rc;
+  if (const int rc = tc_attributes(kernel, kind, mt, sv4, dev)) return rc;
   cudaLaunchConfig_t cfg{};
   cudaLaunchAttribute attr[2];
   tc_config(form, (N + rows - 1) / rows * p.ks, p.ks, (flags & kFlagNoPdl) == 0, &cfg, attr);

@@ -44,6 +44,18 @@ def test_scale_prefetches_are_bounded():
         assert re.search(r"\b%s < p\.KG" % at, cond), (cond, at)
 
 
+def test_scale_prefetches_by_other_warps_are_bounded():
+    """The warps that issue the products prefetch the sector ahead of step i for rows of their tile: a row and a step that exist."""
+    found = [m for s in SOURCES.values() for m in re.finditer(r"prefetch_l2\(p\.S \+ \(size_t\)n \* p\.KG \+ ([^;]*)\);", s)]
+    assert len(found) == sum(s.count("prefetch_l2(p.S") for s in SOURCES.values()) == 2
+    for m in found:
+        before = m.string[:m.start()]
+        assert before.endswith("if (n < p.N) ")
+        step = re.findall(r"if \(([^{}]*)\) \{", before)[-1]
+        assert step in ("(i & 7) == 0 && i + 8 < np", "i % kSectorSteps == 0 && i + kSectorSteps < nkb")
+        assert m.group(1) == ("2 * (pr0 + i) + 16" if "np" in step else "(kb0 + i + kSectorSteps) * (128 / MODE)")
+
+
 def test_questions_ahead_of_work_do_not_wait():
     """A try_wait may suspend the warp for a while: an answer that is only used behind a block's conversion is asked for by
     test_wait, and try_wait stands where nothing else is left to do (in the waits of ptx.cuh and in pairs of questions)."""
