@@ -4,8 +4,8 @@
 // products accumulate in fp32, one rounding at the store.
 //
 // What bounds it: the packed weights' way from HBM (0.5 bytes per weight), and next to it the conversion of every
-// weight (eleven instructions per eight, six of them on the ALU pipe at two cycles).  w4_gemm.cu gives the tokens the 128-row side of the MMA and writes the converted
-// weights to shared memory: with 48 tokens it pads the MMA to 128, sends every weight through shared memory twice and
+// weight (eleven instructions per eight, six of them on the ALU pipe at two cycles).  w4_gemm.cu gives the tokens the 128-row
+// side of the MMA and writes the converted weights to shared memory: with 48 tokens it pads the MMA to 128, sends every weight through shared memory twice and
 // has one CTA per 256 weight rows with no way to fill the chip but fp32 part-tiles in global memory.  Here
 //   * the WEIGHTS are the M side of tcgen05.mma (128 rows per block) and the tokens its N side (16 to 128 columns, a
 //     multiple of 16): the MMA's work follows the token count;
@@ -24,7 +24,8 @@
 // sums.  What bounds it: at 48 tokens the sixteen products of a step take 590 cycles (37 each, whatever the tokens up to 64: the
 // weights' way out of tensor memory) and the conversion 980 per step of either group; a step takes 0.60 us (37888 x 14336 less
 // 37888 x 3584), 1170 cycles at 1965 MHz, so neither hides the other whole; 11 of the 21.7 us are HBM's.  At 112 columns the products take
-// 57 cycles each, 912 a step, and a step 0.82 us, 1610 cycles: nearly one behind the other.  A third group of conversion warps (24 in all, three buffers) changed nothing.
+// 57 cycles each, 912 a step, and a step 0.82 us, 1610 cycles: nearly one behind the other.  A third group of
+// conversion warps (24 in all, three buffers) changed nothing.
 // Warps: 0 packed words (TMA), 1 MMA issue and TMEM, 2 X tiles (TMA), 3 idle, then DW conversion warps, which also do
 // the epilogue.  All rings run on mbarriers with bounded waits; a CTA that gives up records a status, still takes part in
 // the cluster barriers, frees its TMEM and returns.

@@ -23,8 +23,8 @@
 // The chain of a group is what the order in the loop is for: half of a pair's words are converted while the products of the group's last
 // pair run, and the sums of that one are added while this pair's do (2530 -> 2300 cycles per pair of a group; 8192 x 28672 at
 // eight tokens 30.7 -> 28.6 us).  The parts of a cut K go to the CTA that adds them with a barrier of their own instead of the
-// cluster's (4608 x 3584 6.65 -> 5.8 us), tensor memory is freed beside the last sums.  Measured, weights from HBM, us at 4 / 8 / 13 tokens, in brackets before that: 37888 x
-// 3584 15.2 / 15.4 / 16.9 (15.4 / 16.1 / 17.8), 3584 x 18944 12.4 / 12.6 / 14.7 (13.2 / 13.5 / 15.2), 4608 x 3584 at 4 and 13 5.8 and
+// cluster's (4608 x 3584 6.65 -> 5.8 us), tensor memory is freed beside the last sums.  Measured,
+// weights from HBM, us at 4 / 8 / 13 tokens, in brackets before that: 37888 x 3584 15.2 / 15.4 / 16.9 (15.4 / 16.1 / 17.8), 3584 x 18944 12.4 / 12.6 / 14.7 (13.2 / 13.5 / 15.2), 4608 x 3584 at 4 and 13 5.8 and
 // 6.8 (6.65 and 7.2), 57344 x 8192 at 8 57.9 (61.0).
 // Every wait is bounded; a CTA that gives up records a status, still takes part in the cluster barriers and frees its TMEM.
 #include <cuda.h>
@@ -104,7 +104,7 @@ __device__ __forceinline__ void tmem_ld_sums(uint32_t taddr, uint32_t (&d)[16]) 
 }
 
 // MT: token columns (4, 8 or 16).  Four and fewer tokens keep X in 32 bits (three unsigned planes and a signed one), more
-// in 16 (one and one).  MB: blocks of 128 weight rows.  SV: scales per load.
+// in 16 (one and one).  MB: blocks of 128 weight rows.  SV: scales per load.  TOGETHER: a cluster's CTAs leave as one (gemv_tc_launch).
 template <int MB, int MT, int SV, bool TOGETHER = false>
 __global__ void __launch_bounds__(MB == 2 ? 896 : 512, MB == 2 ? 1 : 2)
     w4_gemv_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const TcParams p) {
